@@ -213,8 +213,8 @@ PixelwiseArgs pixelwise_args(const fg_params &p, const fg_derived &d, const PwPl
     a.seed = p.seed;
     a.lognorm = p.radius_dist == FG_RADIUS_LOGNORM;
     a.radius_mean = p.radius_mean;
-    a.log_mu = (double)p.radius_log_mu;
-    a.log_sigma = (double)p.radius_log_sigma;
+    a.log_mu = p.radius_log_mu;
+    a.log_sigma = p.radius_log_sigma;
     return a;
 }
 
@@ -333,8 +333,8 @@ GrainwiseArgs grainwise_args(const fg_params &p, const fg_derived &d, const floa
     a.seed = p.seed;
     a.lognorm = p.radius_dist == FG_RADIUS_LOGNORM;
     a.radius_mean = p.radius_mean;
-    a.log_mu = (double)p.radius_log_mu;
-    a.log_sigma = (double)p.radius_log_sigma;
+    a.log_mu = p.radius_log_mu;
+    a.log_sigma = p.radius_log_sigma;
     return a;
 }
 

@@ -308,9 +308,7 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
             py = iy0 + pi / fw;
             const float lv = a.lam[(long long)py * a.in_w + px];
             if (lv > 0.0f) {
-                rng = pixel_rng(a.seed, px, py);
-                const PoissonParams P = poisson_new((double)lv);
-                left = poisson_sample(P, rng);
+                left = poisson_count(mix3(a.seed, kPixelStream, px, py), lv, rng);
             }
         }
         while (__any_sync(0xffffffffu, left > 0)) {
@@ -498,9 +496,7 @@ __device__ __forceinline__ void grainwise_tile_flat(const GrainwiseArgs &a, int 
             py = iy0 + pi / fw;
             const float lv = a.lam[(long long)py * a.in_w + px];
             if (lv > 0.0f) {
-                rng = pixel_rng(a.seed, px, py);
-                const PoissonParams P = poisson_new((double)lv);
-                left = poisson_sample(P, rng);
+                left = poisson_count(mix3(a.seed, kPixelStream, px, py), lv, rng);
             }
         }
         while (__any_sync(0xffffffffu, left > 0)) {

@@ -81,7 +81,7 @@ struct PixelwiseArgs {
     unsigned long long seed;
     int lognorm;
     float radius_mean;
-    double log_mu, log_sigma;
+    float log_mu, log_sigma;
     int *cancel;                // null, or the in-launch cancellation words (cancel_requested)
     // null, or the plane's emptiness bitmask (the sparse pass's first_draw_screen of every cell):
     // cells [cm_gi0, cm_gi0 + cm_gw) x [cm_gj0, cm_gj0 + 32 cm_ghw), word (c, k) = cellmask[k * cm_gw + c]
@@ -107,7 +107,7 @@ struct GrainwiseArgs {
     unsigned long long seed;
     int lognorm;
     float radius_mean;
-    double log_mu, log_sigma;
+    float log_mu, log_sigma;
     int *work;                  // null: one CTA per tile; else the tile scheduler's area (grainwise_work_ints)
     int parts;                  // CTAs per tile (>= 1; above 1 only for the bitmask variants)
     int *cancel;                // null, or the in-launch cancellation words (cancel_requested)

@@ -41,19 +41,30 @@ __device__ __forceinline__ uint64_t cell_row_hash(uint64_t col, int j) {
     return splitmix64(rotl64(col + (uint64_t)(int64_t)j, 41));
 }
 
+// Grain count of a cell with hash h whose first draw is above its threshold, with the stream left after
+// the Poisson draws.  The rejection regime (lambda * delta^2 >= 12) runs the f64 sampler: no workload's
+// cells reach it (the default cell holds lambda * delta^2 < 4.4 grains).
+__device__ __forceinline__ uint32_t cell_count_drawn(uint64_t h, long long thresh, double exp_lambda, Xoshiro &rng) {
+    uint32_t q = 0u;
+    if (thresh >= 0) {
+        rng = small_seed(h);
+        const uint64_t first = rng.next();
+        // exp(-lambda) to 2^-32 from the integer threshold floor(exp(-lambda) * 2^53)
+        const float e = (float)(uint32_t)(thresh >> 21) * 2.3283064365386963e-10f;
+        if (knuth_count_f32<true>(unit_f32(first), e, rng, q)) return q;
+    }
+    const DrawnCount d = thresh >= 0 ? knuth_count_f64(h, exp_lambda) : poisson_f64(h, (float)-exp_lambda);
+    rng = d.rng;
+    return d.q;
+}
+
 // Grain count of the cell with hash h; when q > 0 the stream is left positioned after the Poisson
 // draws.  q == 0 is decided from the first draw alone: only state words s0 and s3 (seed words 1, 2, 7
 // and 8) enter it.
 __device__ __forceinline__ uint32_t cell_count_h(uint64_t h, long long thresh, double exp_lambda, Xoshiro &rng) {
     const long long v = (long long)(small_first_u64(h) >> 11);
     if (v <= thresh) return 0u;
-    rng = small_seed(h);
-    if (thresh >= 0) {
-        (void)rng.next();  // the first draw, already evaluated
-        return poisson_knuth_tail(u53_unit((uint64_t)v), exp_lambda, rng);
-    }
-    PoissonParams P = poisson_new(-exp_lambda);
-    return poisson_rejection(P, rng);
+    return cell_count_drawn(h, thresh, exp_lambda, rng);
 }
 
 // Grain count of cell (i, j); when q > 0 the stream is left positioned after the Poisson draws.

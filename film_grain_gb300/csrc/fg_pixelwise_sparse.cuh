@@ -211,16 +211,25 @@ __device__ __noinline__ bool sparse_regen_sample(const PixelwiseArgs &a, float x
 // separate first-draw hash).
 __device__ __forceinline__ uint32_t sparse_cell_count(const PixelwiseArgs &a, int i, int j, Xoshiro *rng) {
     const CellParam cp = a.cells[cell_pixel(a, i, j)];
-    Xoshiro r = small_seed(cell_row_hash(cell_col_hash(a.seed, i), j));
-    uint32_t q;
+    const uint64_t h = cell_row_hash(cell_col_hash(a.seed, i), j);
+    Xoshiro r = small_seed(h);
+    uint32_t q = 0u;
+    bool sure = false;
     if (cp.thresh >= 0) {
         // the first draw (above the threshold for every listed cell but one whose seed words 1, 2, 7 and
         // 8 are all zero, which the bitmask lists to be safe)
-        const uint64_t v = r.next() >> 11;
-        q = (long long)v > cp.thresh ? poisson_knuth_tail(u53_unit(v), cp.exp_lambda, r) : 0u;
-    } else {
-        const PoissonParams P = poisson_new(-cp.exp_lambda);
-        q = poisson_rejection(P, r);
+        const uint64_t first = r.next();
+        if ((long long)(first >> 11) <= cp.thresh) {
+            *rng = r;
+            return 0u;
+        }
+        const float e = (float)(uint32_t)(cp.thresh >> 21) * 2.3283064365386963e-10f;
+        sure = knuth_count_f32<true>(unit_f32(first), e, r, q);
+    }
+    if (!sure) {
+        const DrawnCount d = cp.thresh >= 0 ? knuth_count_f64(h, cp.exp_lambda) : poisson_f64(h, (float)-cp.exp_lambda);
+        r = d.rng;
+        q = d.q;
     }
     *rng = r;
     return q;

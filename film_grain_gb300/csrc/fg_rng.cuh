@@ -20,9 +20,11 @@
 
 #if defined(__CUDACC__)
 #define FG_HD __host__ __device__ __forceinline__
+#define FG_HDN static __host__ __device__ __noinline__  // rare paths, out of line
 #define FG_HDC __host__ __device__ constexpr
 #else
 #define FG_HD inline
+#define FG_HDN static inline
 #define FG_HDC constexpr
 #endif
 
@@ -427,10 +429,10 @@ FG_HD double normal_sample(double mean, double sd, Rng &rng) {
 #define FG_EXP_FALLBACK_HOOK()  // counted by the native host checker in tests/native
 #endif
 
+struct FgFloat2 { float x, y; };
 #ifdef __CUDACC__
 static __device__ const float2 g_exp64[49] = FG_EXP64_TABLE_INIT;
 #endif
-struct FgFloat2 { float x, y; };
 static const FgFloat2 h_exp64[49] = FG_EXP64_TABLE_INIT;
 
 FG_HD float ff_fma(float a, float b, float c) {
@@ -451,21 +453,9 @@ FG_HD void ff_fast_two_sum(float a, float b, float &s, float &e) {
 }
 FG_HD float pow2f(int e) { return bits_f32((uint32_t)(e + 127) << 23); }  // e in [-126, 127]
 
-FG_HD float exp_f64_to_f32(double t) {
-    const uint64_t b = f64_bits(t);
-    const uint32_t E = (uint32_t)(b >> 52) & 0x7FFu;
-    if (E < 1023u - 30u) return 1.0f;                // |t| < 2^-30: exp(t) rounds to 1
-    if (E >= 1023u + 4u) {                           // |t| >= 16, inf, nan
-        FG_EXP_FALLBACK_HOOK();
-        return (float)exp(t);
-    }
-    const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;  // t = +-m * 2^(E-1075)
-    const uint32_t neg = (uint32_t)(b >> 63) << 31;
-    const int e0 = (int)E - 1075;                    // in [-82, -49]
-    const float th = bits_f32(neg | ((E - 896u) << 23) | ((uint32_t)(m >> 29) & 0x7FFFFFu));
-    const float tm = bits_f32(f32_bits((float)(uint32_t)((m >> 5) & 0xFFFFFFu) * pow2f(e0 + 5)) | neg);
-    const float tt = bits_f32(f32_bits((float)(uint32_t)(m & 31u) * pow2f(e0)) | neg);
-
+// exp(th + tm + tt) rounded to f32 (|th| < 16, |tm| and |tt| at most an ulp of th); false when the result
+// lies within `margin` (relative) of a rounding midpoint.
+FG_HD bool exp_ff_to_f32(float th, float tm, float tt, float margin, float &out) {
     const float L1 = 0.693115234375f, L2 = 3.1946183e-05f, L3 = 1.646595e-12f;
     const float kf = rintf(FG_FMUL(th, 1.44269504f));
     const float a = FG_FSUB(th, FG_FMUL(kf, L1));    // exact (Sterbenz; k*L1 exact)
@@ -509,17 +499,299 @@ FG_HD float exp_f64_to_f32(double t) {
     const float up = FG_FSUB(bits_f32(fb + 1u), f), dn = FG_FSUB(f, bits_f32(fb - 1u));
     const float half = fl >= 0.0f ? FG_FMUL(0.5f, up) : FG_FMUL(0.5f, dn);
     const float dist = fabsf(FG_FSUB(fabsf(fl), half));
-    if (!(dist > FG_FMUL(f, 9.09494702e-13f)) || !(fabsf(fl) <= half)) {  // within 2^-40 of a midpoint
+    out = f;
+    return dist > FG_FMUL(f, margin) && fabsf(fl) <= half;
+}
+
+FG_HD float exp_f64_to_f32(double t) {
+    const uint64_t b = f64_bits(t);
+    const uint32_t E = (uint32_t)(b >> 52) & 0x7FFu;
+    if (E < 1023u - 30u) return 1.0f;                // |t| < 2^-30: exp(t) rounds to 1
+    if (E >= 1023u + 4u) {                           // |t| >= 16, inf, nan
+        FG_EXP_FALLBACK_HOOK();
+        return (float)exp(t);
+    }
+    const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;  // t = +-m * 2^(E-1075)
+    const uint32_t neg = (uint32_t)(b >> 63) << 31;
+    const int e0 = (int)E - 1075;                    // in [-82, -49]
+    const float th = bits_f32(neg | ((E - 896u) << 23) | ((uint32_t)(m >> 29) & 0x7FFFFFu));
+    const float tm = bits_f32(f32_bits((float)(uint32_t)((m >> 5) & 0xFFFFFFu) * pow2f(e0 + 5)) | neg);
+    const float tt = bits_f32(f32_bits((float)(uint32_t)(m & 31u) * pow2f(e0)) | neg);
+    float f;
+    if (!exp_ff_to_f32(th, tm, tt, 9.09494702e-13f, f)) {  // within 2^-40 of a midpoint
         FG_EXP_FALLBACK_HOOK();
         return (float)exp(t);
     }
     return f;
 }
 
-// The lognormal radius draw: LogNormal::sample (rand_distr 0.4.3) cast to f32.
-template <class Rng>
-FG_HD float lognormal_radius_f32(double mu, double sigma, Rng &rng) {
-    return exp_f64_to_f32(normal_sample(mu, sigma, rng));
+// ------------------------------------------------------------------ samplers on the 32-bit pipes
+// The samplers above are written in the reference's f64 operations.  GB300 issues one warp-wide FP64
+// operation per 16 cycles and SM, so a ziggurat wedge (an f64 exp) or a rejection trial (tan, exp and a
+// log-gamma with seven divisions) costs more than everything else a grain needs.  The samplers below draw
+// the same numbers from the stream and take every decision -- a comparison, a floor, a rounding -- on f32
+// or double-float values with a bound on their error; a decision within the bound of its edge is taken
+// again by the f64 operations, from the same draws.  So counts, radii and the stream's position are the
+// reference's bit for bit, and the f64 operations run for about one grain in 2^11 and one pixel in 10^3.
+// Measured: grain-wise 1250x978, r 0.0465 log-normal, N 36: the kernel's FP64 pipe 74 -> 4 % busy, issue
+// slots 50 -> 74 %, 11.3 -> 8.4 ms; pixel-wise 1024^2 blobs, r 0.025 log-normal, N 256: 44.7 -> 38.2 ms.
+// tests/native/sampler_check.cpp compares them with the f64 samplers draw by draw.
+#ifndef FG_EXACT_HOOK
+#define FG_EXACT_HOOK()  // counted by the native host checker
+#endif
+
+struct DrawnCount {
+    Xoshiro rng;  // the stream after the Poisson draws
+    uint32_t q;
+};
+
+// The first 32 bits of a Standard f64 draw as a float: within 2^-32 + 2^-24 of it (relative).
+FG_HD float unit_f32(uint64_t raw) { return (float)(uint32_t)(raw >> 32) * 2.3283064365386963e-10f; }
+
+// A Knuth count by its f64 operations: the stream of seed h, exp(-lambda) = e.
+FG_HDN DrawnCount knuth_count_f64(uint64_t h, double e) {
+    FG_EXACT_HOOK();
+    DrawnCount d;
+    Xoshiro rng = small_seed(h);
+    const double p = std_f64_from(rng.next());
+    d.q = p > e ? poisson_knuth_tail(p, e, rng) : 0u;
+    d.rng = rng;
+    return d;
+}
+// Poisson(lambda) by its f64 operations, on the stream of seed h.
+FG_HDN DrawnCount poisson_f64(uint64_t h, float lambda) {
+    FG_EXACT_HOOK();
+    DrawnCount d;
+    Xoshiro rng = small_seed(h);
+    const PoissonParams P = poisson_new((double)lambda);
+    d.q = poisson_sample(P, rng);
+    d.rng = rng;
+    return d;
+}
+
+// Knuth's product against e = exp(-lambda) from the first uniform p (the stream stands after it); `q`
+// receives the count and `rng` the position after q + 1 draws.  False when a comparison is too close: p
+// carries one rounding and one 2^-32 cut per factor, e at most 2^-21 relative and 2^-31.
+template <bool kFirstAbove = false>
+FG_HD bool knuth_count_f32(float p, float e, Xoshiro &rng, uint32_t &q) {
+    const float rel = FG_FMUL(e, 1e-5f);  // 80 factors' roundings (2^-23 each)
+    uint32_t n = 0;
+    if (kFirstAbove) {  // the caller knows that the first uniform exceeds e
+        n = 1;
+        p = FG_FMUL(p, unit_f32(rng.next()));
+    }
+    for (;;) {
+        const float m = FG_FADD(rel, FG_FMUL((float)(n + 2), 5e-10f));
+        if (!(p > FG_FADD(e, m))) {
+            q = n;
+            return p < FG_FSUB(e, m);
+        }
+        if (++n > 64) return false;
+        p = FG_FMUL(p, unit_f32(rng.next()));
+    }
+}
+
+#ifdef __CUDA_ARCH__
+FG_HD float fg_sinpif(float x) { return sinpif(x); }
+FG_HD float fg_cospif(float x) { return cospif(x); }
+#else
+FG_HD float fg_sinpif(float x) { return (float)sin(3.14159265358979323846 * (double)x); }
+FG_HD float fg_cospif(float x) { return (float)cos(3.14159265358979323846 * (double)x); }
+#endif
+
+// Stirling's correction ln(r!) - (r ln r - r + ln(2 pi r) / 2) for r >= 1 (Abramowitz & Stegun 6.1.42;
+// after 1 / (1260 r^5) the next term is below 3e-7 from r = 3 on).
+FG_HD float stirling_corr(float r) {
+    if (r < 3.0f) return r < 1.5f ? 0.081061467f : 0.041340696f;  // r = 1, 2
+    const float i = FG_FDIV(1.0f, r), i2 = FG_FMUL(i, i);
+    return FG_FMUL(i, FG_FADD(0.083333333f, FG_FMUL(i2, FG_FADD(-0.0027777778f, FG_FMUL(i2, 7.9365079e-4f)))));
+}
+
+// The rejection sampler (12 <= lambda < 2^16), `rng` at the first draw.  A trial's candidate is
+// floor(lambda + s), s = sqrt(2 lambda) tan(pi x); with lambda = li + lf it is li + floor(lf + s), so its
+// error is that of s alone (4e-7 of it: the tangent's argument is reduced on the integer draw).  The
+// acceptance exponent r ln(lambda) - lnGamma(r + 1) - (lambda ln(lambda) - lnGamma(lambda + 1)) is a
+// difference of two numbers up to 10^5; by Stirling's formula it is
+//   -lambda ((1 + d) ln(1 + d) - d) - ln(1 + d) / 2 - corr(r) + corr(lambda),   d = (r - lambda) / lambda,
+// whose f32 error is about 2.4e-7 |r - lambda|.
+FG_HD bool poisson_reject_f32(float lambda, Xoshiro &rng, uint32_t &q) {
+    const float s2 = sqrtf(FG_FMUL(2.0f, lambda)), inv = FG_FDIV(1.0f, lambda), corr_l = stirling_corr(lambda);
+    const float li = floorf(lambda), lf = FG_FSUB(lambda, li);
+    for (;;) {
+        // tan(pi x), x = v 2^-53: with y = x - 1/2, -cot(pi y), or beyond |y| = 1/4 the tangent of 1/2 - |y|
+        const int64_t w = (int64_t)(rng.next() >> 11) - (1ll << 52);
+        const int64_t aw = w < 0 ? -w : w;
+        if (aw == 0) return false;  // the f64 argument pi / 2 decides on which side of the pole it lies
+        const bool far = aw > (1ll << 51);
+        const float z = FG_FMUL((float)(far ? (1ll << 52) - aw : aw), 1.1102230246251565e-16f);
+        const float sn = fg_sinpif(z), cs = fg_cospif(z);
+        const float t = far ? FG_FDIV(sn, cs) : FG_FDIV(cs, sn);
+        const float c = w < 0 ? t : -t;
+        const float s = FG_FMUL(s2, c), as = fabsf(s);
+        const float err = FG_FADD(FG_FMUL(as, 2e-6f), 2e-6f);
+        if (s < -FG_FADD(lambda, FG_FADD(err, 1.0f))) continue;  // a negative candidate: the next draw
+        if (!(as < 1e6f)) return false;
+        const float g = FG_FADD(lf, s), fl = floorf(g), frac = FG_FSUB(g, fl);
+        if (frac < err || FG_FSUB(1.0f, frac) < err) return false;
+        const float r = FG_FADD(li, fl);
+        if (r < 0.0f) continue;
+        const float dr = FG_FSUB(fl, lf);  // r - lambda
+        float arg;
+        if (r == 0.0f) {
+            arg = FG_FADD(FG_FADD(-lambda, FG_FMUL(0.5f, logf(FG_FMUL(6.2831853f, lambda)))), corr_l);
+        } else {
+            const float d = FG_FMUL(dr, inv), l1 = log1pf(d);
+            const float phi = FG_FSUB(FG_FMUL(FG_FADD(1.0f, d), l1), d);
+            arg = FG_FSUB(FG_FSUB(FG_FADD(corr_l, -FG_FMUL(lambda, phi)), FG_FMUL(0.5f, l1)), stirling_corr(r));
+        }
+        const float check = FG_FMUL(FG_FMUL(0.9f, FG_FADD(1.0f, FG_FMUL(c, c))), expf(arg));
+        const float rel = FG_FADD(2e-5f, FG_FMUL(2e-6f, FG_FADD(fabsf(dr), fabsf(arg))));
+        const float m = FG_FADD(FG_FMUL(check, rel), 1e-9f);
+        const float u = unit_f32(rng.next());
+        if (u > FG_FADD(check, m)) continue;
+        if (!(u < FG_FSUB(check, m))) return false;
+        q = (uint32_t)r;
+        return true;
+    }
+}
+
+// Poisson(lambda) for lambda > 0 on the stream of seed h; `rng` is left after the draws.
+FG_HD uint32_t poisson_count(uint64_t h, float lambda, Xoshiro &rng) {
+    rng = small_seed(h);
+    uint32_t q = 0;
+    bool sure = false;
+    if (lambda < 12.0f) sure = knuth_count_f32(unit_f32(rng.next()), expf(-lambda), rng, q);
+    else if (lambda < 65536.0f) sure = poisson_reject_f32(lambda, rng, q);
+    if (sure) return q;
+    const DrawnCount d = poisson_f64(h, lambda);
+    rng = d.rng;
+    return d.q;
+}
+
+// Ziggurat tables for the f32 decisions: the layer edges as float pairs and the densities.
+struct ZigF32 {
+    FgFloat2 x[257];
+    float f[257];
+};
+constexpr ZigF32 make_zig_f32() {
+    const double x[257] = FG_ZIG_NORM_X_INIT, f[257] = FG_ZIG_NORM_F_INIT;
+    ZigF32 t{};
+    for (int i = 0; i < 257; i++) {
+        t.x[i].x = (float)x[i];
+        t.x[i].y = (float)(x[i] - (double)t.x[i].x);
+        t.f[i] = (float)f[i];
+    }
+    return t;
+}
+#ifdef __CUDACC__
+static __device__ const ZigF32 g_zig32 = make_zig_f32();
+#endif
+static const ZigF32 h_zig32 = make_zig_f32();
+#ifdef __CUDA_ARCH__
+#define FG_ZIG32 g_zig32
+#else
+#define FG_ZIG32 h_zig32
+#endif
+
+// exp(mu + sd z) rounded to f32 by the f64 operations, for the normal draw's value z.
+FG_HDN float radius_from_normal_f64(double z, float mu, float sd) {
+    return exp_f64_to_f32(FG_DADD((double)mu, FG_DMUL((double)sd, z)));
+}
+FG_HD double zig_product(uint64_t bits) {  // u * x_i of a raw draw
+    return FG_DMUL(i51_scaled((int64_t)(bits >> 12) - (int64_t)(1ull << 51)), zig_x((unsigned)(bits & 0xffu)));
+}
+// The f64 decisions of a raw draw: inside its layer; below the density at its wedge draw.
+FG_HDN bool zig_inside_f64(uint64_t bits) {
+    FG_EXACT_HOOK();
+    return fabs(zig_product(bits)) < zig_x((unsigned)(bits & 0xffu) + 1);
+}
+FG_HDN bool zig_wedge_f64(uint64_t bits, uint64_t raw) {
+    FG_EXACT_HOOK();
+    const double x = zig_product(bits);
+    const unsigned i = (unsigned)(bits & 0xffu);
+    const double fi1 = zig_f(i + 1), pdf = exp(FG_DDIV(FG_DMUL(-x, x), 2.0));
+    return FG_DADD(fi1, FG_DMUL(FG_DSUB(zig_f(i), fi1), std_f64_from(raw))) < pdf;
+}
+struct ZigTail {
+    Xoshiro rng;
+    double x;
+};
+FG_HDN ZigTail zig_tail_f64(Xoshiro rng, bool negative) {  // the base layer's tail, beyond R
+    FG_EXACT_HOOK();
+    ZigTail t;
+    double xx = 1.0, yy = 0.0;
+    while (FG_DMUL(-2.0, yy) < FG_DMUL(xx, xx)) {
+        const double x_ = open01_from(rng.next());
+        const double y_ = open01_from(rng.next());
+        xx = FG_DDIV(log(x_), FG_ZIG_NORM_R);
+        yy = log(y_);
+    }
+    t.x = negative ? FG_DSUB(xx, FG_ZIG_NORM_R) : FG_DSUB(FG_ZIG_NORM_R, xx);
+    t.rng = rng;
+    return t;
+}
+
+// u x_i of a raw ziggurat draw as a float pair, to 2^-45.
+FG_HD void zig_product_ff(uint64_t bits, float &xh, float &xl) {
+    const int64_t k = (int64_t)(bits >> 12) - (int64_t)(1ull << 51);  // u = k * 2^-51
+    const float uh = (float)(int32_t)(k >> 28) * 1.1920928955078125e-07f;
+    const float ul = (float)(uint32_t)(k & 0xFFFFFFF) * 4.440892098500626e-16f;
+    const FgFloat2 z = FG_ZIG32.x[(unsigned)(bits & 0xffu)];
+    xh = FG_FMUL(uh, z.x);
+    xl = FG_FADD(ff_fma(uh, z.x, -xh), FG_FADD(FG_FMUL(uh, z.y), FG_FMUL(ul, z.x)));
+}
+
+// The lognormal radius draw, LogNormal::sample (rand_distr 0.4.3) cast to f32, in two steps: the draws from
+// the stream, and the radius they give.  mu and sd are f32 values (the crate's parameters are f32, widened
+// for the distribution).
+struct RadiusDraw {
+    uint64_t bits;  // the accepted raw ziggurat draw
+    float tail;     // the radius itself when the draw came from the base layer's tail, else -1
+};
+FG_HD RadiusDraw lognormal_draw(float mu, float sd, Xoshiro &rng) {
+    RadiusDraw d;
+    d.tail = -1.0f;
+    for (;;) {
+        d.bits = rng.next();
+        const unsigned i = (unsigned)(d.bits & 0xffu);
+        const float w = FG_ZIG32.x[i + 1].x;
+        float xh, xl;
+        zig_product_ff(d.bits, xh, xl);
+        const float ax = fabsf(FG_FADD(xh, xl));
+        if (ax < FG_FMUL(w, 0.9999995f)) return d;
+        if (ax <= FG_FMUL(w, 1.0000005f) && zig_inside_f64(d.bits)) return d;
+        if (i == 0) {  // outside the base layer's rectangle
+            const ZigTail t = zig_tail_f64(rng, (int64_t)d.bits >= 0);  // u < 0: the top bit is clear
+            rng = t.rng;
+            d.tail = radius_from_normal_f64(t.x, mu, sd);
+            return d;
+        }
+        const uint64_t raw = rng.next();
+        const float f1 = FG_ZIG32.f[i + 1];
+        const float lhs = FG_FADD(f1, FG_FMUL(FG_FSUB(FG_ZIG32.f[i], f1), unit_f32(raw)));
+        const float pdf = expf(FG_FMUL(-0.5f, FG_FMUL(ax, ax)));
+        const float gap = FG_FSUB(pdf, lhs);  // both within 2e-6
+        if (gap > 4e-6f || (gap >= -4e-6f && zig_wedge_f64(d.bits, raw))) return d;
+    }
+}
+// t = mu + sd x is kept to 2^-42, so the f32 nearest exp(t) is known unless exp(t) lies within 2^-37 of a
+// rounding midpoint.
+FG_HD float lognormal_radius(const RadiusDraw &d, float mu, float sd) {
+    if (d.tail >= 0.0f) return d.tail;
+    float xh, xl;
+    zig_product_ff(d.bits, xh, xl);
+    const float yh = FG_FMUL(sd, xh);
+    const float yl = FG_FADD(ff_fma(sd, xh, -yh), FG_FMUL(sd, xl));
+    float th, tl;
+    ff_two_sum(mu, yh, th, tl);
+    ff_fast_two_sum(th, FG_FADD(tl, yl), th, tl);
+    const float at = fabsf(th);
+    float r;
+    if (sd <= 4.0f && at < 16.0f && at > 1e-4f && exp_ff_to_f32(th, tl, 0.0f, 7.2759576e-12f, r)) return r;
+    return radius_from_normal_f64(zig_product(d.bits), mu, sd);
+}
+FG_HD float lognormal_radius_f32(float mu, float sd, Xoshiro &rng) {
+    return lognormal_radius(lognormal_draw(mu, sd, rng), mu, sd);
 }
 
 // ChaCha12 keystream reader (StdRng), seeded through rand_core's PCG32 seed_from_u64.

@@ -54,3 +54,17 @@ def test_bitmask_screen_and_row_hash_identities(tmp_path):
     checked, bad, checked2, bad2 = (int(v) for v in out)
     assert checked == 200000 * 13 and bad == 0
     assert checked2 > 6000000 and bad2 == 0
+
+
+def test_samplers_on_32_bit_pipes_match_f64_samplers(tmp_path):
+    """poisson_count, knuth_count_f32 and lognormal_radius_f32 give the f64 samplers' values and stream
+    positions on every stream (both Poisson regimes and the ends of the f32 rejection's range, cell
+    thresholds, radius laws with and without spread), and decide in f64 on few of them: an f32 decision's
+    margin is at most 1e-3 of the pixels wide (5e-10 per factor against exp(-12) = 6e-6, for the largest
+    Knuth lambda) and the ziggurat's tail 3e-4 of the radii."""
+    exe = _compile("sampler_check.cpp", "sampler_check", tmp_path)
+    out = subprocess.run([exe, "20000"], check=True, capture_output=True, text=True).stdout.split()
+    (n1, bad1, f1), (n2, bad2, f2), (n3, bad3, f3) = ([int(v) for v in out[k:k + 3]] for k in (0, 3, 6))
+    assert n1 == 21 * 20000 and bad1 == 0 and f1 < 2e-3 * n1
+    assert n2 > 50000 and bad2 == 0 and f2 < 1e-4 * n2
+    assert n3 == 7 * 400000 and bad3 == 0 and f3 < 1e-3 * n3

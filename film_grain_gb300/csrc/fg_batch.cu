@@ -44,7 +44,8 @@ struct BatchImage {
 
 struct BatchItem {
     int image, x, y;
-    int pad;  // grain-wise: part | parts << 16
+    int part;   // grain-wise: part | parts << 16
+    int chunk;  // grain-wise: sample chunk
 };
 
 // One contiguous range of a segmented elementwise pass.
@@ -191,8 +192,8 @@ __global__ void __launch_bounds__(512, 2) batch_persistent_kernel(const BatchIma
         __syncthreads();
         if (threadIdx.x == 0) s_image = w.image;
         if (s_img.algo == FG_ALGO_PIXEL) pixelwise_block<PwFat>(s_img.pa, w.x, w.y, smem_raw);
-        else if (s_img.small) grainwise_tile<true>(s_img.ga, w.x, w.y, smem_raw, w.pad & 0xFFFF, w.pad >> 16);
-        else grainwise_tile<false>(s_img.ga, w.x, w.y, smem_raw, w.pad & 0xFFFF, w.pad >> 16);
+        else if (s_img.small) grainwise_tile<true>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk);
+        else grainwise_tile<false>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk);
         __syncthreads();
     }
 }
@@ -279,14 +280,14 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
     struct GrainTile {
         double cost;
         BatchItem it;
-        int batches;  // the most CTAs the tile can be split over (its 32-pixel batches)
+        int most_parts;
     };
     std::vector<GrainTile> grain_tiles;
     std::vector<RegenRange> regen;
     long long regen_ctas = 0;
     std::vector<Segment> segs;
     std::vector<Chunk> pre, post;
-    size_t smem = pixelwise_smem_bytes();
+    size_t smem = pixelwise_smem_bytes(), request = smem;
     auto fail = [&](fg_status st) {
         free_batch(b);
         return st;
@@ -342,20 +343,18 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
                 std::min(cell_area * cell_area, block_samples * a.regen_cells) + 1.5 * block_samples;
             for (int by = 0; by < pl.nby; by++)
                 for (int bx = 0; bx < pl.nbx; bx++)
-                    px_work.push_back(CostItem{per_block, BatchItem{i, pl.bx0 + bx, pl.by0 + by, 0}});
+                    px_work.push_back(CostItem{per_block, BatchItem{i, pl.bx0 + bx, pl.by0 + by, 0, 0}});
         } else {
-            const size_t tab_bytes = grain_table_bytes(p.n_samples);
-            std::vector<unsigned char> tab(tab_bytes);
-            grain_table(im.offsets, p.n_samples, tab.data());
-            void *d_tab, *d_mask;
-            FG_BCUDA(dev_alloc(b, tab_bytes, &d_tab), "batch alloc");
-            FG_BCUDA(cudaMemcpy(d_tab, tab.data(), tab_bytes, cudaMemcpyHostToDevice), "H2D");
+            void *d_offs, *d_mask;
+            FG_BCUDA(dev_alloc(b, sizeof(float) * 2 * p.n_samples, &d_offs), "batch alloc");
+            FG_BCUDA(cudaMemcpy(d_offs, im.offsets, sizeof(float) * 2 * p.n_samples, cudaMemcpyHostToDevice), "H2D");
             const size_t mask_bytes = grainwise_mask_bytes(p, d);
             FG_BCUDA(dev_alloc(b, mask_bytes, &d_mask), "batch alloc");
             GrainwiseArgs &a = B.ga;
-            a = grainwise_args(p, d, im.offsets, im.d_lambda, d_tab, (unsigned int *)d_mask, tun.grain_mask_words);
+            a = grainwise_args(p, d, im.offsets, im.d_lambda, (const float *)d_offs, (unsigned int *)d_mask, tun.grain_mask_words);
             B.small = grainwise_small_coords(a) ? 1 : 0;
             smem = std::max(smem, grainwise_smem_bytes(a));
+            request = std::max(request, a.request_bytes);
             segs.push_back(Segment{0, 0, (long long)(mask_bytes / 4), d_mask, nullptr, 0.0f});
             add_chunks(pre, (int)segs.size() - 1, (long long)(mask_bytes / 4));
             segs.push_back(Segment{3, a.words, n_out, d_mask, im.d_out, 1.0f / (float)p.n_samples});
@@ -373,17 +372,19 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
                     } else {
                         lam_sum = 50.0 * (x1 - x0) * (y1 - y0);
                     }
-                    const double cost = lam_sum * (60.0 + 0.3 * p.n_samples) + 20.0 * (x1 - x0) * (y1 - y0);
-                    const int batches = grainwise_variant(a.n) == 0 ? 1 : ((x1 - x0) * (y1 - y0) + 31) / 32;
-                    grain_tiles.push_back(GrainTile{cost, BatchItem{i, tx, ty, 0}, batches});
+                    const int n_chunk = std::min((int)p.n_samples, 32 * a.chunk_words);
+                    const double cost = lam_sum * (60.0 + 0.3 * n_chunk) + 20.0 * (x1 - x0) * (y1 - y0);
+                    const int most = grainwise_most_parts((x1 - x0) * (y1 - y0));
+                    for (int c = 0; c < a.chunks; c++)
+                        grain_tiles.push_back(GrainTile{cost, BatchItem{i, tx, ty, 0, c}, most});
                 }
             }
         }
     }
-    if (smem > 200 * 1024) return fail(set_error(FG_ERR_UNSUPPORTED, "batch tile needs too much shared memory"));
+    if (request > 200 * 1024) return fail(set_error(FG_ERR_UNSUPPORTED, "batch tile needs too much shared memory"));
     // Heavy grain-wise tiles are split over CTAs (part | parts << 16 in the item's last word) so that no
     // item is far above the average share of an SM slot: a tile of cost c gets ceil(c / target) parts,
-    // at most one per kGwWarps of its 32-pixel batches.
+    // at most grainwise_most_parts.
     {
         double total_cost = 0.0;
         for (const GrainTile &g : grain_tiles) total_cost += g.cost;
@@ -393,11 +394,10 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
         FG_BCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
         const double target = total_cost / (8.0 * std::max(1, sms) * std::max(1, tun.ctas_per_sm)) + 1.0;
         for (const GrainTile &g : grain_tiles) {
-            const int most = std::max(1, std::min(g.batches / kGwWarps, 0xFFFF));  // a batch per warp at least
-            const int parts = (int)std::max(1.0, std::min((double)most, std::ceil(g.cost / target)));
+            const int parts = (int)std::max(1.0, std::min((double)g.most_parts, std::ceil(g.cost / target)));
             for (int q = 0; q < parts; q++) {
                 BatchItem it = g.it;
-                it.pad = q | (parts << 16);
+                it.part = q | (parts << 16);
                 work.push_back(CostItem{g.cost / parts, it});
             }
         }

@@ -263,65 +263,57 @@ fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_der
     return FG_OK;
 }
 
-size_t grain_table_bytes(uint32_t n) { return (size_t)n * sizeof(float4) + (kGwBucketCount + 1) * sizeof(int); }
-
-void grain_table(const float *h_offs, uint32_t n, void *blob) {
-    struct Entry {
-        float fx;
-        float4 e;
-    };
-    std::vector<Entry> t(n);
-    for (uint32_t k = 0; k < n; k++) {
-        const float ox = h_offs[2 * k], oy = h_offs[2 * k + 1];
-        float fx = ox - std::floor(ox), fy = oy - std::floor(oy);
-        if (!(fx < 1.0f)) fx = 0.0f;  // a tiny negative offset can round up to 1; cyclically that is 0
-        if (!(fy < 1.0f)) fy = 0.0f;
-        int kb = (int)k;
-        float kf;
-        std::memcpy(&kf, &kb, 4);
-        t[k] = Entry{fx, make_float4(fy, ox, oy, kf)};
-    }
-    std::stable_sort(t.begin(), t.end(), [](const Entry &a, const Entry &b) { return a.fx < b.fx; });
-    float4 *entries = reinterpret_cast<float4 *>(blob);
-    int *bstart = reinterpret_cast<int *>(entries + n);
-    for (uint32_t k = 0; k < n; k++) entries[k] = t[k].e;
-    uint32_t j = 0;
-    for (int b = 0; b <= kGwBucketCount; b++) {
-        const float v = (float)b / (float)kGwBucketCount;
-        while (j < n && t[j].fx < v) j++;
-        bstart[b] = b == kGwBucketCount ? (int)n : (int)j;
-    }
-}
-
 // Shared-memory sample-mask words per grain-wise tile (sets the tile edge).  Measured on GB300 with
 // N = 128 at zoom 2 (1024^2 plane): 6144 words 29.6 ms, 8192 26.3 ms, 12288 28.7 ms, 16384 31.7 ms.
 constexpr int kGrainMaskWords = 8192;
+constexpr int kGrainChunkWords = 8;  // mask words of a chunk at most (kGbMaxWords, fg_grainwise.cuh)
 
 GrainwiseArgs grainwise_args(const fg_params &p, const fg_derived &d, const float *h_offs, const float *d_lam,
-                             const void *d_table, unsigned int *d_gmask, int mask_words) {
+                             const float *d_offs, unsigned int *d_gmask, int mask_words) {
     GrainwiseArgs a;
     std::memset(&a, 0, sizeof a);
     float ext[4];
     offset_extents(h_offs, p.n_samples, ext);
     a.lam = d_lam;
-    a.sorted_offs = reinterpret_cast<const float4 *>(d_table);
-    a.bucket_start = reinterpret_cast<const int *>(reinterpret_cast<const float4 *>(d_table) + p.n_samples);
+    a.offs = reinterpret_cast<const float2 *>(d_offs);
     a.gmask = d_gmask;
     a.in_w = (int)d.input_width; a.in_h = (int)d.input_height;
     a.out_w = (int)d.output_width; a.out_h = (int)d.output_height;
     a.n = (int)p.n_samples;
     a.words = (a.n + 31) / 32;
+    // chunks of equal width, so that no item is much lighter than the others of its tile
+    a.chunks = (a.words + kGrainChunkWords - 1) / kGrainChunkWords;
+    a.chunk_words = (a.words + a.chunks - 1) / a.chunks;
+    a.chunks = (a.words + a.chunk_words - 1) / a.chunk_words;
     // Input tile: its zoomed rectangle should fill about `mask_words` words of shared memory.
     // floor(x0*zoom + tin*zoom) - floor(x0*zoom) <= ceil(tin*zoom), so that bounds the rectangle.
-    const int side = std::max(1, (int)std::floor(std::sqrt((double)mask_words / a.words)));
-    const int tin = std::max(1, (int)std::floor(side / p.zoom));
-    a.tin_w = std::min(tin, a.in_w);
-    a.tin_h = std::min(tin, a.in_h);
-    a.rmax_w = std::max(1, std::min(a.out_w, (int)std::ceil(a.tin_w * (double)p.zoom)));
-    a.rmax_h = std::max(1, std::min(a.out_h, (int)std::ceil(a.tin_h * (double)p.zoom)));
+    auto fit_tile = [&](int words) {
+        const int side = std::max(1, (int)std::floor(std::sqrt((double)mask_words / words)));
+        const int tin = std::max(1, (int)std::floor(side / p.zoom));
+        a.tin_w = std::min(tin, a.in_w);
+        a.tin_h = std::min(tin, a.in_h);
+        a.rmax_w = std::max(1, std::min(a.out_w, (int)std::ceil(a.tin_w * (double)p.zoom)));
+        a.rmax_h = std::max(1, std::min(a.out_h, (int)std::ceil(a.tin_h * (double)p.zoom)));
+    };
+    // What limits a request: 200 KB for a tile's masks with all samples (the rectangle such a tile would
+    // have) beside fixed sizes per offset and filter word, whatever the kernel's own layout and chunks need
+    // (grainwise_smem_bytes: at most 12 KB more than this with one chunk, less with several).
+    fit_tile(a.words);
+    const size_t n = p.n_samples, rect = (size_t)a.rmax_w * a.rmax_h * a.words * sizeof(unsigned int);
+    a.request_bytes = rect + (a.chunks > 1 ? n * 20 + 44108
+                                           : ((n + 1) & ~(size_t)1) * 8 + 7168 * (size_t)(a.words | 1) +
+                                                 ((n + 7) & ~(size_t)7) * 2 + 16);
+    fit_tile(a.chunk_words);
     a.rm = d.rm;
     a.zoom = p.zoom;
-    a.parts = 1;
+    // A grain's draws and filter cost about 400 lane-ops, a pair 100, and a grain has
+    // n (2 (r zoom + 1/128))^2 of them on average.
+    {
+        const double n_chunk = std::min<double>(p.n_samples, 32.0 * a.chunk_words);
+        const double r2 = (double)p.radius_mean * p.radius_mean + (double)p.radius_stddev * p.radius_stddev;
+        const double band = std::min(1.0, 2.0 * (std::sqrt(r2) * p.zoom + 1.0 / 128.0));
+        a.grain_cost = (float)(400.0 + 100.0 * n_chunk * band * band);
+    }
     a.offx_min = ext[0]; a.offx_max = ext[1]; a.offy_min = ext[2]; a.offy_max = ext[3];
     // Rounding margin of the candidate intervals: each of the three f32 roundings between
     // czx + offx and the bounds() comparison moves a value by at most half an ulp of the largest
@@ -343,18 +335,17 @@ size_t grainwise_mask_bytes(const fg_params &p, const fg_derived &d) {
 }
 
 fg_status enqueue_grainwise(const GrainwiseArgs &a, cudaStream_t s) {
-    if (grainwise_smem_bytes(a) > 200 * 1024)
+    if (a.request_bytes > 200 * 1024)
         return set_error(FG_ERR_UNSUPPORTED, "n_samples too large for the grain-wise tile");
     FG_CUDA(cudaMemsetAsync(a.gmask, 0, (size_t)a.out_w * a.out_h * a.words * sizeof(unsigned int), s), "memset mask");
     GrainwiseArgs b = a;
-    DevBuf work;  // the tile scheduler's area, freed in stream order after the launch
-    FG_CUDA(work.alloc(grainwise_work_ints(a) * sizeof(int), s), "alloc tile scheduler");
-    b.work = static_cast<int *>(work.p);
     int dev = 0, sms = 0;
     FG_CUDA(cudaGetDevice(&dev), "device");
     FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-    b.parts = grainwise_parts(a, sms);
-    FG_CUDA(launch_grainwise(b, s), "grainwise kernel");
+    DevBuf work;  // the tile scheduler's area, freed in stream order after the launch
+    FG_CUDA(work.alloc(grainwise_work_ints(a, sms) * sizeof(int), s), "alloc tile scheduler");
+    b.work = static_cast<int *>(work.p);
+    FG_CUDA(launch_grainwise(b, sms, s), "grainwise kernel");
     return FG_OK;
 }
 
@@ -431,13 +422,7 @@ static fg_status render_plane_sync(int algo, const float *lambda, const fg_param
         FG_CUDA(b_out.alloc(sizeof(float) * n_out, s), "alloc out");
         d_out = (float *)b_out.p;
     }
-    if (algo == FG_ALGO_GRAIN) {
-        std::vector<unsigned char> tab(grain_table_bytes(p.n_samples));
-        grain_table(h_offs.data(), p.n_samples, tab.data());
-        FG_CUDA(b_offs.alloc(tab.size(), s), "alloc offsets");
-        FG_CUDA(cudaMemcpyAsync(b_offs.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, s), "offsets H2D");
-        d_offs = (const float *)b_offs.p;
-    } else if (!offs_dev) {
+    if (!offs_dev) {
         FG_CUDA(b_offs.alloc(off_bytes, s), "alloc offsets");
         FG_CUDA(cudaMemcpyAsync(b_offs.p, h_offs.data(), off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
         d_offs = (const float *)b_offs.p;
@@ -513,13 +498,12 @@ FG_API fg_status fg_render_grainwise_async(const float *d_lambda, const fg_param
     if (is_device_ptr(offsets)) return set_error(FG_ERR_INVALID, "offsets must be host memory");
     keep_pool_memory();
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<unsigned char> tab(grain_table_bytes(params->n_samples));
-    grain_table(offsets, params->n_samples, tab.data());
+    const size_t off_bytes = sizeof(float) * 2 * params->n_samples;
     DevBuf b_offs, b_mask;
-    FG_CUDA(b_offs.alloc(tab.size(), s), "alloc offsets");
-    FG_CUDA(cudaMemcpyAsync(b_offs.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, s), "offsets H2D");
+    FG_CUDA(b_offs.alloc(off_bytes, s), "alloc offsets");
+    FG_CUDA(cudaMemcpyAsync(b_offs.p, offsets, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
     FG_CUDA(b_mask.alloc(grainwise_mask_bytes(*params, *derived), s), "alloc sample masks");
-    GrainwiseArgs a = grainwise_args(*params, *derived, offsets, d_lambda, b_offs.p, (unsigned int *)b_mask.p, kGrainMaskWords);
+    GrainwiseArgs a = grainwise_args(*params, *derived, offsets, d_lambda, (const float *)b_offs.p, (unsigned int *)b_mask.p, kGrainMaskWords);
     st = enqueue_grainwise(a, s);
     if (st == FG_OK) st = enqueue_grainwise_epilogue(a, d_out, 0, nullptr, nullptr, nullptr, s);
     return st;
@@ -567,17 +551,10 @@ FG_API fg_status fg_render_image(const float *rgb, int64_t width, int64_t height
     FG_CUDA(b_lam.alloc(sizeof(float) * n_in * nplanes, s), "alloc lambda");
     FG_CUDA(b_out.alloc(sizeof(float) * n_out * nplanes, s), "alloc planes");
     FG_CUDA(b_rgb8.alloc(3 * n_out, s), "alloc rgb8");
-    std::vector<unsigned char> tab;
-    if (algo == FG_ALGO_PIXEL) {
-        FG_CUDA(b_offs.alloc(sizeof(float) * 2 * p.n_samples, s), "alloc offsets");
-        FG_CUDA(cudaMemcpyAsync(b_offs.p, offs_in.data(), sizeof(float) * 2 * p.n_samples, cudaMemcpyHostToDevice, s),
-                "offsets H2D");
-    } else {
-        tab.resize(grain_table_bytes(p.n_samples));
-        grain_table(offs.data(), p.n_samples, tab.data());
-        FG_CUDA(b_offs.alloc(tab.size(), s), "alloc offsets");
-        FG_CUDA(cudaMemcpyAsync(b_offs.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, s), "offsets H2D");
-    }
+    const std::vector<float> &used_offs = algo == FG_ALGO_PIXEL ? offs_in : offs;
+    FG_CUDA(b_offs.alloc(sizeof(float) * 2 * p.n_samples, s), "alloc offsets");
+    FG_CUDA(cudaMemcpyAsync(b_offs.p, used_offs.data(), sizeof(float) * 2 * p.n_samples, cudaMemcpyHostToDevice, s),
+            "offsets H2D");
     float *d_lam = (float *)b_lam.p, *d_out = (float *)b_out.p;
     st = enqueue_split_lambda((const float *)b_rgb.p, (long long)n_in, luma ? 1 : 0, (float *)b_planes.p,
                               (unsigned int *)b_max.p, d.inv_e_pi_r2, d_lam, s);
@@ -616,7 +593,7 @@ FG_API fg_status fg_render_image(const float *rgb, int64_t width, int64_t height
                                    (CellParam *)b_cells.p, (unsigned long long *)b_diag.p, &e, s, true, watch.dev());
         } else {
             unsigned int *plane_mask = (unsigned int *)((unsigned char *)b_cells.p + mask_bytes * c);
-            GrainwiseArgs a = grainwise_args(p, d, offs.data(), d_lam + (size_t)c * n_in, b_offs.p, plane_mask, kGrainMaskWords);
+            GrainwiseArgs a = grainwise_args(p, d, offs.data(), d_lam + (size_t)c * n_in, (const float *)b_offs.p, plane_mask, kGrainMaskWords);
             a.cancel = watch.dev();
             st = enqueue_grainwise(a, s);
             if (st == FG_OK && c == nplanes - 1) {

@@ -10,17 +10,14 @@
 // with the luma colour recombination and u8 packing.
 //
 // Work organisation:
-//   - each warp takes 32 footprint pixels at a time (one per lane, Poisson set-up in step) and
-//     draws their grains one per lane per step; valid grains are compacted into a 64-entry warp
-//     queue with a ballot, and every full batch of 32 is rasterised grain by grain by the whole warp;
+//   - each warp takes 32 footprint pixels at a time (one per lane, Poisson set-up in step) and draws
+//     their grains one per lane per step;
 //   - an offset can put a pixel centre inside a grain's disk only if frac(czx + offx) lies within
-//     radius_out of 1/2 (and likewise for y).  For N <= 256 each lane turns both tests, widened by a
-//     rounding margin and rounded out to 1/128 buckets, into a bitmask over the sample index (two
-//     lookups per axis in per-tile sparse OR tables), ANDs them, and the set bits -- about 1.2x the
-//     true candidates -- go through the warp's list to stage B.  For larger N the offsets are sorted
-//     by frac(offx), the cyclic interval of the sorted table around frac(1/2 - czx) is flattened over
-//     the lanes (stage A) and filtered by the y test.  Stage B runs the reference's exact bounds()
-//     and centre tests on the pairs, one pair per lane;
+//     radius_out of 1/2 (and likewise for y).  Each lane turns both tests, widened by a rounding margin
+//     and rounded out to 1/128 buckets, into a bitmask over the sample index (two lookups per axis in
+//     per-tile sparse OR tables), ANDs them, and the set bits -- about 1.2x the true candidates -- are
+//     dealt over the warp's lanes for stage B: the reference's exact bounds() and centre tests on one
+//     pair per lane.  Above 256 samples a work item takes one chunk of them (fg_grainwise.cuh);
 //   - the lognormal radius is evaluated with the double-float exp (exp_f64_to_f32).
 // Bits are set with shared-memory atomicOr; OR is idempotent and commutative, so the result does not
 // depend on the order.
@@ -34,88 +31,134 @@
 
 namespace fg {
 
-template <bool kSmall, int kVariant>
-__global__ void __launch_bounds__(kGwThreads, 2) grainwise_kernel(const __grid_constant__ GrainwiseArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    grainwise_tile<kSmall, kVariant>(a, blockIdx.x, blockIdx.y, smem_raw, blockIdx.z, a.parts);
-}
-
-// Persistent form: CTAs pull tiles from the scheduler's list (a.work[2..], heaviest first) through the
-// counter a.work[0] until the list is exhausted.
+// Persistent form: CTAs pull work items (tile, part of it, sample chunk) through the counter a.work[0] from
+// the scheduler's list until it is exhausted.
 template <bool kSmall, int kVariant>
 __global__ void __launch_bounds__(kGwThreads, 2) grainwise_persistent_kernel(const __grid_constant__ GrainwiseArgs a,
-                                                                             int ntx, int ntiles) {
+                                                                             int ntx) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_tile;
-    const int parts = a.parts;
+    __shared__ int s_item;
+    const int nitems = a.work[1] * a.chunks;
+    const int2 *items = reinterpret_cast<const int2 *>(a.work + 2);
     for (;;) {
         if (threadIdx.x == 0) {
-            const int i = atomicAdd(a.work, 1);  // item i: part i % parts of the (i / parts)-th tile
-            s_tile = (i < ntiles * parts && !cancel_requested(a.cancel)) ? i : -1;
+            const int i = atomicAdd(a.work, 1);  // chunk i % chunks of the (i / chunks)-th listed part
+            s_item = (i < nitems && !cancel_requested(a.cancel)) ? i : -1;
         }
         __syncthreads();
-        const int i = s_tile;
+        const int i = s_item;
         if (i < 0) break;
-        const int t = a.work[2 + i / parts];
-        grainwise_tile<kSmall, kVariant>(a, t % ntx, t / ntx, smem_raw, i % parts, parts);
+        const int2 it = items[i / a.chunks];  // (tile, part | parts << 16)
+        grainwise_tile<kSmall, kVariant>(a, it.x % ntx, it.x / ntx, smem_raw, it.y & 0xFFFF, it.y >> 16, i % a.chunks);
         __syncthreads();
     }
 }
 
-// Expected cost of each input tile (one warp per tile): its grains (sum of lambda) plus a per-pixel
-// set-up term.
+// Expected lane-ops of each input tile and sample chunk (one warp per tile): its grains (sum of lambda) and
+// its pixels' Poisson set-up (two grain steps: kGwPixelCost).
+constexpr float kGwPixelCost = 800.0f;
 __global__ void grainwise_costs_kernel(const float *__restrict__ lam, int in_w, int in_h, int tin_w, int tin_h, int ntx,
-                                       int ntiles, float *__restrict__ cost) {
+                                       int ntiles, float grain_cost, float *__restrict__ cost) {
     const int tile = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (tile >= ntiles) return;
     const int x0 = (tile % ntx) * tin_w, y0 = (tile / ntx) * tin_h;
     const int w = min(x0 + tin_w, in_w) - x0, n = w * (min(y0 + tin_h, in_h) - y0);
     float sum = 0.0f;
-    for (int i = lane; i < n; i += 32) sum += lam[(long long)(y0 + i / w) * in_w + x0 + i % w];
+    // (clamped: the work list's bound needs finite costs, whatever plane the caller passes)
+    for (int i = lane; i < n; i += 32)
+        sum += fminf(fmaxf(lam[(long long)(y0 + i / w) * in_w + x0 + i % w], 0.0f), 1.0e6f);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) cost[tile] = sum + 4.0f * (float)n;
+    if (lane == 0) cost[tile] = grain_cost * sum + kGwPixelCost * (float)n;
 }
 
-// order[i] = the tile indices by descending cost: a bitonic sort in shared memory (one CTA) for up to
-// kGwSortMax tiles; larger grids keep the natural order.
+// The work list: tiles by descending cost (a bitonic sort in shared memory, one CTA, for up to kGwSortMax
+// tiles; larger grids keep the natural order), each cut into parts of at most `target` lane-ops, the cost
+// an item has when every CTA slot gets kGwItemsPerSlot.  Without the cut, the saturated spots of a blob
+// plane (3 % of the pixels, half of the grains) held the kernel to the end: 1024^2 -> 2048^2, N 128, the
+// heaviest tile ran 14.7 ms while the CTAs were done in 6.6 ms on average; finer cuts than two items per slot
+// repeat the items' set-up and share pixels among more lanes (3 or 4 per slot: 6.5 -> 7.2, 8.0 ms).  A part has no less
+// than kGwItemFloor lane-ops (an item's set-up, about 10 us of a CTA) and a pixel per warp.
+// work[1] = items, then int2 (tile, part | parts << 16).
 constexpr int kGwSortMax = 4096;
-__global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__restrict__ cost, int ntiles,
-                                                               int *__restrict__ order) {
+constexpr int kGwItemsPerSlot = 2;
+constexpr float kGwItemFloor = 2.0e6f;
+__global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__restrict__ cost, int ntiles, int slots,
+                                                               int chunks, int most_parts, int *__restrict__ work) {
     __shared__ float key[kGwSortMax];
     __shared__ int idx[kGwSortMax];
-    const int tid = threadIdx.x;
-    if (ntiles > kGwSortMax) {
-        for (int i = tid; i < ntiles; i += blockDim.x) order[i] = i;
-        return;
-    }
-    int n2 = 2;
-    while (n2 < ntiles) n2 <<= 1;
-    for (int i = tid; i < n2; i += blockDim.x) {
-        key[i] = i < ntiles ? cost[i] : -1.0f;  // costs are >= 0: the padding sorts last
-        idx[i] = i;
-    }
-    __syncthreads();
-    for (int k = 2; k <= n2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < n2; i += blockDim.x) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const bool desc = (i & k) == 0;
-                    if ((key[i] < key[ixj]) == desc) {
-                        const float tk = key[i];
-                        key[i] = key[ixj];
-                        key[ixj] = tk;
-                        const int ti = idx[i];
-                        idx[i] = idx[ixj];
-                        idx[ixj] = ti;
+    __shared__ float wsum[32];
+    __shared__ int wcnt[33];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool sorted = ntiles <= kGwSortMax;
+    float sum = 0.0f;
+    for (int i = tid; i < ntiles; i += blockDim.x) sum += cost[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) wsum[warp] = sum;
+    if (sorted) {
+        int n2 = 2;
+        while (n2 < ntiles) n2 <<= 1;
+        for (int i = tid; i < n2; i += blockDim.x) {
+            key[i] = i < ntiles ? cost[i] : -1.0f;  // costs are >= 0: the padding sorts last
+            idx[i] = i;
+        }
+        __syncthreads();
+        for (int k = 2; k <= n2; k <<= 1) {
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int i = tid; i < n2; i += blockDim.x) {
+                    const int ixj = i ^ j;
+                    if (ixj > i) {
+                        const bool desc = (i & k) == 0;
+                        if ((key[i] < key[ixj]) == desc) {
+                            const float tk = key[i];
+                            key[i] = key[ixj];
+                            key[ixj] = tk;
+                            const int ti = idx[i];
+                            idx[i] = idx[ixj];
+                            idx[ixj] = ti;
+                        }
                     }
                 }
+                __syncthreads();
             }
-            __syncthreads();
         }
     }
-    for (int i = tid; i < ntiles; i += blockDim.x) order[i] = idx[i];
+    __syncthreads();
+    float total = 0.0f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) total += wsum[w];
+    const float target = fmaxf(kGwItemFloor, total * (float)chunks / (float)(slots * kGwItemsPerSlot));
+    int2 *items = reinterpret_cast<int2 *>(work + 2);
+    int base = 0;  // items of the tiles before this round's
+    for (int i0 = 0; i0 < ntiles; i0 += blockDim.x) {
+        const int i = i0 + tid;
+        int tile = 0, parts = 0;
+        if (i < ntiles) {
+            tile = sorted ? idx[i] : i;
+            const float c = sorted ? key[i] : cost[i];
+            parts = max(1, min(most_parts, (int)fminf(ceilf(c / target), 65535.0f)));
+        }
+        int incl = parts;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wcnt[warp] = incl;
+        __syncthreads();
+        int first = base + incl - parts, round = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+            if (w < warp) first += wcnt[w];
+            round += wcnt[w];
+        }
+        for (int q = 0; q < parts; q++) items[first + q] = make_int2(tile, q | (parts << 16));
+        base += round;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        work[0] = 0;
+        work[1] = base;
+    }
 }
 
 // popcount * (1/N) of the sample masks (src/grainwise.rs:114-122), fused with the colour output:
@@ -160,17 +203,6 @@ __global__ void grainwise_epilogue_kernel(const GrainwiseEpilogueArgs a) {
 size_t grainwise_smem_bytes(const GrainwiseArgs &a) { return grainwise_tile_smem_bytes(a); }
 
 // The directed-rounding floor/ceil needs every bounds() argument within +-2^22.
-// CTAs per tile for a stand-alone launch: enough work items to give every SM about eight, never so
-// many that a part has fewer 32-pixel batches than the CTA has warps (bitmask variants only).
-int grainwise_parts(const GrainwiseArgs &a, int sms) {
-    if (grainwise_variant(a.n) == 0) return 1;
-    const int ntiles = grainwise_tile_count(a);
-    const int batches = (a.tin_w * a.tin_h + 31) / 32;
-    const int want = (8 * sms + ntiles - 1) / std::max(1, ntiles);
-    // each part keeps at least one 32-pixel batch per warp: fewer leave warps idle at the tile's end
-    return std::max(1, std::min(std::max(1, batches / kGwWarps), want));
-}
-
 bool grainwise_small_coords(const GrainwiseArgs &a) {
     const float span = (float)max(a.out_w, a.out_h) +
                        fmaxf(fmaxf(-a.offx_min, a.offx_max), fmaxf(-a.offy_min, a.offy_max)) + a.rm * a.zoom + 4.0f;
@@ -181,47 +213,39 @@ int grainwise_tile_count(const GrainwiseArgs &a) {
     return ((a.in_w + a.tin_w - 1) / a.tin_w) * ((a.in_h + a.tin_h - 1) / a.tin_h);
 }
 
-size_t grainwise_work_ints(const GrainwiseArgs &a) { return 2 + 2 * (size_t)grainwise_tile_count(a); }
+// The scheduler's area: item counter, items, then the list -- every tile's share above the first is a target's
+// worth of lane-ops, so there are at most slots * kGwItemsPerSlot of those -- and the tiles' costs.
+static size_t grainwise_list_items(const GrainwiseArgs &a, int sms) {
+    return (size_t)grainwise_tile_count(a) + (size_t)2 * sms * kGwItemsPerSlot + 1;
+}
+size_t grainwise_work_ints(const GrainwiseArgs &a, int sms) {
+    return 2 + 2 * grainwise_list_items(a, sms) + (size_t)grainwise_tile_count(a);
+}
 
-cudaError_t launch_grainwise(const GrainwiseArgs &a, cudaStream_t s) {
+cudaError_t launch_grainwise(const GrainwiseArgs &a, int sms, cudaStream_t s) {
     const size_t smem = grainwise_smem_bytes(a);
     const int ntx = (a.in_w + a.tin_w - 1) / a.tin_w, nty = (a.in_h + a.tin_h - 1) / a.tin_h;
     if (ntx <= 0 || nty <= 0) return cudaSuccess;
     const bool small = grainwise_small_coords(a);
-    const int v = grainwise_variant(a.n);
-    cudaError_t e;
-    if (!a.work) {
-        void (*k)(GrainwiseArgs);
-        if (small) k = v == 4 ? grainwise_kernel<true, 4> : (v == 8 ? grainwise_kernel<true, 8> : grainwise_kernel<true, 0>);
-        else k = v == 4 ? grainwise_kernel<false, 4> : (v == 8 ? grainwise_kernel<false, 8> : grainwise_kernel<false, 0>);
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k<<<dim3(ntx, nty, std::max(1, a.parts)), kGwThreads, smem, s>>>(a);
-        return cudaGetLastError();
-    }
+    const int v = grainwise_variant(a.chunk_words);
     // tile scheduler: costs from lambda, heaviest first, persistent CTAs
-    const int ntiles = ntx * nty;
-    float *cost = reinterpret_cast<float *>(a.work + 2 + ntiles);
-    e = cudaMemsetAsync(a.work, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
-    grainwise_costs_kernel<<<(ntiles + 7) / 8, 256, 0, s>>>(a.lam, a.in_w, a.in_h, a.tin_w, a.tin_h, ntx, ntiles, cost);
-    grainwise_order_kernel<<<1, 1024, 0, s>>>(cost, ntiles, a.work + 2);
-    void (*k)(GrainwiseArgs, int, int);
-    if (small)
-        k = v == 4 ? grainwise_persistent_kernel<true, 4>
-                   : (v == 8 ? grainwise_persistent_kernel<true, 8> : grainwise_persistent_kernel<true, 0>);
-    else
-        k = v == 4 ? grainwise_persistent_kernel<false, 4>
-                   : (v == 8 ? grainwise_persistent_kernel<false, 8> : grainwise_persistent_kernel<false, 0>);
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per_sm = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int ntiles = ntx * nty, slots = 2 * sms;
+    float *cost = reinterpret_cast<float *>(a.work + 2 + 2 * grainwise_list_items(a, sms));
+    grainwise_costs_kernel<<<(ntiles + 7) / 8, 256, 0, s>>>(a.lam, a.in_w, a.in_h, a.tin_w, a.tin_h, ntx, ntiles,
+                                                            a.grain_cost, cost);
+    grainwise_order_kernel<<<1, 1024, 0, s>>>(cost, ntiles, slots, a.chunks, grainwise_most_parts(a.tin_w * a.tin_h),
+                                              a.work);
+    void (*k)(GrainwiseArgs, int);
+    if (!small) k = grainwise_persistent_kernel<false, kGbMaxWords>;  // coordinates beyond 2^22: one variant
+    else if (v == 1) k = grainwise_persistent_kernel<true, 1>;
+    else if (v == 2) k = grainwise_persistent_kernel<true, 2>;
+    else if (v == 4) k = grainwise_persistent_kernel<true, 4>;
+    else k = grainwise_persistent_kernel<true, kGbMaxWords>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kGwThreads, smem);
     if (e != cudaSuccess) return e;
-    const int grid = std::max(1, std::min(ntiles * std::max(1, a.parts), sms * std::max(1, per_sm)));
-    k<<<grid, kGwThreads, smem, s>>>(a, ntx, ntiles);
+    k<<<sms * std::max(1, per_sm), kGwThreads, smem, s>>>(a, ntx);
     return cudaGetLastError();
 }
 

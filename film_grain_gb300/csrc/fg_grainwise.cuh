@@ -1,6 +1,8 @@
 // fg_grainwise.cuh -- device code of the grain-wise integrator (src/grainwise.rs:12-142), shared by
 // the standalone kernel (fg_grainwise.cu) and the batched persistent kernel (fg_batch.cu).
 #pragma once
+#include <algorithm>
+
 #include "fg_kernels.cuh"
 #include "fg_rng.cuh"
 #include "fg_color.cuh"
@@ -9,16 +11,16 @@ namespace fg {
 
 constexpr int kGwThreads = 512;
 constexpr int kGwWarps = kGwThreads / 32;
-constexpr int kGwQueue = 64;     // grains per warp queue (a full batch of 32 plus a partial step)
-constexpr int kGwList = 256;     // surviving (grain, offset) pairs per warp list
-constexpr int kGwBuckets = kGwBucketCount;
 
-// The CTA's shared-memory mask covers the output rectangle [rx0, rx0 + rw) x [ry0, ry0 + rh); bits of
-// other output pixels go straight to the global mask.
+// The CTA's shared-memory mask covers the output rectangle [rx0, rx0 + rw) x [ry0, ry0 + rh) with the
+// `words` mask words of one sample chunk per pixel; bits of other output pixels go straight to the
+// global mask.
 struct GwTile {
     int rx0, ry0, rw, rh, words, out_w;
+    float frx0, fry0, frw, frh;      // the rectangle as floats
     float flast_x, flast_y;          // last output column / row as floats
-    unsigned int *gmask;             // out_w x out_h x words
+    unsigned int *gmask;             // the chunk's first word of out_w x out_h x gwords
+    int gwords;
 };
 
 // floor / ceil of an f32.  With kSmall (every coordinate within +-2^22) they are one directed-rounding
@@ -47,144 +49,68 @@ __device__ __forceinline__ bool gw_range(float c, float r, float lo_t, float hi_
 }
 
 // Stage B: the reference's exact bounds() on both axes, then its centre tests and bit sets
-// (src/grainwise.rs:69-101) for one (grain, offset) pair.  G = (czx, czy, radius_out, -),
-// e = (frac(offy), offx, offy, k).
+// (src/grainwise.rs:69-101) for one (grain, offset) pair: grain (czx, czy, ro) = zoomed centre and
+// radius, offset o, sample k of the chunk.  Most pairs have one pixel or none in their bounds, so the loops
+// test their end after the body.  Pixels of the tile's rectangle are integers below 2^24, so their index is
+// taken in f32.
 template <bool kSmall>
-__device__ __forceinline__ void gw_splat(const GwTile &T, unsigned int *mask, const float4 G, const float4 e) {
-    const float ro = G.z;
-    const float ty = FG_FADD(G.y, e.z);
+__device__ __forceinline__ void gw_splat(const GwTile &T, unsigned int *mask, float czx, float czy, float ro,
+                                         const float2 o, int k) {
+    const float tx = FG_FADD(czx, o.x), ty = FG_FADD(czy, o.y);
     float y0, y1, x0, x1;
-    if (!gw_range<kSmall>(ty, ro, 0.0f, T.flast_y, y0, y1)) return;
-    const float tx = FG_FADD(G.x, e.y);
-    if (!gw_range<kSmall>(tx, ro, 0.0f, T.flast_x, x0, x1)) return;
+    const bool in_y = gw_range<kSmall>(ty, ro, 0.0f, T.flast_y, y0, y1);
+    const bool in_x = gw_range<kSmall>(tx, ro, 0.0f, T.flast_x, x0, x1);
+    if (!(in_x && in_y)) return;
     const float rsq = FG_FMUL(ro, ro);
-    const int k = __float_as_int(e.w);
-    const unsigned bit = 1u << (k & 31);
-    const int word = k >> 5;
-    int oy = (int)y0;
-    for (float fyv = y0; fyv <= y1; fyv = FG_FADD(fyv, 1.0f), oy++) {
-        const float dy = FG_FSUB(FG_FADD(fyv, 0.5f), ty);
+    for (float fy = y0;;) {
+        const float dy = FG_FSUB(FG_FADD(fy, 0.5f), ty);
         const float dysq = FG_FMUL(dy, dy);
-        if (dysq > rsq) continue;
-        int ox = (int)x0;
-        for (float fxv = x0; fxv <= x1; fxv = FG_FADD(fxv, 1.0f), ox++) {
-            const float dx = FG_FSUB(FG_FADD(fxv, 0.5f), tx);
-            if (FG_FADD(FG_FMUL(dx, dx), dysq) <= rsq) {
-                const int lx = ox - T.rx0, ly = oy - T.ry0;
-                if ((unsigned)lx < (unsigned)T.rw && (unsigned)ly < (unsigned)T.rh)
-                    atomicOr(mask + (ly * T.rw + lx) * T.words + word, bit);
-                else
-                    atomicOr(T.gmask + ((long long)oy * T.out_w + ox) * T.words + word, bit);
+        if (dysq <= rsq) {
+            for (float fx = x0;;) {
+                const float dx = FG_FSUB(FG_FADD(fx, 0.5f), tx);
+                if (FG_FADD(FG_FMUL(dx, dx), dysq) <= rsq) {
+                    const float lx = FG_FSUB(fx, T.frx0), ly = FG_FSUB(fy, T.fry0);
+                    const unsigned bit = 1u << (k & 31);
+                    if (lx >= 0.0f && lx < T.frw && ly >= 0.0f && ly < T.frh)
+                        atomicOr(mask + (int)FG_FADD(FG_FMUL(ly, T.frw), lx) * T.words + (k >> 5), bit);
+                    else
+                        atomicOr(T.gmask + ((long long)(int)fy * T.out_w + (int)fx) * T.gwords + (k >> 5), bit);
+                }
+                if (!(fx < x1)) break;
+                fx = FG_FADD(fx, 1.0f);
             }
         }
+        if (!(fy < y1)) break;
+        fy = FG_FADD(fy, 1.0f);
     }
 }
 
-// Candidate ranges of one grain in the sorted offset table: the entries whose frac(offx) lies in the
-// cyclic interval [c - h, c + h], c = frac(1/2 - czx), h = radius_out + margin, rounded out to whole
-// buckets of the index `bstart` (bstart[b] = first entry with frac >= b / kGwBuckets).  Entries the
-// rounding adds are harmless: every entry still goes through the exact reference test.  Packed as
-// (first | end << 16) for the two pieces of the cyclic interval.
-__device__ __forceinline__ uint2 gw_candidates(const int *bstart, int n, float czx, float ro, float eps) {
-    const float h = FG_FADD(ro, eps);
-    if (h >= 0.5f) return make_uint2((unsigned)n << 16, 0u);
-    const float fz = FG_FSUB(czx, floorf(czx));     // exact
-    float c = FG_FSUB(0.5f, fz);
-    if (c < 0.0f) c = FG_FADD(c, 1.0f);
-    const float lo = FG_FSUB(c, h), hi = FG_FADD(c, h);
-    const float nb = (float)kGwBuckets;
-    int s0, e0, s1 = 0, e1 = 0;
-    if (lo < 0.0f) {  // [0, hi] and [lo + 1, 1)
-        s0 = 0;
-        e0 = bstart[min(kGwBuckets - 1, (int)(hi * nb)) + 1];
-        s1 = bstart[min(kGwBuckets - 1, max(0, (int)(FG_FADD(lo, 1.0f) * nb)))];
-        e1 = n;
-    } else if (hi >= 1.0f) {  // [lo, 1) and [0, hi - 1]
-        s0 = bstart[min(kGwBuckets - 1, (int)(lo * nb))];
-        e0 = n;
-        e1 = bstart[min(kGwBuckets - 1, max(0, (int)(FG_FSUB(hi, 1.0f) * nb))) + 1];
-    } else {
-        s0 = bstart[min(kGwBuckets - 1, (int)(lo * nb))];
-        e0 = bstart[min(kGwBuckets - 1, (int)(hi * nb)) + 1];
-    }
-    return make_uint2((unsigned)s0 | ((unsigned)e0 << 16), (unsigned)s1 | ((unsigned)e1 << 16));
-}
-
-// Stage B over the warp's survivor list: one (grain, offset) pair per lane.
-template <bool kSmall>
-__device__ __forceinline__ void gw_drain(const GwTile &T, unsigned int *mask, const float4 *tab, const float4 *q,
-                                         const unsigned *list, int &ln, int lane) {
-    for (int b = 0; b < ln; b += 32) {
-        if (b + lane < ln) {
-            const unsigned v = list[b + lane];
-            gw_splat<kSmall>(T, mask, q[v >> 16], tab[v & 0xFFFFu]);
-        }
-    }
-    ln = 0;
-    __syncwarp();
-}
-
-// Stage A over one batch of `count` queued grains: the (grain, candidate offset) pairs are flattened
-// across the lanes (every lane busy).  A pair can set a bit only if some pixel row lies within
-// radius_out of ty = czy + offy, i.e. only if frac(offy) lies within h = radius_out + margin of
-// cy = frac(1/2 - czy) on the unit circle; that test filters the pairs, and the survivors -- (grain,
-// table index) -- are compacted into the warp's list for the exact stage B.
-template <bool kSmall>
-__device__ __forceinline__ void gw_raster_batch(const GwTile &T, unsigned int *mask, const float4 *tab,
-                                                const float *fy, const float4 *q, const uint2 *qr, int count,
-                                                int *cpre, unsigned *list, int &ln, float eps, int lane) {
-    int c = 0;
-    if (lane < count) {
-        const uint2 r = qr[lane];
-        c = (int)(r.x >> 16) - (int)(r.x & 0xFFFFu) + (int)(r.y >> 16) - (int)(r.y & 0xFFFFu);
-    }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, c, o);
-        if (lane >= o) c += y;
-    }
-    const int total = __shfl_sync(0xffffffffu, c, 31);
-    cpre[lane + 1] = c;
-    if (lane == 0) cpre[0] = 0;
-    __syncwarp();
-    int g = 0;
-    for (int base = 0; base < total; base += 32) {
-        const int t = base + lane;
-        bool surv = false;
-        unsigned item = 0;
-        if (t < total) {
-            while (cpre[g + 1] <= t) g++;
-            const uint2 r = qr[g];
-            const int o = t - cpre[g];
-            const int n0 = (int)(r.x >> 16) - (int)(r.x & 0xFFFFu);
-            const int i = o < n0 ? (int)(r.x & 0xFFFFu) + o : (int)(r.y & 0xFFFFu) + (o - n0);
-            const float2 gy = *reinterpret_cast<const float2 *>(&q[g].z);  // (radius_out, cy)
-            const float h = FG_FADD(gy.x, eps);
-            const float d = fabsf(FG_FSUB(fy[i], gy.y));
-            surv = d <= h || d >= FG_FSUB(1.0f, h);
-            item = ((unsigned)g << 16) | (unsigned)i;
-        }
-        const unsigned sb = __ballot_sync(0xffffffffu, surv);
-        if (surv) list[ln + __popc(sb & ((1u << lane) - 1u))] = item;
-        ln += __popc(sb);
-        __syncwarp();
-        if (ln > kGwList - 32) gw_drain<kSmall>(T, mask, tab, q, list, ln, lane);
-    }
-    gw_drain<kSmall>(T, mask, tab, q, list, ln, lane);
-}
-
-// ------------------------------------------------------------------ bitmask candidate filter (N <= 256)
-// For N <= 256 the candidate offsets of a grain are found as a bitmask over the sample index k: the
-// unit interval of frac(offset) is cut into 128 buckets, and for each axis a sparse table holds, for
-// every bucket b and level L, the OR of the sample masks of buckets b .. b + 2^L - 1 (cyclic).  The
+// ------------------------------------------------------------------ bitmask candidate filter
+// The candidate offsets of a grain are found as a bitmask over the sample index k: the unit interval of
+// frac(offset) is cut into 128 buckets, and for each axis a sparse table holds, for every bucket b and
+// level L, the OR of the sample masks of buckets b .. b + 2^(L+1) - 1 (cyclic).  The
 // cyclic interval [c - h, c + h] of an axis test, rounded out to whole buckets, is the OR of two table
-// entries; the AND of the x and y masks is a superset of the pairs that pass both of the tests the
-// flattened stage A applies (so of every pair that can set a bit), and those pairs go to stage B.
+// entries; the AND of the x and y masks is a superset of every pair that can set a bit (a pixel centre
+// lies within radius_out of the offset grain centre on both axes), and those pairs go to stage B.
+// The masks take kGbMaxWords words at most (256 samples).  More samples are cut into chunks of equal
+// width, and a work item renders one chunk of its tile: it draws the grains again (150 to 250 lane-ops
+// of the about 1000 a grain costs with its pairs) and keeps the filter, the tables and the tile's
+// masks small.  A 311x205 plane at zoom 1.5, N 400, r 0.08: 16.0 ms with one item per tile for all
+// samples, listing (grain, offset) pairs from a sorted offset table, 6.4 ms with two chunks of 200 (1.7 ms
+// with the rest of this file).
 constexpr int kGbBuckets = 128;
-constexpr int kGbLevels = 7;     // spans 1 .. 64 buckets; 128 or more is the full mask
-constexpr int kGbMaxWords = 8;   // N <= 256
+constexpr int kGbLevels = 6;     // spans 2 .. 64 buckets (a span of 1 takes 2); 128 or more is the full mask
+constexpr int kGbMaxWords = 8;   // samples of a chunk: at most 256
 
-__host__ __device__ inline bool grainwise_uses_bits(int n) { return n <= 32 * kGbMaxWords; }
+// A warp's pair queue (gw_process): the candidate (grain, sample) pairs of its lanes' grains, taken
+// out 32 at a time, and the grains they belong to.  Fewer than 32 pairs stay between steps, so the last
+// kGwGrains = 31 + 32 grains pushed (and one) are all that the queue can name.
+constexpr int kGwPairs = 256;    // queue entries: grain slot << 8 | sample of the chunk
+constexpr int kGwGrains = 64;    // grain slots: zoomed centre and radius
+struct GwQueue {
+    float gx[kGwGrains], gy[kGwGrains], gr[kGwGrains];
+    unsigned short pair[kGwPairs];
+};
 
 // Words between consecutive table entries: W rounded up to odd, so that the lanes of a warp reading
 // word w of the entries of different buckets b hit different banks ((b * S + w) mod 32 is one-to-one
@@ -210,9 +136,9 @@ __device__ __forceinline__ void gb_axis_mask(const unsigned *tab, int W, int S, 
         return;
     }
     const int b0 = blo & (kGbBuckets - 1);
-    const int L = 31 - __clz(len);
+    const int L = 30 - __clz(len | 2);  // spans of 2^(L+1) <= len buckets (2 for len = 1)
     const unsigned *e0 = tab + (L * kGbBuckets + b0) * S;
-    const unsigned *e1 = tab + (L * kGbBuckets + ((b0 + len - (1 << L)) & (kGbBuckets - 1))) * S;
+    const unsigned *e1 = tab + (L * kGbBuckets + ((b0 + max(len, 2) - (2 << L)) & (kGbBuckets - 1))) * S;
 #pragma unroll
     for (int w = 0; w < MW; w++) {
         const unsigned v = w < W ? (e0[w] | e1[w]) : 0u;
@@ -220,20 +146,44 @@ __device__ __forceinline__ void gb_axis_mask(const unsigned *tab, int W, int S, 
     }
 }
 
-// Part `part` of `parts` of a tile: a contiguous range of its 32-pixel batches (a heavy tile is split
-// over several CTAs, each with its own copy of the tile's masks; OR makes the result the same).
+// Stage B on queue entries [head, head + 32) of a warp, `n` of them valid.
+template <bool kSmall>
+__device__ __forceinline__ void gw_process(const GwTile &T, unsigned int *mask, const float2 *offk, const GwQueue &Q,
+                                           int head, int n, int lane) {
+    if (lane < n) {
+        const unsigned e = Q.pair[head + lane];
+        const int g = (int)(e >> 8), k = (int)(e & 0xFFu);
+        gw_splat<kSmall>(T, mask, Q.gx[g], Q.gy[g], Q.gr[g], offk[k], k);
+    }
+}
+
+// Chunk `chunk` of the samples over part `part` of `parts` of a tile: a contiguous range of its pixels (a
+// heavy tile is split over several CTAs, each with its own copy of the tile's masks; OR makes the result
+// the same).  Each step of a warp draws one grain per lane.  In a part with enough pixels for the CTA's
+// warps a lane has a pixel of its own; in a smaller one g = 2 .. 32 lanes share a pixel: they hold the same
+// stream, draw its next g grains one after another, and each keeps one.  The draws (36 lane-ops for the
+// centre, about 90 with a log-normal radius) are then repeated in g lanes, but a pixel's grains are a serial
+// chain of whole steps, and a step's filter and pairs cost several times its draws (311x205, N 400: 4.9 -> 1.7 ms; 128x96, N 32:
+// 0.88 -> 0.39 ms; filling the warps 1.5 or 2 times over instead of once was slower, 6.5 -> 7.0 and 8.0 ms
+// on the 1024^2 -> 2048^2 plane).
+// A group whose pixel is done takes the next one once half of the warp's groups wait (the Poisson set-up runs
+// for all of them at once), so that pixels of unequal lambda keep the lanes busy.
 template <bool kSmall, int MW>
 __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int tile_x, int tile_y,
-                                                    unsigned char *smem_raw, int part, int parts) {
-    const int W = (a.n + 31) >> 5;
-    float2 *offk = reinterpret_cast<float2 *>(smem_raw);                         // [n] (offx, offy) by k
+                                                    unsigned char *smem_raw, int part, int parts, int chunk) {
+    const int k0 = 32 * chunk * a.chunk_words;                 // the chunk's samples: [k0, k0 + n)
+    const int n = min(a.n - k0, 32 * a.chunk_words);
+    const int W = (n + 31) >> 5;
+    float2 *offk = reinterpret_cast<float2 *>(smem_raw);                       // [n] (offx, offy) by k
     const int S = gb_entry_stride(W);
-    unsigned *tabx = reinterpret_cast<unsigned *>(offk + ((a.n + 1) & ~1));     // [levels][buckets][S]
+    unsigned *tabx = reinterpret_cast<unsigned *>(offk + ((n + 1) & ~1));     // [levels][buckets][S]
     unsigned *taby = tabx + kGbLevels * kGbBuckets * S;
     unsigned short *bk = reinterpret_cast<unsigned short *>(taby + kGbLevels * kGbBuckets * S);  // [n] buckets
-    int *next_px = reinterpret_cast<int *>(bk + ((a.n + 7) & ~7));             // [4]: batch counter
-    unsigned int *mask = reinterpret_cast<unsigned int *>(next_px + 4);
+    int *next_px = reinterpret_cast<int *>(bk + ((n + 7) & ~7));               // [4]: the next pixel
+    GwQueue *queues = reinterpret_cast<GwQueue *>(next_px + 4);                // [warps]
+    unsigned int *mask = reinterpret_cast<unsigned int *>(queues + kGwWarps);
     const int tid = threadIdx.x, lane = tid & 31;
+    GwQueue &Q = queues[tid >> 5];
 
     const int ix0 = tile_x * a.tin_w, iy0 = tile_y * a.tin_h;
     const int ix1 = min(ix0 + a.tin_w, a.in_w), iy1 = min(iy0 + a.tin_h, a.in_h);
@@ -244,38 +194,45 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
     T.rh = min(a.rmax_h, min(a.out_h, (int)floorf((float)iy1 * a.zoom)) - T.ry0);
     T.rw = max(T.rw, 0);
     T.rh = max(T.rh, 0);
-    T.words = a.words;
+    T.frx0 = (float)T.rx0;
+    T.fry0 = (float)T.ry0;
+    T.frw = (float)T.rw;
+    T.frh = (float)T.rh;
+    T.words = W;
     T.out_w = a.out_w;
     T.flast_x = (float)(a.out_w - 1);
     T.flast_y = (float)(a.out_h - 1);
-    T.gmask = a.gmask;
-    const int region_words = T.rw * T.rh * a.words;
+    T.gmask = a.gmask + chunk * a.chunk_words;
+    T.gwords = a.words;
+    const int region_words = T.rw * T.rh * W;
 
-    // offsets by sample index, and each sample's x / y bucket
-    for (int i = tid; i < a.n; i += kGwThreads) {
-        const float4 e = a.sorted_offs[i];  // (frac(offy), offx, offy, k)
-        const int k = __float_as_int(e.w);
-        offk[k] = make_float2(e.y, e.z);
-        float fx = FG_FSUB(e.y, floorf(e.y));
+    // the chunk's offsets, and each sample's x / y bucket
+    for (int k = tid; k < n; k += kGwThreads) {
+        const float2 o = a.offs[k0 + k];
+        offk[k] = o;
+        float fx = FG_FSUB(o.x, floorf(o.x)), fy = FG_FSUB(o.y, floorf(o.y));
         if (!(fx < 1.0f)) fx = 0.0f;  // a tiny negative offset rounds up to 1; cyclically that is 0
-        bk[k] =(unsigned short)((int)FG_FMUL(fx, (float)kGbBuckets) | ((int)FG_FMUL(e.x, (float)kGbBuckets) << 8));
+        if (!(fy < 1.0f)) fy = 0.0f;
+        bk[k] = (unsigned short)((int)FG_FMUL(fx, (float)kGbBuckets) | ((int)FG_FMUL(fy, (float)kGbBuckets) << 8));
     }
     for (int t = tid; t < region_words; t += kGwThreads) mask[t] = 0u;
     const int fw = ix1 - ix0, total = fw * (iy1 - iy0);
-    const int nbatch = (total + 31) >> 5;
-    const int px_begin = 32 * (int)(((long long)nbatch * part) / parts);
-    const int px_end = min(total, 32 * (int)(((long long)nbatch * (part + 1)) / parts));
+    const int px_begin = (int)(((long long)total * part) / parts);
+    const int px_end = (int)(((long long)total * (part + 1)) / parts);
     if (tid == 0) *next_px = px_begin;
+    int g = 1;  // lanes per pixel
+    while (g < 32 && g * (px_end - px_begin) < kGwThreads) g *= 2;
+    const int sub = lane & (g - 1);
+    // level 0: two buckets each
+    for (int t = tid; t < kGbBuckets * S; t += kGwThreads) tabx[t] = taby[t] = 0u;
     __syncthreads();
-    for (int t = tid; t < 2 * kGbBuckets * W; t += kGwThreads) {  // level 0: one bucket each
-        const int axis = t / (kGbBuckets * W), r = t - axis * kGbBuckets * W;
-        const int b = r / W, w = r - b * W;
-        unsigned bits = 0u;
-        for (int j = 0; j < 32; j++) {
-            const int k = w * 32 + j;
-            if (k < a.n && ((bk[k] >> (8 * axis)) & 0xFF) == b) bits |= 1u << j;
-        }
-        (axis ? taby : tabx)[b * S + w] = bits;
+    for (int k = tid; k < n; k += kGwThreads) {
+        const int bx = bk[k] & 0xFF, by = bk[k] >> 8, w = k >> 5;
+        const unsigned bit = 1u << (k & 31);
+        atomicOr(&tabx[bx * S + w], bit);
+        atomicOr(&tabx[((bx + kGbBuckets - 1) & (kGbBuckets - 1)) * S + w], bit);
+        atomicOr(&taby[by * S + w], bit);
+        atomicOr(&taby[((by + kGbBuckets - 1) & (kGbBuckets - 1)) * S + w], bit);
     }
     __syncthreads();
     for (int L = 1; L < kGbLevels; L++) {
@@ -283,7 +240,7 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
             const int axis = t / (kGbBuckets * W), r = t - axis * kGbBuckets * W;
             const int b = r / W, w = r - b * W;
             unsigned *tb = axis ? taby : tabx;
-            const int b2 = (b + (1 << (L - 1))) & (kGbBuckets - 1);
+            const int b2 = (b + (1 << L)) & (kGbBuckets - 1);
             tb[(L * kGbBuckets + b) * S + w] = tb[((L - 1) * kGbBuckets + b) * S + w] |
                                                tb[((L - 1) * kGbBuckets + b2) * S + w];
         }
@@ -292,37 +249,59 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
 
     const UniformF32 U = uniform_f32_new(0.0f, 1.0f);
     const float zoom = a.zoom;
+    uint32_t left = 0;  // grains of this group's pixel still to draw
+    int px = 0, py = 0;
+    Xoshiro rng = {0, 0, 0, 0};
+    bool more = true;   // the part may still have pixels (warp-uniform)
+    int qn = 0;         // pairs in the warp's queue (below 32 between steps)
+    int gn = 0;         // grains pushed so far
     for (;;) {
-        // the next 32 footprint pixels of this part (a shared counter balances the warps), one per
-        // lane, Poisson set-up in step across the warp
-        int base = 0;
-        if (lane == 0) base = atomicAdd(next_px, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= px_end) break;
-        const int pi = base + lane;
-        uint32_t left = 0;
-        int px = 0, py = 0;
-        Xoshiro rng = {0, 0, 0, 0};
-        if (pi < px_end) {
-            px = ix0 + pi % fw;
-            py = iy0 + pi / fw;
-            const float lv = a.lam[(long long)py * a.in_w + px];
-            if (lv > 0.0f) {
-                left = poisson_count(mix3(a.seed, kPixelStream, px, py), lv, rng);
+        const unsigned busy = __ballot_sync(0xffffffffu, left > 0);
+        if (more && __popc(busy) <= 16) {
+            const unsigned idle = ~busy;
+            const int want = __popc(idle) / g;  // groups without a pixel
+            int base = 0;
+            if (lane == 0) base = atomicAdd(next_px, want);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            more = base + want < px_end;
+            const int pi = base + __popc(idle & ((1u << (lane & ~(g - 1))) - 1u)) / g;
+            if (((idle >> lane) & 1u) && pi < px_end) {
+                px = ix0 + pi % fw;
+                py = iy0 + pi / fw;
+                const float lv = a.lam[(long long)py * a.in_w + px];
+                if (lv > 0.0f) left = poisson_count(mix3(a.seed, kPixelStream, px, py), lv, rng);
             }
+            continue;
         }
-        while (__any_sync(0xffffffffu, left > 0)) {
-            // one grain per lane; its candidate samples as a bitmask
+        if (busy == 0u) break;
+        {
+            // the group's next g grains, one kept by each lane
+            bool have = false;
+            float ux = 0.0f, uy = 0.0f;
+            RadiusDraw rd = {0ull, -1.0f};
+            for (int t = 0; t < g; t++) {
+                if (left > 0) {
+                    left--;
+                    const float vx = uniform_f32_from(U, rng.next()), vy = uniform_f32_from(U, rng.next());
+                    RadiusDraw vd = {0ull, -1.0f};
+                    if (a.lognorm) vd = lognormal_draw(a.log_mu, a.log_sigma, rng);
+                    if (t == sub) {
+                        have = true;
+                        ux = vx;
+                        uy = vy;
+                        rd = vd;
+                    }
+                }
+            }
+            // its candidate samples as a bitmask
             unsigned m[MW];
 #pragma unroll
             for (int w = 0; w < MW; w++) m[w] = 0u;
             int cnt = 0;
             float gx = 0.0f, gy = 0.0f, gr = 0.0f;  // this lane's grain: zoomed centre, zoomed radius
-            if (left > 0) {
-                left--;
-                const float cx = FG_FADD((float)px, uniform_f32_from(U, rng.next()));
-                const float cy = FG_FADD((float)py, uniform_f32_from(U, rng.next()));
-                float r = a.lognorm ? lognormal_radius_f32(a.log_mu, a.log_sigma, rng) : a.radius_mean;
+            if (have) {
+                const float cx = FG_FADD((float)px, ux), cy = FG_FADD((float)py, uy);
+                float r = a.lognorm ? lognormal_radius(rd, a.log_mu, a.log_sigma) : a.radius_mean;
                 if (r > a.rm) r = a.rm;
                 if (r > 0.0f) {
                     const float ro = FG_FMUL(r, zoom);
@@ -336,17 +315,15 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
                         gy = czy;
                         gr = ro;
                         const float h = FG_FADD(ro, a.frac_eps);
-                        gb_axis_mask<MW, false>(tabx, W, S, cxf, h, a.n, m);
-                        gb_axis_mask<MW, true>(taby, W, S, cyf, h, a.n, m);
+                        gb_axis_mask<MW, false>(tabx, W, S, cxf, h, n, m);
+                        gb_axis_mask<MW, true>(taby, W, S, cyf, h, n, m);
 #pragma unroll
                         for (int w = 0; w < MW; w++) cnt += __popc(m[w]);
                     }
                 }
             }
-            // this step's (grain, sample) pairs, 32 at a time: pair p belongs to the first lane whose
-            // inclusive candidate count exceeds p (a binary search over shuffled prefixes), and is the
-            // (p - exclusive count)-th set bit of that lane's mask.  Every lane stays converged and the
-            // grains never leave the registers of the lanes that drew them.
+            // this step's (grain, sample) pairs go to the warp's queue, each lane's at its prefix of the counts,
+            // and leave it 32 at a time (every lane busy), the last few staying for the next step
             int incl = cnt;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -354,215 +331,103 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
                 if (lane >= o) incl += y;
             }
             const int tot = __shfl_sync(0xffffffffu, incl, 31);
-            for (int b = 0; b < tot; b += 32) {
-                const int p = b + lane;
-                int src = 0;
+            if (tot == 0) continue;
+            const unsigned with = __ballot_sync(0xffffffffu, cnt > 0);
+            const int slot = (gn + __popc(with & ((1u << lane) - 1u))) & (kGwGrains - 1);
+            gn += __popc(with);
+            if (cnt > 0) {
+                Q.gx[slot] = gx;
+                Q.gy[slot] = gy;
+                Q.gr[slot] = gr;
+            }
+            for (int done = 0; done < tot;) {
+                // the lanes whose pairs still fit, in lane order
+                const unsigned fit = __ballot_sync(0xffffffffu, incl - done <= kGwPairs - qn);
+                const int upto = fit ? __shfl_sync(0xffffffffu, incl, 31 - __clz(fit)) : 0;
+                if (upto <= done) {
+                    // one lane's pairs alone overflow the queue (grains that reach most samples): the lanes
+                    // take their own pairs, which are about as many on each.  The queue is emptied too: its
+                    // pairs would outlive their grains' slots.
+                    gw_process<kSmall>(T, mask, offk, Q, 0, qn, lane);
+                    qn = 0;
+                    __syncwarp();
+                    const bool mine = incl - cnt >= done;
 #pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int v = __shfl_sync(0xffffffffu, incl, src + step - 1);
-                    if (v <= p) src += step;
+                    for (int w = 0; w < MW; w++) {
+                        unsigned v = mine ? m[w] : 0u;
+                        while (v) {
+                            const int k = 32 * w + __ffs(v) - 1;
+                            v &= v - 1u;
+                            gw_splat<kSmall>(T, mask, gx, gy, gr, offk[k], k);
+                        }
+                    }
+                    break;
                 }
-                int j = p - (__shfl_sync(0xffffffffu, incl, src) - __shfl_sync(0xffffffffu, cnt, src));
-                unsigned word = 0u;
-                int wsel = 0;
+                if (cnt > 0 && incl - cnt >= done && incl <= upto) {
+                    unsigned short *q = Q.pair + qn + (incl - cnt - done);
 #pragma unroll
-                for (int w = 0; w < MW; w++) {
-                    const unsigned mw = __shfl_sync(0xffffffffu, m[w], src);
-                    const int c = __popc(mw);
-                    if (wsel == w) {
-                        if (j < c) word = mw;
-                        else { j -= c; wsel = w + 1; }
+                    for (int w = 0; w < MW; w++) {
+                        unsigned v = m[w];
+                        while (v) {
+                            *q++ = (unsigned short)((slot << 8) | (32 * w + __ffs(v) - 1));
+                            v &= v - 1u;
+                        }
                     }
                 }
-                int bit = 0;  // the j-th set bit of `word`
-#pragma unroll
-                for (int half = 16; half > 0; half >>= 1) {
-                    const int c = __popc(word & ((1u << half) - 1u));
-                    if (j >= c) {
-                        j -= c;
-                        bit += half;
-                        word >>= half;
-                    }
-                }
-                const float sx = __shfl_sync(0xffffffffu, gx, src);
-                const float sy = __shfl_sync(0xffffffffu, gy, src);
-                const float sr = __shfl_sync(0xffffffffu, gr, src);
-                if (p < tot) {
-                    const int k = wsel * 32 + bit;
-                    const float2 o = offk[k];
-                    gw_splat<kSmall>(T, mask, make_float4(sx, sy, sr, 0.0f), make_float4(0.0f, o.x, o.y, __int_as_float(k)));
+                qn += upto - done;
+                done = upto;
+                __syncwarp();
+                int head = 0;
+                for (; head + 32 <= qn; head += 32) gw_process<kSmall>(T, mask, offk, Q, head, 32, lane);
+                if (head > 0) {  // the rest moves to the front
+                    const unsigned short e = Q.pair[head + lane < qn ? head + lane : head - 1];
+                    __syncwarp();
+                    if (head + lane < qn) Q.pair[lane] = e;
+                    qn -= head;
+                    __syncwarp();
                 }
             }
         }
     }
+    gw_process<kSmall>(T, mask, offk, Q, 0, qn, lane);
     __syncthreads();
 
     // OR the rectangle's words into the global mask (other CTAs' spills land there too).
     for (int t = tid; t < region_words; t += kGwThreads) {
         const unsigned v = mask[t];
         if (v) {
-            const int w = t % a.words, px = t / a.words;
+            const int w = t % W, px = t / W;
             const int lx = px % T.rw, ly = px / T.rw;
-            atomicOr(a.gmask + ((long long)(T.ry0 + ly) * a.out_w + (T.rx0 + lx)) * a.words + w, v);
+            atomicOr(T.gmask + ((long long)(T.ry0 + ly) * a.out_w + (T.rx0 + lx)) * a.words + w, v);
         }
     }
 }
-
-inline size_t grainwise_bits_smem_bytes(const GrainwiseArgs &a) {
-    const size_t W = (size_t)(a.n + 31) / 32;
-    return (size_t)((a.n + 1) & ~1) * sizeof(float2) +
-           2 * (size_t)kGbLevels * kGbBuckets * gb_entry_stride((int)W) * sizeof(unsigned) +
-           (size_t)((a.n + 7) & ~7) * sizeof(unsigned short) + 4 * sizeof(int) +
-           (size_t)a.rmax_w * a.rmax_h * a.words * sizeof(unsigned int);
-}
-
-// The tile variant for n samples: 4 or 8 = the bitmask filter with that many mask words, 0 = the
-// flattened stage A (n > 256).
-__host__ __device__ inline int grainwise_variant(int n) { return n <= 128 ? 4 : (grainwise_uses_bits(n) ? 8 : 0); }
-
-template <bool kSmall>
-__device__ __forceinline__ void grainwise_tile_flat(const GrainwiseArgs &a, int tile_x, int tile_y,
-                                                    unsigned char *smem_raw);
-
-// One input tile of the grain-wise kernel (all threads of the CTA; `smem_raw` holds its shared memory).
-// kVariant: grainwise_variant(a.n), or -1 to dispatch at run time (the batched kernel).
-// parts > 1 splits the tile's pixels over CTAs (bitmask variants only; the flat variant takes whole tiles).
-template <bool kSmall, int kVariant = -1>
-__device__ __forceinline__ void grainwise_tile(const GrainwiseArgs &a, int tile_x, int tile_y,
-                                               unsigned char *smem_raw, int part = 0, int parts = 1) {
-    const int v = kVariant >= 0 ? kVariant : grainwise_variant(a.n);
-    if (v == 4) grainwise_tile_bits<kSmall, 4>(a, tile_x, tile_y, smem_raw, part, parts);
-    else if (v == 8) grainwise_tile_bits<kSmall, kGbMaxWords>(a, tile_x, tile_y, smem_raw, part, parts);
-    else grainwise_tile_flat<kSmall>(a, tile_x, tile_y, smem_raw);
-}
-
-template <bool kSmall>
-__device__ __forceinline__ void grainwise_tile_flat(const GrainwiseArgs &a, int tile_x, int tile_y,
-                                                    unsigned char *smem_raw) {
-    float4 *tab = reinterpret_cast<float4 *>(smem_raw);                   // [n] offsets, by frac(offx)
-    float4 *queue = tab + a.n;                                            // [warps][kGwQueue] grains
-    uint2 *qrange = reinterpret_cast<uint2 *>(queue + kGwWarps * kGwQueue); // [warps][kGwQueue]
-    unsigned *lists = reinterpret_cast<unsigned *>(qrange + kGwWarps * kGwQueue);  // [warps][kGwList]
-    float *fy = reinterpret_cast<float *>(lists + kGwWarps * kGwList);    // [n] frac(offy), table order
-    int *cpre = reinterpret_cast<int *>(fy + a.n);                        // [warps][33]
-    int *bstart = cpre + kGwWarps * 33;                                   // [kGwBuckets + 1]
-    unsigned int *mask = reinterpret_cast<unsigned int *>(bstart + kGwBuckets + 3);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-    // This CTA's input tile and the output rectangle its mask covers (the zoomed tile).
-    const int ix0 = tile_x * a.tin_w, iy0 = tile_y * a.tin_h;
-    const int ix1 = min(ix0 + a.tin_w, a.in_w), iy1 = min(iy0 + a.tin_h, a.in_h);
-    GwTile T;
-    T.rx0 = min(a.out_w, (int)floorf((float)ix0 * a.zoom));
-    T.ry0 = min(a.out_h, (int)floorf((float)iy0 * a.zoom));
-    T.rw = min(a.rmax_w, min(a.out_w, (int)floorf((float)ix1 * a.zoom)) - T.rx0);
-    T.rh = min(a.rmax_h, min(a.out_h, (int)floorf((float)iy1 * a.zoom)) - T.ry0);
-    T.rw = max(T.rw, 0);
-    T.rh = max(T.rh, 0);
-    T.words = a.words;
-    T.out_w = a.out_w;
-    T.flast_x = (float)(a.out_w - 1);
-    T.flast_y = (float)(a.out_h - 1);
-    T.gmask = a.gmask;
-    const int region_words = T.rw * T.rh * a.words;
-
-    for (int k = tid; k < a.n; k += kGwThreads) {
-        const float4 e = a.sorted_offs[k];
-        tab[k] = e;
-        fy[k] = e.x;
-    }
-    for (int t = tid; t < region_words; t += kGwThreads) mask[t] = 0u;
-    for (int b = tid; b <= kGwBuckets; b += kGwThreads) bstart[b] = a.bucket_start[b];
-    __syncthreads();
-
-    const int fw = ix1 - ix0, total = fw * (iy1 - iy0);
-    const UniformF32 U = uniform_f32_new(0.0f, 1.0f);
-    const float zoom = a.zoom;
-    float4 *q = queue + warp * kGwQueue;
-    uint2 *qr = qrange + warp * kGwQueue;
-    unsigned *list = lists + warp * kGwList;
-    int *wc = cpre + warp * 33;
-
-    int qn = 0;  // warp-uniform grain-queue fill
-    int ln = 0;  // warp-uniform survivor-list fill
-    for (int base = warp * 32; base < total; base += kGwThreads) {
-        // one footprint pixel per lane, Poisson set-up in step across the warp
-        const int pi = base + lane;
-        uint32_t left = 0;
-        int px = 0, py = 0;
-        Xoshiro rng = {0, 0, 0, 0};
-        if (pi < total) {
-            px = ix0 + pi % fw;
-            py = iy0 + pi / fw;
-            const float lv = a.lam[(long long)py * a.in_w + px];
-            if (lv > 0.0f) {
-                left = poisson_count(mix3(a.seed, kPixelStream, px, py), lv, rng);
-            }
-        }
-        while (__any_sync(0xffffffffu, left > 0)) {
-            bool valid = false;
-            float4 G;
-            uint2 R;
-            if (left > 0) {
-                left--;
-                const float cx = FG_FADD((float)px, uniform_f32_from(U, rng.next()));
-                const float cy = FG_FADD((float)py, uniform_f32_from(U, rng.next()));
-                float r = a.lognorm ? lognormal_radius_f32(a.log_mu, a.log_sigma, rng) : a.radius_mean;
-                if (r > a.rm) r = a.rm;
-                if (r > 0.0f) {
-                    const float ro = FG_FMUL(r, zoom);
-                    if (ro > 0.0f) {
-                        valid = true;
-                        const float czy = FG_FMUL(cy, zoom);
-                        float cyf = FG_FSUB(0.5f, FG_FSUB(czy, floorf(czy)));  // frac(1/2 - czy)
-                        if (cyf < 0.0f) cyf = FG_FADD(cyf, 1.0f);
-                        G = make_float4(FG_FMUL(cx, zoom), czy, ro, cyf);
-                        R = gw_candidates(bstart, a.n, G.x, ro, a.frac_eps);
-                    }
-                }
-            }
-            const unsigned vb = __ballot_sync(0xffffffffu, valid);
-            if (valid) {
-                const int slot = qn + __popc(vb & ((1u << lane) - 1u));
-                q[slot] = G;
-                qr[slot] = R;
-            }
-            qn += __popc(vb);
-            __syncwarp();
-            if (qn >= 32) {
-                gw_raster_batch<kSmall>(T, mask, tab, fy, q, qr, 32, wc, list, ln, a.frac_eps, lane);
-                __syncwarp();
-                if (lane + 32 < qn) {
-                    q[lane] = q[lane + 32];
-                    qr[lane] = qr[lane + 32];
-                }
-                qn -= 32;
-                __syncwarp();
-            }
-        }
-    }
-    if (qn > 0) gw_raster_batch<kSmall>(T, mask, tab, fy, q, qr, qn, wc, list, ln, a.frac_eps, lane);
-    __syncthreads();
-
-    // OR the rectangle's words into the global mask (other CTAs' spills land there too).
-    for (int t = tid; t < region_words; t += kGwThreads) {
-        const unsigned v = mask[t];
-        if (v) {
-            const int w = t % a.words, px = t / a.words;
-            const int lx = px % T.rw, ly = px / T.rw;
-            atomicOr(a.gmask + ((long long)(T.ry0 + ly) * a.out_w + (T.rx0 + lx)) * a.words + w, v);
-        }
-    }
-}
-
 
 // Shared-memory bytes of one grain-wise tile.
 inline size_t grainwise_tile_smem_bytes(const GrainwiseArgs &a) {
-    if (grainwise_uses_bits(a.n)) return grainwise_bits_smem_bytes(a);
-    return (size_t)a.n * sizeof(float4) + (size_t)kGwWarps * kGwQueue * sizeof(float4) +
-           (size_t)kGwWarps * kGwQueue * sizeof(uint2) + (size_t)kGwWarps * kGwList * sizeof(unsigned) +
-           (size_t)a.n * sizeof(float) + ((size_t)kGwWarps * 33 + kGwBuckets + 3) * sizeof(int) +
-           (size_t)a.rmax_w * a.rmax_h * a.words * sizeof(unsigned int);
+    const size_t W = (size_t)a.chunk_words, n = std::min<size_t>((size_t)a.n, 32 * W);
+    return ((n + 1) & ~(size_t)1) * sizeof(float2) +
+           2 * (size_t)kGbLevels * kGbBuckets * gb_entry_stride((int)W) * sizeof(unsigned) +
+           ((n + 7) & ~(size_t)7) * sizeof(unsigned short) + 4 * sizeof(int) + kGwWarps * sizeof(GwQueue) +
+           (size_t)a.rmax_w * a.rmax_h * W * sizeof(unsigned int);
+}
+
+// The most CTAs a tile of `px` pixels is split over: one pixel for each warp.
+inline int grainwise_most_parts(int px) { return std::max(1, std::min(px / kGwWarps, 0x7FFF)); }
+
+// The tile variant for chunks of `words` mask words: the words a grain's candidate mask holds in registers.
+__host__ __device__ inline int grainwise_variant(int words) {
+    return words <= 1 ? 1 : words <= 2 ? 2 : words <= 4 ? 4 : kGbMaxWords;
+}
+
+// One input tile of the grain-wise kernel (all threads of the CTA; `smem_raw` holds its shared memory).
+// kVariant: grainwise_variant(a.chunk_words), or -1 to dispatch at run time (the batched kernel).
+template <bool kSmall, int kVariant = -1>
+__device__ __forceinline__ void grainwise_tile(const GrainwiseArgs &a, int tile_x, int tile_y,
+                                               unsigned char *smem_raw, int part, int parts, int chunk) {
+    if (kVariant > 0) grainwise_tile_bits<kSmall, kVariant < 0 ? 1 : kVariant>(a, tile_x, tile_y, smem_raw, part, parts, chunk);
+    else if (kSmall && a.chunk_words <= 2) grainwise_tile_bits<kSmall, 2>(a, tile_x, tile_y, smem_raw, part, parts, chunk);
+    else grainwise_tile_bits<kSmall, kGbMaxWords>(a, tile_x, tile_y, smem_raw, part, parts, chunk);
 }
 
 }  // namespace fg

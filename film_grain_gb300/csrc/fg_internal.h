@@ -24,12 +24,8 @@ fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_der
                             const float *d_offs_in, float *d_out, CellParam *d_cells, unsigned long long *d_diag,
                             const EpilogueArgs *colour, cudaStream_t s, bool may_allocate = true,
                             int *d_cancel = nullptr);
-// The grain-wise offset table: n entries (frac(offy), offx, offy, k) sorted by frac(offx), followed by
-// the bucket index over frac(offx) (kGwBucketCount + 1 ints).
-size_t grain_table_bytes(uint32_t n);
-void grain_table(const float *h_offs, uint32_t n, void *blob);
 GrainwiseArgs grainwise_args(const fg_params &p, const fg_derived &d, const float *h_offs, const float *d_lam,
-                             const void *d_table, unsigned int *d_gmask, int mask_words);
+                             const float *d_offs, unsigned int *d_gmask, int mask_words);
 bool grainwise_small_coords(const GrainwiseArgs &a);
 size_t grainwise_mask_bytes(const fg_params &p, const fg_derived &d);
 fg_status enqueue_grainwise(const GrainwiseArgs &a, cudaStream_t s);

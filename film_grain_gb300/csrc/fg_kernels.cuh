@@ -90,15 +90,13 @@ struct PixelwiseArgs {
     int cm_gi0, cm_gj0, cm_gw, cm_ghw;
 };
 
-constexpr int kGwBucketCount = 256;  // bucket index over the frac(offx)-sorted offsets
-
 struct GrainwiseArgs {
     const float *lam;           // in_w x in_h
-    const float4 *sorted_offs;  // [n] (frac(offy), offx, offy, k as int bits), ascending frac(offx)
-    const int *bucket_start;    // [kGwBucketCount + 1]: first entry with frac(offx) >= b / kGwBucketCount
+    const float2 *offs;         // offsets [n]
     unsigned int *gmask;        // out_w x out_h x words sample masks (zeroed before the launch)
     int in_w, in_h, out_w, out_h;
     int n, words;               // words = ceil(n/32)
+    int chunk_words, chunks;    // a work item takes the samples of one chunk of chunk_words mask words
     int tin_w, tin_h;           // input tile of one CTA
     int rmax_w, rmax_h;         // bound of the zoomed tile rectangle held in shared memory
     float rm, zoom;
@@ -108,8 +106,9 @@ struct GrainwiseArgs {
     int lognorm;
     float radius_mean;
     float log_mu, log_sigma;
-    int *work;                  // null: one CTA per tile; else the tile scheduler's area (grainwise_work_ints)
-    int parts;                  // CTAs per tile (>= 1; above 1 only for the bitmask variants)
+    int *work;                  // the tile scheduler's area (grainwise_work_ints)
+    float grain_cost;           // lane-ops of a grain in one chunk (the tile scheduler's cost model)
+    size_t request_bytes;       // size of the request, for its limit (grainwise_request_bytes)
     int *cancel;                // null, or the in-launch cancellation words (cancel_requested)
 };
 
@@ -154,11 +153,10 @@ size_t pixelwise_cellmask_bytes(const PixelwiseArgs &a, int nby);
 bool pixelwise_prefers_regen(const PixelwiseArgs &a);
 cudaError_t launch_pixelwise_regen(const PixelwiseArgs &a, cudaStream_t s);
 size_t pixelwise_smem_bytes();  // the fat configuration (the batched kernel's pixel-wise items)
-cudaError_t launch_grainwise(const GrainwiseArgs &a, cudaStream_t s);
+cudaError_t launch_grainwise(const GrainwiseArgs &a, int sms, cudaStream_t s);
 size_t grainwise_smem_bytes(const GrainwiseArgs &a);
 int grainwise_tile_count(const GrainwiseArgs &a);
-size_t grainwise_work_ints(const GrainwiseArgs &a);  // scheduler area: counter, pad, order[tiles], cost[tiles]
-int grainwise_parts(const GrainwiseArgs &a, int sms);
+size_t grainwise_work_ints(const GrainwiseArgs &a, int sms);  // the tile scheduler's area (GrainwiseArgs::work)
 cudaError_t launch_grainwise_epilogue(const GrainwiseEpilogueArgs &a, cudaStream_t s);
 cudaError_t launch_epilogue(const EpilogueArgs &a, cudaStream_t s);
 cudaError_t launch_rgb_pack(const float *p0, const float *p1, const float *p2, int n, unsigned char *out,

@@ -273,3 +273,22 @@ def test_device_tensors_in_and_out(cuda, fgl, orc):
     torch.cuda.synchronize()
     want, _ = orc.render("grain", lam, op, od, offs)
     assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [256, 257, 289, 512, 577])
+def test_grainwise_sample_chunks(cuda, fgl, orc, n):
+    """More samples than one chunk's masks hold: one chunk full, a last chunk of one sample's word, chunks of
+    unequal width, two full ones, three."""
+    _check("grain", fgl, orc, _blobs(37, 29), radius=0.07, n=n, zoom=1.5, seed=n)
+
+
+@pytest.mark.parametrize("w,h,zoom,radius,n,dist", [
+    (3, 1, 1.0, 0.05, 64, "const"),       # fewer pixels than warps: 32 lanes to a pixel
+    (61, 9, 1.0, 0.02, 33, "lognorm"),    # saturated ramp end: parts of a few pixels, groups of 2 to 16 lanes
+    (300, 40, 0.5, 0.04, 16, "lognorm"),  # one tile, lanes with a pixel each and refills
+    (33, 35, 2.0, 0.4, 200, "const"),     # a grain reaches most samples: the pair queue overflows
+])
+def test_grainwise_lane_groups_and_queue(cuda, fgl, orc, w, h, zoom, radius, n, dist):
+    plane = workloads.ramp_noise(w, h, 5)
+    _check("grain", fgl, orc, plane, radius=radius, n=n, zoom=zoom, dist=dist, sd=0.4 * radius if dist == "lognorm" else 0.0,
+           seed=41)

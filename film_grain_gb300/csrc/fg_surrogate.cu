@@ -466,8 +466,8 @@ static cudaError_t launch_conv_t(const SgConvArgs &a, int total, cudaStream_t s)
 
 // fg_sg_tc.cu: the residual conv on the tcgen05 tensor cores (TMA-staged rows, accumulator in tensor
 // memory); cudaErrorNotSupported when its preconditions fail.
-cudaError_t launch_sg_conv32_tc(const void *in, const void *w, const float *bias, void *out, void *aux, int nb, int H,
-                                int W, cudaStream_t s);
+cudaError_t launch_sg_conv32_tc(const void *in, const void *w, const float *bias, const void *res, const void *relu,
+                                void *out, void *out2, int nb, int H, int W, cudaStream_t s);
 
 static fg_status launch_conv(int32_t kind, const SgConvArgs &a, int nb, cudaStream_t s) {
     const long long blocks = (long long)nb * a.tiles_per_img;
@@ -479,7 +479,7 @@ static fg_status launch_conv(int32_t kind, const SgConvArgs &a, int nb, cudaStre
     case FG_SG_CONV_RESIDUAL:
         // the residual is the conv's own input (every residual layer of the network): tensor cores
         e = a.res == a.in && a.in_cstride == 32
-                ? launch_sg_conv32_tc(a.in, a.w, a.bias, a.out, a.aux, nb, a.H, a.W, s)
+                ? launch_sg_conv32_tc(a.in, a.w, a.bias, nullptr, nullptr, a.out, a.aux, nb, a.H, a.W, s)
                 : cudaErrorNotSupported;
         if (e == cudaErrorNotSupported) {
             cudaGetLastError();
@@ -487,7 +487,14 @@ static fg_status launch_conv(int32_t kind, const SgConvArgs &a, int nb, cudaStre
         }
         break;
     case FG_SG_CONV_OUTPUT: e = launch_conv_t<32, 8, kSgOutput>(a, total, s); break;
-    case FG_SG_CONV_DGRAD_RESIDUAL: e = launch_conv_t<32, 32, kSgLinearAdd>(a, total, s); break;
+    case FG_SG_CONV_DGRAD_RESIDUAL:
+        e = a.in_cstride == 32 ? launch_sg_conv32_tc(a.in, a.w, nullptr, a.res, nullptr, a.out, nullptr, nb, a.H, a.W, s)
+                               : cudaErrorNotSupported;
+        if (e == cudaErrorNotSupported) {
+            cudaGetLastError();
+            e = launch_conv_t<32, 32, kSgLinearAdd>(a, total, s);
+        }
+        break;
     case FG_SG_CONV_DGRAD_OUTPUT: e = launch_conv_t<16, 32, kSgLinear>(a, total, s); break;
     default: return set_error(FG_ERR_INVALID, "unknown surrogate conv kind");
     }

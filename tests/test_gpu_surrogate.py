@@ -82,6 +82,40 @@ def test_forward_matches_oracle(sg, cuda, shape):
     assert np.array_equal(y_inf.view(np.uint32), y.view(np.uint32)), "fg_sg_infer differs from the layer calls"
 
 
+def _conv_inputs(torch, nb, h, w, seed):
+    rng = np.random.default_rng(seed)
+    bf = lambda a: sr.bf16_round(a.astype(np.float32))
+    x = bf(np.maximum(rng.normal(0, 1, (nb, h, w, 32)), 0))
+    return (x, bf(rng.normal(0, 0.06, (32, 9, 32))), rng.normal(0, 0.1, 32).astype(np.float32),
+            bf(rng.normal(0, 1, (nb, h, w, 32))))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 9, 128), (3, 17, 129), (700, 3, 5), (1, 400, 130)])
+def test_tensor_core_convs_match_oracle(sg, cuda, fgl, shape):
+    """The residual conv with its ReLU output and the data gradient on the tensor cores: one pixel, one full
+    column tile, a column tile of one pixel, row ranges that span many images, ranges longer than the
+    accumulator ring.  Outputs are f32 sums rounded to bf16: within one bf16 step (2^-7) of the oracle's,
+    plus 2e-5 for 288 products of f32 rounding."""
+    torch = cuda
+    nb, h, w = shape
+    x, wt, b, res = _conv_inputs(torch, nb, h, w, 3)
+    dev = lambda a: torch.from_numpy(a).cuda().to(torch.bfloat16)
+    X, Wt, R, B = dev(x), dev(wt), dev(res), torch.from_numpy(b).cuda()
+    out, aux = torch.empty_like(X), torch.empty_like(X)
+    st = torch.cuda.current_stream().cuda_stream
+    call = lambda kind, r, o, a: fgl.lib().fg_sg_conv_forward(kind, X.data_ptr(), 32, Wt.data_ptr(), B.data_ptr(),
+                                                              r.data_ptr(), None, o.data_ptr(), a, None, nb, h, w, st)
+    close = lambda got, want: np.all(np.abs(got.float().cpu().numpy() - want) <= 2.0**-7 * np.abs(want) + 2e-5)
+    z = sr.conv(x, wt)
+    relu = np.maximum(z + b, 0)
+    assert call(sg.CONV_RESIDUAL, X, out, aux.data_ptr()) == 0
+    assert close(out, x + relu) and close(aux, relu)
+    assert call(sg.CONV_DGRAD_RESIDUAL, R, out, None) == 0
+    assert close(out, res + z)
+    assert call(sg.CONV_DGRAD_RESIDUAL, R, R, None) == 0  # in place, as the backward pass runs it
+    assert torch.equal(R, out)
+
+
 @pytest.mark.parametrize("shape", [(2, 16, 32), (2, 19, 41)])
 def test_gradients_match_oracle(sg, cuda, shape):
     """Every parameter gradient within 3e-2 relative L2 of the oracle's (bf16 activations, f32 sums)."""

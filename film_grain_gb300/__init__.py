@@ -193,6 +193,8 @@ SIGNATURES = {
                                          _P(ctypes.c_float)]),
     "fg_sg_conv_forward": (ctypes.c_int, [ctypes.c_int32, _vp, ctypes.c_int32, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                           ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, _vp]),
+    "fg_sg_conv_dgrad": (ctypes.c_int, [ctypes.c_int32, _vp, ctypes.c_int32, _vp, _vp, _vp, _vp, _vp, ctypes.c_int32,
+                                        ctypes.c_int32, ctypes.c_int32, _vp]),
     "fg_sg_conv_wgrad": (ctypes.c_int, [ctypes.c_int32, _vp, ctypes.c_int32, _vp, ctypes.c_int32, _vp, _vp,
                                         ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, _vp]),
     "fg_sg_mask_grad": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int64, _vp]),

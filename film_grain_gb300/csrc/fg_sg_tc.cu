@@ -1,9 +1,13 @@
-// fg_sg_tc.cu -- the surrogate's 32 -> 32 convs on the fifth-generation tensor cores.
+// fg_sg_tc.cu -- the surrogate's convs on the fifth-generation tensor cores.
 //
-// NHWC bf16 activations with 32 channels, weights [cout 32][tap 9][cin 32] bf16, f32 accumulation:
-//   residual       out = in + relu(conv3x3(in) + b)      (aux, for training: the ReLU output)
-//   data gradient  out = res + conv3x3(in)               (masked: out where relu > 0, else 0)
+// NHWC bf16 activations, weights [cout][tap 9][cin] bf16, f32 accumulation (channels in -> out):
+//   input          16 -> 32  out = relu(conv3x3(in) + b)
+//   residual       32 -> 32  out = in + relu(conv3x3(in) + b)      (aux, for training: the ReLU output)
+//   output         32 -> 1   f32 out = u + conv3x3(in) + b
+//   data gradient  32 -> 32  out = res + conv3x3(in)               (masked, a second output: out where the
+//                  16 -> 32  out = conv3x3(in)                      layer's ReLU output is positive, else 0)
 //
+// Taking the 32 -> 32 conv (the others differ in their channel counts):
 // An implicit GEMM over row tiles of M = 128 pixels.  An input row y contributes to the output rows y + 1, y
 // and y - 1 (taps ky = 0, 1, 2), so the three taps' weights stand side by side as one B operand of
 // N = 96 columns, ordered ky = 2, 1, 0, and the accumulators of consecutive output rows stand side by side in
@@ -24,118 +28,69 @@
 // neighbouring threads write eight bank groups) and leave by TMA, which also cuts them at the image's edge;
 // written directly, a thread's own 64 bytes would touch each 32-byte sector twice.
 //
-// Measured at 3 x 1024^2 pixels (403 MB, 60 us at the measured copy rate): 18 MMAs of N 32 per row 128 us;
-// this split, one epilogue group and rows as 16-byte TMA pieces 95 us; two groups 92 us; the MMAs issued by a
-// converged warp 78 us (call by call 139 -> 81 us).  What is left is shared-memory traffic: 8.5 MMAs a row
-// with the overwriting and wrapping ones, 7 KB each, and 33 KB of rows in and out against 128 B per clock.
+// Measured, 32 -> 32 at 3 x 1024^2 pixels (403 MB, 60 us at the measured copy rate): 18 MMAs of N 32 per row
+// 128 us; this split with one epilogue group and rows as 16-byte TMA pieces 95 us; two groups 92 us; the MMAs
+// issued by a converged warp 78 us; with constant operands inside a run 72 us (call by call 139 -> 76 us).
+// 720p, 3 planes, a layer 122 -> 62 us, the input conv 90 -> 45 us, the output conv 106 -> 50 us (both on mma.sync
+// before).  What is left: the MMA warp's own instructions (a row's 8.5 MMAs with the overwriting and wrapping
+// ones are issued in about 900 of its 1590 cycles) and shared-memory traffic.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out records the fact in g_sg_tc_timeout, writes NaN
 // outputs for the CTA's rows not yet written, waits (bounded) for its own copies and MMAs, frees its tensor
 // memory and returns.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <cudaTypedefs.h>
-#include <stdint.h>
-
 #include <algorithm>
-#include <mutex>
+#include <type_traits>
 
+#include "../../include/film_grain_gb300.h"
 #include "fg_internal.h"
+#include "fg_sg_tc.cuh"
 
 namespace fg {
 
-typedef __nv_bfloat16 bf16;
-
 constexpr int kTcPx = 128;          // output pixels of one row tile (the MMA's M)
 constexpr int kTcHalo = kTcPx + 2;  // input pixels of one row at most
-constexpr int kTcRowBytes = 17 * 512;  // 130 x 64 bytes, to the 512 bytes that the 64-byte swizzle repeats over
 constexpr int kTcSlots = 6;         // input rows in flight
-constexpr int kTcAcc = 8;           // accumulator rows (32 columns each) in tensor memory
-constexpr uint32_t kTcTmemCols = 32 * kTcAcc;
-constexpr int kTcWOff = kTcSlots * kTcRowBytes;
-constexpr int kTcWBytes = 36 * 32 * 16;
-constexpr int kTcStageOff = kTcWOff + kTcWBytes;
-constexpr int kTcStageBytes = 2048;              // a warp's 32 pixels
-constexpr int kTcThreads = 320;                  // loader, MMA issuer, two groups of four epilogue warps
+constexpr int kTcAcc = 8;           // accumulator rows in tensor memory
+constexpr int kTcStageBytes = 2048; // a warp's 32 pixels of 32 channels
+constexpr int kTcThreads = 320;     // loader, MMA issuer, two groups of four epilogue warps
 // barriers: rows full, rows free (MMA), rows free (epilogue), accumulators full, accumulators free, drain
 constexpr int kTcBars = 3 * kTcSlots + 2 * kTcAcc + 1;
-// SM cycles a wait on an mbarrier may take before it gives up (about a second)
-constexpr long long kTcWaitCycles = 2000000000ll;
-
 __device__ int g_sg_tc_timeout;
 
-enum TcMode { kTcResidual = 0, kTcResidualAux = 1, kTcDgrad = 2, kTcDgradMasked = 3 };
+enum TcMode { kTcInput, kTcResidual, kTcResidualAux, kTcOutput, kTcDgrad, kTcDgradMasked, kTcLinear, kTcLinearMasked };
 
-__host__ __device__ constexpr int tc_outputs(int mode) { return mode == kTcResidualAux || mode == kTcDgradMasked ? 2 : 1; }
-__host__ __device__ constexpr int tc_bar_off(int mode) { return kTcStageOff + 8 * tc_outputs(mode) * kTcStageBytes; }
-constexpr int tc_smem(int mode) { return tc_bar_off(mode) + 8 * kTcBars + 16 + 128; }
-
-// Instruction descriptor of tcgen05.mma kind::f16: D f32 (bits 4-5 = 1), A and B bf16 (bits 7-9 and
-// 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bit 17, M >> 4 at bit 24.
-__device__ __forceinline__ uint32_t tc_idesc(uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Shared-memory matrix descriptor, no swizzle: start address, leading (K-direction core-matrix) byte
-// offset, stride (M/N-direction core-matrix) byte offset, each >> 4; descriptor version 1 at bit 46.
-__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// Bounded wait for the completion of the phase with the given parity; false when the limit ran out or
-// another warp gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int *abort) {
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-        if (mbar_try(bar, parity)) return true;
-        if (*abort || clock64() - t0 > kTcWaitCycles) return false;
-    }
-}
-// The MMA warp runs as one: every lane holds the same operands and the leader's predicate guards the
-// instruction itself.  (Issued by one lane inside a branch, the operands went through vector registers and
-// an MMA took about 250 cycles to issue, five times its own time.)
-__device__ __forceinline__ void tc_commit(uint32_t bar, bool leader) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
-        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
-        "r"(leader ? 1u : 0u)
-        : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc, bool leader) {
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u), "r"(leader ? 1u : 0u)
-        : "memory");
-}
+// Sizes of a mode.  A row slot holds kTcHalo pixels, rounded up to what the swizzle repeats over (8 pixels).
+template <int MODE>
+struct TcCfg {
+    static constexpr bool kRelu = MODE == kTcInput || MODE == kTcResidual || MODE == kTcResidualAux;
+    static constexpr bool kRes = MODE == kTcResidual || MODE == kTcResidualAux;       // the addend is the input row
+    static constexpr bool kAdd = MODE == kTcDgrad || MODE == kTcDgradMasked;          // another tensor
+    static constexpr bool kMask = MODE == kTcDgradMasked || MODE == kTcLinearMasked;
+    static constexpr bool kTwo = MODE == kTcResidualAux || kMask;
+    static constexpr bool kF32 = MODE == kTcOutput;
+    static constexpr int kCin = MODE == kTcInput || MODE == kTcLinear || MODE == kTcLinearMasked ? 16 : 32;
+    static constexpr int kHalves = kCin / 16;        // MMAs' K steps per tap
+    static constexpr int kChunks = kCin / 8;         // 16-byte channel chunks per pixel
+    static constexpr int kPxBytes = 2 * kCin;
+    static constexpr int kRowBytes = (kTcHalo + 7) / 8 * 8 * kPxBytes;
+    static constexpr int kCols = kF32 ? 16 : 32;     // accumulator columns of an output row
+    static constexpr int kCout = kF32 ? 8 : 32;      // output channels the weights have
+    static constexpr int kWRows = MODE == kTcLinearMasked ? 8 : 32;  // output channels of a masked gradient's layer
+    static constexpr int kBlock = 3 * kCols * 16;    // weights of one (kx, chunk): rows ky = 2, 1, 0
+    static constexpr uint64_t kSwizzle = kCin == 32 ? 4ull : 6ull;  // 64- or 32-byte swizzle
+    static constexpr int kWOff = kTcSlots * kRowBytes;
+    static constexpr int kStageOff = (kWOff + 3 * kChunks * kBlock + 511) / 512 * 512;
+    static constexpr int kBarOff = kStageOff + (kF32 ? 0 : 8 * (kTwo ? 2 : 1) * kTcStageBytes);
+    static constexpr int kSmem = kBarOff + 8 * kTcBars + 16 + 128;
+    static constexpr uint32_t kTmemCols = kCols * kTcAcc;
+};
 
 struct TcArgs {
     const bf16 *w;
-    const float *bias;       // residual modes
+    const float *bias;
     const bf16 *res, *relu;  // data-gradient modes: the addend, and the mask's ReLU output
+    const float *u;          // output mode
+    float *out_f32;
     bf16 *out, *out2;        // out2: aux, or the masked gradient
     int nb, H, W, tiles_x;
     int box_px;              // pixels of an input row box (even, <= kTcHalo)
@@ -184,17 +139,17 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                                                                      const __grid_constant__ CUtensorMap tmap_out2,
                                                                      const __grid_constant__ TcArgs a) {
     extern __shared__ __align__(1024) unsigned char tc_sm[];
-    constexpr bool kRes = MODE == kTcResidual || MODE == kTcResidualAux;  // the addend is the input itself
-    constexpr bool kTwo = MODE == kTcResidualAux || MODE == kTcDgradMasked;
+    using C = TcCfg<MODE>;
+    constexpr bool kRes = C::kRes, kTwo = C::kTwo;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sbase = smem_u32(tc_sm);
-    const uint32_t bars = sbase + tc_bar_off(MODE);
+    const uint32_t bars = sbase + C::kBarOff;
     const uint32_t full = bars, free_mma = full + 8 * kTcSlots, free_epi = free_mma + 8 * kTcSlots,
                    acc_full = free_epi + 8 * kTcSlots, acc_free = acc_full + 8 * kTcAcc, drain = acc_free + 8 * kTcAcc;
-    volatile int *s_abort = reinterpret_cast<volatile int *>(tc_sm + tc_bar_off(MODE) + 8 * kTcBars);
+    volatile int *s_abort = reinterpret_cast<volatile int *>(tc_sm + C::kBarOff + 8 * kTcBars);
     const uint32_t tmem_slot = bars + 8 * kTcBars + 4;
-    float *s_bias = reinterpret_cast<float *>(tc_sm + tc_bar_off(MODE) + 8 * kTcBars + 16);
-    if (kRes && tid < 32) s_bias[tid] = a.bias[tid];
+    float *s_bias = reinterpret_cast<float *>(tc_sm + C::kBarOff + 8 * kTcBars + 16);
+    if ((C::kRelu && tid < 32) || (C::kF32 && tid == 0)) s_bias[tid] = a.bias[tid];
 
     if (tid == 0) {
         for (int i = 0; i < kTcSlots; i++) {
@@ -212,25 +167,43 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tmem_slot),
-                     "r"(kTcTmemCols)
+                     "r"(C::kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    // weights: element (co, tap = 3 ky + kx, ci) to block (kx, ci / 8), row 32 (2 - ky) + co
-    for (int e = tid; e < 32 * 36; e += kTcThreads) {
-        const int co = e / 36, kc = e - co * 36, tap = kc >> 2, c = kc & 3, ky = tap / 3, kx = tap - 3 * ky;
-        const uint4 v = *reinterpret_cast<const uint4 *>(a.w + co * 288 + kc * 8);
-        *reinterpret_cast<uint4 *>(tc_sm + kTcWOff + ((kx * 4 + c) * 96 + 32 * (2 - ky) + co) * 16) = v;
+    // weights: element (co, tap = 3 ky + kx, ci) to block (kx, ci / 8), row kCols (2 - ky) + co
+    for (int e = tid; e < C::kCols * 9 * C::kChunks; e += kTcThreads) {
+        const int co = e / (9 * C::kChunks), kc = e - co * (9 * C::kChunks), tap = kc / C::kChunks,
+                  c = kc - tap * C::kChunks, ky = tap / 3, kx = tap - 3 * ky;
+        if (C::kMask) break;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (co < C::kCout) v = *reinterpret_cast<const uint4 *>(a.w + (co * 9 + tap) * C::kCin + 8 * c);
+        *reinterpret_cast<uint4 *>(tc_sm + C::kWOff + (kx * C::kChunks + c) * C::kBlock +
+                                   (C::kCols * (2 - ky) + co) * 16) = v;
+    }
+    // the masked data gradients take the layer's own weights [cout kWRows][9][32]: turned around (tap 8 - tap)
+    // and transposed here, 32 lanes reading one row's 32 input channels
+    if (C::kMask) {
+        for (int e = tid; e < 32 * 9 * C::kChunks; e += kTcThreads) {
+            const int n = e & 31, tc = e >> 5, tap = tc / C::kChunks, c = tc - tap * C::kChunks, ky = tap / 3,
+                      kx = tap - 3 * ky;
+            uint4 v;
+            bf16 *b = reinterpret_cast<bf16 *>(&v);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                b[j] = 8 * c + j < C::kWRows ? a.w[((8 * c + j) * 9 + 8 - tap) * 32 + n] : __float2bfloat16(0.0f);
+            *reinterpret_cast<uint4 *>(tc_sm + C::kWOff + (kx * C::kChunks + c) * C::kBlock + (32 * (2 - ky) + n) * 16) = v;
+        }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the weights, for the tensor cores
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tc_sm + tc_bar_off(MODE) + 8 * kTcBars + 4);
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tc_sm + C::kBarOff + 8 * kTcBars + 4);
 
     const long long total = (long long)a.nb * a.tiles_x * a.H;
     const long long t0 = total * blockIdx.x / gridDim.x, t1 = total * (blockIdx.x + 1) / gridDim.x;
-    const uint32_t row_bytes = (uint32_t)a.box_px * 64;
+    const uint32_t row_bytes = (uint32_t)a.box_px * C::kPxBytes;
     // Input rows are numbered q = 0, 1, ... over the CTA's runs (a run of R output rows has R + 2), output
     // rows n; row q is in slot q % kTcSlots, row n in accumulator n % kTcAcc.
     long long t = t0;
@@ -256,7 +229,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     mbar_expect_tx(full + 8 * s, row_bytes);
                     asm volatile(
                         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
-                        "%3, %4, %5}], [%6];\n" ::"r"(sbase + (uint32_t)(s * kTcRowBytes)),
+                        "%3, %4, %5}], [%6];\n" ::"r"(sbase + (uint32_t)(s * C::kRowBytes)),
                         "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(r.x0 - 1), "r"(r.y0 - 1 + i), "r"(r.img),
                         "r"(full + 8 * s)
                         : "memory");
@@ -266,9 +239,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
         }
         __syncwarp();
     } else if (warp == 1) {
-        const bool leader = lane == 0;
-        const uint64_t a0 = tc_desc(sbase, 16, 512) | (4ull << 61);  // 64-byte swizzle, rows of 64 bytes
-        const uint64_t b0 = tc_desc(sbase + kTcWOff, 1536, 128);
+        const uint64_t a0 = tc_desc(sbase, 16, 8 * C::kPxBytes) | (C::kSwizzle << 61);
+        const uint64_t b0 = tc_desc(sbase + C::kWOff, C::kBlock, 128);
         int q = 0, n0 = 0;  // n0: output rows of the runs before
         bool ok = true;
         while (ok && tc_run(a, t, t1, r)) {
@@ -288,42 +260,72 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint64_t ad = a0 + (uint64_t)(s * (kTcRowBytes >> 4));
-                // rows [o, o + cnt) of the window: accumulator columns from 32 ((n0 + o) % kTcAcc), weight
-                // rows from 32 (2 - ky)
+                const uint64_t ad = a0 + (uint64_t)(s * (C::kRowBytes >> 4));
+                // rows [o, o + cnt) of the window: accumulator columns from kCols ((n0 + o) % kTcAcc), weight
+                // rows from kCols (2 - ky)
                 const int w0 = (n0 + o0) % kTcAcc, cnt = o1 - o0 + 1, head = min(cnt, kTcAcc - w0);
-                const uint64_t bd0 = b0 + (uint64_t)(32 * (2 - (i - o0)));
-                const uint32_t d0 = tmem + 32u * (uint32_t)w0;
+                const uint64_t bd0 = b0 + (uint64_t)(C::kCols * (2 - (i - o0)));
+                const uint32_t d0 = tmem + C::kCols * (uint32_t)w0;
+                // Inside a run the window is three rows, the last one fresh: everything but the row slot and
+                // the accumulator column is a constant of the loop, for each place of the wrap.
+                auto inner = [&](auto head_c) {
+                    constexpr int kHead = decltype(head_c)::value;  // rows before the wrap
 #pragma unroll
-                for (int kx = 0; kx < 3; kx++)
+                    for (int kx = 0; kx < 3; kx++)
 #pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        const uint64_t av = ad + (uint64_t)(4 * kx + 2 * j);
-                        const uint64_t bv = bd0 + (uint64_t)((kx * 4 + 2 * j) * 96);
-                        if (kx == 0 && j == 0 && fresh) {
-                            const int old = cnt - 1, h = min(old, head);
-                            if (h > 0) tc_mma(d0, av, bv, tc_idesc(32u * h), true, leader);
-                            if (old > h) tc_mma(tmem, av, bv + 32u * h, tc_idesc(32u * (old - h)), true, leader);
-                            tc_mma(tmem + 32u * (uint32_t)((n0 + o1) % kTcAcc), av, bv + 32u * old, tc_idesc(32u), false,
-                                   leader);
-                        } else {
-                            tc_mma(d0, av, bv, tc_idesc(32u * head), true, leader);
-                            if (cnt > head) tc_mma(tmem, av, bv + 32u * head, tc_idesc(32u * (cnt - head)), true, leader);
+                        for (int j = 0; j < C::kHalves; j++) {
+                            const uint64_t av = ad + (uint64_t)((kx * C::kPxBytes + 32 * j) >> 4);
+                            const uint64_t bv = b0 + (uint64_t)((kx * C::kChunks + 2 * j) * (C::kBlock >> 4));
+                            if (kx == 0 && j == 0) {
+                                constexpr int kOld = kHead < 2 ? kHead : 2;
+                                tc_mma(d0, av, bv, tc_idesc(C::kCols * kOld), true);
+                                if (kOld < 2) tc_mma(tmem, av, bv + C::kCols, tc_idesc(C::kCols), true);
+                                tc_mma(kHead == 3 ? d0 + 2 * C::kCols : tmem + (2 - kHead) * C::kCols, av,
+                                       bv + 2 * C::kCols, tc_idesc(C::kCols), false);
+                            } else {
+                                tc_mma(d0, av, bv, tc_idesc(C::kCols * kHead), true);
+                                if (kHead < 3)
+                                    tc_mma(tmem, av, bv + C::kCols * kHead, tc_idesc(C::kCols * (3 - kHead)), true);
+                            }
                         }
-                    }
-                tc_commit(free_mma + 8 * s, leader);
-                if (i >= 2) tc_commit(acc_full + 8 * ((n0 + i - 2) % kTcAcc), leader);
+                };
+                if (fresh && cnt == 3 && head >= 3) inner(std::integral_constant<int, 3>());
+                else if (fresh && cnt == 3 && head == 2) inner(std::integral_constant<int, 2>());
+                else if (fresh && cnt == 3) inner(std::integral_constant<int, 1>());
+                else {
+#pragma unroll
+                    for (int kx = 0; kx < 3; kx++)
+#pragma unroll
+                        for (int j = 0; j < C::kHalves; j++) {
+                            const uint64_t av = ad + (uint64_t)((kx * C::kPxBytes + 32 * j) >> 4);
+                            const uint64_t bv = bd0 + (uint64_t)((kx * C::kChunks + 2 * j) * (C::kBlock >> 4));
+                            if (kx == 0 && j == 0 && fresh) {
+                                const int old = cnt - 1, h = min(old, head);
+                                if (h > 0) tc_mma(d0, av, bv, tc_idesc(C::kCols * h), true);
+                                if (old > h)
+                                    tc_mma(tmem, av, bv + C::kCols * h, tc_idesc(C::kCols * (old - h)), true);
+                                tc_mma(tmem + C::kCols * (uint32_t)((n0 + o1) % kTcAcc), av, bv + C::kCols * old,
+                                       tc_idesc(C::kCols), false);
+                            } else {
+                                tc_mma(d0, av, bv, tc_idesc(C::kCols * head), true);
+                                if (cnt > head)
+                                    tc_mma(tmem, av, bv + C::kCols * head, tc_idesc(C::kCols * (cnt - head)), true);
+                            }
+                        }
+                }
+                tc_commit(free_mma + 8 * s);
+                if (i >= 2) tc_commit(acc_full + 8 * ((n0 + i - 2) % kTcAcc));
             }
             n0 += r.rows;
         }
-        tc_commit(drain, leader);
+        tc_commit(drain);
         __syncwarp();
     } else {
         // two groups of four warps take the output rows in turn: one row's way through the epilogue is
         // about 2000 cycles of latency, and a group alone left every unit of the SM below 50 % busy
         const int quad = warp & 3;  // the tensor-memory lanes this warp may read
         const int group = (warp - 2) >> 2;
-        unsigned char *stage = tc_sm + kTcStageOff + (warp - 2) * (tc_outputs(MODE) * kTcStageBytes);
+        unsigned char *stage = tc_sm + C::kStageOff + (warp - 2) * ((kTwo ? 2 : 1) * kTcStageBytes);
         const int m = quad * 32 + lane;
         int q = 0, n = 0;
         bool ok = true;
@@ -342,12 +344,14 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                 const int x = r.x0 + m, y = r.y0 + o, acc = n % kTcAcc;
                 const size_t p = ((size_t)r.img * a.H + y) * a.W + x;
                 uint4 rv[4], mv[4];
-                if (!kRes && x < a.W) {
+                float uv = 0.0f;
+                if (x < a.W) {
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
-                        rv[c] = *reinterpret_cast<const uint4 *>(a.res + p * 32 + 8 * c);
-                        if (kTwo) mv[c] = __ldg(reinterpret_cast<const uint4 *>(a.relu + p * 32 + 8 * c));
+                        if (C::kAdd) rv[c] = *reinterpret_cast<const uint4 *>(a.res + p * 32 + 8 * c);
+                        if (C::kMask) mv[c] = __ldg(reinterpret_cast<const uint4 *>(a.relu + p * 32 + 8 * c));
                     }
+                    if (C::kF32) uv = a.u[p];
                 }
                 ok = ok && mbar_wait(acc_full + 8 * acc, (uint32_t)((n / kTcAcc) & 1), s_abort);
                 const int qi = q + o + 1, s = qi % kTcSlots;  // the input row at the output's place
@@ -357,16 +361,27 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     *s_abort = 1;
                     if (x < a.W) {  // a failed launch cannot pass for a result
                         const uint4 nan4 = make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
+                        if (C::kF32) a.out_f32[p] = __int_as_float(0x7fc00000);
 #pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            *reinterpret_cast<uint4 *>(a.out + p * 32 + 8 * c) = nan4;
+                        for (int c = 0; c < (C::kF32 ? 0 : 4); c++) {
+                            if (a.out) *reinterpret_cast<uint4 *>(a.out + p * 32 + 8 * c) = nan4;
                             if (kTwo) *reinterpret_cast<uint4 *>(a.out2 + p * 32 + 8 * c) = nan4;
                         }
                     }
                     continue;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t tcol = tmem + C::kCols * (uint32_t)acc + ((uint32_t)(quad * 32) << 16);
                 uint32_t v[32];
+                if (C::kF32) {
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(v[0]) : "r"(tcol));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_free + 8 * acc);
+                    if (x < a.W) a.out_f32[p] = uv + __uint_as_float(v[0]) + s_bias[0];
+                    continue;
+                }
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
                     "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
@@ -376,10 +391,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                       "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
                       "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
                       "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(tmem + 32u * (uint32_t)acc + ((uint32_t)(quad * 32) << 16)));
+                    : "r"(tcol));
                 if (kRes) {
                     // chunk c of pixel i lies at chunk c ^ (i / 2 % 4) of its 64 bytes (the swizzle)
-                    const unsigned char *rp = tc_sm + s * kTcRowBytes + (m + 1) * 64;
+                    const unsigned char *rp = tc_sm + s * C::kRowBytes + (m + 1) * 64;
 #pragma unroll
                     for (int c = 0; c < 4; c++)
                         rv[c] = *reinterpret_cast<const uint4 *>(rp + ((c ^ (((m + 1) >> 1) & 3)) << 4));
@@ -389,10 +404,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                 // the stage's previous row has been read
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(acc_free + 8 * acc);
-                    if (kRes) mbar_arrive(free_epi + 8 * s);
-                }
+                if (lane == 0) mbar_arrive(acc_free + 8 * acc);
                 uint4 ov[4], av[4];
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
@@ -404,26 +416,31 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     for (int k = 0; k < 4; k++) {
                         const int ch = 8 * c + 2 * k;
                         float2 z = make_float2(__uint_as_float(v[ch]), __uint_as_float(v[ch + 1]));
-                        if (kRes) {
+                        if (C::kRelu) {
                             z = add2(z, *reinterpret_cast<const float2 *>(&s_bias[ch]));
                             z = make_float2(fmaxf(z.x, 0.0f), fmaxf(z.y, 0.0f));
                         }
                         if (MODE == kTcResidualAux) a2[k] = __float22bfloat162_rn(z);
-                        o2[k] = __float22bfloat162_rn(add2(z, __bfloat1622float2(r2[k])));
-                        if (MODE == kTcDgradMasked) {
+                        if (kRes || C::kAdd) z = add2(z, __bfloat1622float2(r2[k]));
+                        o2[k] = __float22bfloat162_rn(z);
+                        if (C::kMask) {
                             const float2 mf = __bfloat1622float2(m2[k]);
                             a2[k].x = mf.x > 0.0f ? o2[k].x : __float2bfloat16(0.0f);
                             a2[k].y = mf.y > 0.0f ? o2[k].y : __float2bfloat16(0.0f);
                         }
                     }
                 }
-                tc_stage(stage, lane, ov);
+                if (!C::kMask || a.out) tc_stage(stage, lane, ov);
                 if (kTwo) tc_stage(stage + kTcStageBytes, lane, av);
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
+                    // Only now: the staged values prove that the warp's reads of the row slot have returned.  An
+                    // arrival right behind the loads can pass them, and a halo row outside the image (filled
+                    // with zeros at once) then overwrites what they are about to read.
+                    if (kRes) mbar_arrive(free_epi + 8 * s);
                     if (x < a.W) {  // the box is cut at the image's edge
-                        tma_store(&tmap_out, stage, x, y, r.img);
+                        if (!C::kMask || a.out) tma_store(&tmap_out, stage, x, y, r.img);
                         if (kTwo) tma_store(&tmap_out2, stage + kTcStageBytes, x, y, r.img);
                     }
                     asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
@@ -454,78 +471,77 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTcTmemCols)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(C::kTmemCols)
                      : "memory");
     }
 }
 
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static std::once_flag once;
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        else
-            cudaGetLastError();
-    });
-    return fn;
-}
-
 template <int MODE>
-static cudaError_t launch_tc(const CUtensorMap (&tm)[3], const TcArgs &a, cudaStream_t s) {
+static cudaError_t launch_tc(const void *in, int in_cstride, TcArgs a, cudaStream_t s) {
+    using C = TcCfg<MODE>;
+    PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (!encode) return cudaErrorNotSupported;
+    CUtensorMap tm[3];  // input rows, and 32-pixel boxes of the outputs
+    const void *base[3] = {in, C::kF32 ? in : (a.out ? a.out : a.out2), C::kTwo ? a.out2 : (C::kF32 ? in : a.out)};
+    for (int k = 0; k < 3; k++) {
+        const cuuint64_t ch = k == 0 || C::kF32 ? C::kCin : 32, px = k == 0 || C::kF32 ? 2 * (cuuint64_t)in_cstride : 64;
+        const cuuint64_t dims[4] = {ch, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.nb};
+        const cuuint64_t strides[3] = {px, (cuuint64_t)a.W * px, (cuuint64_t)a.H * a.W * px};
+        const cuuint32_t box[4] = {(cuuint32_t)ch, k == 0 ? (cuuint32_t)a.box_px : 32u, 1, 1};
+        const cuuint32_t estr[4] = {1, 1, 1, 1};
+        if (encode(&tm[k], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base[k]), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorNotSupported;
+    }
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(sg_conv32_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem(MODE));
+        e = cudaFuncSetAttribute(sg_conv32_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
     if (e != cudaSuccess) return e;
     const long long rows = (long long)a.nb * a.tiles_x * a.H;
     const long long grid = std::min<long long>(rows, 2ll * std::max(1, sms));
-    sg_conv32_tc_kernel<MODE><<<(unsigned)grid, kTcThreads, tc_smem(MODE), s>>>(tm[0], tm[1], tm[2], a);
+    sg_conv32_tc_kernel<MODE><<<(unsigned)grid, kTcThreads, C::kSmem, s>>>(tm[0], tm[1], tm[2], a);
     return cudaGetLastError();
 }
 
-// The 32 -> 32 convs on the tensor cores.  res == null: out = in + relu(conv(in) + bias), out2 (may be null)
-// = the ReLU output.  Else out = res + conv(in), out2 (may be null) = out where relu > 0; res may be out.
-// 32 channels per pixel, out and out2 distinct from in.  Returns cudaErrorNotSupported when the buffers are
-// not 16-byte aligned or the tensor map cannot be made (the caller's mma.sync kernel runs instead).
-cudaError_t launch_sg_conv32_tc(const void *in, const void *w, const float *bias, const void *res, const void *relu,
-                                void *out, void *out2, int nb, int H, int W, cudaStream_t s) {
+// A surrogate conv on the tensor cores, by the C-ABI's kinds.  For the residual kind res is the input itself; res
+// may be out in the data gradient; out2 (may be null) is the ReLU output (residual) or the gradient masked by
+// `relu` (then w are the layer's own weights, else already turned around, and out may be null).  Returns cudaErrorNotSupported when the buffers overlap otherwise or are not 16-byte aligned, or
+// the tensor maps cannot be made (the caller's mma.sync kernels run instead).
+cudaError_t launch_sg_conv_tc(int kind, const void *in, int in_cstride, const void *w, const float *bias, const void *res,
+                              const float *u, const void *relu, void *out, void *out2, float *out_f32, int nb, int H,
+                              int W, cudaStream_t s) {
     if (nb <= 0 || H <= 0 || W <= 0) return cudaSuccess;
     const void *ptrs[] = {in, w, res, relu, out, out2};
     for (const void *p : ptrs)
         if (reinterpret_cast<uintptr_t>(p) & 15u) return cudaErrorNotSupported;
-    if (in == out || in == out2 || (out2 && (out2 == out || out2 == res))) return cudaErrorNotSupported;
-    PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-    if (!encode) return cudaErrorNotSupported;
+    if (in == out || (out2 && (in == out2 || out2 == out || out2 == res))) return cudaErrorNotSupported;
+    if (kind == FG_SG_CONV_RESIDUAL && (res != in || in_cstride != 32)) return cudaErrorNotSupported;
     TcArgs a;
     a.w = static_cast<const bf16 *>(w);
     a.bias = bias;
     a.res = static_cast<const bf16 *>(res);
     a.relu = static_cast<const bf16 *>(relu);
+    a.u = u;
+    a.out_f32 = out_f32;
     a.out = static_cast<bf16 *>(out);
     a.out2 = static_cast<bf16 *>(out2);
     a.nb = nb; a.H = H; a.W = W;
     a.tiles_x = (W + kTcPx - 1) / kTcPx;
-    a.box_px = std::min(kTcHalo, (W + 3) & ~1);  // W + 2 halo pixels, rounded up to even (128-byte rows)
-    CUtensorMap tm[3];  // input rows, and 32-pixel boxes of the outputs
-    const void *base[3] = {in, out, out2 ? out2 : out};
-    for (int k = 0; k < 3; k++) {
-        const cuuint64_t dims[4] = {32, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)nb};
-        const cuuint64_t strides[3] = {64, (cuuint64_t)W * 64, (cuuint64_t)H * W * 64};
-        const cuuint32_t box[4] = {32, k == 0 ? (cuuint32_t)a.box_px : 32u, 1, 1};
-        const cuuint32_t estr[4] = {1, 1, 1, 1};
-        if (encode(&tm[k], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base[k]), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorNotSupported;
+    a.box_px = std::min(kTcHalo, (W + 9) & ~7);  // W + 2 halo pixels, in whole swizzle periods
+    switch (kind) {
+    case FG_SG_CONV_INPUT: return launch_tc<kTcInput>(in, in_cstride, a, s);
+    case FG_SG_CONV_RESIDUAL:
+        return out2 ? launch_tc<kTcResidualAux>(in, in_cstride, a, s) : launch_tc<kTcResidual>(in, in_cstride, a, s);
+    case FG_SG_CONV_OUTPUT: return launch_tc<kTcOutput>(in, in_cstride, a, s);
+    case FG_SG_CONV_DGRAD_RESIDUAL:
+        return out2 ? launch_tc<kTcDgradMasked>(in, in_cstride, a, s) : launch_tc<kTcDgrad>(in, in_cstride, a, s);
+    case FG_SG_CONV_DGRAD_OUTPUT:
+        return out2 ? launch_tc<kTcLinearMasked>(in, in_cstride, a, s) : launch_tc<kTcLinear>(in, in_cstride, a, s);
+    default: return cudaErrorNotSupported;
     }
-    if (!res) return out2 ? launch_tc<kTcResidualAux>(tm, a, s) : launch_tc<kTcResidual>(tm, a, s);
-    return out2 ? launch_tc<kTcDgradMasked>(tm, a, s) : launch_tc<kTcDgrad>(tm, a, s);
 }
 
 // Whether a tensor-core conv ran out of an mbarrier wait since the last call (and clears the flag).

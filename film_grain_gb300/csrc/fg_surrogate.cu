@@ -464,39 +464,35 @@ static cudaError_t launch_conv_t(const SgConvArgs &a, int total, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// fg_sg_tc.cu: the residual conv on the tcgen05 tensor cores (TMA-staged rows, accumulator in tensor
-// memory); cudaErrorNotSupported when its preconditions fail.
-cudaError_t launch_sg_conv32_tc(const void *in, const void *w, const float *bias, const void *res, const void *relu,
-                                void *out, void *out2, int nb, int H, int W, cudaStream_t s);
+// fg_sg_tc.cu: the convs on the tcgen05 tensor cores (TMA-staged rows, accumulators in tensor memory);
+// cudaErrorNotSupported when the preconditions fail.
+cudaError_t launch_sg_conv_tc(int kind, const void *in, int in_cstride, const void *w, const float *bias, const void *res,
+                              const float *u, const void *relu, void *out, void *out2, float *out_f32, int nb, int H,
+                              int W, cudaStream_t s);
+
+// fg_sg_wgrad.cu: the weight gradients on the tensor cores (cudaErrorNotSupported as above).
+cudaError_t launch_sg_wgrad_tc(int kind, const void *g, int g_cstride, const void *x, int x_cstride, float *dw, float *db,
+                               int nb, int H, int W, cudaStream_t s);
 
 static fg_status launch_conv(int32_t kind, const SgConvArgs &a, int nb, cudaStream_t s) {
     const long long blocks = (long long)nb * a.tiles_per_img;
     if (blocks > 0x7FFFFFFFll) return set_error(FG_ERR_UNSUPPORTED, "surrogate batch too large");
     const int total = (int)blocks;
-    cudaError_t e;
-    switch (kind) {
-    case FG_SG_CONV_INPUT: e = launch_conv_t<16, 32, kSgRelu>(a, total, s); break;
-    case FG_SG_CONV_RESIDUAL:
-        // the residual is the conv's own input (every residual layer of the network): tensor cores
-        e = a.res == a.in && a.in_cstride == 32
-                ? launch_sg_conv32_tc(a.in, a.w, a.bias, nullptr, nullptr, a.out, a.aux, nb, a.H, a.W, s)
-                : cudaErrorNotSupported;
-        if (e == cudaErrorNotSupported) {
-            cudaGetLastError();
-            e = launch_conv_t<32, 32, kSgResidual>(a, total, s);
+    if (kind < FG_SG_CONV_INPUT || kind > FG_SG_CONV_DGRAD_OUTPUT)
+        return set_error(FG_ERR_INVALID, "unknown surrogate conv kind");
+    void *aux = kind == FG_SG_CONV_RESIDUAL ? a.aux : nullptr;
+    const void *res = kind == FG_SG_CONV_RESIDUAL || kind == FG_SG_CONV_DGRAD_RESIDUAL ? a.res : nullptr;
+    cudaError_t e = launch_sg_conv_tc(kind, a.in, a.in_cstride, a.w, a.bias, res, a.res_f32, nullptr, a.out, aux, a.out_f32,
+                                      nb, a.H, a.W, s);
+    if (e == cudaErrorNotSupported) {  // e.g. an input that is its own output's buffer, or a residual of another tensor
+        cudaGetLastError();
+        switch (kind) {
+        case FG_SG_CONV_INPUT: e = launch_conv_t<16, 32, kSgRelu>(a, total, s); break;
+        case FG_SG_CONV_RESIDUAL: e = launch_conv_t<32, 32, kSgResidual>(a, total, s); break;
+        case FG_SG_CONV_OUTPUT: e = launch_conv_t<32, 8, kSgOutput>(a, total, s); break;
+        case FG_SG_CONV_DGRAD_RESIDUAL: e = launch_conv_t<32, 32, kSgLinearAdd>(a, total, s); break;
+        default: e = launch_conv_t<16, 32, kSgLinear>(a, total, s); break;
         }
-        break;
-    case FG_SG_CONV_OUTPUT: e = launch_conv_t<32, 8, kSgOutput>(a, total, s); break;
-    case FG_SG_CONV_DGRAD_RESIDUAL:
-        e = a.in_cstride == 32 ? launch_sg_conv32_tc(a.in, a.w, nullptr, a.res, nullptr, a.out, nullptr, nb, a.H, a.W, s)
-                               : cudaErrorNotSupported;
-        if (e == cudaErrorNotSupported) {
-            cudaGetLastError();
-            e = launch_conv_t<32, 32, kSgLinearAdd>(a, total, s);
-        }
-        break;
-    case FG_SG_CONV_DGRAD_OUTPUT: e = launch_conv_t<16, 32, kSgLinear>(a, total, s); break;
-    default: return set_error(FG_ERR_INVALID, "unknown surrogate conv kind");
     }
     return e == cudaSuccess ? FG_OK : cuda_error(e, "surrogate conv launch");
 }
@@ -528,6 +524,24 @@ FG_API fg_status fg_sg_conv_forward(int32_t kind, const void *in, int32_t in_cst
     return launch_conv(kind, a, nb, (cudaStream_t)stream);
 }
 
+FG_API fg_status fg_sg_conv_dgrad(int32_t kind, const void *g, int32_t g_cstride, const void *w, const void *res,
+                                  const void *relu, void *out, void *masked, int32_t nb, int32_t height, int32_t width,
+                                  void *stream) {
+    if (nb <= 0 || height <= 0 || width <= 0) return set_error(FG_ERR_INVALID, "empty surrogate batch");
+    if (kind != FG_SG_CONV_DGRAD_RESIDUAL && kind != FG_SG_CONV_DGRAD_OUTPUT)
+        return set_error(FG_ERR_INVALID, "surrogate dgrad: unknown conv kind");
+    const bool add = kind == FG_SG_CONV_DGRAD_RESIDUAL;
+    if (!g || !w || !relu || !masked || (add && !res) || (g_cstride % 8) != 0 || g_cstride < (add ? 32 : 16))
+        return set_error(FG_ERR_INVALID, "surrogate dgrad: missing buffer or channel stride");
+    const cudaError_t e = launch_sg_conv_tc(kind, g, g_cstride, w, nullptr, add ? res : nullptr, nullptr, relu, out, masked,
+                                            nullptr, nb, height, width, (cudaStream_t)stream);
+    if (e == cudaErrorNotSupported) {
+        cudaGetLastError();
+        return set_error(FG_ERR_INVALID, "surrogate dgrad: buffers must be 16-byte aligned and distinct");
+    }
+    return e == cudaSuccess ? FG_OK : cuda_error(e, "surrogate dgrad launch");
+}
+
 FG_API fg_status fg_sg_conv_wgrad(int32_t kind, const void *gout, int32_t g_cstride, const void *x, int32_t x_cstride,
                                   float *dw, float *db, int32_t nb, int32_t height, int32_t width, void *stream) {
     if (nb <= 0 || height <= 0 || width <= 0 || !gout || !x || !dw || !db)
@@ -543,6 +557,13 @@ FG_API fg_status fg_sg_conv_wgrad(int32_t kind, const void *gout, int32_t g_cstr
     cudaStream_t s = (cudaStream_t)stream;
     auto G = static_cast<const bf16 *>(gout);
     auto X = static_cast<const bf16 *>(x);
+    const int need_g = kind == FG_SG_CONV_OUTPUT ? 8 : 32, need_x = kind == FG_SG_CONV_INPUT ? 16 : 32;
+    if (kind >= FG_SG_CONV_INPUT && kind <= FG_SG_CONV_OUTPUT && g_cstride >= need_g && x_cstride >= need_x) {
+        e = launch_sg_wgrad_tc(kind, gout, g_cstride, x, x_cstride, dw, db, nb, height, width, s);
+        if (e == cudaSuccess) return FG_OK;
+        if (e != cudaErrorNotSupported) return cuda_error(e, "surrogate wgrad launch");
+        cudaGetLastError();  // misaligned buffers or channel strides: the mma.sync kernel below
+    }
     switch (kind) {
     case FG_SG_CONV_INPUT:
         if (g_cstride < 32 || x_cstride < 16) return set_error(FG_ERR_INVALID, "surrogate wgrad: channel stride");

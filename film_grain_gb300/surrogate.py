@@ -83,8 +83,6 @@ class SurrogateNet:
         self.ema = self.w32.clone()  # exponential moving average of the weights (what inference ships)
         self.decay = torch.zeros_like(self.w32)  # decoupled weight decay per parameter (none)
         self._ws: Dict[Tuple[int, int, int], dict] = {}
-        self._wt_res = torch.zeros(CH * 9 * CH, dtype=torch.bfloat16, device=self.device)
-        self._wt_out = torch.zeros(CH * 9 * CH_IN, dtype=torch.bfloat16, device=self.device)
 
     # ------------------------------------------------------------------ views
     def _np_view(self, flat: np.ndarray, name: str) -> np.ndarray:
@@ -162,6 +160,7 @@ class SurrogateNet:
                           dy=torch.empty((nb, h, w, CH_IN), dtype=bf, device=dev),
                           dh=torch.empty((nb, h, w, CH), dtype=bf, device=dev),
                           dz=torch.empty((nb, h, w, CH), dtype=bf, device=dev),
+                          dz2=torch.empty((nb, h, w, CH), dtype=bf, device=dev),
                           loss=torch.zeros(1, dtype=torch.float32, device=dev))
             same_mode = [k for k in self._ws if k[3] == train]
             if len(same_mode) >= 2:  # two shapes per mode stay resident (grain training uses two)
@@ -225,17 +224,21 @@ class SurrogateNet:
         hs, rs = ws["hs"], ws["rs"]
         _raise(L.fg_sg_conv_wgrad(CONV_OUTPUT, ws["dy"].data_ptr(), CH_IN, hs[self.n_res].data_ptr(), CH,
                                   self._ptr(g, "w_out"), self._ptr(g, "b_out"), nb, h, w, s))
-        _raise(L.fg_sg_flip_weights(self._ptr(self.wbf, "w_out"), self._wt_out.data_ptr(), CH_OUT, CH, CH_IN, CH, s))
-        dh, dz = ws["dh"], ws["dz"]
-        self._conv(CONV_DGRAD_OUTPUT, ws["dy"], CH_IN, self._wt_out.data_ptr(), None, None, None, dh, None, None,
-                   nb, h, w)
+        dh, dz, dz2 = ws["dh"], ws["dz"], ws["dz2"]
+
+        def dgrad(kind, g_out, w_ptr, layer, dst, masked):
+            """The gradient before the conv of `layer` (n_res: the output conv) into dst and, through the ReLU of
+            the layer before it, into masked."""
+            relu = rs[layer - 1] if layer > 0 else hs[0]
+            _raise(L.fg_sg_conv_dgrad(kind, g_out.data_ptr(), g_out.shape[-1], w_ptr, dh.data_ptr(), relu.data_ptr(),
+                                      None if dst is None else dst.data_ptr(), masked.data_ptr(), nb, h, w, s))
+
+        dgrad(CONV_DGRAD_OUTPUT, ws["dy"], self._ptr(self.wbf, "w_out"), self.n_res, dh, dz)
         for l in range(self.n_res - 1, -1, -1):
-            _raise(L.fg_sg_mask_grad(dh.data_ptr(), rs[l].data_ptr(), dz.data_ptr(), dz.numel(), s))
             _raise(L.fg_sg_conv_wgrad(CONV_RESIDUAL, dz.data_ptr(), CH, hs[l].data_ptr(), CH,
                                       self._ptr(g, "w_res", l), self._ptr(g, "b_res", l), nb, h, w, s))
-            _raise(L.fg_sg_flip_weights(self._ptr(self.wbf, "w_res", l), self._wt_res.data_ptr(), CH, CH, CH, CH, s))
-            self._conv(CONV_DGRAD_RESIDUAL, dz, CH, self._wt_res.data_ptr(), None, dh, None, dh, None, None, nb, h, w)
-        _raise(L.fg_sg_mask_grad(dh.data_ptr(), hs[0].data_ptr(), dz.data_ptr(), dz.numel(), s))
+            dgrad(CONV_DGRAD_RESIDUAL, dz, self._ptr(self.wbf, "w_res", l), l, dh if l > 0 else None, dz2)
+            dz, dz2 = dz2, dz
         _raise(L.fg_sg_conv_wgrad(CONV_INPUT, dz.data_ptr(), CH, ws["x"].data_ptr(), CH_IN, self._ptr(g, "w_in"),
                                   self._ptr(g, "b_in"), nb, h, w, s))
 

@@ -287,6 +287,14 @@ typedef struct fg_sg_net {
 FG_API fg_status fg_sg_conv_forward(int32_t kind, const void *in, int32_t in_cstride, const void *w, const float *bias,
                                     const void *res, const float *res_f32, void *out, void *aux, float *out_f32,
                                     int32_t nb, int32_t height, int32_t width, void *stream);
+/* The data gradient of a layer and, through the ReLU before it, of the layer's predecessor, in one pass.
+ * kind DGRAD_RESIDUAL: g has 32 channels, w are the residual layer's own weights [32][9][32],
+ * out = res + conv_t(g); DGRAD_OUTPUT: g has 16 (8 used), w are the output conv's [8][9][32], out = conv_t(g)
+ * (res unused).  masked = relu > 0 ? out : 0, relu the predecessor's ReLU output.  bf16, 32 channels; res may be
+ * out, out may be NULL, masked is distinct from every input; all buffers 16-byte aligned. */
+FG_API fg_status fg_sg_conv_dgrad(int32_t kind, const void *g, int32_t g_cstride, const void *w, const void *res,
+                                  const void *relu, void *out, void *masked, int32_t nb, int32_t height, int32_t width,
+                                  void *stream);
 /* Adds the weight and bias gradients of a forward conv of `kind` (INPUT, RESIDUAL or OUTPUT) into the
  * f32 buffers dw [cout][9][cin] and db [cout]: gout is the gradient at the conv output (before the
  * bias, channel stride g_cstride), x the conv input (channel stride x_cstride). */

@@ -186,6 +186,9 @@ extern "C" {
     pub fn fg_sg_conv_forward(kind: i32, input: *const c_void, in_cstride: i32, w: *const c_void, bias: *const f32,
                               res: *const c_void, res_f32: *const f32, out: *mut c_void, aux: *mut c_void,
                               out_f32: *mut f32, nb: i32, height: i32, width: i32, stream: *mut c_void) -> i32;
+    pub fn fg_sg_conv_dgrad(kind: i32, g: *const c_void, g_cstride: i32, w: *const c_void, res: *const c_void,
+                            relu: *const c_void, out: *mut c_void, masked: *mut c_void, nb: i32, height: i32, width: i32,
+                            stream: *mut c_void) -> i32;
     pub fn fg_sg_conv_wgrad(kind: i32, gout: *const c_void, g_cstride: i32, x: *const c_void, x_cstride: i32,
                             dw: *mut f32, db: *mut f32, nb: i32, height: i32, width: i32, stream: *mut c_void) -> i32;
     pub fn fg_sg_mask_grad(dh: *const c_void, relu: *const c_void, g: *mut c_void, n: i64, stream: *mut c_void) -> i32;

@@ -116,6 +116,71 @@ def test_tensor_core_convs_match_oracle(sg, cuda, fgl, shape):
     assert torch.equal(R, out)
 
 
+def test_tensor_core_conv_repeats_bit_for_bit(sg, cuda, fgl):
+    """Back-to-back launches over many small images (whose halo rows outside the image are filled with zeros at
+    once, the tightest reuse of a row slot) all equal the first."""
+    torch = cuda
+    nb, h, w = 256, 64, 64
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    X = torch.randn((nb, h, w, 32), generator=gen, device="cuda").relu_().to(torch.bfloat16)
+    Wt = (torch.randn((32, 9, 32), generator=gen, device="cuda") * 0.05).to(torch.bfloat16)
+    B = torch.zeros(32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    outs = [(torch.empty_like(X), torch.empty_like(X)) for _ in range(8)]
+    for _ in range(6):
+        for out, aux in outs:
+            assert fgl.lib().fg_sg_conv_forward(sg.CONV_RESIDUAL, X.data_ptr(), 32, Wt.data_ptr(), B.data_ptr(), X.data_ptr(),
+                                                None, out.data_ptr(), aux.data_ptr(), None, nb, h, w, st) == 0
+        torch.cuda.synchronize()
+        for out, aux in outs:
+            assert torch.equal(aux, outs[0][1]) and torch.equal(out, outs[0][0])
+            # the sum's two roundings (r and out, one bf16 step each)
+            assert bool(((out.float() - X.float() - aux.float()).abs() <= 2.0**-7 * out.float().abs()).all())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 9, 128), (3, 17, 129), (300, 3, 5)])
+def test_tensor_core_dgrad_and_wgrad_match_oracle(sg, cuda, fgl, shape):
+    """The masked data gradients and the weight gradients of the three conv kinds on the tensor cores.  Data
+    gradients: one bf16 step (2^-7) plus 2e-5; the mask exactly.  Weight gradients: f32 sums of up to
+    n = nb h w products (here n <= 4500) in another order, each within n 2^-23 of the sum of magnitudes."""
+    torch = cuda
+    nb, h, w = shape
+    x, wt, _, res = _conv_inputs(torch, nb, h, w, 7)
+    rng = np.random.default_rng(8)
+    g = sr.bf16_round(rng.normal(0, 1, (nb, h, w, 32)).astype(np.float32))
+    relu = np.maximum(rng.normal(0, 1, (nb, h, w, 32)), 0).astype(np.float32)
+    dy = np.zeros((nb, h, w, 16), np.float32)
+    dy[..., 0] = g[..., 0]
+    w_out = np.zeros((8, 9, 32), np.float32)
+    w_out[0] = wt[0]
+    dev = lambda a: torch.from_numpy(a).cuda().to(torch.bfloat16)
+    G, X, R, Wt, M, DY, WO = dev(g), dev(x), dev(res), dev(wt), dev(relu), dev(dy), dev(w_out)
+    out, masked = torch.empty_like(G), torch.empty_like(G)
+    L, st = fgl.lib(), torch.cuda.current_stream().cuda_stream
+    close = lambda got, want: np.all(np.abs(got.float().cpu().numpy() - want) <= 2.0**-7 * np.abs(want) + 2e-5)
+    for kind, gout, wts, want in ((sg.CONV_DGRAD_RESIDUAL, G, Wt, res + sr.conv_dgrad(g, wt)),
+                                  (sg.CONV_DGRAD_OUTPUT, DY, WO, sr.conv_dgrad(dy[..., :8], w_out))):
+        for dst in (out, None):
+            assert L.fg_sg_conv_dgrad(kind, gout.data_ptr(), gout.shape[-1], wts.data_ptr(), R.data_ptr(), M.data_ptr(),
+                                      None if dst is None else out.data_ptr(), masked.data_ptr(), nb, h, w, st) == 0
+            if dst is not None:
+                assert close(out, want)
+            assert torch.equal(masked, torch.where(M > 0, out, torch.zeros_like(out)))
+    x16 = torch.zeros((nb, h, w, 16), dtype=torch.bfloat16, device="cuda")
+    x16[..., :3] = X[..., :3]
+    for kind, gout, xin, co, ci in ((sg.CONV_RESIDUAL, G, X, 32, 32), (sg.CONV_INPUT, G, x16, 32, 16),
+                                    (sg.CONV_OUTPUT, DY, X, 8, 32)):
+        dw = torch.zeros((co, 9, ci), device="cuda")
+        db = torch.zeros(co, device="cuda")
+        assert L.fg_sg_conv_wgrad(kind, gout.data_ptr(), gout.shape[-1], xin.data_ptr(), xin.shape[-1], dw.data_ptr(),
+                                  db.data_ptr(), nb, h, w, st) == 0
+        gn, xn = gout.float().cpu().numpy()[..., :co].astype(np.float64), xin.float().cpu().numpy().astype(np.float64)
+        bound = nb * h * w * 2.0**-23
+        assert np.all(np.abs(dw.cpu().numpy() - sr.conv_wgrad(gn, xn)) <= bound * sr.conv_wgrad(np.abs(gn), np.abs(xn)))
+        flat = gn.reshape(-1, co)
+        assert np.all(np.abs(db.cpu().numpy() - flat.sum(0)) <= bound * np.abs(flat).sum(0))
+
+
 @pytest.mark.parametrize("shape", [(2, 16, 32), (2, 19, 41)])
 def test_gradients_match_oracle(sg, cuda, shape):
     """Every parameter gradient within 3e-2 relative L2 of the oracle's (bf16 activations, f32 sums)."""

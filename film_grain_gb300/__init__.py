@@ -401,7 +401,8 @@ class _Cancel:
         self.flag = ctypes.c_int32(1 if (cancel is not None and cancel()) else 0)
         self._stop = threading.Event()
         self._thread = None
-        if cancel is not None and not self.flag.value:
+        self._polled = cancel is not None
+        if self._polled and not self.flag.value:
             def watch():
                 while not self._stop.wait(0.001):
                     if cancel():
@@ -412,7 +413,8 @@ class _Cancel:
 
     @property
     def ptr(self):
-        return ctypes.addressof(self.flag)
+        # without a closure the library is given no flag, and its kernels none to look at
+        return ctypes.addressof(self.flag) if self._polled else None
 
     def __enter__(self):
         return self

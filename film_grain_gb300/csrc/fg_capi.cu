@@ -2,7 +2,6 @@
 // whole-image orchestration of render_from_workspace_impl (src/lib.rs:134-173).
 #include <algorithm>
 #include <atomic>
-#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -46,27 +45,28 @@ bool is_device_ptr(const void *p) {
 
 static bool cancelled(const volatile int32_t *cancel) { return cancel && *cancel != 0; }
 
-// ------------------------------------------------------------------ in-launch cancellation
-// The caller's cancel flag is ordinary host memory that the GPU cannot be assumed to reach, so while a
-// synchronous render runs a watcher thread polls it (every 200 us) and mirrors a non-zero value into
-// a word of mapped pinned memory that the kernels read (cancel_requested).  The words come from one
-// pinned block kept for the life of the process, one 64-byte line per render in flight.
-class CancelSlots {
+// ------------------------------------------------------------------ a synchronous render's host side
+// One 64-byte line of pinned, mapped host memory per synchronous render in flight, from one block kept for
+// the life of the process.  Words 0 and 1 are the in-launch cancellation words (cancel_requested): the
+// caller's cancel flag is ordinary host memory that the GPU cannot be assumed to reach, so it is mirrored
+// into word 0.  The rest receives the diagnostic counters (a copy into pageable memory would block the
+// host until the stream reached it).
+class HostLines {
   public:
-    static CancelSlots &get() {
-        static CancelSlots s;
+    static HostLines &get() {
+        static HostLines s;
         return s;
     }
     int *acquire() {
         std::lock_guard<std::mutex> lock(mu_);
         if (!base_) {
             void *p = nullptr;
-            if (cudaHostAlloc(&p, kSlots * kLine, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            if (cudaHostAlloc(&p, kLines * kLine, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
                 cudaGetLastError();
                 return nullptr;  // no in-launch polling; the flag is still read between launches
             }
             base_ = static_cast<int *>(p);
-            for (int i = kSlots - 1; i >= 0; i--) free_.push_back(i);
+            for (int i = kLines - 1; i >= 0; i--) free_.push_back(i);
         }
         if (free_.empty()) return nullptr;
         int *w = base_ + free_.back() * (kLine / sizeof(int));
@@ -81,61 +81,70 @@ class CancelSlots {
     }
 
   private:
-    static constexpr int kSlots = 256;
+    static constexpr int kLines = 256;
     static constexpr size_t kLine = 64;
+    static_assert(2 * sizeof(int) + kPwDiagWords * sizeof(unsigned long long) <= kLine, "line too short");
     std::mutex mu_;
     int *base_ = nullptr;
     std::vector<int> free_;
 };
 
-class CancelWatch {
+// The calling thread waits for its render here, and mirrors the cancel flag while it waits.  (A watcher
+// thread that slept 200 us between its looks cost every call its start and up to 200 us in its join: a
+// 96 x 64 plane whose launches span 208 us took 432 us.)
+class HostSide {
   public:
-    explicit CancelWatch(const volatile int32_t *cancel) : cancel_(cancel) {
-        if (!cancel) return;
-        host_ = CancelSlots::get().acquire();
-        if (!host_) return;
+    HostSide(const volatile int32_t *cancel, cudaStream_t s)
+        : cancel_(cancel), stream_(s), line_(HostLines::get().acquire()) {
+        if (!cancel || !line_) return;
         void *d = nullptr;
-        if (cudaHostGetDevicePointer(&d, host_, 0) != cudaSuccess) {
+        if (cudaHostGetDevicePointer(&d, line_, 0) != cudaSuccess) {
             cudaGetLastError();
-            CancelSlots::get().release(host_);
-            host_ = nullptr;
             return;
         }
         dev_ = static_cast<int *>(d);
-        thread_ = std::thread([this] {
-            while (!done_.load(std::memory_order_acquire)) {
-                if (*cancel_ != 0) {
-                    ((volatile int *)host_)[0] = 1;
-                    return;
-                }
-                std::this_thread::sleep_for(std::chrono::microseconds(200));
-            }
-        });
     }
-    // Called once the render's work on the GPU has finished (or failed).
-    ~CancelWatch() {
-        if (thread_.joinable()) {
-            done_.store(true, std::memory_order_release);
-            thread_.join();
-        }
-        if (host_) CancelSlots::get().release(host_);
+    // An early return waits here: the kernels and the counters' copy write the line.
+    ~HostSide() {
+        if (!waited_) cudaStreamSynchronize(stream_);
+        if (line_) HostLines::get().release(line_);
     }
-    CancelWatch(const CancelWatch &) = delete;
-    CancelWatch &operator=(const CancelWatch &) = delete;
-    int *dev() const { return dev_; }
+    HostSide(const HostSide &) = delete;
+    HostSide &operator=(const HostSide &) = delete;
+    int *cancel_words() const { return dev_; }
+    // where the counters' copy lands: pinned when there is a line
+    unsigned long long *diag() {
+        return line_ ? reinterpret_cast<unsigned long long *>(line_ + 2) : diag_;
+    }
     // whether a CTA stopped on the flag
-    bool stopped() const { return host_ && ((volatile int *)host_)[1] != 0; }
+    bool stopped() const { return line_ && ((volatile int *)line_)[1] != 0; }
+    // until the work queued so far has finished
+    cudaError_t wait() {
+        waited_ = true;
+        if (!dev_) return cudaStreamSynchronize(stream_);
+        for (;;) {
+            const cudaError_t e = cudaStreamQuery(stream_);
+            if (e != cudaErrorNotReady) return e;
+            cudaGetLastError();
+            if (*cancel_ != 0) {
+                ((volatile int *)line_)[0] = 1;
+                return cudaStreamSynchronize(stream_);
+            }
+            std::this_thread::yield();
+        }
+    }
 
   private:
     const volatile int32_t *cancel_;
-    int *host_ = nullptr;
+    cudaStream_t stream_;
+    int *line_;
+    bool waited_ = false;
     int *dev_ = nullptr;
-    std::atomic<bool> done_{false};
-    std::thread thread_;
+    unsigned long long diag_[kPwDiagWords];
 };
 
-static fg_status cancelled_error(const CancelWatch &w) {
-    return set_error(FG_ERR_CANCELLED, w.stopped() ? "cancelled (stopped inside a kernel)" : "cancelled");
+static fg_status cancelled_error(const HostSide &h) {
+    return set_error(FG_ERR_CANCELLED, h.stopped() ? "cancelled (stopped inside a kernel)" : "cancelled");
 }
 
 void offset_extents(const float *offs, uint32_t n, float ext[4]) {
@@ -231,28 +240,61 @@ struct DevBuf {
     }
 };
 
-fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_derived &d, const float *h_offs_in,
-                            const float *d_offs_in, float *d_out, CellParam *d_cells, unsigned long long *d_diag,
-                            const EpilogueArgs *colour, cudaStream_t s, bool may_allocate, int *d_cancel) {
+// The parts of a render's device memory, laid out one after the other in one allocation (each alloc and
+// free is some microseconds of host time before the first launch): add() gives a part's byte offset.
+struct Layout {
+    size_t bytes = 0;
+    size_t add(size_t n) {
+        const size_t at = bytes;
+        bytes = at + ((n + 255) & ~(size_t)255);
+        return at;
+    }
+};
+
+// A pixel-wise plane's scratch: the counters and the deferred list (its header beside them, so that both
+// are cleared together), the offsets, the cell table and, last, the sparse pass's bitmask.
+struct PwScratch {
+    PwPlan plan;
+    size_t diag, offs, cells, mask, mask_bytes;
+    PwScratch(const fg_params &p, const fg_derived &d, const float *h_offs_in, Layout *l) {
+        plan = plan_pixelwise(p, d, h_offs_in, 4);
+        const PixelwiseArgs a = pixelwise_args(p, d, plan, nullptr, nullptr, nullptr, nullptr, nullptr);
+        diag = l->add(sizeof(PwCounters) + (size_t)plan.nbx * plan.nby * sizeof(int));
+        offs = l->add(sizeof(float) * 2 * p.n_samples);
+        cells = l->add(sizeof(CellParam) * (size_t)d.input_width * d.input_height);
+        mask_bytes = pixelwise_cellmask_bytes(a, plan.nby);
+        mask = l->add(mask_bytes);
+    }
+    // the layout's allocation, without the bitmask where that finds no room (the plane takes the lean pass)
+    cudaError_t alloc(DevBuf *b, const Layout &l, cudaStream_t s) {
+        cudaError_t e = b->alloc(l.bytes, s);
+        if (e != cudaErrorMemoryAllocation || !mask_bytes) return e;
+        cudaGetLastError();
+        mask_bytes = 0;
+        return b->alloc(mask, s);
+    }
+    PwBuffers at(void *base) const {
+        char *c = static_cast<char *>(base);
+        PwBuffers w;
+        w.counters = reinterpret_cast<PwCounters *>(c + diag);
+        w.offs = reinterpret_cast<float *>(c + offs);
+        w.cells = reinterpret_cast<CellParam *>(c + cells);
+        w.listed = true;
+        w.mask = mask_bytes ? reinterpret_cast<unsigned int *>(c + mask) : nullptr;
+        return w;
+    }
+};
+
+fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_derived &d, const PwPlan &pl,
+                            const PwBuffers &w, float *d_out, const EpilogueArgs *colour, cudaStream_t s,
+                            int *d_cancel) {
     const int in_w = (int)d.input_width, in_h = (int)d.input_height;
     const int out_w = (int)d.output_width, out_h = (int)d.output_height;
-    const PwPlan pl = plan_pixelwise(p, d, h_offs_in, 4);
-    FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, d_cells, s), "cell params");
-    FG_CUDA(cudaMemsetAsync(d_out, 0, sizeof(float) * (size_t)out_w * out_h, s), "memset");
-    PixelwiseArgs a = pixelwise_args(p, d, pl, d_lam, d_cells, d_offs_in, d_out, d_diag);
+    FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, w.cells, d_out, (long long)out_w * out_h, w.counters, s),
+            "cell params");
+    PixelwiseArgs a = pixelwise_args(p, d, pl, d_lam, w.cells, w.offs, d_out, w.counters->diag);
     a.cancel = d_cancel;
-    DevBuf defer;  // the first pass's list of deferred root blocks (none without allocation: fat CTAs only)
-    DevBuf cellmask;  // the sparse pass's emptiness bitmask of the plane's cells
-    if (may_allocate) {
-        FG_CUDA(defer.alloc((2 + (size_t)pl.nbx * pl.nby) * sizeof(int), s), "alloc defer list");
-        const size_t mask_bytes = pixelwise_cellmask_bytes(a, pl.nby);
-        if (mask_bytes && cellmask.alloc(mask_bytes, s) != cudaSuccess) {
-            cudaGetLastError();  // no room for the bitmask: the plane takes the lean pass
-            cellmask.p = nullptr;
-        }
-    }
-    FG_CUDA(launch_pixelwise(a, pl.nby, static_cast<int *>(defer.p), static_cast<unsigned int *>(cellmask.p), s),
-            "pixelwise kernel");
+    FG_CUDA(launch_pixelwise(a, pl.nby, w.listed ? w.counters->list : nullptr, w.mask, s), "pixelwise kernel");
     EpilogueArgs e;
     if (colour) e = *colour;
     else std::memset(&e, 0, sizeof e);
@@ -330,22 +372,29 @@ GrainwiseArgs grainwise_args(const fg_params &p, const fg_derived &d, const floa
     return a;
 }
 
+// A grain-wise plane's scheduler area and a device's SM count for it.
+static fg_status grainwise_work_bytes(const GrainwiseArgs &a, size_t *bytes, int *sms) {
+    int dev = 0;
+    FG_CUDA(cudaGetDevice(&dev), "device");
+    FG_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
+    *bytes = grainwise_work_ints(a, *sms) * sizeof(int);
+    return FG_OK;
+}
+
+static fg_status check_grainwise(const GrainwiseArgs &a) {
+    if (a.request_bytes > 200 * 1024)
+        return set_error(FG_ERR_UNSUPPORTED, "n_samples too large for the grain-wise tile");
+    return FG_OK;
+}
+
 size_t grainwise_mask_bytes(const fg_params &p, const fg_derived &d) {
     return (size_t)d.output_width * d.output_height * ((p.n_samples + 31) / 32) * sizeof(unsigned int);
 }
 
-fg_status enqueue_grainwise(const GrainwiseArgs &a, cudaStream_t s) {
-    if (a.request_bytes > 200 * 1024)
-        return set_error(FG_ERR_UNSUPPORTED, "n_samples too large for the grain-wise tile");
+// a.work: the scheduler's area (grainwise_work_bytes)
+static fg_status enqueue_grainwise(const GrainwiseArgs &a, int sms, cudaStream_t s) {
     FG_CUDA(cudaMemsetAsync(a.gmask, 0, (size_t)a.out_w * a.out_h * a.words * sizeof(unsigned int), s), "memset mask");
-    GrainwiseArgs b = a;
-    int dev = 0, sms = 0;
-    FG_CUDA(cudaGetDevice(&dev), "device");
-    FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-    DevBuf work;  // the tile scheduler's area, freed in stream order after the launch
-    FG_CUDA(work.alloc(grainwise_work_ints(a, sms) * sizeof(int), s), "alloc tile scheduler");
-    b.work = static_cast<int *>(work.p);
-    FG_CUDA(launch_grainwise(b, sms, s), "grainwise kernel");
+    FG_CUDA(launch_grainwise(a, sms, s), "grainwise kernel");
     return FG_OK;
 }
 
@@ -399,56 +448,70 @@ static fg_status render_plane_sync(int algo, const float *lambda, const fg_param
     cudaStream_t s = (cudaStream_t)stream;
     const fg_params &p = *params;
     const fg_derived &d = *derived;
-    CancelWatch watch(cancel);
+    HostSide host(cancel, s);
     const size_t n_in = (size_t)d.input_width * d.input_height, n_out = (size_t)d.output_width * d.output_height;
     const size_t off_bytes = sizeof(float) * 2 * p.n_samples;
 
-    std::vector<float> h_offs(2 * (size_t)p.n_samples);
-    const bool offs_dev = is_device_ptr(offsets);
-    if (offs_dev) FG_CUDA(cudaMemcpy(h_offs.data(), offsets, off_bytes, cudaMemcpyDeviceToHost), "offsets D2H");
-    else std::memcpy(h_offs.data(), offsets, off_bytes);
-
-    DevBuf b_lam, b_out, b_offs, b_cells, b_diag;
-    const float *d_lam = lambda;
-    float *d_out = out;
-    const float *d_offs = offsets;
-    if (!is_device_ptr(lambda)) {
-        FG_CUDA(b_lam.alloc(sizeof(float) * n_in, s), "alloc lambda");
-        FG_CUDA(cudaMemcpyAsync(b_lam.p, lambda, sizeof(float) * n_in, cudaMemcpyHostToDevice, s), "lambda H2D");
-        d_lam = (const float *)b_lam.p;
+    const bool offs_dev = is_device_ptr(offsets), lam_dev = is_device_ptr(lambda), out_dev = is_device_ptr(out);
+    std::vector<float> h_copy;
+    const float *h_offs = offsets;
+    if (offs_dev) {
+        h_copy.resize(2 * (size_t)p.n_samples);
+        FG_CUDA(cudaMemcpy(h_copy.data(), offsets, off_bytes, cudaMemcpyDeviceToHost), "offsets D2H");
+        h_offs = h_copy.data();
     }
-    const bool out_dev = is_device_ptr(out);
-    if (!out_dev) {
-        FG_CUDA(b_out.alloc(sizeof(float) * n_out, s), "alloc out");
-        d_out = (float *)b_out.p;
-    }
-    if (!offs_dev) {
-        FG_CUDA(b_offs.alloc(off_bytes, s), "alloc offsets");
-        FG_CUDA(cudaMemcpyAsync(b_offs.p, h_offs.data(), off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
-        d_offs = (const float *)b_offs.p;
-    }
+    DevBuf b;
+    Layout l;
+    const size_t at_lam = lam_dev ? 0 : l.add(sizeof(float) * n_in), at_out = out_dev ? 0 : l.add(sizeof(float) * n_out);
+    auto planes = [&](const float **d_lam, float **d_out) -> fg_status {
+        *d_lam = lambda;
+        *d_out = out;
+        if (!lam_dev) {
+            float *dst = reinterpret_cast<float *>(static_cast<char *>(b.p) + at_lam);
+            FG_CUDA(cudaMemcpyAsync(dst, lambda, sizeof(float) * n_in, cudaMemcpyHostToDevice, s), "lambda H2D");
+            *d_lam = dst;
+        }
+        if (!out_dev) *d_out = reinterpret_cast<float *>(static_cast<char *>(b.p) + at_out);
+        return FG_OK;
+    };
+    const float *d_lam;
+    float *d_out;
     if (algo == FG_ALGO_PIXEL) {
-        FG_CUDA(b_cells.alloc(sizeof(CellParam) * n_in, s), "alloc cell table");
-        FG_CUDA(b_diag.alloc(sizeof(unsigned long long) * kPwDiagWords, s), "alloc diag");
-        FG_CUDA(cudaMemsetAsync(b_diag.p, 0, sizeof(unsigned long long) * kPwDiagWords, s), "memset diag");
-        st = enqueue_pixelwise(d_lam, p, d, h_offs.data(), d_offs, d_out, (CellParam *)b_cells.p,
-                               (unsigned long long *)b_diag.p, nullptr, s, true, watch.dev());
+        PwScratch scratch(p, d, h_offs, &l);
+        FG_CUDA(scratch.alloc(&b, l, s), "alloc render");
+        const PwBuffers w = scratch.at(b.p);
+        FG_CUDA(cudaMemcpyAsync(w.offs, h_offs, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
+        if ((st = planes(&d_lam, &d_out)) != FG_OK) return st;
+        st = enqueue_pixelwise(d_lam, p, d, scratch.plan, w, d_out, nullptr, s, host.cancel_words());
+        if (st != FG_OK) return st;
+        FG_CUDA(cudaMemcpyAsync(host.diag(), w.counters->diag, sizeof g_pw_diag, cudaMemcpyDeviceToHost, s), "diag D2H");
     } else {
-        FG_CUDA(b_cells.alloc(grainwise_mask_bytes(p, d), s), "alloc sample masks");
-        GrainwiseArgs a = grainwise_args(p, d, h_offs.data(), d_lam, d_offs, (unsigned int *)b_cells.p, kGrainMaskWords);
-        a.cancel = watch.dev();
-        st = enqueue_grainwise(a, s);
+        GrainwiseArgs a = grainwise_args(p, d, h_offs, nullptr, nullptr, nullptr, kGrainMaskWords);
+        size_t work_bytes;
+        int sms;
+        if ((st = check_grainwise(a)) != FG_OK) return st;
+        if ((st = grainwise_work_bytes(a, &work_bytes, &sms)) != FG_OK) return st;
+        const size_t at_offs = l.add(off_bytes), at_work = l.add(work_bytes), at_mask = l.add(grainwise_mask_bytes(p, d));
+        FG_CUDA(b.alloc(l.bytes, s), "alloc render");
+        char *base = static_cast<char *>(b.p);
+        FG_CUDA(cudaMemcpyAsync(base + at_offs, h_offs, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
+        if ((st = planes(&d_lam, &d_out)) != FG_OK) return st;
+        a.lam = d_lam;
+        a.offs = reinterpret_cast<const float2 *>(base + at_offs);
+        a.work = reinterpret_cast<int *>(base + at_work);
+        a.gmask = reinterpret_cast<unsigned int *>(base + at_mask);
+        a.cancel = host.cancel_words();
+        st = enqueue_grainwise(a, sms, s);
         if (st == FG_OK) st = enqueue_grainwise_epilogue(a, d_out, 0, nullptr, nullptr, nullptr, s);
+        if (st != FG_OK) return st;
     }
-    if (st != FG_OK) {
-        cudaStreamSynchronize(s);
-        return st;
+    FG_CUDA(host.wait(), "render");
+    if (!out_dev) {
+        FG_CUDA(cudaMemcpyAsync(out, d_out, sizeof(float) * n_out, cudaMemcpyDeviceToHost, s), "out D2H");
+        FG_CUDA(cudaStreamSynchronize(s), "render");
     }
-    if (!out_dev) FG_CUDA(cudaMemcpyAsync(out, d_out, sizeof(float) * n_out, cudaMemcpyDeviceToHost, s), "out D2H");
-    if (algo == FG_ALGO_PIXEL)
-        FG_CUDA(cudaMemcpyAsync(g_pw_diag, b_diag.p, sizeof g_pw_diag, cudaMemcpyDeviceToHost, s), "diag D2H");
-    FG_CUDA(cudaStreamSynchronize(s), "render");
-    if (cancelled(cancel)) return cancelled_error(watch);
+    if (algo == FG_ALGO_PIXEL) std::memcpy(g_pw_diag, host.diag(), sizeof g_pw_diag);
+    if (cancelled(cancel)) return cancelled_error(host);
     clear_error();
     return FG_OK;
 }
@@ -478,16 +541,14 @@ FG_API fg_status fg_render_pixelwise_async(const float *d_lambda, const fg_param
     if (is_device_ptr(offsets_input)) return set_error(FG_ERR_INVALID, "offsets_input must be host memory");
     keep_pool_memory();
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t n_in = (size_t)derived->input_width * derived->input_height;
-    const size_t off_bytes = sizeof(float) * 2 * params->n_samples;
-    DevBuf b_offs, b_cells, b_diag;
-    FG_CUDA(b_offs.alloc(off_bytes, s), "alloc offsets");
-    FG_CUDA(cudaMemcpyAsync(b_offs.p, offsets_input, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
-    FG_CUDA(b_cells.alloc(sizeof(CellParam) * n_in, s), "alloc cell table");
-    FG_CUDA(b_diag.alloc(sizeof(unsigned long long) * kPwDiagWords, s), "alloc diag");
-    FG_CUDA(cudaMemsetAsync(b_diag.p, 0, sizeof(unsigned long long) * kPwDiagWords, s), "memset diag");
-    return enqueue_pixelwise(d_lambda, *params, *derived, offsets_input, (const float *)b_offs.p, d_out,
-                             (CellParam *)b_cells.p, (unsigned long long *)b_diag.p, nullptr, s);
+    DevBuf b;
+    Layout l;
+    PwScratch scratch(*params, *derived, offsets_input, &l);
+    FG_CUDA(scratch.alloc(&b, l, s), "alloc render");
+    const PwBuffers w = scratch.at(b.p);
+    FG_CUDA(cudaMemcpyAsync(w.offs, offsets_input, sizeof(float) * 2 * params->n_samples, cudaMemcpyHostToDevice, s),
+            "offsets H2D");
+    return enqueue_pixelwise(d_lambda, *params, *derived, scratch.plan, w, d_out, nullptr, s, nullptr);
 }
 
 FG_API fg_status fg_render_grainwise_async(const float *d_lambda, const fg_params *params, const fg_derived *derived,
@@ -499,12 +560,22 @@ FG_API fg_status fg_render_grainwise_async(const float *d_lambda, const fg_param
     keep_pool_memory();
     cudaStream_t s = (cudaStream_t)stream;
     const size_t off_bytes = sizeof(float) * 2 * params->n_samples;
-    DevBuf b_offs, b_mask;
-    FG_CUDA(b_offs.alloc(off_bytes, s), "alloc offsets");
-    FG_CUDA(cudaMemcpyAsync(b_offs.p, offsets, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
-    FG_CUDA(b_mask.alloc(grainwise_mask_bytes(*params, *derived), s), "alloc sample masks");
-    GrainwiseArgs a = grainwise_args(*params, *derived, offsets, d_lambda, (const float *)b_offs.p, (unsigned int *)b_mask.p, kGrainMaskWords);
-    st = enqueue_grainwise(a, s);
+    GrainwiseArgs a = grainwise_args(*params, *derived, offsets, d_lambda, nullptr, nullptr, kGrainMaskWords);
+    size_t work_bytes;
+    int sms;
+    if ((st = check_grainwise(a)) != FG_OK) return st;
+    if ((st = grainwise_work_bytes(a, &work_bytes, &sms)) != FG_OK) return st;
+    DevBuf b;
+    Layout l;
+    const size_t at_offs = l.add(off_bytes), at_work = l.add(work_bytes),
+                 at_mask = l.add(grainwise_mask_bytes(*params, *derived));
+    FG_CUDA(b.alloc(l.bytes, s), "alloc render");
+    char *base = static_cast<char *>(b.p);
+    FG_CUDA(cudaMemcpyAsync(base + at_offs, offsets, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
+    a.offs = reinterpret_cast<const float2 *>(base + at_offs);
+    a.work = reinterpret_cast<int *>(base + at_work);
+    a.gmask = reinterpret_cast<unsigned int *>(base + at_mask);
+    st = enqueue_grainwise(a, sms, s);
     if (st == FG_OK) st = enqueue_grainwise_epilogue(a, d_out, 0, nullptr, nullptr, nullptr, s);
     return st;
 }
@@ -537,78 +608,84 @@ FG_API fg_status fg_render_image(const float *rgb, int64_t width, int64_t height
 
     keep_pool_memory();
     cudaStream_t s = (cudaStream_t)stream;
-    CancelWatch watch(cancel);
-    DevBuf b_lam, b_out, b_rgb8, b_rgb, b_planes, b_max, b_offs, b_cells, b_diag;
+    HostSide host(cancel, s);
     // the cropped interleaved RGB to the device, then the colour split, the plane maxima and lambda
     // there (fg_lambda.cu): no host pass over the image
-    FG_CUDA(b_rgb.alloc(sizeof(float) * 3 * n_in, s), "alloc rgb");
-    FG_CUDA(cudaMemcpy2DAsync(b_rgb.p, sizeof(float) * 3 * (size_t)cw, rgb + 3 * ((size_t)y0 * width + x0),
+    DevBuf b;
+    Layout l;
+    const size_t at_rgb = l.add(sizeof(float) * 3 * n_in), at_planes = l.add(sizeof(float) * 3 * n_in),
+                 at_max = l.add(sizeof(unsigned int) * 3), at_lam = l.add(sizeof(float) * n_in * nplanes),
+                 at_out = l.add(sizeof(float) * n_out * nplanes), at_rgb8 = l.add(3 * n_out);
+    const std::vector<float> &used_offs = algo == FG_ALGO_PIXEL ? offs_in : offs;
+    const size_t off_bytes = sizeof(float) * 2 * p.n_samples;
+    const size_t mask_bytes = algo == FG_ALGO_GRAIN ? grainwise_mask_bytes(p, d) : 0;
+    std::unique_ptr<PwScratch> pw;  // one plane after the other in the same scratch
+    GrainwiseArgs ga;
+    std::memset(&ga, 0, sizeof ga);
+    size_t at_offs = 0, at_work = 0, at_mask = 0;
+    int sms = 0;
+    if (algo == FG_ALGO_PIXEL) {
+        pw.reset(new PwScratch(p, d, offs_in.data(), &l));
+        at_offs = pw->offs;
+        FG_CUDA(pw->alloc(&b, l, s), "alloc render");
+    } else {
+        ga = grainwise_args(p, d, offs.data(), nullptr, nullptr, nullptr, kGrainMaskWords);
+        size_t work_bytes;
+        if ((st = check_grainwise(ga)) != FG_OK) return st;
+        if ((st = grainwise_work_bytes(ga, &work_bytes, &sms)) != FG_OK) return st;
+        at_offs = l.add(off_bytes);
+        at_work = l.add(work_bytes);
+        at_mask = l.add(mask_bytes * nplanes);
+        FG_CUDA(b.alloc(l.bytes, s), "alloc render");
+    }
+    char *base = static_cast<char *>(b.p);
+    float *d_rgb = reinterpret_cast<float *>(base + at_rgb), *d_planes = reinterpret_cast<float *>(base + at_planes);
+    float *d_lam = reinterpret_cast<float *>(base + at_lam), *d_out = reinterpret_cast<float *>(base + at_out);
+    unsigned char *d_rgb8 = reinterpret_cast<unsigned char *>(base + at_rgb8);
+    FG_CUDA(cudaMemcpyAsync(base + at_offs, used_offs.data(), off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
+    FG_CUDA(cudaMemcpy2DAsync(d_rgb, sizeof(float) * 3 * (size_t)cw, rgb + 3 * ((size_t)y0 * width + x0),
                               sizeof(float) * 3 * (size_t)width, sizeof(float) * 3 * (size_t)cw, (size_t)ch,
                               cudaMemcpyHostToDevice, s),
             "rgb H2D");
-    FG_CUDA(b_planes.alloc(sizeof(float) * 3 * n_in, s), "alloc planes");
-    FG_CUDA(b_max.alloc(sizeof(unsigned int) * 3, s), "alloc plane maxima");
-    FG_CUDA(b_lam.alloc(sizeof(float) * n_in * nplanes, s), "alloc lambda");
-    FG_CUDA(b_out.alloc(sizeof(float) * n_out * nplanes, s), "alloc planes");
-    FG_CUDA(b_rgb8.alloc(3 * n_out, s), "alloc rgb8");
-    const std::vector<float> &used_offs = algo == FG_ALGO_PIXEL ? offs_in : offs;
-    FG_CUDA(b_offs.alloc(sizeof(float) * 2 * p.n_samples, s), "alloc offsets");
-    FG_CUDA(cudaMemcpyAsync(b_offs.p, used_offs.data(), sizeof(float) * 2 * p.n_samples, cudaMemcpyHostToDevice, s),
-            "offsets H2D");
-    float *d_lam = (float *)b_lam.p, *d_out = (float *)b_out.p;
-    st = enqueue_split_lambda((const float *)b_rgb.p, (long long)n_in, luma ? 1 : 0, (float *)b_planes.p,
-                              (unsigned int *)b_max.p, d.inv_e_pi_r2, d_lam, s);
-    if (st != FG_OK) {
-        cudaStreamSynchronize(s);
-        return st;
-    }
-    float *d_cb = nullptr, *d_cr = nullptr;
-    if (luma) {
-        d_cb = (float *)b_planes.p + n_in;
-        d_cr = d_cb + n_in;
-    }
-    const size_t mask_bytes = algo == FG_ALGO_GRAIN ? grainwise_mask_bytes(p, d) : 0;
-    if (algo == FG_ALGO_PIXEL) {
-        FG_CUDA(b_cells.alloc(sizeof(CellParam) * n_in, s), "alloc cell table");
-        FG_CUDA(b_diag.alloc(sizeof(unsigned long long) * kPwDiagWords, s), "alloc diag");
-        FG_CUDA(cudaMemsetAsync(b_diag.p, 0, sizeof(unsigned long long) * kPwDiagWords, s), "memset diag");
-    } else {
-        FG_CUDA(b_cells.alloc(mask_bytes * nplanes, s), "alloc sample masks");
-    }
+    st = enqueue_split_lambda(d_rgb, (long long)n_in, luma ? 1 : 0, d_planes,
+                              reinterpret_cast<unsigned int *>(base + at_max), d.inv_e_pi_r2, d_lam, s);
+    if (st != FG_OK) return st;
+    float *d_cb = luma ? d_planes + n_in : nullptr, *d_cr = luma ? d_cb + n_in : nullptr;
     for (int c = 0; c < nplanes; c++) {
         if (cancelled(cancel)) {
-            cudaStreamSynchronize(s);
-            return cancelled_error(watch);
+            host.wait();
+            return cancelled_error(host);
         }
         float *d_plane = d_out + (size_t)c * n_out;
         if (algo == FG_ALGO_PIXEL) {
             EpilogueArgs e;
             std::memset(&e, 0, sizeof e);
             if (luma) {
-                e.mode = 1; e.out_rgb8 = (unsigned char *)b_rgb8.p; e.cb = d_cb; e.cr = d_cr;
+                e.mode = 1; e.out_rgb8 = d_rgb8; e.cb = d_cb; e.cr = d_cr;
             } else if (c == 2) {
-                e.mode = 2; e.out_rgb8 = (unsigned char *)b_rgb8.p; e.p0 = d_out; e.p1 = d_out + n_out;
+                e.mode = 2; e.out_rgb8 = d_rgb8; e.p0 = d_out; e.p1 = d_out + n_out;
             }
-            st = enqueue_pixelwise(d_lam + (size_t)c * n_in, p, d, offs_in.data(), (const float *)b_offs.p, d_plane,
-                                   (CellParam *)b_cells.p, (unsigned long long *)b_diag.p, &e, s, true, watch.dev());
+            st = enqueue_pixelwise(d_lam + (size_t)c * n_in, p, d, pw->plan, pw->at(base), d_plane, &e, s,
+                                   host.cancel_words());
         } else {
-            unsigned int *plane_mask = (unsigned int *)((unsigned char *)b_cells.p + mask_bytes * c);
-            GrainwiseArgs a = grainwise_args(p, d, offs.data(), d_lam + (size_t)c * n_in, (const float *)b_offs.p, plane_mask, kGrainMaskWords);
-            a.cancel = watch.dev();
-            st = enqueue_grainwise(a, s);
+            GrainwiseArgs a = ga;
+            a.lam = d_lam + (size_t)c * n_in;
+            a.offs = reinterpret_cast<const float2 *>(base + at_offs);
+            a.work = reinterpret_cast<int *>(base + at_work);
+            a.gmask = reinterpret_cast<unsigned int *>(base + at_mask + mask_bytes * c);
+            a.cancel = host.cancel_words();
+            st = enqueue_grainwise(a, sms, s);
             if (st == FG_OK && c == nplanes - 1) {
-                a.gmask = (unsigned int *)b_cells.p;  // all planes' masks, consecutive
-                st = enqueue_grainwise_epilogue(a, nullptr, luma ? 1 : 2, (unsigned char *)b_rgb8.p, d_cb, d_cr, s);
+                a.gmask = reinterpret_cast<unsigned int *>(base + at_mask);  // all planes' masks, consecutive
+                st = enqueue_grainwise_epilogue(a, nullptr, luma ? 1 : 2, d_rgb8, d_cb, d_cr, s);
             }
         }
-        if (st != FG_OK) {
-            cudaStreamSynchronize(s);
-            return st;
-        }
+        if (st != FG_OK) return st;
     }
-    FG_CUDA(cudaMemcpyAsync(out_rgb8, b_rgb8.p, 3 * n_out, cudaMemcpyDeviceToHost, s), "rgb8 D2H");
+    FG_CUDA(host.wait(), "render");
+    FG_CUDA(cudaMemcpyAsync(out_rgb8, d_rgb8, 3 * n_out, cudaMemcpyDeviceToHost, s), "rgb8 D2H");
     FG_CUDA(cudaStreamSynchronize(s), "render");
-    if (cancelled(cancel)) return cancelled_error(watch);
+    if (cancelled(cancel)) return cancelled_error(host);
     if (stats) fill_stats(p, d, algo, stats);
     clear_error();
     return FG_OK;

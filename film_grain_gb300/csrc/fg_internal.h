@@ -20,15 +20,21 @@ void offset_extents(const float *offs, uint32_t n, float ext[4]);
 PwPlan plan_pixelwise(const fg_params &p, const fg_derived &d, const float *h_offs_in, int max_block_log2);
 PixelwiseArgs pixelwise_args(const fg_params &p, const fg_derived &d, const PwPlan &pl, const float *d_lam,
                              const CellParam *d_cells, const float *d_offs_in, float *d_out, unsigned long long *d_diag);
-fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_derived &d, const float *h_offs_in,
-                            const float *d_offs_in, float *d_out, CellParam *d_cells, unsigned long long *d_diag,
-                            const EpilogueArgs *colour, cudaStream_t s, bool may_allocate = true,
-                            int *d_cancel = nullptr);
+// The device memory of a pixel-wise plane beside its input and output.
+struct PwBuffers {
+    PwCounters *counters;  // cleared by the enqueued work
+    float *offs;           // the input-space offsets, already there
+    CellParam *cells;
+    bool listed;           // the deferred list follows the counters (else: fat CTAs over every block)
+    unsigned int *mask;    // null, or the sparse pass's bitmask (pixelwise_cellmask_bytes)
+};
+fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_derived &d, const PwPlan &pl,
+                            const PwBuffers &w, float *d_out, const EpilogueArgs *colour, cudaStream_t s,
+                            int *d_cancel);
 GrainwiseArgs grainwise_args(const fg_params &p, const fg_derived &d, const float *h_offs, const float *d_lam,
                              const float *d_offs, unsigned int *d_gmask, int mask_words);
 bool grainwise_small_coords(const GrainwiseArgs &a);
 size_t grainwise_mask_bytes(const fg_params &p, const fg_derived &d);
-fg_status enqueue_grainwise(const GrainwiseArgs &a, cudaStream_t s);
 fg_status enqueue_grainwise_epilogue(const GrainwiseArgs &a, float *d_out, int mode, unsigned char *d_rgb8,
                                      const float *d_cb, const float *d_cr, cudaStream_t s);
 

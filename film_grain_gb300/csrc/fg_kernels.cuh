@@ -37,6 +37,13 @@ constexpr int kPwMaxLevel = 3;     // block subdivision depth on grain overflow
 // [1] blocks without a staged window, [2] block subdivisions, [3] blocks run, [4] sparse blocks whose
 // samples ran sample-major, [5] sparse blocks that ran grain-major.
 constexpr int kPwDiagWords = 6;
+
+// A pixel-wise plane's counters, and the header of its deferred list: [0] the next entry the fat pass
+// takes, [1] the number of entries, which follow in list[2..] where a list is kept.
+struct PwCounters {
+    unsigned long long diag[kPwDiagWords];
+    int list[2];
+};
 // A block regenerates per sample (no staging) when its samples' reach, in cells, is below
 // kPwRegenSparse x its window's cells, or below kPwRegenOverflow x them once the window overflows
 // with more than kPwRegenDense of its cells non-empty.
@@ -54,7 +61,7 @@ constexpr float kPwRegenRankLd = 0.3f;
 constexpr float kPwRegenFlatLd = 1.1f;
 
 // In-launch cancellation: `cancel` is null or two words of mapped pinned host memory.  Word 0 is set
-// by the library's host watcher once the caller's cancel flag turns non-zero; the persistent passes
+// by the waiting host thread once the caller's cancel flag turns non-zero; the persistent passes
 // read it once per work item they pull (the block passes once per block) and stop, and a CTA that
 // stops on it sets word 1.
 #ifdef __CUDACC__
@@ -141,9 +148,11 @@ struct LogfTableDev {
     int shift;
 };
 
-cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, cudaStream_t s);
-// defer: null (fat CTAs over every block) or a buffer of 2 + nbx*nby ints (lean pass, then fat CTAs
-// over the deferred blocks).
+// The cell table, and the plane's output and counters set to zero beside it.
+cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, float *out,
+                               long long n_out, PwCounters *counters, cudaStream_t s);
+// defer: null (fat CTAs over every block) or PwCounters::list, cleared, with nbx*nby ints behind it (lean
+// pass, then fat CTAs over the deferred blocks).
 // cellmask: null, or pixelwise_cellmask_bytes(a, nby) bytes for the sparse pass's plane bitmask (the
 // plane then takes the sparse pass, else the lean pass).
 cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsigned int *cellmask, cudaStream_t s);

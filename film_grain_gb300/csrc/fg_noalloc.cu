@@ -30,7 +30,7 @@ namespace fg {
 
 constexpr size_t kNaCellsBytes = (size_t)FG_NOALLOC_MAX_INPUT_PIXELS * sizeof(CellParam);
 constexpr size_t kNaOffsBytes = (size_t)FG_NOALLOC_MAX_SAMPLES * 2 * sizeof(float);
-constexpr size_t kNaDiagBytes = kPwDiagWords * sizeof(unsigned long long);
+constexpr size_t kNaDiagBytes = sizeof(PwCounters);
 constexpr size_t kNaScratchBytes = kNaCellsBytes + kNaOffsBytes + kNaDiagBytes;
 
 // The shared scratch of every fg_render_pixelwise_noalloc call on a device.
@@ -118,19 +118,20 @@ extern "C" FG_API fg_status fg_render_pixelwise_noalloc(const float *d_lambda, c
     unsigned char *scratch = nullptr;
     st = noalloc_scratch(&scratch);
     if (st != FG_OK) return st;
-    CellParam *cells = reinterpret_cast<CellParam *>(scratch);
-    float *offs = reinterpret_cast<float *>(scratch + kNaCellsBytes);
-    unsigned long long *diag = reinterpret_cast<unsigned long long *>(scratch + kNaCellsBytes + kNaOffsBytes);
+    PwBuffers w;
+    w.cells = reinterpret_cast<CellParam *>(scratch);
+    w.offs = reinterpret_cast<float *>(scratch + kNaCellsBytes);
+    w.counters = reinterpret_cast<PwCounters *>(scratch + kNaCellsBytes + kNaOffsBytes);
+    w.listed = false;
+    w.mask = nullptr;
     cudaStream_t s = (cudaStream_t)stream;
-    // The array keeps the previous call's contents: the offsets are overwritten here, the cell table
-    // by the cell-parameter kernel, and the counters must start at zero.
-    cudaError_t e = cudaMemcpyAsync(offs, offsets_input, sizeof(float) * 2 * params->n_samples,
-                                    cudaMemcpyHostToDevice, s);
+    // The array keeps the previous call's contents: the offsets are overwritten here, the cell table and
+    // the counters by the cell-parameter kernel.
+    const cudaError_t e = cudaMemcpyAsync(w.offs, offsets_input, sizeof(float) * 2 * params->n_samples,
+                                          cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_error(e, "offsets H2D");
-    e = cudaMemsetAsync(diag, 0, kNaDiagBytes, s);
-    if (e != cudaSuccess) return cuda_error(e, "clear counters");
-    st = enqueue_pixelwise(d_lambda, *params, *derived, offsets_input, offs, d_out, cells, diag, nullptr, s,
-                           /*may_allocate=*/false);
+    st = enqueue_pixelwise(d_lambda, *params, *derived, plan_pixelwise(*params, *derived, offsets_input, 4), w, d_out,
+                           nullptr, s, nullptr);
     if (st == FG_OK) clear_error();
     return st;
 }

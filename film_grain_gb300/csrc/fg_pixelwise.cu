@@ -35,8 +35,14 @@
 namespace fg {
 
 // ------------------------------------------------------------------ per-pixel Poisson set-up
-__global__ void cell_params_kernel(const float *__restrict__ lam, int n, float delta, CellParam *__restrict__ cells) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The output and the counters are cleared here too: each memset of its own was 6 us of a small plane's 208 us
+// between its first and last launch, which are bound by the host's enqueueing.
+__global__ void cell_params_kernel(const float *__restrict__ lam, long long n, float delta,
+                                   CellParam *__restrict__ cells, float *__restrict__ out, long long n_out,
+                                   PwCounters *__restrict__ counters) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (long long)(sizeof(PwCounters) / sizeof(int))) reinterpret_cast<int *>(counters)[i] = 0;
+    if (i < n_out) out[i] = 0.0f;
     if (i >= n) return;
     float l = lam[i];
     CellParam c;
@@ -59,10 +65,12 @@ __global__ void cell_params_kernel(const float *__restrict__ lam, int n, float d
     cells[i] = c;
 }
 
-cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, cudaStream_t s) {
-    int n = in_w * in_h;
-    if (n <= 0) return cudaSuccess;
-    cell_params_kernel<<<(n + 255) / 256, 256, 0, s>>>(lam, n, delta, cells);
+cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, float *out,
+                               long long n_out, PwCounters *counters, cudaStream_t s) {
+    const long long n = (long long)in_w * in_h;
+    const long long grid = (std::max(n, n_out) + 255) / 256;  // 256 threads and more: all words of the counters
+    if (grid <= 0) return cudaSuccess;
+    cell_params_kernel<<<(unsigned)grid, 256, 0, s>>>(lam, n, delta, cells, out, n_out, counters);
     return cudaGetLastError();
 }
 
@@ -330,8 +338,6 @@ cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsign
         pixelwise_kernel<PwFat><<<(unsigned)nblocks, PwFat::kThreads, fat_smem, s>>>(a, nullptr);
         return cudaGetLastError();
     }
-    e = cudaMemsetAsync(defer, 0, 2 * sizeof(int), s);  // [0] the fat pass's counter, [1] the list's count
-    if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -51,15 +51,11 @@ constexpr float kPwRegenSparse = 1.0f;
 constexpr float kPwRegenOverflow = 4.0f;
 constexpr float kPwRegenDense = 0.4f;
 // The per-sample kernel replaces the block kernel for a whole plane when an interior root block's
-// samples reach fewer than kPwRegenKernel x its window's cells (and a sample's range fits 64 cells).
+// samples reach fewer than kPwRegenKernel x its window's cells (and a sample's range fits 64 cells): 700 x 500
+// ramps cross at 2.1 to 2.7 (radius 0.05: N 100 at 2.1 runs 2.92 ms against the block passes' 3.40, N 128 at
+// 2.7 3.66 against 3.63; radius 0.07: N 64 at 2.6 1.92 against 1.96), blobs at 2.1 (2.29 against 2.27).
 constexpr int kPwRegenThreads = 256;
-constexpr float kPwRegenKernel = 1.5f;
-// Forms of the per-sample kernel by a warp's expected grains per cell (λδ²), from timings of uniform
-// planes (r 0.025-0.1, N 16-256): lane-major dealing up to 0.3, rank-major dealing up to 1.1 (u 0.7:
-// 11 % faster, u 0.9: 27 % faster than its neighbours), the flattened loop above (u 0.99).
-constexpr float kPwRegenRankLd = 0.3f;
-constexpr float kPwRegenFlatLd = 1.1f;
-
+constexpr float kPwRegenKernel = 2.05f;
 // In-launch cancellation: `cancel` is null or two words of mapped pinned host memory.  Word 0 is set
 // by the waiting host thread once the caller's cancel flag turns non-zero; the persistent passes
 // read it once per work item they pull (the block passes once per block) and stop, and a CTA that
@@ -90,7 +86,7 @@ struct PixelwiseArgs {
     float radius_mean;
     float log_mu, log_sigma;
     int *cancel;                // null, or the in-launch cancellation words (cancel_requested)
-    // null, or the plane's emptiness bitmask (the sparse pass's first_draw_screen of every cell):
+    // null, or the plane's emptiness bitmask (the sparse pass's first_draw_maybe of every cell):
     // cells [cm_gi0, cm_gi0 + cm_gw) x [cm_gj0, cm_gj0 + 32 cm_ghw), word (c, k) = cellmask[k * cm_gw + c]
     // holding rows cm_gj0 + 32k .. + 31 of column cm_gi0 + c
     const unsigned int *cellmask;

@@ -153,12 +153,15 @@ __global__ void __launch_bounds__(kPwKChunk) sort_offsets_kernel(const float2 *_
     }
 }
 
-// The plane's emptiness bitmask (pixelwise_sparse_block step 0): one thread per mask word.
-__global__ void __launch_bounds__(256) cell_mask_kernel(const __grid_constant__ PixelwiseArgs a, const PwSparseGrid g,
-                                                        unsigned int *__restrict__ cellmask) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.gw * g.ghw) return;
-    cell_mask_word(a, g, t, cellmask);
+// The plane's emptiness bitmask (pixelwise_sparse_block step 0): one thread per mask word, row_ctas CTAs to a
+// word row.
+constexpr int kMaskThreads = 256;
+__global__ void __launch_bounds__(kMaskThreads) cell_mask_kernel(const __grid_constant__ PixelwiseArgs a,
+                                                                 const PwSparseGrid g, int row_ctas,
+                                                                 unsigned int *__restrict__ cellmask) {
+    const int k = (int)(blockIdx.x / (unsigned)row_ctas);
+    const int c = (int)(blockIdx.x % (unsigned)row_ctas) * kMaskThreads + (int)threadIdx.x;
+    if ((c & ~31) < g.gw) cell_mask_word(a, g, c, k, cellmask);  // whole warps
 }
 
 static int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
@@ -301,7 +304,7 @@ bool pixelwise_prefers_regen(const PixelwiseArgs &a) {
     // a sample's range must fit the 64-bit cell mask of pixelwise_pixel
     const double axis = std::floor(2.0 * (double)a.rm / (double)a.delta) + 2.0;
     if (!(axis * axis <= 64.0)) return false;
-    // cell indices of every sample must stay far inside int (the flattened loop's range arithmetic)
+    // cell indices of every sample must stay far inside int (the range arithmetic)
     const double reach = (double)std::max(a.out_w, a.out_h) / a.zoom +
                          std::max({std::fabs(a.offx_min), std::fabs(a.offx_max), std::fabs(a.offy_min),
                                    std::fabs(a.offy_max)}) + a.rm + 2.0;
@@ -346,8 +349,8 @@ cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsign
     const bool sparse = cellmask && plan_sparse(a, nby, sms, &g);
     if (sparse) {
         g.cellmask = cellmask;
-        const long long words = (long long)g.gw * g.ghw;
-        cell_mask_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(a, g, cellmask);
+        const int row_ctas = (g.gw + kMaskThreads - 1) / kMaskThreads;
+        cell_mask_kernel<<<(unsigned)((long long)row_ctas * g.ghw), kMaskThreads, 0, s>>>(a, g, row_ctas, cellmask);
         PixelwiseArgs as = a;  // the sparse pass reads the offsets sorted by x
         char *scratch = reinterpret_cast<char *>(cellmask);
         as.offs = reinterpret_cast<const float2 *>(scratch + sparse_mask_bytes(g));

@@ -78,14 +78,38 @@ __device__ __forceinline__ float radius_draw(const PixelwiseArgs &a, Xoshiro &rn
     return lognormal_radius_f32(a.log_mu, a.log_sigma, rng);
 }
 
-// Index of the lambda pixel of cell (i, j): the cell origin's pixel, clamped to the plane
-// (src/pixelwise.rs:69-72).
+// Lambda pixel of a cell's origin on one axis, clamped to the plane's n pixels (src/pixelwise.rs:69-72): the
+// clamp on floats, which hold 0..n-1 exactly (n <= 2^24), so that the conversion is a 32-bit one.
+__device__ __forceinline__ int cell_axis_pixel(int i, float delta, int n) {
+    return (int)fminf(fmaxf(floorf(FG_FMUL((float)i, delta)), 0.0f), (float)(n - 1));
+}
+
+// Index of the lambda pixel of cell (i, j).
 __device__ __forceinline__ long long cell_pixel(const PixelwiseArgs &a, int i, int j) {
-    float sx = FG_FMUL((float)i, a.delta), sy = FG_FMUL((float)j, a.delta);
-    long long ix = (long long)floorf(sx), iy = (long long)floorf(sy);
-    ix = ix < 0 ? 0 : (ix > a.in_w - 1 ? a.in_w - 1 : ix);
-    iy = iy < 0 ? 0 : (iy > a.in_h - 1 ? a.in_h - 1 : iy);
-    return iy * (long long)a.in_w + ix;
+    return (long long)cell_axis_pixel(j, a.delta, a.in_h) * a.in_w + cell_axis_pixel(i, a.delta, a.in_w);
+}
+
+// The cells of an offset's rows for the output row of a warp: all its lanes have the same y.
+struct PixelRows {
+    float yg;
+    int j0, nj;    // first cell row and their number; nj 0: none, -1: more than 8, or of more than two pixel rows
+    int iy0;       // lambda pixel row of cell row j0
+    unsigned up;   // bit dj: cell row j0 + dj lies in pixel row iy0 + 1
+};
+__device__ __forceinline__ PixelRows pixel_rows(const PixelwiseArgs &a, int y, float oy) {
+    PixelRows w;
+    w.yg = xg_of(y, a.inv_zoom, oy);
+    w.j0 = f2i_floor(FG_FDIV(FG_FSUB(w.yg, a.rm), a.delta));
+    const int j1 = f2i_floor(FG_FDIV(FG_FADD(w.yg, a.rm), a.delta));
+    w.nj = w.j0 > j1 ? 0 : (j1 - w.j0 >= 8 ? -1 : j1 - w.j0 + 1);
+    w.iy0 = cell_axis_pixel(w.j0, a.delta, a.in_h);
+    w.up = 0u;
+    for (int dj = 1; dj < w.nj; dj++) {
+        const int d = cell_axis_pixel(w.j0 + dj, a.delta, a.in_h) - w.iy0;
+        if (d > 1) w.nj = -1;
+        else if (d == 1) w.up |= 1u << dj;
+    }
+    return w;
 }
 
 // One cell of the reference's per-sample loop: does a grain of cell (i, j), whose lambda pixel has
@@ -125,279 +149,147 @@ static __device__ bool eval_regen(const PixelwiseArgs &a, const UniformF32 &U, f
     return false;
 }
 
+// A warp's queue of cells to regenerate (pixelwise_pixel_queue).
+struct RegenQueue {
+    uint2 e[64];        // ring: cell column; owner lane | sample << 5 | cell row - j0 << 10
+    unsigned hit[32];   // per sample of the current 32: the lanes whose sample is covered
+};
+
 // Hit count of output pixel (x, y) over its N samples by the reference's per-sample loop
 // (src/pixelwise.rs:30-38 around evaluate_indicator, src/pixelwise.rs:47-106), for sparse and
 // moderately dense grains.  Called by all 32 lanes of a warp (neighbouring pixels; `valid` false for
-// lanes past the row's end, which take part without samples); the lanes take the samples in step, and
-// each sample runs in two phases:
-//   1. every cell of its range gets the emptiness test alone (the first uniform against the Poisson
-//      threshold, cell_count_h): the same short work on every lane, one column hash per column; the
-//      non-empty cells go to a 64-bit mask, cell (i0 + di, j0 + dj) at bit di * 8 + dj with the middle
-//      cell swapped into bit 0;
-//   2. the (lane, non-empty cell) pairs of the whole warp are dealt out 32 at a time, each lane
-//      regenerating one cell's grains against its owner's sample and ORing a hit back to the owner.
-//      Lane-major order (kRankMajor false; sparse grains, few pairs): pair p goes to lane p % 32, which
-//      finds its owner by a shuffle binary search over the inclusive counts and the cell by a
-//      rank-select in the owner's mask (pairs of owners already covered are skipped).  Rank-major
-//      order (moderately dense grains): each round deals every uncovered lane's lowest pending cell,
-//      then their second cells, and so on, so that a sample covered by its middle cell drops out
-//      before the rest of its cells are dealt.
+// lanes past the row's end, which take part without samples); the lanes take the samples in step:
+//   1. every cell of a sample's range gets the emptiness screen alone (first_draw_maybe): the same short work
+//      on every lane, one column hash per column; the cells that may hold grains go to a 64-bit mask, cell
+//      (i0 + di, j0 + dj) at bit di * 8 + dj with the middle cell swapped into bit 0.  The rows of a sample
+//      (pixel_rows: two divisions, conversions for each row) are the same on every lane, so each lane
+//      computes them for one of 32 samples; a range lies in one lambda pixel, or straddles two on an axis
+//      (a conversion per cell, on the unit of 16 lanes a cycle, costs as much as the screen);
+//   2. rank by rank -- every lane's lowest pending cell, the middle one when it holds grains, then their next
+//      -- the lanes put their cells into the warp's queue, and whenever it holds 32 each lane regenerates
+//      one of them against its owner's sample.  What is left waits for the next sample's cells, so only
+//      the last round of 32 samples runs with idle lanes; a sample that turns out covered leaves its
+//      pending cells out.
 // Coverage is an OR over the cells, so neither the order nor the dealing changes it.  A range wider
-// than 8 cells on an axis (outside the plane-level choice of this path) runs the plain loop instead.
-template <bool kRankMajor>
-__device__ __forceinline__ uint32_t pixelwise_pixel_split(const PixelwiseArgs &a, const UniformF32 &U, int x, int y,
-                                                          bool valid) {
+// than 8 cells on an axis (outside the plane-level choice of this path) or than two lambda pixels runs the
+// plain loop instead.
+// What bounds it: the shifts, xors and multiplies of the screens' hashes and of the regenerated cells' draws.
+__device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a, const UniformF32 &U, int x, int y,
+                                                          bool valid, RegenQueue &Q) {
     if (!(a.rm > 0.0f)) return 0u;
     const int lane = threadIdx.x & 31;
     uint32_t hits = 0;
-    for (int k = 0; k < a.n; k++) {
-        float xg = 0.0f, yg = 0.0f;
-        int i0 = 0, j0 = 0, mid = 0;
-        unsigned long long m = 0ull;
-        bool hit = false;
-        if (valid) {
-            const float2 o = a.offs[k];
-            xg = xg_of(x, a.inv_zoom, o.x);
-            yg = xg_of(y, a.inv_zoom, o.y);
-            i0 = f2i_floor(FG_FDIV(FG_FSUB(xg, a.rm), a.delta));
-            const int i1 = f2i_floor(FG_FDIV(FG_FADD(xg, a.rm), a.delta));
-            j0 = f2i_floor(FG_FDIV(FG_FSUB(yg, a.rm), a.delta));
-            const int j1 = f2i_floor(FG_FDIV(FG_FADD(yg, a.rm), a.delta));
-            if (i0 <= i1 && j0 <= j1) {  // else no cell (src/pixelwise.rs:60-62)
-                const int ni = i1 - i0 + 1, nj = j1 - j0 + 1;
-                if (ni > 8 || nj > 8) {
-                    hit = eval_regen(a, U, xg, yg, i0, i1, j0, j1);
-                } else {
-                    // phase 1
-                    mid = ((ni - 1) >> 1) * 8 + ((nj - 1) >> 1);
-                    // (the screen may pass a cell whose seed words are all zero: phase 2 counts it exactly)
-                    long long pix = -1;
-                    uint64_t bound = 0;
-                    for (int di = 0; di < ni; di++) {
-                        const int i = i0 + di;
-                        const uint64_t colh = cell_col_hash(a.seed, i);
-                        for (int dj = 0; dj < nj; dj++) {
-                            const int j = j0 + dj;
-                            const long long p = cell_pixel(a, i, j);
-                            if (p != pix) {
-                                pix = p;
-                                bound = screen_bound(a.cells[p].thresh);
+    PixelRows rows = {0.0f, 0, 0, 0, 0u};
+    int head = 0, queued = 0;  // uniform
+    Q.hit[lane] = 0u;
+    __syncwarp();
+    for (int kb = 0; kb < a.n; kb += 32) {
+        const int nk = min(32, a.n - kb);
+        if (lane < nk) rows = pixel_rows(a, y, a.offs[kb + lane].y);
+        // the first `count` cells of the queue, one per lane
+        auto run = [&](int count) {
+            bool live = lane < count;
+            const uint2 e = Q.e[(head + (live ? lane : 0)) & 63];
+            const int owner = (int)(e.y & 31u), ks = (int)((e.y >> 5) & 31u), dj = (int)(e.y >> 10), i = (int)e.x;
+            const float yg = __shfl_sync(0xffffffffu, rows.yg, ks);
+            const int j = __shfl_sync(0xffffffffu, rows.j0, ks) + dj;
+            const unsigned up = __shfl_sync(0xffffffffu, rows.up, ks);
+            const int iy = __shfl_sync(0xffffffffu, rows.iy0, ks) + (int)((up >> dj) & 1u);
+            live = live && !((Q.hit[ks] >> owner) & 1u);
+            if (live) {
+                const float xg = xg_of(x - lane + owner, a.inv_zoom, a.offs[kb + ks].x);
+                const CellParam cp = a.cells[(long long)iy * a.in_w + cell_axis_pixel(i, a.delta, a.in_w)];
+                if (regen_cell(a, U, xg, yg, i, j, cell_col_hash(a.seed, i), cp)) atomicOr(&Q.hit[ks], 1u << owner);
+            }
+            __syncwarp();
+            head += count;
+            queued -= count;
+        };
+        for (int ks = 0; ks < nk; ks++) {
+            const int j0 = __shfl_sync(0xffffffffu, rows.j0, ks), nj = __shfl_sync(0xffffffffu, rows.nj, ks);
+            const int iy0 = __shfl_sync(0xffffffffu, rows.iy0, ks);
+            const unsigned up = __shfl_sync(0xffffffffu, rows.up, ks);
+            int i0 = 0, mid = 0;
+            unsigned long long m = 0ull;
+            if (valid && nj != 0) {  // nj == 0: no cell (src/pixelwise.rs:60-62)
+                const float xg = xg_of(x, a.inv_zoom, a.offs[kb + ks].x);
+                i0 = f2i_floor(FG_FDIV(FG_FSUB(xg, a.rm), a.delta));
+                const int i1 = f2i_floor(FG_FDIV(FG_FADD(xg, a.rm), a.delta));
+                const int ni = i1 - i0 + 1;
+                if (ni > 0) {
+                    const int ix0 = cell_axis_pixel(i0, a.delta, a.in_w), ix1 = cell_axis_pixel(i1, a.delta, a.in_w);
+                    if (ni > 8 || nj < 0 || ix1 - ix0 > 1) {
+                        const float yg = xg_of(y, a.inv_zoom, a.offs[kb + ks].y);
+                        if (eval_regen(a, U, xg, yg, i0, i1, f2i_floor(FG_FDIV(FG_FSUB(yg, a.rm), a.delta)),
+                                       f2i_floor(FG_FDIV(FG_FADD(yg, a.rm), a.delta))))
+                            atomicOr(&Q.hit[ks], 1u << lane);
+                    } else {
+                        mid = ((ni - 1) >> 1) * 8 + ((nj - 1) >> 1);
+                        const CellParam *row0 = a.cells + (long long)iy0 * a.in_w, *row1 = up ? row0 + a.in_w : row0;
+                        uint32_t b0 = maybe_bound(row0[ix0].thresh), b1 = maybe_bound(row1[ix0].thresh);
+                        int ix = ix0;
+                        for (int di = 0; di < ni; di++) {
+                            const int i = i0 + di;
+                            if (ix != ix1 && cell_axis_pixel(i, a.delta, a.in_w) == ix1) {
+                                ix = ix1;
+                                b0 = maybe_bound(row0[ix1].thresh);
+                                b1 = maybe_bound(row1[ix1].thresh);
                             }
-                            const int idx = di * 8 + dj;
-                            const int pos = idx == mid ? 0 : (idx == 0 ? mid : idx);
-                            if (first_draw_screen(cell_row_hash(colh, j), bound)) m |= 1ull << pos;
+                            const uint64_t colh = cell_col_hash(a.seed, i);
+                            unsigned col = 0u;
+                            for (int dj = 0; dj < nj; dj++)
+                                col |= (first_draw_maybe(cell_row_hash(colh, j0 + dj), ((up >> dj) & 1u) ? b1 : b0) ? 1u : 0u)
+                                       << dj;
+                            m |= (unsigned long long)col << (8 * di);
                         }
+                        // the middle cell and cell (0, 0) change places
+                        const unsigned long long d = (m ^ (m >> mid)) & 1ull;
+                        m ^= d | (d << mid);
                     }
                 }
             }
-        }
-        if (kRankMajor) {
-            // phase 2: the warp's pairs, 32 per round in rank-major order: first every uncovered lane's
-            // lowest pending cell (the middle one when it holds grains), then their second cells, and so
-            // on, so that a covered sample drops out before its further cells are dealt.
+            __syncwarp();
             for (;;) {
-                const bool live = m != 0ull && !hit;
-                const int mine = live ? __popcll((long long)m) : 0;
-                int owner = -1, rank = 0, before = 0, assigned = 0;
-                for (int r = 0; before < 32; r++) {
-                    const unsigned mask_r = __ballot_sync(0xffffffffu, mine > r);
-                    const int c = __popc(mask_r);
-                    if (c == 0) break;
-                    if (mine > r && before + __popc(mask_r & ((1u << lane) - 1u)) < 32) assigned++;
-                    if (owner < 0 && lane < before + c) {
-                        // the (lane - before)-th set bit of mask_r
-                        int q = lane - before, bit = 0;
-                        unsigned w = mask_r;
-#pragma unroll
-                        for (int half = 16; half > 0; half >>= 1) {
-                            const int cl = __popc(w & ((1u << half) - 1u));
-                            if (q >= cl) {
-                                q -= cl;
-                                bit += half;
-                                w >>= half;
-                            }
-                        }
-                        owner = bit;
-                        rank = r;
-                    }
-                    before += c;
+                const unsigned pending = __ballot_sync(0xffffffffu, m != 0ull);
+                if (pending == 0u) break;
+                if (m != 0ull) {
+                    const int pos = __ffsll((long long)m) - 1;
+                    m &= m - 1ull;
+                    const int idx = pos == 0 ? mid : (pos == mid ? 0 : pos);
+                    Q.e[(head + queued + __popc(pending & ((1u << lane) - 1u))) & 63] =
+                        make_uint2((unsigned)(i0 + (idx >> 3)),
+                                   (unsigned)lane | ((unsigned)ks << 5) | ((unsigned)(idx & 7) << 10));
                 }
-                if (before == 0) break;  // no lane has a pending cell
-                const int src = owner < 0 ? 0 : owner;
-                const unsigned mlo = __shfl_sync(0xffffffffu, (unsigned)m, src);
-                const unsigned mhi = __shfl_sync(0xffffffffu, (unsigned)(m >> 32), src);
-                const float sx = __shfl_sync(0xffffffffu, xg, src), sy = __shfl_sync(0xffffffffu, yg, src);
-                const int si0 = __shfl_sync(0xffffffffu, i0, src), sj0 = __shfl_sync(0xffffffffu, j0, src);
-                const int smid = __shfl_sync(0xffffffffu, mid, src);
-                bool h = false;
-                if (owner >= 0) {
-                    // the rank-th set bit of the owner's pending mask
-                    int r = rank;
-                    unsigned word = mlo;
-                    int base = 0;
-                    const int c = __popc(mlo);
-                    if (r >= c) {
-                        r -= c;
-                        word = mhi;
-                        base = 32;
-                    }
-                    int bit = 0;
-#pragma unroll
-                    for (int half = 16; half > 0; half >>= 1) {
-                        const int cl = __popc(word & ((1u << half) - 1u));
-                        if (r >= cl) {
-                            r -= cl;
-                            bit += half;
-                            word >>= half;
-                        }
-                    }
-                    const int pos = base + bit;
-                    const int idx = pos == 0 ? smid : (pos == smid ? 0 : pos);
-                    const int i = si0 + (idx >> 3), j = sj0 + (idx & 7);
-                    h = regen_cell(a, U, sx, sy, i, j, cell_col_hash(a.seed, i), a.cells[cell_pixel(a, i, j)]);
+                queued += __popc(pending);
+                __syncwarp();
+                if (queued >= 32) {
+                    run(32);
+                    if ((Q.hit[ks] >> lane) & 1u) m = 0ull;
                 }
-                const unsigned hm = __reduce_or_sync(0xffffffffu, h ? (1u << src) : 0u);
-                hit = hit || ((hm >> lane) & 1u) != 0u;
-                for (int t = 0; t < assigned; t++) m &= m - 1ull;  // this round dealt the lowest `assigned` cells
-            }
-        } else {
-            // phase 2: the warp's pairs, 32 at a time in lane-major order
-            const int cnt = __popcll((long long)m);
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int tot = __shfl_sync(0xffffffffu, incl, 31);
-            for (int b = 0; b < tot; b += 32) {
-                const int p = b + lane;
-                int src = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int v = __shfl_sync(0xffffffffu, incl, src + step - 1);
-                    if (v <= p) src += step;
-                }
-                src = min(src, 31);
-                int r = p - (__shfl_sync(0xffffffffu, incl, src) - __shfl_sync(0xffffffffu, cnt, src));
-                const unsigned mlo = __shfl_sync(0xffffffffu, (unsigned)m, src);
-                const unsigned mhi = __shfl_sync(0xffffffffu, (unsigned)(m >> 32), src);
-                const bool done = __shfl_sync(0xffffffffu, hit ? 1 : 0, src) != 0;
-                const float sx = __shfl_sync(0xffffffffu, xg, src), sy = __shfl_sync(0xffffffffu, yg, src);
-                const int si0 = __shfl_sync(0xffffffffu, i0, src), sj0 = __shfl_sync(0xffffffffu, j0, src);
-                const int smid = __shfl_sync(0xffffffffu, mid, src);
-                bool h = false;
-                if (p < tot && !done) {
-                    // the r-th set bit of the owner's mask
-                    unsigned word = mlo;
-                    int base = 0;
-                    const int c = __popc(mlo);
-                    if (r >= c) {
-                        r -= c;
-                        word = mhi;
-                        base = 32;
-                    }
-                    int bit = 0;
-#pragma unroll
-                    for (int half = 16; half > 0; half >>= 1) {
-                        const int cl = __popc(word & ((1u << half) - 1u));
-                        if (r >= cl) {
-                            r -= cl;
-                            bit += half;
-                            word >>= half;
-                        }
-                    }
-                    const int pos = base + bit;
-                    const int idx = pos == 0 ? smid : (pos == smid ? 0 : pos);
-                    const int i = si0 + (idx >> 3), j = sj0 + (idx & 7);
-                    h = regen_cell(a, U, sx, sy, i, j, cell_col_hash(a.seed, i), a.cells[cell_pixel(a, i, j)]);
-                }
-                const unsigned hm = __reduce_or_sync(0xffffffffu, h ? (1u << src) : 0u);
-                hit = hit || ((hm >> lane) & 1u) != 0u;
             }
         }
-        hits += hit ? 1u : 0u;
-    }
-    return hits;
-}
-
-// The same hit count for dense grains, where most samples are covered by the first cells they
-// visit: the loop is flattened so that each iteration visits ONE cell of the current sample and a
-// lane moves on to its next sample as soon as the current one is decided.  Each sample visits its
-// middle cell first, then the rest of its range column by column.
-__device__ __forceinline__ uint32_t pixelwise_pixel_flat(const PixelwiseArgs &a, const UniformF32 &U, int x,
-                                                         int y) {
-    if (!(a.rm > 0.0f)) return 0u;
-    uint32_t hits = 0;
-    int k = 0;
-    float xg = 0.0f, yg = 0.0f;
-    int i0 = 0, j0 = 0, ni = 0, nj = 0, ic = 0, jc = 0, ri = 0, rj = 0;
-    bool active = false, first = false;
-    int col_i = 0;
-    bool have_col = false;
-    uint64_t colh = 0;
-    long long pix = -1;
-    CellParam cp;
-    cp.thresh = 0; cp.exp_lambda = 0.0;
-    while (true) {
-        if (!active) {
-            if (k >= a.n) break;
-            const float2 o = a.offs[k];
-            xg = xg_of(x, a.inv_zoom, o.x);
-            yg = xg_of(y, a.inv_zoom, o.y);
-            i0 = f2i_floor(FG_FDIV(FG_FSUB(xg, a.rm), a.delta));
-            const int i1 = f2i_floor(FG_FDIV(FG_FADD(xg, a.rm), a.delta));
-            j0 = f2i_floor(FG_FDIV(FG_FSUB(yg, a.rm), a.delta));
-            const int j1 = f2i_floor(FG_FDIV(FG_FADD(yg, a.rm), a.delta));
-            if (i0 > i1 || j0 > j1) {  // src/pixelwise.rs:60-62
-                k++;
-                continue;
-            }
-            ni = i1 - i0 + 1;
-            nj = j1 - j0 + 1;
-            ic = (ni - 1) >> 1;
-            jc = (nj - 1) >> 1;
-            ri = 0; rj = 0;
-            first = true;
-            active = true;
-        }
-        const int i = i0 + (first ? ic : ri), j = j0 + (first ? jc : rj);
-        if (!have_col || i != col_i) {
-            col_i = i;
-            have_col = true;
-            colh = cell_col_hash(a.seed, i);
-        }
-        const long long p = cell_pixel(a, i, j);
-        if (p != pix) {
-            pix = p;
-            cp = a.cells[p];
-        }
-        const bool hit = regen_cell(a, U, xg, yg, i, j, colh, cp);
-        if (first) {
-            first = false;
-        } else if (++rj == nj) {
-            rj = 0;
-            ++ri;
-        }
-        if (ri == ic && rj == jc && ++rj == nj) {  // the middle cell went first: skip it
-            rj = 0;
-            ++ri;
-        }
-        if (hit || ri >= ni) {
-            hits += hit ? 1u : 0u;
-            k++;
-            active = false;
+        if (queued > 0) run(queued);
+        // word ks holds sample ks's lanes: lane b counts the words with bit b
+        const unsigned w = Q.hit[lane];
+        __syncwarp();
+        Q.hit[lane] = 0u;
+        for (int b = 0; b < 32; b++) {
+            const unsigned c = __ballot_sync(0xffffffffu, (w >> b) & 1u);
+            if (lane == b) hits += __popc(c);
         }
     }
     return hits;
 }
 
 // The per-sample path for the kPwRegenThreads pixels [x0, x0 + kPwRegenThreads) of row y (one per
-// thread of the CTA): each warp (32 neighbouring pixels) votes on its pixels' expected grains per cell
-// λδ² and takes the flattened form when most exceed kPwRegenFlatLd, the rank-major two-phase form when
-// most exceed kPwRegenRankLd, else the lane-major two-phase form, and writes the hit counts.  Thread 0 adds the CTA's samples and the CTA to the diagnostics
-// (regenerated samples, unstaged blocks, blocks).
+// thread of the CTA).  Thread 0 adds the CTA's samples and the CTA to the diagnostics (regenerated samples,
+// unstaged blocks, blocks).
+// One form for every density.  Before it, warps went by their grains per cell: cells dealt sample by sample
+// (lane- or rank-major), where a sample of 32 lanes left its last round of 32 cells half empty, and above 1.1 a
+// loop that visited one cell at a time.  GB300, radius 0.025, N 64: 1021 x 763 blobs 4.03 -> 2.82 ms,
+// 700 x 500 ramp 3.09 -> 1.86 ms (1.94 with the loop kept above 1.1).
 __device__ __forceinline__ void pixelwise_regen_pixels(const PixelwiseArgs &a, int x0, int y) {
+    __shared__ RegenQueue queues[kPwRegenThreads / 32];
     const int x = x0 + (int)threadIdx.x;
     if (threadIdx.x == 0) {
         const int px = min(kPwRegenThreads, a.out_w - x0);
@@ -405,24 +297,10 @@ __device__ __forceinline__ void pixelwise_regen_pixels(const PixelwiseArgs &a, i
         atomicAdd(&a.diag[1], 1ull);
         atomicAdd(&a.diag[3], 1ull);
     }
-    float ld = 0.0f;  // expected grains per cell at this pixel
-    if (x < a.out_w) {
-        const int xi = min(a.in_w - 1, max(0, (int)floorf(((float)x + 0.5f) * a.inv_zoom)));
-        const int yi = min(a.in_h - 1, max(0, (int)floorf(((float)y + 0.5f) * a.inv_zoom)));
-        ld = a.lam[(long long)yi * a.in_w + xi] * a.delta * a.delta;
-    }
-    const bool flat = __popc(__ballot_sync(0xffffffffu, ld > kPwRegenFlatLd)) >= 16;
-    const bool rank_major = __popc(__ballot_sync(0xffffffffu, ld > kPwRegenRankLd)) >= 16;
     const bool valid = x < a.out_w;
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
-    if (flat) {
-        if (!valid) return;
-        a.out[(long long)y * a.out_w + x] = (float)pixelwise_pixel_flat(a, U, x, y);
-    } else {
-        const uint32_t hits = rank_major ? pixelwise_pixel_split<true>(a, U, x, y, valid)    // all 32 lanes
-                                         : pixelwise_pixel_split<false>(a, U, x, y, valid);
-        if (valid) a.out[(long long)y * a.out_w + x] = (float)hits;
-    }
+    const uint32_t hits = pixelwise_pixel_queue(a, U, x, y, valid, queues[threadIdx.x >> 5]);  // all 32 lanes
+    if (valid) a.out[(long long)y * a.out_w + x] = (float)hits;
 }
 
 // Block-wide exclusive scan of one int per thread (any blockDim.x that is a multiple of 32, <= 1024).
@@ -651,7 +529,8 @@ __device__ __forceinline__ bool pixelwise_block(const PixelwiseArgs &a, int root
                 const int lane = tid & 31;
                 int ci = c0 / (int)Hc, cj = c0 % (int)Hc;
                 int col = -1, pix = -1;
-                uint64_t colh = 0, bound = 0;
+                uint64_t colh = 0;
+                uint32_t bound = 0;
                 const bool from_mask = a.cellmask != nullptr && wi0 >= a.cm_gi0 &&
                                        wi0 + (int)Wc <= a.cm_gi0 + a.cm_gw && wj0 >= a.cm_gj0 &&
                                        wj0 + (int)Hc <= a.cm_gj0 + 32 * a.cm_ghw;
@@ -679,11 +558,11 @@ __device__ __forceinline__ bool pixelwise_block(const PixelwiseArgs &a, int root
                             const int p = S.rowiy[cj] * a.in_w + S.colix[ci];
                             if (p != pix) {
                                 pix = p;
-                                bound = screen_bound(a.cells[p].thresh);
+                                bound = maybe_bound(a.cells[p].thresh);
                             }
-                            nonempty = first_draw_screen(cell_row_hash(colh, wj0 + cj), bound);
+                            nonempty = first_draw_maybe(cell_row_hash(colh, wj0 + cj), bound);
                         }
-                        // (a cell whose seed words are all zero may pass: A2 counts it exactly)
+                        // (an empty cell may pass: A2 counts it exactly)
                         if (!nonempty) S.pre[rc] = 0;
                         if (++cj == (int)Hc) {
                             cj = 0;

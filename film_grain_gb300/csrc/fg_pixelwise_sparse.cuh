@@ -129,74 +129,45 @@ struct PwSparseGrid {
     float gm_grain_cost, gm_sample_cost;  // modelled instructions per staged grain / per owned sample
 };
 
-// The plane's emptiness bitmask (step 0): thread t = (word row k = t / gw, column c = t % gw).
-__device__ __forceinline__ void cell_mask_word(const PixelwiseArgs &a, const PwSparseGrid &g, long long t,
+// The plane's emptiness bitmask (step 0): word (column c, word row k), the lanes of a warp taking neighbouring
+// columns of one word row (all 32 lanes; those past the last column write nothing).
+// What bounds it: the shifts, xors and multiplies of the row hash and the screen, once per cell.
+__device__ __forceinline__ void cell_mask_word(const PixelwiseArgs &a, const PwSparseGrid &g, int c, int k,
                                                unsigned int *cellmask) {
-    const int c = (int)(t % g.gw), k = (int)(t / g.gw);
-    const int i = g.gi0 + c;
+    const int i = g.gi0 + c, jb = g.gj0 + 32 * k, lane = (int)(threadIdx.x & 31);
     const uint64_t colh = cell_col_hash(a.seed, i);
-    // the cell's lambda pixel, clamped to the plane (cell_pixel); cell coordinates stay far inside int,
-    // so the clamp is done on floats and the conversion is a 32-bit one
-    const int ix = (int)fminf(fmaxf(floorf(FG_FMUL((float)i, a.delta)), 0.0f), (float)(a.in_w - 1));
-    auto iy_of = [&](int j) {
-        return (int)fminf(fmaxf(floorf(FG_FMUL((float)j, a.delta)), 0.0f), (float)(a.in_h - 1));
-    };
-    const int jb = g.gj0 + 32 * k;
-    // iy_of is nondecreasing in j (rounding and floor are monotone), so the word's 32 rows take at most
-    // a few pixel rows: one when the first and last agree, two when they differ by one (the boundary
-    // found by bisection); otherwise each row is looked up
-    const int iy0 = iy_of(jb), iy1 = iy_of(jb + 31);
-    const long long t0 = a.cells[(long long)iy0 * a.in_w + ix].thresh;
+    const CellParam *cells = a.cells + cell_axis_pixel(i, a.delta, a.in_w);
+    // the word's 32 rows have the same lambda pixel rows on every lane: lane r converts row r, and the
+    // rows where a new one starts cut the word into runs
+    const int iy = cell_axis_pixel(jb + lane, a.delta, a.in_h);
+    const int above = __shfl_up_sync(0xffffffffu, iy, 1);  // lane 0: its own
+    const unsigned starts = __ballot_sync(0xffffffffu, iy != above);
     // The row stage of mix3 is fmix64(rotl64(col + j, 41) + phi).  With base = col + jb, when adding
     // r < 32 carries nothing out of base's low 23 bits, rotl64(base + r, 41) = rotl64(base, 41) + r * 2^41,
     // so the row hash's input is one constant plus r * 2^41 (only its high word changes); a word whose
     // rows would carry (31 in 2^23) takes the row hash as is.
     const uint64_t base = colh + (uint64_t)(int64_t)jb;
     const uint64_t c0 = rotl64(base, 41) + kPhi;
-    auto scan = [&](auto row_hash) {
-        unsigned int word = 0;
-        if (iy1 <= iy0 + 1) {
-            int rb = 32;  // first row of pixel row iy1
-            long long t1 = t0;
-            if (iy1 != iy0) {
-                int lo = 1, hi = 31;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (iy_of(jb + mid) == iy1) hi = mid;
-                    else lo = mid + 1;
-                }
-                rb = lo;
-                t1 = a.cells[(long long)iy1 * a.in_w + ix].thresh;
-            }
-            // the first-draw test as first_draw_screen: a cell whose seed words are all zero is listed and
-            // counted exactly by the sparse pass (sparse_cell_count)
-            auto bit = [&](int r, uint64_t m) -> unsigned { return (first_draw_screen(row_hash(r), m) ? 1u : 0u) << r; };
-            // rows before rb take pixel row iy0's threshold, the others iy1's
-            const uint64_t m0 = screen_bound(t0), m1 = screen_bound(t1);
+    const bool plain = (base & 0x7FFFFFull) <= 0x7FFFFFull - 31;
+    unsigned int word = 0;
+    for (int r0 = 0; r0 < 32;) {
+        const unsigned later = starts & (r0 < 31 ? ~0u << (r0 + 1) : 0u);
+        const int r1 = later ? __ffs(later) - 1 : 32;
+        const uint32_t bound = maybe_bound(cells[(long long)__shfl_sync(0xffffffffu, iy, r0) * a.in_w].thresh);
+        // the few empty cells that the screen lists are counted exactly by the passes that read the
+        // bitmask (sparse_cell_count, cell_count_h)
+        if (plain) {
 #pragma unroll 4
-            for (int r = 0; r < rb; r++) word |= bit(r, m0);
-#pragma unroll 4
-            for (int r = rb; r < 32; r++) word |= bit(r, m1);
+            for (int r = r0; r < r1; r++)
+                word |= (first_draw_maybe(fmix64(c0 + ((uint64_t)r << 41)), bound) ? 1u : 0u) << r;
         } else {
-            int iy_prev = iy0;
-            long long thresh = t0;
-#pragma unroll 4
-            for (int r = 0; r < 32; r++) {
-                const int iy = iy_of(jb + r);
-                if (iy != iy_prev) {
-                    iy_prev = iy;
-                    thresh = a.cells[(long long)iy * a.in_w + ix].thresh;
-                }
-                const long long v = (long long)(small_first_u64(row_hash(r)) >> 11);
-                word |= (v > thresh ? 1u : 0u) << r;
-            }
+            for (int r = r0; r < r1; r++)
+                word |= (first_draw_maybe(cell_row_hash(colh, jb + r), bound) ? 1u : 0u) << r;
         }
-        return word;
-    };
-    const unsigned int word = (base & 0x7FFFFFull) <= 0x7FFFFFull - 31
-                                  ? scan([&](int r) { return fmix64(c0 + ((uint64_t)r << 41)); })
-                                  : scan([&](int r) { return cell_row_hash(colh, jb + r); });
-    cellmask[t] = word;
+        __syncwarp();
+        r0 = r1;
+    }
+    if (c < g.gw) cellmask[(long long)k * g.gw + c] = word;
 }
 
 // The reference's per-sample loop for a sample the staged window cannot serve (out of line: rare).

@@ -186,6 +186,24 @@ FG_HD bool first_draw_screen(uint64_t h, uint64_t bound) {
     const uint64_t s3 = pcg_pair(pcg_word<7>(h), pcg_word<8>(h));
     return rotl64(s0 + s3, 23) + s0 - 1ull >= bound;
 }
+// The same screen from seed words 2 and 8 alone, which passes every cell that first_draw_screen passes and,
+// of the others, about one in 2^8.  The high word of r1 is
+//   (((w2 + w8) << 23) + w2) + (c1 << 23) + ((w1 + w7) >> 9) + c2   (mod 2^32)
+// with carries c1, c2 in {0, 1}: the bracket plus at most 2^24.  So r1 - 1 >= bound implies that the
+// bracket is at least (bound >> 32) - 2^24 (a bracket that would pass 2^32 is above that too), and an
+// all-zero seed has bracket 0: the comparison of the bracket minus one holds for both.  Half of the
+// seed words and no 64-bit sums: 41 instructions a cell instead of 73, and the pipes that the shifts,
+// xors and multiplies share are what bounds a screen.
+FG_HD uint32_t maybe_bound(long long thresh) {
+    if (thresh < 0) return 0u;
+    if (thresh >= (1ll << 53) - 1) return ~0u;  // passes a bracket of 0 alone
+    const uint32_t hi = (uint32_t)(((((uint64_t)thresh + 1ull) << 11) - 1ull) >> 32);
+    return hi > (1u << 24) ? hi - (1u << 24) - 1u : 0u;
+}
+FG_HD bool first_draw_maybe(uint64_t h, uint32_t bound) {
+    const uint32_t w2 = pcg_word<2>(h), w8 = pcg_word<8>(h);
+    return ((w2 + w8) << 23) + w2 - 1u >= bound;
+}
 // src/rng.rs:26-29 / 31-34
 FG_HD Xoshiro cell_rng(uint64_t seed, int32_t i, int32_t j) { return small_seed(mix3(seed, kCellStream, i, j)); }
 FG_HD Xoshiro pixel_rng(uint64_t seed, int32_t i, int32_t j) { return small_seed(mix3(seed, kPixelStream, i, j)); }

@@ -292,3 +292,16 @@ def test_grainwise_lane_groups_and_queue(cuda, fgl, orc, w, h, zoom, radius, n, 
     plane = workloads.ramp_noise(w, h, 5)
     _check("grain", fgl, orc, plane, radius=radius, n=n, zoom=zoom, dist=dist, sd=0.4 * radius if dist == "lognorm" else 0.0,
            seed=41)
+
+
+@pytest.mark.parametrize("w,h,radius,cell,zoom,n", [
+    (41, 37, 0.02, None, 1.0, 33),    # per-sample kernel: rows of one lambda pixel and of two, two batches of 32
+    (37, 29, 0.05, 0.31, 1.3, 5),     # three or four cells to a pixel, runs of a word's rows of three
+    (70, 45, 0.45, 0.29, 0.5, 8),     # ranges over two pixels and more
+    (64, 33, 0.4, 1.0, 1.0, 64),      # a lambda pixel row for every row of a bitmask word
+    (300, 9, 0.3, 1.7, 1.0, 48),      # pixel rows left out between cell rows, more columns than a CTA
+    (33, 70, 0.11, 0.07, 2.0, 100),   # runs that end inside a word
+])
+def test_pixelwise_screened_cells(cuda, fgl, orc, w, h, radius, cell, zoom, n):
+    """The lambda pixels of a cell column's rows: in the plane's bitmask and in the per-sample kernel."""
+    _check("pixel", fgl, orc, _blobs(w, h), radius=radius, cell=cell, zoom=zoom, n=n, seed=13)

@@ -56,6 +56,17 @@ def test_bitmask_screen_and_row_hash_identities(tmp_path):
     assert checked2 > 6000000 and bad2 == 0
 
 
+def test_screen_by_two_seed_words_misses_no_cell(tmp_path):
+    """first_draw_maybe passes every cell that first_draw_screen passes, and few others: its bracket is below
+    the first output by at most 2^24 of 2^32, so at most one in 2^8 of all cells, and half that on average
+    over the carry and the low words (8 standard deviations of slack on 1.8 million cells: 2^-7)."""
+    exe = _compile("maybe_check.cpp", "maybe_check", tmp_path)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()
+    checked, missed, checked2, extra = (int(v) for v in out)
+    assert checked == 200000 * 18 and missed == 0
+    assert checked2 == 200000 * 9 and 0 < extra < checked2 / 128
+
+
 def test_samplers_on_32_bit_pipes_match_f64_samplers(tmp_path):
     """poisson_count, knuth_count_f32 and lognormal_radius_f32 give the f64 samplers' values and stream
     positions on every stream (both Poisson regimes and the ends of the f32 rejection's range, cell

@@ -56,6 +56,15 @@ constexpr float kPwRegenDense = 0.4f;
 // 2.7 3.66 against 3.63; radius 0.07: N 64 at 2.6 1.92 against 1.96), blobs at 2.1 (2.29 against 2.27).
 constexpr int kPwRegenThreads = 256;
 constexpr float kPwRegenKernel = 2.05f;
+// Small planes on their own (pixelwise_takes_regen): below kPwRegenSmallVisits cell visits and kPwRegenSmall
+// windows.  Ramps of radius 0.1 and 0.2 on the per-sample kernel against the block passes, us of a whole call:
+// 96 x 64 N 32 (1.8 million visits) 116 / 257, N 64 119 / 301, 160 x 120 N 64 (11 million) 183 / 385, 256 x 256
+// N 64 (38 million) 458 / 550.  The line lies well below where the two meet, so that the small planes on which
+// the tests hold the block passes against the oracle stay with them.  kPwRegenWarps: the warps per SM below
+// which the kernel splits the samples (96 x 64 N 32 without the split: 226 us).
+constexpr double kPwRegenSmallVisits = 4.5e6;
+constexpr float kPwRegenSmall = 5.0f;
+constexpr double kPwRegenWarps = 32.0;
 // In-launch cancellation: `cancel` is null or two words of mapped pinned host memory.  Word 0 is set
 // by the waiting host thread once the caller's cancel flag turns non-zero; the persistent passes
 // read it once per work item they pull (the block passes once per block) and stop, and a CTA that
@@ -154,9 +163,9 @@ cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta
 cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsigned int *cellmask, cudaStream_t s);
 // Scratch bytes of the sparse pass's plane bitmask for this plane; 0 when the plane does not take it.
 size_t pixelwise_cellmask_bytes(const PixelwiseArgs &a, int nby);
-// Whether a plane runs on the per-sample kernel instead of the block kernel, and its launch.
+// Whether a plane runs on the per-sample kernel instead of the block kernel: in a batch, and on its own.
 bool pixelwise_prefers_regen(const PixelwiseArgs &a);
-cudaError_t launch_pixelwise_regen(const PixelwiseArgs &a, cudaStream_t s);
+bool pixelwise_takes_regen(const PixelwiseArgs &a);
 size_t pixelwise_smem_bytes();  // the fat configuration (the batched kernel's pixel-wise items)
 cudaError_t launch_grainwise(const GrainwiseArgs &a, int sms, cudaStream_t s);
 size_t grainwise_smem_bytes(const GrainwiseArgs &a);

@@ -230,7 +230,7 @@ static size_t sparse_gm_idx_at(const PwSparseGrid &g, int n) {
 }
 
 size_t pixelwise_cellmask_bytes(const PixelwiseArgs &a, int nby) {
-    if (pixelwise_prefers_regen(a)) return 0;
+    if (pixelwise_takes_regen(a)) return 0;
     PwSparseGrid g;
     const int sms = sm_count();  // without a device (planning only): the GB300's 152
     if (!plan_sparse(a, nby, sms > 0 ? sms : 152, &g)) return 0;
@@ -286,40 +286,64 @@ __global__ void __launch_bounds__(PwFat::kThreads, PwFat::kCtasPerSm)
     }
 }
 
-// Per-sample kernel: one thread per output pixel (pixelwise_regen_pixels); no shared memory, no
-// barriers.  CTA b covers pixels [256 (b % row_ctas), +256) of row b / row_ctas.
+// Per-sample kernel: one thread per output pixel and part of its samples (pixelwise_regen_pixels); no barriers.
+// CTA b covers pixels [256 (c % row_ctas), +256) of row c / row_ctas, c = b / parts, and samples
+// [per (b % parts), +per).
 __global__ void __launch_bounds__(kPwRegenThreads) pixelwise_regen_kernel(const __grid_constant__ PixelwiseArgs a,
-                                                                          int row_ctas) {
+                                                                          int row_ctas, int parts, int per) {
     if (a.cancel) {  // once per warp: the warp's lanes work in step, so the whole warp stops
         int stop = 0;
         if ((threadIdx.x & 31) == 0) stop = cancel_requested(a.cancel) ? 1 : 0;
         if (__shfl_sync(0xffffffffu, stop, 0)) return;
     }
-    pixelwise_regen_pixels(a, (int)(blockIdx.x % (unsigned)row_ctas) * kPwRegenThreads,
-                           (int)(blockIdx.x / (unsigned)row_ctas));
+    const unsigned c = blockIdx.x / (unsigned)parts;
+    const int k0 = (int)(blockIdx.x % (unsigned)parts) * per;
+    pixelwise_regen_pixels(a, (int)(c % (unsigned)row_ctas) * kPwRegenThreads, (int)(c / (unsigned)row_ctas), k0,
+                           min(a.n, k0 + per));
 }
 
-bool pixelwise_prefers_regen(const PixelwiseArgs &a) {
-    if (!(a.rm > 0.0f)) return true;  // nothing can cover a sample: the per-sample loop exits at once
-    // a sample's range must fit the 64-bit cell mask of pixelwise_pixel
+// The reach of an interior root block's samples, in windows of cells; infinite where the per-sample kernel cannot
+// take the plane, 0 where it has nothing to do.
+static double regen_reach(const PixelwiseArgs &a) {
+    if (!(a.rm > 0.0f)) return 0.0;  // nothing can cover a sample: the per-sample loop exits at once
+    // a sample's range must fit the 64-bit cell mask of pixelwise_pixel_queue
     const double axis = std::floor(2.0 * (double)a.rm / (double)a.delta) + 2.0;
-    if (!(axis * axis <= 64.0)) return false;
+    if (!(axis * axis <= 64.0)) return HUGE_VAL;
     // cell indices of every sample must stay far inside int (the range arithmetic)
     const double reach = (double)std::max(a.out_w, a.out_h) / a.zoom +
                          std::max({std::fabs(a.offx_min), std::fabs(a.offx_max), std::fabs(a.offy_min),
                                    std::fabs(a.offy_max)}) + a.rm + 2.0;
-    if (reach / a.delta > 1.0e9) return false;
+    if (reach / a.delta > 1.0e9) return HUGE_VAL;
     // an interior root block: its samples' reach in cells against its staged window
     const double samples = (double)a.bsize * a.bsize * a.zoom * a.zoom * a.n;
     const double edge = std::floor((a.bsize + 2.0 * a.rm) / a.delta) + 1.0;
-    return samples * a.regen_cells < kPwRegenKernel * edge * edge;
+    return samples * a.regen_cells / (edge * edge);
 }
 
-cudaError_t launch_pixelwise_regen(const PixelwiseArgs &a, cudaStream_t s) {
+bool pixelwise_prefers_regen(const PixelwiseArgs &a) { return regen_reach(a) < kPwRegenKernel; }
+
+// The planes that one render gives to the per-sample kernel: besides the ones of pixelwise_prefers_regen, small
+// ones, whose block passes are a chain of a few CTAs' latencies (bitmask, sparse blocks, the dense blocks left
+// over) while the per-sample kernel spreads their samples over the chip.
+bool pixelwise_takes_regen(const PixelwiseArgs &a) {
+    if (pixelwise_prefers_regen(a)) return true;
+    const double visits = (double)a.out_w * a.out_h * a.n * a.regen_cells;
+    return visits < kPwRegenSmallVisits && regen_reach(a) < kPwRegenSmall;
+}
+
+static cudaError_t launch_pixelwise_regen(const PixelwiseArgs &a, cudaStream_t s) {
     const long long row_ctas = (a.out_w + kPwRegenThreads - 1) / kPwRegenThreads;
     const long long grid = row_ctas * a.out_h;
     if (grid <= 0) return cudaSuccess;
-    pixelwise_regen_kernel<<<(unsigned)grid, kPwRegenThreads, 0, s>>>(a, (int)row_ctas);
+    // A warp alone on its scheduler takes 3.6 us a sample, most of it waiting: with fewer warps than
+    // kPwRegenWarps per SM the samples are split, into parts of four and more (each part ends with a round
+    // of less than 32 cells).
+    const int sms = sm_count();
+    const double warps = (double)((a.out_w + 31) / 32) * a.out_h;
+    const double want = warps > 0 ? kPwRegenWarps * (double)std::max(1, sms) / warps : 1.0;
+    const int per = std::max(4, (int)std::ceil(a.n / std::max(1.0, want)));
+    const int parts = (a.n + per - 1) / per;
+    pixelwise_regen_kernel<<<(unsigned)(grid * parts), kPwRegenThreads, 0, s>>>(a, (int)row_ctas, parts, per);
     return cudaGetLastError();
 }
 
@@ -329,7 +353,7 @@ static cudaError_t set_smem(K k, size_t smem) {
 }
 
 cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsigned int *cellmask, cudaStream_t s) {
-    if (pixelwise_prefers_regen(a)) return launch_pixelwise_regen(a, s);
+    if (pixelwise_takes_regen(a)) return launch_pixelwise_regen(a, s);
     const size_t lean_smem = sizeof(PwShared<PwLean>), fat_smem = sizeof(PwShared<PwFat>);
     cudaError_t e = set_smem(pixelwise_kernel<PwLean>, lean_smem);
     if (e == cudaSuccess) e = set_smem(pixelwise_kernel<PwFat>, fat_smem);

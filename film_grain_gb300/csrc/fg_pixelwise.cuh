@@ -155,9 +155,8 @@ struct RegenQueue {
     unsigned hit[32];   // per sample of the current 32: the lanes whose sample is covered
 };
 
-// Hit count of output pixel (x, y) over its N samples by the reference's per-sample loop
-// (src/pixelwise.rs:30-38 around evaluate_indicator, src/pixelwise.rs:47-106), for sparse and
-// moderately dense grains.  Called by all 32 lanes of a warp (neighbouring pixels; `valid` false for
+// Hit count of output pixel (x, y) over its samples [k0, k1) by the reference's per-sample loop
+// (src/pixelwise.rs:30-38 around evaluate_indicator, src/pixelwise.rs:47-106).  Called by all 32 lanes of a warp (neighbouring pixels; `valid` false for
 // lanes past the row's end, which take part without samples); the lanes take the samples in step:
 //   1. every cell of a sample's range gets the emptiness screen alone (first_draw_maybe): the same short work
 //      on every lane, one column hash per column; the cells that may hold grains go to a 64-bit mask, cell
@@ -175,7 +174,7 @@ struct RegenQueue {
 // plain loop instead.
 // What bounds it: the shifts, xors and multiplies of the screens' hashes and of the regenerated cells' draws.
 __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a, const UniformF32 &U, int x, int y,
-                                                          bool valid, RegenQueue &Q) {
+                                                          bool valid, int k0, int k1, RegenQueue &Q) {
     if (!(a.rm > 0.0f)) return 0u;
     const int lane = threadIdx.x & 31;
     uint32_t hits = 0;
@@ -183,8 +182,8 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
     int head = 0, queued = 0;  // uniform
     Q.hit[lane] = 0u;
     __syncwarp();
-    for (int kb = 0; kb < a.n; kb += 32) {
-        const int nk = min(32, a.n - kb);
+    for (int kb = k0; kb < k1; kb += 32) {
+        const int nk = min(32, k1 - kb);
         if (lane < nk) rows = pixel_rows(a, y, a.offs[kb + lane].y);
         // the first `count` cells of the queue, one per lane
         auto run = [&](int count) {
@@ -282,25 +281,30 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
 }
 
 // The per-sample path for the kPwRegenThreads pixels [x0, x0 + kPwRegenThreads) of row y (one per
-// thread of the CTA).  Thread 0 adds the CTA's samples and the CTA to the diagnostics (regenerated samples,
-// unstaged blocks, blocks).
+// thread of the CTA) and their samples [k0, k1): all N of them, or a part, whose hits add up in the plane
+// (whole numbers: exact).  The CTA of the first part adds the pixels' samples and itself to the diagnostics
+// (regenerated samples, unstaged blocks, blocks).
 // One form for every density.  Before it, warps went by their grains per cell: cells dealt sample by sample
 // (lane- or rank-major), where a sample of 32 lanes left its last round of 32 cells half empty, and above 1.1 a
 // loop that visited one cell at a time.  GB300, radius 0.025, N 64: 1021 x 763 blobs 4.03 -> 2.82 ms,
 // 700 x 500 ramp 3.09 -> 1.86 ms (1.94 with the loop kept above 1.1).
-__device__ __forceinline__ void pixelwise_regen_pixels(const PixelwiseArgs &a, int x0, int y) {
+__device__ __forceinline__ void pixelwise_regen_pixels(const PixelwiseArgs &a, int x0, int y, int k0, int k1) {
     __shared__ RegenQueue queues[kPwRegenThreads / 32];
     const int x = x0 + (int)threadIdx.x;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && k0 == 0) {
         const int px = min(kPwRegenThreads, a.out_w - x0);
         atomicAdd(&a.diag[0], (unsigned long long)px * (unsigned long long)a.n);
         atomicAdd(&a.diag[1], 1ull);
         atomicAdd(&a.diag[3], 1ull);
     }
+    if (x - (int)(threadIdx.x & 31) >= a.out_w) return;  // whole warps
     const bool valid = x < a.out_w;
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
-    const uint32_t hits = pixelwise_pixel_queue(a, U, x, y, valid, queues[threadIdx.x >> 5]);  // all 32 lanes
-    if (valid) a.out[(long long)y * a.out_w + x] = (float)hits;
+    const uint32_t hits = pixelwise_pixel_queue(a, U, x, y, valid, k0, k1, queues[threadIdx.x >> 5]);  // all 32 lanes
+    if (!valid) return;
+    float *out = a.out + (long long)y * a.out_w + x;
+    if (k1 - k0 == a.n) *out = (float)hits;
+    else if (hits) atomicAdd(out, (float)hits);
 }
 
 // Block-wide exclusive scan of one int per thread (any blockDim.x that is a multiple of 32, <= 1024).

@@ -305,3 +305,13 @@ def test_grainwise_lane_groups_and_queue(cuda, fgl, orc, w, h, zoom, radius, n, 
 def test_pixelwise_screened_cells(cuda, fgl, orc, w, h, radius, cell, zoom, n):
     """The lambda pixels of a cell column's rows: in the plane's bitmask and in the per-sample kernel."""
     _check("pixel", fgl, orc, _blobs(w, h), radius=radius, cell=cell, zoom=zoom, n=n, seed=13)
+
+
+@pytest.mark.parametrize("n", [1, 4, 5, 31, 33, 100])
+def test_pixelwise_small_plane_parts(cuda, fgl, orc, n):
+    """A small plane on the per-sample kernel, its samples in parts of four and more over several warps."""
+    plane = _blobs(35, 9)
+    p, d, *_ = _setup(fgl, orc, plane, radius=0.2, n=n, seed=3)
+    if n <= 5:
+        assert fgl.pixelwise_kernel_count(p, d) == 3
+    _check("pixel", fgl, orc, plane, radius=0.2, n=n, seed=3)

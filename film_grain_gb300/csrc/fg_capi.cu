@@ -255,7 +255,7 @@ struct Layout {
 // are cleared together), the offsets, the cell table and, last, the sparse pass's bitmask.
 struct PwScratch {
     PwPlan plan;
-    size_t diag, offs, cells, mask, mask_bytes;
+    size_t diag, offs, cells, mask, mask_bytes, bits, bits_bytes;
     PwScratch(const fg_params &p, const fg_derived &d, const float *h_offs_in, Layout *l) {
         plan = plan_pixelwise(p, d, h_offs_in, 4);
         const PixelwiseArgs a = pixelwise_args(p, d, plan, nullptr, nullptr, nullptr, nullptr, nullptr);
@@ -264,13 +264,15 @@ struct PwScratch {
         cells = l->add(sizeof(CellParam) * (size_t)d.input_width * d.input_height);
         mask_bytes = pixelwise_cellmask_bytes(a, plan.nby);
         mask = l->add(mask_bytes);
+        bits_bytes = mask_bytes ? pixelwise_stream_bytes(a, plan.nby) : 0;
+        bits = l->add(bits_bytes);
     }
     // the layout's allocation, without the bitmask where that finds no room (the plane takes the lean pass)
     cudaError_t alloc(DevBuf *b, const Layout &l, cudaStream_t s) {
         cudaError_t e = b->alloc(l.bytes, s);
         if (e != cudaErrorMemoryAllocation || !mask_bytes) return e;
         cudaGetLastError();
-        mask_bytes = 0;
+        mask_bytes = bits_bytes = 0;
         return b->alloc(mask, s);
     }
     PwBuffers at(void *base) const {
@@ -281,6 +283,8 @@ struct PwScratch {
         w.cells = reinterpret_cast<CellParam *>(c + cells);
         w.listed = true;
         w.mask = mask_bytes ? reinterpret_cast<unsigned int *>(c + mask) : nullptr;
+        w.bits = bits_bytes ? reinterpret_cast<unsigned int *>(c + bits) : nullptr;
+        w.bits_bytes = bits_bytes;
         return w;
     }
 };
@@ -290,15 +294,19 @@ fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_der
                             int *d_cancel) {
     const int in_w = (int)d.input_width, in_h = (int)d.input_height;
     const int out_w = (int)d.output_width, out_h = (int)d.output_height;
-    FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, w.cells, d_out, (long long)out_w * out_h, w.counters, s),
+    FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, w.cells, d_out, w.bits ? 0 : (long long)out_w * out_h,
+                               w.counters, s),
             "cell params");
+    if (w.bits) FG_CUDA(cudaMemsetAsync(w.bits, 0, w.bits_bytes, s), "clear bits");
     PixelwiseArgs a = pixelwise_args(p, d, pl, d_lam, w.cells, w.offs, d_out, w.counters->diag);
     a.cancel = d_cancel;
-    FG_CUDA(launch_pixelwise(a, pl.nby, w.listed ? w.counters->list : nullptr, w.mask, s), "pixelwise kernel");
+    FG_CUDA(launch_pixelwise(a, pl.nby, w.listed ? w.counters : nullptr, w.mask, w.bits, s), "pixelwise kernel");
     EpilogueArgs e;
     if (colour) e = *colour;
     else std::memset(&e, 0, sizeof e);
     e.plane = d_out;
+    e.bits = w.bits;
+    e.words = (int)((p.n_samples + 31) / 32);
     e.out_w = out_w; e.out_h = out_h; e.in_w = in_w; e.in_h = in_h;
     e.inv_samples = 1.0f / (float)p.n_samples;
     FG_CUDA(launch_epilogue(e, s), "pixelwise epilogue");

@@ -27,6 +27,8 @@ struct PwBuffers {
     CellParam *cells;
     bool listed;           // the deferred list follows the counters (else: fat CTAs over every block)
     unsigned int *mask;    // null, or the sparse pass's bitmask (pixelwise_cellmask_bytes)
+    unsigned int *bits;    // null, or the stream pass's bits (pixelwise_stream_bytes)
+    size_t bits_bytes;
 };
 fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_derived &d, const PwPlan &pl,
                             const PwBuffers &w, float *d_out, const EpilogueArgs *colour, cudaStream_t s,

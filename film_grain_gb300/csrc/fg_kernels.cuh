@@ -34,14 +34,15 @@ constexpr int kPwKChunk = 256;     // offsets per sample-assignment chunk
 constexpr int kPwFootMax = 1024;   // per-block output-pixel counters
 constexpr int kPwMaxLevel = 3;     // block subdivision depth on grain overflow
 // Pixel-wise diagnostic counters (PixelwiseArgs::diag): [0] samples evaluated on the per-sample path,
-// [1] blocks without a staged window, [2] block subdivisions, [3] blocks run, [4] sparse blocks whose
-// samples ran sample-major, [5] sparse blocks that ran grain-major.
+// [1] blocks without a staged window, [2] block subdivisions, [3] blocks and tiles run, [4] blocks of the sparse
+// pass, [5] tiles of the stream pass.
 constexpr int kPwDiagWords = 6;
 
 // A pixel-wise plane's counters, and the header of its deferred list: [0] the next entry the fat pass
 // takes, [1] the number of entries, which follow in list[2..] where a list is kept.
 struct PwCounters {
     unsigned long long diag[kPwDiagWords];
+    int tile, unused;  // the next tile of the stream pass
     int list[2];
 };
 // A block regenerates per sample (no staging) when its samples' reach, in cells, is below
@@ -65,6 +66,14 @@ constexpr float kPwRegenKernel = 2.05f;
 constexpr double kPwRegenSmallVisits = 4.5e6;
 constexpr float kPwRegenSmall = 5.0f;
 constexpr double kPwRegenWarps = 32.0;
+// The stream pass (fg_pixelwise_stream.cuh): planes of kPwStreamPixels output pixels and more, and the grains per
+// output pixel, in multiples of N, above which a segment's samples go to the per-sample kernel -- with ranges of
+// up to 4 cells an axis, and wider ones, whose samples look at more cells.  Log-normal 0.025 at 1024^2, N 256:
+// at 2 N 20.7 ms, 4 N 18.9, 6 N 20.2, 10 N 21.1; 1080p radius 0.1 N 32: at 1.3 N 2.19 ms, 2 N 2.10, 3 N 2.02;
+// 1000^2 ramp, the same grain: 1.68, 1.58, 1.70.
+constexpr double kPwStreamPixels = 8192.0;
+constexpr float kPwStreamDense = 2.0f, kPwStreamDenseWide = 4.0f;
+
 // In-launch cancellation: `cancel` is null or two words of mapped pinned host memory.  Word 0 is set
 // by the waiting host thread once the caller's cancel flag turns non-zero; the persistent passes
 // read it once per work item they pull (the block passes once per block) and stop, and a CTA that
@@ -137,7 +146,9 @@ struct GrainwiseEpilogueArgs {
 
 // Epilogue of the pixel-wise path: counts -> value (and optional colour packing).
 struct EpilogueArgs {
-    float *plane;               // counts in, values out (in place)
+    float *plane;               // counts in (unless bits), values out (in place)
+    const unsigned int *bits;   // null, or the samples' bits: `words` words a pixel
+    int words;
     int out_w, out_h, in_w, in_h;
     float inv_samples;
     unsigned char *out_rgb8;    // null: values only
@@ -156,11 +167,15 @@ struct LogfTableDev {
 // The cell table, and the plane's output and counters set to zero beside it.
 cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, float *out,
                                long long n_out, PwCounters *counters, cudaStream_t s);
-// defer: null (fat CTAs over every block) or PwCounters::list, cleared, with nbx*nby ints behind it (lean
-// pass, then fat CTAs over the deferred blocks).
+// counters: null (fat CTAs over every block) or cleared, with nbx*nby ints behind them (lean or sparse pass,
+// then fat CTAs over the deferred blocks).
 // cellmask: null, or pixelwise_cellmask_bytes(a, nby) bytes for the sparse pass's plane bitmask (the
 // plane then takes the sparse pass, else the lean pass).
-cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsigned int *cellmask, cudaStream_t s);
+// bits: null, or pixelwise_stream_bytes(a, nby) cleared bytes (with cellmask: the plane takes the stream pass,
+// which gives the samples' bits instead of the counts).
+cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, PwCounters *counters, unsigned int *cellmask,
+                             unsigned int *bits, cudaStream_t s);
+size_t pixelwise_stream_bytes(const PixelwiseArgs &a, int nby);
 // Scratch bytes of the sparse pass's plane bitmask for this plane; 0 when the plane does not take it.
 size_t pixelwise_cellmask_bytes(const PixelwiseArgs &a, int nby);
 // Whether a plane runs on the per-sample kernel instead of the block kernel: in a batch, and on its own.

@@ -124,6 +124,7 @@ extern "C" FG_API fg_status fg_render_pixelwise_noalloc(const float *d_lambda, c
     w.counters = reinterpret_cast<PwCounters *>(scratch + kNaCellsBytes + kNaOffsBytes);
     w.listed = false;
     w.mask = nullptr;
+    w.bits = nullptr;
     cudaStream_t s = (cudaStream_t)stream;
     // The array keeps the previous call's contents: the offsets are overwritten here, the cell table and
     // the counters by the cell-parameter kernel.

@@ -1,8 +1,9 @@
 // fg_pixelwise.cu -- the pixel-wise coverage estimator (src/pixelwise.rs:11-106) for sm_103a.
 //
 // The reference loops pixel -> offset sample -> cell -> grain and regenerates every cell's grains
-// from its cell_rng each time a sample visits it.  A plane takes one of two kernels
-// (pixelwise_prefers_regen): the per-sample kernel keeps that loop, one thread per output pixel
+// from its cell_rng each time a sample visits it.  A plane takes one of three ways.  The stream pass
+// (fg_pixelwise_stream.cuh) generates each grain once and finds the samples it covers: planes whose grains
+// reach less than half an output pixel.  The per-sample kernel keeps that loop, one thread per output pixel
 // (pixelwise_regen_pixels in fg_pixelwise.cuh), for planes whose samples reach fewer cells than a
 // staged window would hold (small radii, few samples per pixel); the block kernels regroup the work by
 // where the samples land: sample (pixel x,y; offset k) has the input-space point
@@ -31,6 +32,7 @@
 #include "fg_color.cuh"
 #include "fg_pixelwise.cuh"
 #include "fg_pixelwise_sparse.cuh"
+#include "fg_pixelwise_stream.cuh"
 
 namespace fg {
 
@@ -98,58 +100,55 @@ __global__ void __launch_bounds__(PwSparse::kThreads, PwSparse::kCtasPerSm)
 }
 
 // The offsets in ascending x (ties by index: a permutation even with NaNs), for the sparse pass's
-// lanes (sparse_sample_pass); with gm_ent, also the grain-major form's table of the sorted offsets by
-// phase bin (frac(o.x * zoom), frac(o.y * zoom)): entries bin-major (ties by sorted index), each
-// entry's sorted index, and each bin's first entry (sparse_grain_pass).  One CTA of kPwKChunk threads;
-// n <= kPwKChunk.
+// lanes (sparse_sample_pass).  One CTA of kPwKChunk threads; n <= kPwKChunk.
 __device__ __forceinline__ unsigned offset_sort_key(float v) {
     const unsigned b = __float_as_uint(v);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);  // the float order as an unsigned order
 }
-__device__ __forceinline__ int offset_phase_bin(float v) {  // v = o * zoom
-    constexpr int B = PwSparse::kGmBins;
-    const float f = v - floorf(v);  // [0, 1]: 1 only when v is just below an integer
-    return min((int)(f * (float)B), B - 1);
-}
-__global__ void __launch_bounds__(kPwKChunk) sort_offsets_kernel(const float2 *__restrict__ offs, int n, float zoom,
-                                                                 float2 *__restrict__ sorted,
-                                                                 float4 *__restrict__ gm_ent, int *__restrict__ gm_idx) {
-    constexpr int B = PwSparse::kGmBins;
-    __shared__ float2 s_sorted[kPwKChunk];
-    __shared__ int s_bin[kPwKChunk];
+__global__ void __launch_bounds__(kPwKChunk) sort_offsets_kernel(const float2 *__restrict__ offs, int n,
+                                                                 float2 *__restrict__ sorted) {
     const int k = threadIdx.x;
-    if (k < n) {
-        const float2 o = offs[k];
-        const unsigned key = offset_sort_key(o.x);
-        int rank = 0;
-        for (int j = 0; j < n; j++) {
-            const unsigned kj = offset_sort_key(offs[j].x);
-            rank += (kj < key || (kj == key && j < k)) ? 1 : 0;
-        }
-        sorted[rank] = o;
-        s_sorted[rank] = o;
+    if (k >= n) return;
+    const float2 o = offs[k];
+    const unsigned key = offset_sort_key(o.x);
+    int rank = 0;
+    for (int j = 0; j < n; j++) {
+        const unsigned kj = offset_sort_key(offs[j].x);
+        rank += (kj < key || (kj == key && j < k)) ? 1 : 0;
     }
-    if (!gm_ent) return;  // uniform
+    sorted[rank] = o;
+}
+
+// The stream pass's tables: block 0 the offsets and their phase masks, the others the dense segments, a warp
+// each.
+struct StreamSetup {
+    int segs, nw;  // nw: words of a mask
+    float limit, w_max;
+    unsigned char *dense;
+    int *count, *list;
+    float4 *ent;
+    unsigned int *masks;
+};
+__global__ void __launch_bounds__(kPwKChunk) stream_setup_kernel(const __grid_constant__ PixelwiseArgs a,
+                                                                 const __grid_constant__ StreamSetup t) {
+    if (blockIdx.x > 0) {
+        stream_classify(a, (long long)(blockIdx.x - 1) * (kPwKChunk / 32) + threadIdx.x / 32, t.segs, t.limit, t.dense,
+                        t.count, t.list);
+        return;
+    }
+    __shared__ float s_oz[2][kPwKChunk];
+    if ((int)threadIdx.x < a.n) {
+        const float2 o = a.offs[threadIdx.x];
+        const float4 e = make_float4(o.x, o.y, FG_FMUL(o.x, a.zoom), FG_FMUL(o.y, a.zoom));
+        t.ent[threadIdx.x] = e;
+        s_oz[0][threadIdx.x] = e.z;
+        s_oz[1][threadIdx.x] = e.w;
+    }
     __syncthreads();
-    float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    int bin = 0;
-    if (k < n) {
-        const float2 o = s_sorted[k];
-        e = make_float4(o.x, o.y, o.x * zoom, o.y * zoom);
-        bin = offset_phase_bin(e.w) * B + offset_phase_bin(e.z);
-        s_bin[k] = bin;
-    }
-    __syncthreads();
-    if (k < n) {
-        int pos = 0;
-        for (int j = 0; j < n; j++) pos += (s_bin[j] < bin || (s_bin[j] == bin && j < k)) ? 1 : 0;
-        gm_ent[pos] = e;
-        gm_idx[pos] = k;
-    }
-    for (int b = k; b <= B * B; b += blockDim.x) {
-        int first = 0;
-        for (int j = 0; j < n; j++) first += s_bin[j] < b ? 1 : 0;
-        gm_idx[n + b] = first;
+    for (int w = threadIdx.x; w < phase_table_words(t.nw); w += blockDim.x) {
+        const int word = w % t.nw, bucket = w / t.nw % kPhaseBuckets, cls = w / t.nw / kPhaseBuckets % kPhaseClasses;
+        const int axis = w / t.nw / kPhaseBuckets / kPhaseClasses;
+        t.masks[w] = phase_mask_word(s_oz[axis], a.n, bucket, cls, word, t.w_max);
     }
 }
 
@@ -195,10 +194,6 @@ static bool plan_sparse(const PixelwiseArgs &a, int nby, int sms, PwSparseGrid *
         const int gi0 = window_lo((float)sbx0 * bs, a) - 2, gi1 = window_hi((float)(sbx1 + 1) * bs, a) + 2;
         const int gj0 = window_lo((float)sby0 * bs, a) - 2, gj1 = window_hi((float)(sby1 + 1) * bs, a) + 2;
         g->cellmask = nullptr;
-        g->gm_ent = nullptr;
-        g->gm_idx = nullptr;
-        g->gm_eps = g->gm_grain_cost = g->gm_sample_cost = 0.0f;
-        g->gm_noslow = 0;
         g->gi0 = gi0;
         g->gj0 = gj0;
         g->gw = gi1 - gi0 + 1;
@@ -218,52 +213,76 @@ static int sm_count() {
     return sms;
 }
 
-// The sparse pass's scratch, each part 16-byte aligned: the bitmask, the offsets sorted by x, the
-// grain-major form's entries (float4) and its index (entry offsets, then bin starts).
+// The sparse pass's scratch, each part 16-byte aligned: the bitmask, the offsets sorted by x -- or the stream
+// pass's: the bitmask, the offsets (float4), their phase masks, the list of dense segments and their flags.
 static size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
 static size_t sparse_mask_bytes(const PwSparseGrid &g) { return align16((size_t)g.gw * g.ghw * sizeof(unsigned int)); }
-static size_t sparse_gm_ent_at(const PwSparseGrid &g, int n) {
-    return sparse_mask_bytes(g) + align16((size_t)n * sizeof(float2));
+static int stream_words(int n) { return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8; }  // words of the kernel's variant
+static size_t stream_masks_at(const PwSparseGrid &g, int n) {
+    return sparse_mask_bytes(g) + align16((size_t)n * sizeof(float4));
 }
-static size_t sparse_gm_idx_at(const PwSparseGrid &g, int n) {
-    return sparse_gm_ent_at(g, n) + (size_t)n * sizeof(float4);
+static size_t stream_list_at(const PwSparseGrid &g, int n) {
+    return stream_masks_at(g, n) + phase_table_words(stream_words(n)) * sizeof(unsigned int);
+}
+
+// The stream pass's plane conditions and tiles.  A grain reaches at most rm * zoom output pixels; the candidate
+// pixel of an offset is exact while that reach plus the f32 rounding of the pixel coordinates (eps: a few
+// ulps of the largest coordinate) stays below half a pixel, and the rounding to an integer by adding
+// 1.5 * 2^23 needs coordinates below 2^22.
+// Planes below kPwStreamPixels stay with the sparse and fat passes, whose forms the tests hold against the oracle
+// there.
+// Tiles: the largest of 512 .. 32 cells an edge whose footprint's bits leave room for many CTAs an SM and whose
+// tiles give every CTA slot several; chunks are split while a warp would get few.
+static bool plan_stream(const PixelwiseArgs &a, const PwSparseGrid &g, int sms, PwStreamGrid *t) {
+    if ((double)a.out_w * a.out_h < kPwStreamPixels) return false;
+    const double ext = std::max({std::fabs(a.offx_min), std::fabs(a.offx_max), std::fabs(a.offy_min),
+                                 std::fabs(a.offy_max)});
+    const double coord = (double)std::max(a.out_w, a.out_h) + ext * a.zoom + 2.0;
+    const double eps = coord * 0x1p-21 + 0x1p-20;
+    if (!(coord < 0x1p21) || !((double)a.rm * a.zoom + eps <= 0.4)) return false;
+    t->eps = (float)eps;
+    // the roundings of xg, of xg +- rm, of the cell's origin and of the divisions: a few ulps of the largest
+    // input coordinate
+    const double grid = (double)std::max(a.out_w, a.out_h) * a.inv_zoom + ext + a.rm + 2.0;
+    t->near_rm = (float)(a.rm - 16.0 * grid * 0x1p-23);
+    t->nw = (a.n + 31) / 32;
+    if ((double)a.out_w * a.out_h * t->nw * 4.0 > kCellMaskMaxBytes) return false;
+    t->gi0 = g.gi0; t->gj0 = g.gj0; t->gw = g.gw; t->ghw = g.ghw;
+    t->segs = (a.out_w + 31) / 32;
+    t->sub = 1;
+    while (t->sub < 8 && (double)t->gw / 32.0 * t->ghw * t->sub < 128.0 * sms) t->sub *= 2;
+    for (int T = 512; T >= 32; T >>= 1) {
+        auto edge = [&](float lo, float hi) {
+            return std::floor(((double)T * a.delta + 2.0 * a.rm + (double)hi - (double)lo) * a.zoom) + 8.0;
+        };
+        const double words = edge(a.offx_min, a.offx_max) * edge(a.offy_min, a.offy_max) * t->nw;
+        t->tile = T;
+        t->ntx = (t->gw + T - 1) / T;
+        t->nty = (32 * t->ghw + T - 1) / T;
+        if (words <= (T == 32 ? 12288.0 : 4096.0) && (T == 32 || (double)t->ntx * t->nty >= 32.0 * sms)) {
+            t->fp_words = (int)words;
+            return (double)t->ntx * t->nty < 2.0e9;
+        }
+    }
+    return false;
 }
 
 size_t pixelwise_cellmask_bytes(const PixelwiseArgs &a, int nby) {
     if (pixelwise_takes_regen(a)) return 0;
     PwSparseGrid g;
-    const int sms = sm_count();  // without a device (planning only): the GB300's 152
-    if (!plan_sparse(a, nby, sms > 0 ? sms : 152, &g)) return 0;
-    const int bins = PwSparse::kGmBins * PwSparse::kGmBins;
-    return sparse_gm_idx_at(g, a.n) + (size_t)(a.n + bins + 1) * sizeof(int);
+    PwStreamGrid t;
+    const int sms = sm_count() > 0 ? sm_count() : 152;  // without a device (planning only): the GB300's 152
+    if (!plan_sparse(a, nby, sms, &g)) return 0;
+    if (plan_stream(a, g, sms, &t)) return stream_list_at(g, a.n) + (size_t)t.segs * a.out_h * (sizeof(int) + 1);
+    return sparse_mask_bytes(g) + (size_t)a.n * sizeof(float2);
 }
 
-// The grain-major form's plane conditions and cost model (sparse_grain_pass).  A grain reaches at most
-// rm * zoom output pixels; the candidate pixel of an offset is exact while that reach plus the f32
-// rounding of the pixel coordinates (eps: a few ulps of the largest coordinate) stays below half a
-// pixel, and the rounding to an integer by adding 1.5 * 2^23 needs coordinates below 2^22.  Costs, in
-// units fitted to timings of both forms (on the 4096^2 planes at r 0.025 log-normal N 256 grain-major
-// is faster for every block; on the 256^2 ramp at r 0.12 N 64 it is slower for the dense blocks): a
-// grain pays its set-up and, per candidate, a disk test and its share of the listed hits, for
-// n (2 (r_mean zoom + eps) + 1/bins)^2 candidates on average; a sample pays the scan of its cell
-// range's columns.
-static bool plan_grain_major(const PixelwiseArgs &a, PwSparseGrid *g) {
-    const double ext = std::max({std::fabs(a.offx_min), std::fabs(a.offx_max), std::fabs(a.offy_min),
-                                 std::fabs(a.offy_max)});
-    const double coord = (double)std::max(a.out_w, a.out_h) + ext * a.zoom + 2.0;
-    const double eps = coord * 0x1p-21 + 0x1p-20;
-    g->gm_eps = (float)eps;
-    const double reach = (double)a.rm * a.zoom;
-    if (!(coord < 0x1p21) || !(reach + eps <= 0.4)) return false;
-    // a sample's range spans floor((xg + rm) / delta) - floor((xg - rm) / delta) cells: 2 rm / delta + 1
-    // and the rounding of xg +- rm and of the divisions (a few ulps of the largest grid coordinate)
-    const double grid = (double)std::max(a.out_w, a.out_h) * a.inv_zoom + ext + a.rm + 2.0;
-    const double span = 2.0 * a.rm / a.delta + 1.0 + 8.0 * grid * 0x1p-23 / a.delta;
-    g->gm_noslow = span <= 30.0 ? 1 : 0;
-    const double band = 2.0 * ((double)a.radius_mean * a.zoom + eps) + 1.0 / PwSparse::kGmBins;
-    g->gm_grain_cost = (float)(60.0 + 40.0 * a.n * band * band);
-    g->gm_sample_cost = (float)(40.0 + 9.0 * (2.0 * a.rm / a.delta + 1.0));
-    return true;
+size_t pixelwise_stream_bytes(const PixelwiseArgs &a, int nby) {
+    if (pixelwise_takes_regen(a)) return 0;
+    PwSparseGrid g;
+    PwStreamGrid t;
+    const int sms = sm_count() > 0 ? sm_count() : 152;
+    return plan_sparse(a, nby, sms, &g) && plan_stream(a, g, sms, &t) ? (size_t)a.out_w * a.out_h * t.nw * 4 : 0;
 }
 
 // The root blocks the lean pass deferred, in fat CTAs: persistent, each CTA taking the next listed
@@ -352,16 +371,74 @@ static cudaError_t set_smem(K k, size_t smem) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsigned int *cellmask, cudaStream_t s) {
+template <int NW>
+static cudaError_t launch_stream(const PixelwiseArgs &a, const PwStreamGrid &t, int sms, cudaStream_t s) {
+    const size_t smem = sizeof(PwStreamShared<NW>) + (size_t)t.fp_words * sizeof(unsigned int);
+    cudaError_t e = set_smem(pixelwise_stream_kernel<NW>, smem);
+    int per_sm = 0;
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pixelwise_stream_kernel<NW>, PwStream::kThreads, smem);
+    if (e != cudaSuccess) return e;
+    const long long grid = std::min<long long>((long long)t.ntx * t.nty, (long long)sms * std::max(1, per_sm));
+    pixelwise_stream_kernel<NW><<<(unsigned)grid, PwStream::kThreads, smem, s>>>(a, t);
+    return cudaGetLastError();
+}
+
+// The plane's bits, its emptiness bitmask (g) written: the tables, the stream pass and the per-sample kernel over
+// the dense segments.
+static cudaError_t launch_pixelwise_stream(const PixelwiseArgs &a, const PwSparseGrid &g, PwStreamGrid t,
+                                           PwCounters *counters, unsigned int *scratch, unsigned int *bits, int sms,
+                                           cudaStream_t s) {
+    char *base = reinterpret_cast<char *>(scratch);
+    const int nw = stream_words(a.n);
+    const long long nseg = (long long)t.segs * a.out_h;
+    StreamSetup u;
+    u.segs = t.segs;
+    u.nw = nw;
+    u.ent = reinterpret_cast<float4 *>(base + sparse_mask_bytes(g));
+    u.masks = reinterpret_cast<unsigned int *>(base + stream_masks_at(g, a.n));
+    u.list = reinterpret_cast<int *>(base + stream_list_at(g, a.n));
+    u.dense = reinterpret_cast<unsigned char *>(u.list + nseg);
+    u.count = &counters->list[1];
+    // the per-sample kernel's limits, as pixelwise_prefers_regen
+    const double axis = std::floor(2.0 * (double)a.rm / (double)a.delta) + 2.0;
+    u.limit = std::isfinite(regen_reach(a))
+                  ? (axis > 4.0 ? kPwStreamDenseWide : kPwStreamDense) * (float)a.n * a.zoom * a.zoom
+                  : HUGE_VALF;
+    u.w_max = FG_FMUL(FG_FMUL(a.rm, a.zoom), 1.000008f) + t.eps;  // (stream_candidates' half-width of radius rm, rounded up)
+    t.cellmask = g.cellmask;
+    t.ent = u.ent;
+    t.masks = u.masks;
+    t.class_scale = (float)kPhaseClasses / u.w_max;
+    t.bits = bits;
+    t.next = &counters->tile;
+    t.dense = u.dense;
+    t.dense_count = u.count;
+    constexpr int kSegs = kPwKChunk / 32;
+    stream_setup_kernel<<<(unsigned)(1 + (nseg + kSegs - 1) / kSegs), kPwKChunk, 0, s>>>(a, u);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    e = nw == 1   ? launch_stream<1>(a, t, sms, s)
+        : nw == 2 ? launch_stream<2>(a, t, sms, s)
+        : nw == 4 ? launch_stream<4>(a, t, sms, s)
+                  : launch_stream<8>(a, t, sms, s);
+    if (e != cudaSuccess) return e;
+    const long long ctas = std::min<long long>((nseg + 7) / 8, 4LL * std::max(1, sms));
+    pixelwise_dense_kernel<<<(unsigned)ctas, kPwRegenThreads, 0, s>>>(a, bits, t.nw, t.segs, &counters->list[0], u.count,
+                                                                     u.list);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, PwCounters *counters, unsigned int *cellmask,
+                             unsigned int *bits, cudaStream_t s) {
     if (pixelwise_takes_regen(a)) return launch_pixelwise_regen(a, s);
     const size_t lean_smem = sizeof(PwShared<PwLean>), fat_smem = sizeof(PwShared<PwFat>);
-    cudaError_t e = set_smem(pixelwise_kernel<PwLean>, lean_smem);
-    if (e == cudaSuccess) e = set_smem(pixelwise_kernel<PwFat>, fat_smem);
-    if (e == cudaSuccess) e = set_smem(pixelwise_deferred_kernel, fat_smem);
-    if (e != cudaSuccess) return e;
     const long long nblocks = (long long)a.nbx * nby;
     if (nblocks <= 0) return cudaSuccess;
-    if (!defer) {
+    cudaError_t e;
+    if (!counters) {
+        e = set_smem(pixelwise_kernel<PwFat>, fat_smem);
+        if (e != cudaSuccess) return e;
         pixelwise_kernel<PwFat><<<(unsigned)nblocks, PwFat::kThreads, fat_smem, s>>>(a, nullptr);
         return cudaGetLastError();
     }
@@ -369,33 +446,33 @@ cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsign
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
+    int *list = &counters->list[1];  // the count, then the deferred root blocks
     PwSparseGrid g;
     const bool sparse = cellmask && plan_sparse(a, nby, sms, &g);
     if (sparse) {
         g.cellmask = cellmask;
         const int row_ctas = (g.gw + kMaskThreads - 1) / kMaskThreads;
         cell_mask_kernel<<<(unsigned)((long long)row_ctas * g.ghw), kMaskThreads, 0, s>>>(a, g, row_ctas, cellmask);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        PwStreamGrid t;
+        if (bits && plan_stream(a, g, sms, &t)) return launch_pixelwise_stream(a, g, t, counters, cellmask, bits, sms, s);
         PixelwiseArgs as = a;  // the sparse pass reads the offsets sorted by x
-        char *scratch = reinterpret_cast<char *>(cellmask);
-        as.offs = reinterpret_cast<const float2 *>(scratch + sparse_mask_bytes(g));
-        float4 *gm_ent = nullptr;
-        int *gm_idx = nullptr;
-        if (plan_grain_major(a, &g)) {
-            gm_ent = reinterpret_cast<float4 *>(scratch + sparse_gm_ent_at(g, a.n));
-            gm_idx = reinterpret_cast<int *>(scratch + sparse_gm_idx_at(g, a.n));
-            g.gm_ent = gm_ent;
-            g.gm_idx = gm_idx;
-        }
-        sort_offsets_kernel<<<1, kPwKChunk, 0, s>>>(a.offs, a.n, a.zoom, const_cast<float2 *>(as.offs), gm_ent, gm_idx);
+        float2 *sorted = reinterpret_cast<float2 *>(reinterpret_cast<char *>(cellmask) + sparse_mask_bytes(g));
+        as.offs = sorted;
+        sort_offsets_kernel<<<1, kPwKChunk, 0, s>>>(a.offs, a.n, sorted);
         const size_t sparse_smem = sizeof(PwSparseShared);
         e = set_smem(pixelwise_sparse_kernel, sparse_smem);
         if (e != cudaSuccess) return e;
         pixelwise_sparse_kernel<<<(unsigned)((long long)g.nsbx * g.nsby), PwSparse::kThreads, sparse_smem, s>>>(
-            as, g, nby, defer + 1);
+            as, g, nby, list);
     } else {
-        pixelwise_kernel<PwLean><<<(unsigned)nblocks, PwLean::kThreads, lean_smem, s>>>(a, defer + 1);
+        e = set_smem(pixelwise_kernel<PwLean>, lean_smem);
+        if (e != cudaSuccess) return e;
+        pixelwise_kernel<PwLean><<<(unsigned)nblocks, PwLean::kThreads, lean_smem, s>>>(a, list);
     }
     e = cudaGetLastError();
+    if (e == cudaSuccess) e = set_smem(pixelwise_deferred_kernel, fat_smem);
     if (e != cudaSuccess) return e;
     const long long grid = std::min<long long>(nblocks, (long long)std::max(1, sms) * PwFat::kCtasPerSm);
     PixelwiseArgs ad = a;  // after the sparse pass, the fat pass reads cell emptiness from its bitmask
@@ -406,7 +483,7 @@ cudaError_t launch_pixelwise(const PixelwiseArgs &a, int nby, int *defer, unsign
         ad.cm_gw = g.gw;
         ad.cm_ghw = g.ghw;
     }
-    pixelwise_deferred_kernel<<<(unsigned)grid, PwFat::kThreads, fat_smem, s>>>(ad, defer + 1);
+    pixelwise_deferred_kernel<<<(unsigned)grid, PwFat::kThreads, fat_smem, s>>>(ad, list);
     return cudaGetLastError();
 }
 
@@ -415,7 +492,16 @@ __global__ void epilogue_kernel(const EpilogueArgs a) {
     long long n = (long long)a.out_w * a.out_h;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float v = FG_FMUL(a.plane[i], a.inv_samples);  // sum * inv_samples (src/pixelwise.rs:38)
+    float count;
+    if (a.bits) {
+        const unsigned int *m = a.bits + i * a.words;
+        int c = 0;
+        for (int w = 0; w < a.words; w++) c += __popc(m[w]);
+        count = (float)c;
+    } else {
+        count = a.plane[i];
+    }
+    const float v = FG_FMUL(count, a.inv_samples);  // sum * inv_samples (src/pixelwise.rs:38)
     a.plane[i] = v;
     if (!a.out_rgb8) return;
     unsigned char *o = a.out_rgb8 + 3 * i;

@@ -153,10 +153,12 @@ static __device__ bool eval_regen(const PixelwiseArgs &a, const UniformF32 &U, f
 struct RegenQueue {
     uint2 e[64];        // ring: cell column; owner lane | sample << 5 | cell row - j0 << 10
     unsigned hit[32];   // per sample of the current 32: the lanes whose sample is covered
+    unsigned short pair[64];  // ring of samples whose outer cells are due: owner lane | sample << 5
 };
 
 // Hit count of output pixel (x, y) over its samples [k0, k1) by the reference's per-sample loop
-// (src/pixelwise.rs:30-38 around evaluate_indicator, src/pixelwise.rs:47-106).  Called by all 32 lanes of a warp (neighbouring pixels; `valid` false for
+// (src/pixelwise.rs:30-38 around evaluate_indicator, src/pixelwise.rs:47-106), and when `bits` is given (the
+// pixel's words; the samples then lie in one word) the hits' bits.  Called by all 32 lanes of a warp (neighbouring pixels; `valid` false for
 // lanes past the row's end, which take part without samples); the lanes take the samples in step:
 //   1. every cell of a sample's range gets the emptiness screen alone (first_draw_maybe): the same short work
 //      on every lane, one column hash per column; the cells that may hold grains go to a 64-bit mask, cell
@@ -168,13 +170,17 @@ struct RegenQueue {
 //      -- the lanes put their cells into the warp's queue, and whenever it holds 32 each lane regenerates
 //      one of them against its owner's sample.  What is left waits for the next sample's cells, so only
 //      the last round of 32 samples runs with idle lanes; a sample that turns out covered leaves its
-//      pending cells out.
+//      pending cells out;
+//   3. ranges wider than 3 x 3 cells (log-normal radii reach three times their mean) are screened in two
+//      steps: the middle cells of all 32 samples first, then the outer cells of the samples that are not
+//      covered yet, dealt to the lanes 32 samples at a time.
 // Coverage is an OR over the cells, so neither the order nor the dealing changes it.  A range wider
 // than 8 cells on an axis (outside the plane-level choice of this path) or than two lambda pixels runs the
 // plain loop instead.
 // What bounds it: the shifts, xors and multiplies of the screens' hashes and of the regenerated cells' draws.
 __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a, const UniformF32 &U, int x, int y,
-                                                          bool valid, int k0, int k1, RegenQueue &Q) {
+                                                          bool valid, int k0, int k1, RegenQueue &Q,
+                                                          unsigned int *bits = nullptr) {
     if (!(a.rm > 0.0f)) return 0u;
     const int lane = threadIdx.x & 31;
     uint32_t hits = 0;
@@ -204,30 +210,38 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
             head += count;
             queued -= count;
         };
-        for (int ks = 0; ks < nk; ks++) {
+        // Cells of sample ks of lane `owner` that may hold grains -- the middle 3 x 3 of its range, or the others --
+        // into the queue, rank by rank.  Returns whether its range is wider than that.
+        auto screen = [&](int owner, int ks, bool live, bool middle) -> bool {
             const int j0 = __shfl_sync(0xffffffffu, rows.j0, ks), nj = __shfl_sync(0xffffffffu, rows.nj, ks);
             const int iy0 = __shfl_sync(0xffffffffu, rows.iy0, ks);
             const unsigned up = __shfl_sync(0xffffffffu, rows.up, ks);
             int i0 = 0, mid = 0;
             unsigned long long m = 0ull;
-            if (valid && nj != 0) {  // nj == 0: no cell (src/pixelwise.rs:60-62)
-                const float xg = xg_of(x, a.inv_zoom, a.offs[kb + ks].x);
+            bool wide = false;
+            if (live && nj != 0) {  // nj == 0: no cell (src/pixelwise.rs:60-62)
+                const float xg = xg_of(x - lane + owner, a.inv_zoom, a.offs[kb + ks].x);
                 i0 = f2i_floor(FG_FDIV(FG_FSUB(xg, a.rm), a.delta));
                 const int i1 = f2i_floor(FG_FDIV(FG_FADD(xg, a.rm), a.delta));
                 const int ni = i1 - i0 + 1;
                 if (ni > 0) {
                     const int ix0 = cell_axis_pixel(i0, a.delta, a.in_w), ix1 = cell_axis_pixel(i1, a.delta, a.in_w);
                     if (ni > 8 || nj < 0 || ix1 - ix0 > 1) {
-                        const float yg = xg_of(y, a.inv_zoom, a.offs[kb + ks].y);
-                        if (eval_regen(a, U, xg, yg, i0, i1, f2i_floor(FG_FDIV(FG_FSUB(yg, a.rm), a.delta)),
-                                       f2i_floor(FG_FDIV(FG_FADD(yg, a.rm), a.delta))))
-                            atomicOr(&Q.hit[ks], 1u << lane);
+                        if (middle) {
+                            const float yg = xg_of(y, a.inv_zoom, a.offs[kb + ks].y);
+                            if (eval_regen(a, U, xg, yg, i0, i1, f2i_floor(FG_FDIV(FG_FSUB(yg, a.rm), a.delta)),
+                                           f2i_floor(FG_FDIV(FG_FADD(yg, a.rm), a.delta))))
+                                atomicOr(&Q.hit[ks], 1u << owner);
+                        }
                     } else {
-                        mid = ((ni - 1) >> 1) * 8 + ((nj - 1) >> 1);
+                        const int mi = (ni - 1) >> 1, mj = (nj - 1) >> 1;
+                        mid = mi * 8 + mj;
+                        wide = ni > 3 || nj > 3;
                         const CellParam *row0 = a.cells + (long long)iy0 * a.in_w, *row1 = up ? row0 + a.in_w : row0;
                         uint32_t b0 = maybe_bound(row0[ix0].thresh), b1 = maybe_bound(row1[ix0].thresh);
                         int ix = ix0;
-                        for (int di = 0; di < ni; di++) {
+                        const int di1 = middle ? min(mi + 2, ni) : ni, dj1 = middle ? min(mj + 2, nj) : nj;
+                        for (int di = middle ? max(mi - 1, 0) : 0; di < di1; di++) {
                             const int i = i0 + di;
                             if (ix != ix1 && cell_axis_pixel(i, a.delta, a.in_w) == ix1) {
                                 ix = ix1;
@@ -236,9 +250,11 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
                             }
                             const uint64_t colh = cell_col_hash(a.seed, i);
                             unsigned col = 0u;
-                            for (int dj = 0; dj < nj; dj++)
+                            for (int dj = middle ? max(mj - 1, 0) : 0; dj < dj1; dj++) {
+                                if (!middle && abs(di - mi) <= 1 && abs(dj - mj) <= 1) continue;  // in the first step
                                 col |= (first_draw_maybe(cell_row_hash(colh, j0 + dj), ((up >> dj) & 1u) ? b1 : b0) ? 1u : 0u)
                                        << dj;
+                            }
                             m |= (unsigned long long)col << (8 * di);
                         }
                         // the middle cell and cell (0, 0) change places
@@ -257,13 +273,37 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
                     const int idx = pos == 0 ? mid : (pos == mid ? 0 : pos);
                     Q.e[(head + queued + __popc(pending & ((1u << lane) - 1u))) & 63] =
                         make_uint2((unsigned)(i0 + (idx >> 3)),
-                                   (unsigned)lane | ((unsigned)ks << 5) | ((unsigned)(idx & 7) << 10));
+                                   (unsigned)owner | ((unsigned)ks << 5) | ((unsigned)(idx & 7) << 10));
                 }
                 queued += __popc(pending);
                 __syncwarp();
                 if (queued >= 32) {
                     run(32);
-                    if ((Q.hit[ks] >> lane) & 1u) m = 0ull;
+                    if ((Q.hit[ks] >> owner) & 1u) m = 0ull;
+                }
+            }
+            return wide;
+        };
+        bool wide = false;
+        for (int ks = 0; ks < nk; ks++) wide = screen(lane, ks, valid, true) || wide;
+        if (__any_sync(0xffffffffu, wide)) {
+            if (queued > 0) run(queued);
+            int phead = 0, pairs = 0;
+            for (int ks = 0; ks < nk; ks++) {
+                const bool due = valid && !((Q.hit[ks] >> lane) & 1u);
+                const unsigned d = __ballot_sync(0xffffffffu, due);
+                if (due) Q.pair[(phead + pairs + __popc(d & ((1u << lane) - 1u))) & 63] = (unsigned short)(lane | (ks << 5));
+                pairs += __popc(d);
+                __syncwarp();
+                if (pairs >= 32 || (ks == nk - 1 && pairs > 0)) {
+                    do {
+                        const int c = min(pairs, 32);
+                        const unsigned pr = Q.pair[(phead + (lane < c ? lane : 0)) & 63];
+                        __syncwarp();
+                        phead += c;
+                        pairs -= c;
+                        screen((int)(pr & 31u), (int)(pr >> 5), lane < c, false);
+                    } while (ks == nk - 1 && pairs > 0);
                 }
             }
         }
@@ -274,7 +314,10 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
         Q.hit[lane] = 0u;
         for (int b = 0; b < 32; b++) {
             const unsigned c = __ballot_sync(0xffffffffu, (w >> b) & 1u);
-            if (lane == b) hits += __popc(c);
+            if (lane == b) {
+                hits += __popc(c);
+                if (bits && c) atomicOr(bits + (k0 >> 5), c << (k0 & 31));
+            }
         }
     }
     return hits;

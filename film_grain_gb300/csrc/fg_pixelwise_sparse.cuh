@@ -15,15 +15,11 @@
 //   2. the set bits, ranked in column-major order, list the non-empty cells; their grain counts (the
 //      Poisson draws of src/pixelwise.rs:77-82) are prefix-summed into a CSR over the list and their
 //      grains (centre, radius^2) regenerated into shared memory;
-//   3. sample-major: each thread takes the owned pixels of one offset (or a share of them) and runs the
+//   3. each thread takes the owned pixels of one offset (or a share of them) and runs the
 //      reference's per-sample test: for each cell column i0..i1 of the sample's range
 //      (src/pixelwise.rs:55-58), the bits of rows j0..j1 are cut from the mask, and when any is set
 //      their grains -- contiguous in the CSR, since cells of one column follow each other in the list
 //      -- get the disk test dx*dx + dy*dy <= r*r (src/pixelwise.rs:96-99);
-//      or grain-major (sparse_grain_pass), when a grain's reach is below half an output pixel and the
-//      cost model favours it: a warp takes 32 staged grains, lists the candidate samples within their
-//      radii through a table of the offsets binned by their phase, gives the candidates the same disk
-//      test 32 at a time, and sets a bit per covered sample whose range holds the grain's cell;
 //   4. hit counts go to per-pixel shared counters, then to the output plane (integers, exact in f32).
 // The indicator is an OR over the grains of the sample's cells, so the result equals the reference's
 // early-exit loop bit for bit.
@@ -39,10 +35,6 @@ struct PwSparse {
     static constexpr int kMaskWords = 1280;  // window bitmask, columns an odd number of words apart
     static constexpr int kRowsMax = 256;     // window rows
     static constexpr int kRangeSlots = 4;    // tabulated cell ranges per offset and axis
-    static constexpr int kGmBins = 16;       // phase bins per axis of the grain-major form's offset table
-    static constexpr int kGmBitsWords = 1024;  // owned-sample bits of the grain-major form
-    static constexpr int kGmHitMax = 2560;     // disk tests passed, listed for the hits' pass
-    static constexpr int kGmPairs = 256;       // a warp's queue of (grain, entry) candidates
 };
 
 // Mask words per window column in shared memory: the column's words rounded up to an odd count, so
@@ -67,23 +59,9 @@ struct PwSparseWindow {
     unsigned short list[PwSparse::kListMax];     // non-empty cells: window index i * Hc + j, column-major
     unsigned int gsc[PwSparse::kListMax];        // per listed cell: first grain | grain count << 16
 };
-// Step 3 in the grain-major form (sparse_grain_major), written once the window's cells are read.
-struct PwSparseGrainMajor {
-    float4 ent[kPwKChunk];                       // the offsets by phase bin: o.x, o.y, o.x * zoom, o.y * zoom
-    unsigned short k[kPwKChunk];                 // the entry's offset (index into the x-sorted offsets)
-    unsigned short start[PwSparse::kGmBins * PwSparse::kGmBins + 8];  // first entry of each bin, then n
-    int base[kPwKChunk];                         // first bit of each offset's owned samples
-    unsigned int bits[PwSparse::kGmBitsWords];   // one per owned sample: covered by a grain already
-    unsigned int hits[PwSparse::kGmHitMax];      // (grain, entry) pairs that passed the disk test
-    unsigned short pairs[(PwSparse::kThreads / 32) * PwSparse::kGmPairs];  // per warp: lane << 8 | entry
-};
-
 struct PwSparseShared {
     float4 grains[PwSparse::kGrainMax];          // centre, r^2, window cell (i - wi0) | (j - wj0) << 16 as bits
-    union {
-        PwSparseWindow w;
-        PwSparseGrainMajor gm;
-    };
+    PwSparseWindow w;
     int4 rect[kPwKChunk];                       // owned pixel rectangle per offset: xa, xe, ya, ye
     // cell ranges (sparse_range_code) of the first kRangeSlots columns and rows of each offset's
     // rectangle: entry [slot * n + k]
@@ -94,14 +72,9 @@ struct PwSparseShared {
                                                 // column stored hs = sparse_col_stride(hw) words apart
     int fx0, fx1, fy0, fy1, nsamples;           // owned-pixel footprint, owned samples
     int rw_min, rw_max, rh_min, rh_max;         // extremes of the offsets' rectangle widths and heights
-    int stop, ngrains, any_slow;                // any_slow: a tabulated range code is kRangeSlow
-    int nhits;                                  // disk tests passed in the grain-major form
+    int stop, ngrains;
     float est_grains, est_cells;
 };
-
-static_assert(sizeof(PwSparseGrainMajor) <= sizeof(PwSparseWindow), "the grain-major tables fit the window's space");
-static_assert(PwSparse::kGrainMax <= 2048, "a listed hit holds the grain in 11 bits");
-static_assert(kPwKChunk <= 256, "a queued candidate holds the entry in 8 bits");
 
 // The CTA's PwSparseShared: the start of its dynamic shared memory, named through the shared array
 // itself, so that the out-of-line functions below address it as shared memory (a reference passed in
@@ -121,12 +94,6 @@ struct PwSparseGrid {
     int sbx0, sby0, nsbx, nsby;
     const unsigned int *cellmask;
     int gi0, gj0, gw, ghw;
-    // the grain-major form of step 3 (sparse_grain_major); gm_ent null when the plane does not allow it
-    const float4 *gm_ent;   // [n] the x-sorted offsets by phase bin (PwSparseGrainMajor::ent)
-    const int *gm_idx;      // [n] each entry's offset, then [kGmBins^2 + 1] each bin's first entry
-    float gm_eps;           // rounding margin of a grain's phase band, in output pixels
-    int gm_noslow;          // no sample's cell range can span more than 32 cells (none leaves its window)
-    float gm_grain_cost, gm_sample_cost;  // modelled instructions per staged grain / per owned sample
 };
 
 // The plane's emptiness bitmask (step 0): word (column c, word row k), the lanes of a warp taking neighbouring
@@ -316,177 +283,6 @@ __device__ __noinline__ void sparse_samples(const PixelwiseArgs &a) {
     }
 }
 
-// A disk test of the grain-major form passed: grain (window cell `cell`) covers the sample of offset
-// entry e at pixel (rx, ry).  The sample counts when this block owns it, its cell ranges lie inside the
-// window (else pass 1 decides it), the grain's cell lies in its ranges -- the cells the reference
-// visits for it (src/pixelwise.rs:55-58) -- and no other grain covered it before.  The ranges come
-// from the table, or beyond its slots are computed as the table's entries are.
-__device__ __forceinline__ void sparse_gm_hit(const PixelwiseArgs &a, PwSparseShared &S, int e, unsigned cell, float rx,
-                                              float ry) {
-    using C = PwSparse;
-    const int k = S.gm.k[e];
-    const int x = (int)rx, y = (int)ry;
-    const int4 R = S.rect[k];
-    if (x < R.x || x >= R.y || y < R.z || y >= R.w) return;  // another block's sample
-    const int sx = x - R.x, sy = y - R.z;
-    unsigned cx, cy;
-    if (sx < C::kRangeSlots) cx = S.range_x[sx * a.n + k];
-    else cx = sparse_range_code(xg_of(x, a.inv_zoom, S.gm.ent[e].x), a.rm, a.delta, S.wi0, S.wi1);
-    if (sy < C::kRangeSlots) cy = S.range_y[sy * a.n + k];
-    else cy = sparse_range_code(xg_of(y, a.inv_zoom, S.gm.ent[e].y), a.rm, a.delta, S.wj0, S.wj1);
-    if (cx == kRangeSlow || cy == kRangeSlow) return;
-    if ((cell & 0xFFFFu) - (cx & 0x7FFu) > (cx >> 11) || (cell >> 16) - (cy & 0x7FFu) > (cy >> 11)) return;
-    const int idx = S.gm.base[k] + sy * (R.y - R.x) + sx;
-    const unsigned bit = 1u << (idx & 31);
-    if (!(atomicOr(&S.gm.bits[idx >> 5], bit) & bit)) sparse_count_hit(a, S, x, y);
-}
-
-// Step 3, grain-major: each thread takes staged grains and finds the owned samples within their radius.
-// Sample k of pixel x lies at xg = (x + 0.5) / zoom - o.x, so a grain at gx can cover only the pixel
-// x = rint(gx * zoom - 0.5 + o.x * zoom) of each offset (its reach r * zoom is below half a pixel), and
-// only offsets whose phase frac(o.x * zoom) lies within r * zoom + eps of frac(0.5 - gx * zoom) reach
-// it: the offsets are binned by their two phases (kGmBins^2 bins), and a grain visits the bins its
-// phase band covers.  Every candidate gets the reference's disk test on the reference's xg, yg
-// (src/pixelwise.rs:96-99); the band only has to contain every pixel that can pass it.  A sample's
-// covering grains are OR-ed through its bit, so the count equals the sample-major form's.
-// The pixel coordinate of offset entry O that grain coordinate p = g * zoom - 0.5 can reach, as a float:
-// p + o * zoom rounded to an integer by adding and removing 1.5 * 2^23.
-__device__ __forceinline__ float gm_pixel(float p, float oz) {
-    constexpr float kRint = 12582912.0f;
-    return FG_FSUB(FG_FADD(FG_FADD(p, oz), kRint), kRint);
-}
-
-// A passed disk test is listed as grain | entry << 11 and decided after the pass, the list dealt across
-// all lanes (the decision reads the rectangle, the ranges and the bit; in the pass a warp would run it
-// for a few lanes at a time, and a lane deciding its own tests leaves the warp as slow as its busiest
-// lane: both measured slower); once the list is full a test is decided on the spot.
-__device__ __forceinline__ void gm_pass_test(const PixelwiseArgs &a, PwSparseShared &S, int t, int e) {
-    using C = PwSparse;
-    const float4 G = S.grains[t];
-    const float4 O = S.gm.ent[e];
-    const float px = FG_FSUB(FG_FMUL(G.x, a.zoom), 0.5f), py = FG_FSUB(FG_FMUL(G.y, a.zoom), 0.5f);
-    const float rx = gm_pixel(px, O.z), ry = gm_pixel(py, O.w);
-    // xg_of of pixel (rx, ry): rx + 0.5 is exact
-    const float dx = FG_FSUB(FG_FSUB(FG_FMUL(FG_FADD(rx, 0.5f), a.inv_zoom), O.x), G.x);
-    const float dy = FG_FSUB(FG_FSUB(FG_FMUL(FG_FADD(ry, 0.5f), a.inv_zoom), O.y), G.y);
-    if (FG_FADD(FG_FMUL(dx, dx), FG_FMUL(dy, dy)) <= G.z) {
-        const int slot = atomicAdd(&S.nhits, 1);
-        if (slot < C::kGmHitMax) S.gm.hits[slot] = (unsigned)t | ((unsigned)e << 11);
-        else sparse_gm_hit(a, S, e, __float_as_uint(G.w), rx, ry);
-    }
-}
-
-// A warp takes 32 grains at a time, one per lane: each lane finds its grain's band of bins and counts
-// the entries in them (3.5 on the large frame, 0 to 8 typically), the warp lists its (grain, entry)
-// candidates in its queue at the lanes' prefix of the counts, and then tests the listed candidates 32
-// at a time, every lane busy (a lane testing its own grain's candidates leaves the warp waiting for its
-// busiest lane); a round with more candidates than the queue holds is tested lane by lane.
-__device__ __noinline__ void sparse_grain_pass(const PixelwiseArgs &a, const PwSparseGrid &g) {
-    PwSparseShared &S = sparse_smem();
-    using C = PwSparse;
-    constexpr int B = PwSparse::kGmBins;
-    PwSparseGrainMajor &M = S.gm;
-    const float z = a.zoom, zr = a.zoom * 1.0000039f;  // (1 + 2^-18): sqrt's rounding
-    const int ng = S.ngrains, lane = threadIdx.x & 31;
-    unsigned short *Q = M.pairs + (threadIdx.x >> 5) * C::kGmPairs;
-    for (int t0 = threadIdx.x & ~31; t0 < ng; t0 += blockDim.x) {  // warp-uniform bounds (the shuffles)
-        const int t = t0 + lane;
-        int bx0 = 0, bx1 = -1, by0 = 0, by1 = -1;  // an empty band unless the grain can cover a sample
-        if (t < ng) {
-            const float4 G = S.grains[t];
-            if (G.z >= 0.0f) {  // a radius <= 0 (r^2 = -1) covers nothing
-                const float w = fmaf(sqrtf(G.z), zr, g.gm_eps);  // half-width of the phase band
-                const float px = FG_FSUB(FG_FMUL(G.x, z), 0.5f), py = FG_FSUB(FG_FMUL(G.y, z), 0.5f);
-                float lx = FG_FSUB(FG_FSUB(floorf(px), px), w), ly = FG_FSUB(FG_FSUB(floorf(py), py), w);
-                lx = FG_FSUB(lx, floorf(lx));  // the band starts at phase lx in [0, 1) and spans 2w
-                ly = FG_FSUB(ly, floorf(ly));
-                bx0 = min((int)(lx * (float)B), B - 1);
-                bx1 = (int)((lx + 2.0f * w) * (float)B);
-                by0 = min((int)(ly * (float)B), B - 1);
-                by1 = (int)((ly + 2.0f * w) * (float)B);
-            }
-        }
-        // the band's entries: bins bx0..bx1 of bin rows by0..by1, bins past the last wrapping to the first
-        auto for_each_range = [&](auto f) {
-            for (int by = by0; by <= by1; by++) {
-                const int row = (by & (B - 1)) * B;
-                f(M.start[row + bx0], M.start[row + min(bx1, B - 1) + 1]);
-                if (bx1 >= B) f(M.start[row], M.start[row + bx1 - B + 1]);
-            }
-        };
-        int cnt = 0;
-        for_each_range([&](int e0, int e1) { cnt += e1 - e0; });
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        if (total <= C::kGmPairs) {
-            int q = incl - cnt;
-            for_each_range([&](int e0, int e1) {
-                for (int e = e0; e < e1; e++) Q[q++] = (unsigned short)((lane << 8) | e);
-            });
-            __syncwarp();
-            for (int i = lane; i < total; i += 32) {
-                const unsigned pr = Q[i];
-                gm_pass_test(a, S, t0 + (int)(pr >> 8), (int)(pr & 0xFFu));
-            }
-            __syncwarp();  // the queue is read before the next round writes it
-        } else {
-            for_each_range([&](int e0, int e1) {
-                for (int e = e0; e < e1; e++) gm_pass_test(a, S, t, e);
-            });
-        }
-    }
-    __syncthreads();
-    const int nh = min(S.nhits, C::kGmHitMax);
-    for (int h = threadIdx.x; h < nh; h += blockDim.x) {
-        const unsigned tok = M.hits[h];
-        const int e = (int)(tok >> 11);
-        const float4 G = S.grains[tok & 0x7FFu];
-        const float4 O = M.ent[e];
-        const float rx = gm_pixel(FG_FSUB(FG_FMUL(G.x, z), 0.5f), O.z);
-        const float ry = gm_pixel(FG_FSUB(FG_FMUL(G.y, z), 0.5f), O.w);
-        sparse_gm_hit(a, S, e, __float_as_uint(G.w), rx, ry);
-    }
-}
-
-// Step 3 in the grain-major form: the owned samples' bit bases (a scan of the rectangles' areas), the
-// phase-binned offsets, then the grains' pass.  Samples whose range leaves the window go to the
-// per-sample loop as in the sample-major form: with every rectangle inside the range table the
-// ownership pass saw them (any_slow); otherwise the plane's ranges span too few cells for any
-// (gm_noslow).
-__device__ __noinline__ void sparse_grain_major(const PixelwiseArgs &a, const PwSparseGrid &g) {
-    PwSparseShared &S = sparse_smem();
-    using C = PwSparse;
-    const int tid = threadIdx.x, nthreads = blockDim.x;
-    PwSparseGrainMajor &M = S.gm;
-    int area = 0;
-    if (tid < a.n) {  // n <= kPwKChunk = the CTA size
-        const int4 R = S.rect[tid];
-        if (R.y > R.x && R.w > R.z) area = (R.y - R.x) * (R.w - R.z);
-    }
-    int total;
-    const int base = block_excl_scan(area, S.wsum, &total);
-    if (tid < a.n) M.base[tid] = base;
-    for (int e = tid; e < a.n; e += nthreads) {
-        M.ent[e] = g.gm_ent[e];
-        M.k[e] = (unsigned short)g.gm_idx[e];
-    }
-    for (int b = tid; b <= C::kGmBins * C::kGmBins; b += nthreads) M.start[b] = (unsigned short)g.gm_idx[a.n + b];
-    for (int w = tid; w < (total + 31) >> 5; w += nthreads) M.bits[w] = 0u;
-    if (tid == 0) S.nhits = 0;
-    __syncthreads();
-    if (!(a.rm > 0.0f)) return;  // a grain radius is at most rm: nothing can cover a sample
-    sparse_grain_pass(a, g);
-    if (S.any_slow) {  // uniform
-        const unsigned slow = sparse_sample_pass<1>(a, S);
-        if (slow) atomicAdd(&a.diag[0], (unsigned long long)slow);
-    }
-}
-
 __device__ __noinline__ void sparse_slow_sample(const PixelwiseArgs &a, float xg, float yg, int x, int y) {
     PwSparseShared &S = sparse_smem();
     const int i0 = f2i_floor(FG_FDIV(FG_FSUB(xg, a.rm), a.delta));
@@ -609,7 +405,6 @@ __device__ __noinline__ int pixelwise_sparse_block(const PixelwiseArgs &a, const
         S.est_cells = 0.0f;
         S.fx0 = 0x7fffffff; S.fx1 = -1; S.fy0 = 0x7fffffff; S.fy1 = -1; S.nsamples = 0;
         S.rw_min = 0x7fffffff; S.rw_max = -1; S.rh_min = 0x7fffffff; S.rh_max = -1;
-        S.any_slow = 0;
     }
     __syncthreads();
     // ---- expected grains and non-empty cells of the window: lambda integrated over its rectangle (a
@@ -647,7 +442,6 @@ __device__ __noinline__ int pixelwise_sparse_block(const PixelwiseArgs &a, const
     {
         int lx0 = 0x7fffffff, lx1 = -1, ly0 = 0x7fffffff, ly1 = -1, ns = 0;
         int wmin = 0x7fffffff, wmax = -1, hmin = 0x7fffffff, hmax = -1;
-        bool slow = false;
         for (int k = tid; k < a.n; k += nthreads) {
             const float2 o = a.offs[k];
             const int xa = first_at_least(X0, a.out_w, a.inv_zoom, a.zoom, o.x);
@@ -659,12 +453,10 @@ __device__ __noinline__ int pixelwise_sparse_block(const PixelwiseArgs &a, const
             for (int s2 = 0; s2 < min(xe - xa, C::kRangeSlots); s2++) {
                 const unsigned c = sparse_range_code(xg_of(xa + s2, a.inv_zoom, o.x), a.rm, a.delta, wi0, wi1);
                 S.range_x[s2 * a.n + k] = (unsigned short)c;
-                slow |= c == kRangeSlow;
             }
             for (int s2 = 0; s2 < min(ye - ya, C::kRangeSlots); s2++) {
                 const unsigned c = sparse_range_code(xg_of(ya + s2, a.inv_zoom, o.y), a.rm, a.delta, wj0, wj1);
                 S.range_y[s2 * a.n + k] = (unsigned short)c;
-                slow |= c == kRangeSlow;
             }
             wmin = min(wmin, xe - xa); wmax = max(wmax, xe - xa);
             hmin = min(hmin, ye - ya); hmax = max(hmax, ye - ya);
@@ -683,9 +475,7 @@ __device__ __noinline__ int pixelwise_sparse_block(const PixelwiseArgs &a, const
         wmax = __reduce_max_sync(0xffffffffu, wmax);
         hmin = __reduce_min_sync(0xffffffffu, hmin);
         hmax = __reduce_max_sync(0xffffffffu, hmax);
-        slow = __any_sync(0xffffffffu, slow);
         if (lane == 0) {
-            if (slow) S.any_slow = 1;
             if (ns > 0) {
                 atomicAdd(&S.nsamples, ns);
                 atomicMin(&S.fx0, lx0); atomicMax(&S.fx1, lx1);
@@ -738,14 +528,8 @@ __device__ __noinline__ int pixelwise_sparse_block(const PixelwiseArgs &a, const
     // ---- 2. non-empty cells, their counts and grains
     if (!sparse_stage(a)) return 1;
 
-    // ---- 3. the owned samples: grain-major when the plane allows it, the samples whose range leaves the
-    // window are known (the plane has none, or every rectangle fits the range table), the samples fit the
-    // bit array and the cost model favours it; else sample-major
-    const bool gm = g.gm_ent && (g.gm_noslow || (S.rw_max <= C::kRangeSlots && S.rh_max <= C::kRangeSlots)) &&
-                    S.nsamples <= 32 * C::kGmBitsWords &&
-                    (float)S.ngrains * g.gm_grain_cost < (float)S.nsamples * g.gm_sample_cost;
-    if (gm) sparse_grain_major(a, g);
-    else sparse_samples(a);
+    // ---- 3. the owned samples
+    sparse_samples(a);
     __syncthreads();
 
     // ---- 4. flush the per-pixel counts
@@ -757,7 +541,7 @@ __device__ __noinline__ int pixelwise_sparse_block(const PixelwiseArgs &a, const
     }
     if (tid == 0) {
         atomicAdd(&a.diag[3], 1ull);
-        atomicAdd(&a.diag[gm ? 5 : 4], 1ull);
+        atomicAdd(&a.diag[4], 1ull);
     }
     return 0;
 }

@@ -315,3 +315,33 @@ def test_pixelwise_small_plane_parts(cuda, fgl, orc, n):
     if n <= 5:
         assert fgl.pixelwise_kernel_count(p, d) == 3
     _check("pixel", fgl, orc, plane, radius=0.2, n=n, seed=3)
+
+
+@pytest.mark.parametrize("w,h,radius,dist,zoom,n,cell", [
+    (128, 70, 0.15, "const", 1.0, 32, None),     # a word of bits a pixel
+    (131, 67, 0.15, "const", 1.0, 33, None),     # two
+    (97, 101, 0.1, "const", 1.0, 65, None),      # four
+    (97, 101, 0.08, "lognorm", 1.0, 129, None),  # eight; ranges of several cells
+    (103, 91, 0.05, "lognorm", 1.0, 256, None),
+    (200, 180, 0.7, "const", 0.5, 50, None),     # grains wider than an input pixel
+    (41, 33, 0.12, "const", 3.0, 40, None),      # reach 0.36 of a pixel
+    (120, 90, 0.3, "const", 1.0, 64, 1.0),       # cells of a pixel, the rejection regime
+    (110, 90, 0.3, "const", 1.0, 20, 0.04),      # ranges of 16 cells: no per-sample kernel
+])
+def test_pixelwise_stream_pass(cuda, fgl, orc, w, h, radius, dist, zoom, n, cell):
+    """The stream pass: widths off the segments and tiles, every variant of words, dark, middle and saturated
+    areas (the last on the per-sample kernel, where its ranges allow)."""
+    plane = _blobs(w, h)
+    plane[: h // 3, : w // 2] = 1.0
+    plane[h // 2:, : w // 5] = 0.0
+    kw = dict(radius=radius, dist=dist, sd=0.4 * radius if dist == "lognorm" else 0.0, zoom=zoom, n=n, cell=cell, seed=9)
+    p, d, *_ = _setup(fgl, orc, plane, **kw)
+    assert fgl.pixelwise_kernel_count(p, d) == 6
+    _check("pixel", fgl, orc, plane, **kw)
+    assert fgl.pixelwise_sparse_forms()[1] > 0
+
+
+def test_pixelwise_stream_all_dense_and_empty(cuda, fgl, orc):
+    _check("pixel", fgl, orc, np.ones((96, 100), np.float32), radius=0.1, n=64, seed=3)
+    assert fgl.pixelwise_diagnostics()[0] == 96 * 100 * 64  # every segment on the per-sample kernel
+    _check("pixel", fgl, orc, np.zeros((96, 100), np.float32), radius=0.1, n=64, seed=3)

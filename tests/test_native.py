@@ -67,6 +67,18 @@ def test_screen_by_two_seed_words_misses_no_cell(tmp_path):
     assert checked2 == 200000 * 9 and 0 < extra < checked2 / 128
 
 
+def test_phase_masks_hold_every_offset_in_reach(tmp_path):
+    """The stream pass's masks: no offset within a grain's half-width is left out, and the ones that pass beyond
+    those fit the buckets and classes: a half-width counts as up to a quarter of the largest more, and the
+    fraction as up to 1/128 off, so on average over uniform half-widths (half the largest, w_max 0.02..0.4) at
+    most twice the offsets pass."""
+    exe = _compile("phase_check.cpp", "phase_check", tmp_path)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()
+    checked, missed, passed, counted = (int(v) for v in out)
+    assert checked == 400 * 6 * (1 + 31 + 32 + 33 + 64 + 100 + 256) and missed == 0
+    assert counted <= passed < 2 * counted
+
+
 def test_samplers_on_32_bit_pipes_match_f64_samplers(tmp_path):
     """poisson_count, knuth_count_f32 and lognormal_radius_f32 give the f64 samplers' values and stream
     positions on every stream (both Poisson regimes and the ends of the f32 rejection's range, cell

@@ -294,10 +294,10 @@ fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_der
                             int *d_cancel) {
     const int in_w = (int)d.input_width, in_h = (int)d.input_height;
     const int out_w = (int)d.output_width, out_h = (int)d.output_height;
-    FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, w.cells, d_out, w.bits ? 0 : (long long)out_w * out_h,
-                               w.counters, s),
+    FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, w.cells,
+                               w.bits ? w.bits : reinterpret_cast<unsigned int *>(d_out),
+                               w.bits ? (long long)(w.bits_bytes / sizeof(int)) : (long long)out_w * out_h, w.counters, s),
             "cell params");
-    if (w.bits) FG_CUDA(cudaMemsetAsync(w.bits, 0, w.bits_bytes, s), "clear bits");
     PixelwiseArgs a = pixelwise_args(p, d, pl, d_lam, w.cells, w.offs, d_out, w.counters->diag);
     a.cancel = d_cancel;
     FG_CUDA(launch_pixelwise(a, pl.nby, w.listed ? w.counters : nullptr, w.mask, w.bits, s), "pixelwise kernel");

@@ -164,9 +164,10 @@ struct LogfTableDev {
     int shift;
 };
 
-// The cell table, and the plane's output and counters set to zero beside it.
-cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, float *out,
-                               long long n_out, PwCounters *counters, cudaStream_t s);
+// The cell table, and n_clear words (the output's floats, or the samples' bits) and the counters set to zero
+// beside it.
+cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, unsigned int *clear,
+                               long long n_clear, PwCounters *counters, cudaStream_t s);
 // counters: null (fat CTAs over every block) or cleared, with nbx*nby ints behind them (lean or sparse pass,
 // then fat CTAs over the deferred blocks).
 // cellmask: null, or pixelwise_cellmask_bytes(a, nby) bytes for the sparse pass's plane bitmask (the

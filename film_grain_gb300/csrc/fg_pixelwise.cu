@@ -37,14 +37,15 @@
 namespace fg {
 
 // ------------------------------------------------------------------ per-pixel Poisson set-up
-// The output and the counters are cleared here too: each memset of its own was 6 us of a small plane's 208 us
+// What the later kernels add to -- the output or the bits, and the counters -- is cleared here too: each memset
+// of its own was 6 us of the 208 us of a small plane
 // between its first and last launch, which are bound by the host's enqueueing.
 __global__ void cell_params_kernel(const float *__restrict__ lam, long long n, float delta,
-                                   CellParam *__restrict__ cells, float *__restrict__ out, long long n_out,
-                                   PwCounters *__restrict__ counters) {
+                                   CellParam *__restrict__ cells, unsigned int *__restrict__ clear,
+                                   long long n_clear, PwCounters *__restrict__ counters) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < (long long)(sizeof(PwCounters) / sizeof(int))) reinterpret_cast<int *>(counters)[i] = 0;
-    if (i < n_out) out[i] = 0.0f;
+    if (i < n_clear) clear[i] = 0u;
     if (i >= n) return;
     float l = lam[i];
     CellParam c;
@@ -67,12 +68,12 @@ __global__ void cell_params_kernel(const float *__restrict__ lam, long long n, f
     cells[i] = c;
 }
 
-cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, float *out,
-                               long long n_out, PwCounters *counters, cudaStream_t s) {
+cudaError_t launch_cell_params(const float *lam, int in_w, int in_h, float delta, CellParam *cells, unsigned int *clear,
+                               long long n_clear, PwCounters *counters, cudaStream_t s) {
     const long long n = (long long)in_w * in_h;
-    const long long grid = (std::max(n, n_out) + 255) / 256;  // 256 threads and more: all words of the counters
+    const long long grid = (std::max(n, n_clear) + 255) / 256;  // 256 threads and more: all words of the counters
     if (grid <= 0) return cudaSuccess;
-    cell_params_kernel<<<(unsigned)grid, 256, 0, s>>>(lam, n, delta, cells, out, n_out, counters);
+    cell_params_kernel<<<(unsigned)grid, 256, 0, s>>>(lam, n, delta, cells, clear, n_clear, counters);
     return cudaGetLastError();
 }
 
@@ -249,8 +250,6 @@ static bool plan_stream(const PixelwiseArgs &a, const PwSparseGrid &g, int sms, 
     if ((double)a.out_w * a.out_h * t->nw * 4.0 > kCellMaskMaxBytes) return false;
     t->gi0 = g.gi0; t->gj0 = g.gj0; t->gw = g.gw; t->ghw = g.ghw;
     t->segs = (a.out_w + 31) / 32;
-    t->sub = 1;
-    while (t->sub < 8 && (double)t->gw / 32.0 * t->ghw * t->sub < 128.0 * sms) t->sub *= 2;
     for (int T = 512; T >= 32; T >>= 1) {
         auto edge = [&](float lo, float hi) {
             return std::floor(((double)T * a.delta + 2.0 * a.rm + (double)hi - (double)lo) * a.zoom) + 8.0;
@@ -261,6 +260,9 @@ static bool plan_stream(const PixelwiseArgs &a, const PwSparseGrid &g, int sms, 
         t->nty = (32 * t->ghw + T - 1) / T;
         if (words <= (T == 32 ? 12288.0 : 4096.0) && (T == 32 || (double)t->ntx * t->nty >= 32.0 * sms)) {
             t->fp_words = (int)words;
+            // parts of a tile's chunks: one or two for each of its eight warps
+            const int chunks = (T / 32) * (T / 32);
+            t->sub = chunks >= 16 ? 1 : chunks >= 4 ? 4 : 8;
             return (double)t->ntx * t->nty < 2.0e9;
         }
     }
@@ -424,8 +426,12 @@ static cudaError_t launch_pixelwise_stream(const PixelwiseArgs &a, const PwSpars
                   : launch_stream<8>(a, t, sms, s);
     if (e != cudaSuccess) return e;
     const long long ctas = std::min<long long>((nseg + 7) / 8, 4LL * std::max(1, sms));
-    pixelwise_dense_kernel<<<(unsigned)ctas, kPwRegenThreads, 0, s>>>(a, bits, t.nw, t.segs, &counters->list[0], u.count,
-                                                                     u.list);
+    // Parts of eight samples: the last round of a part's cells is partly idle, which parts of four pay more often
+    // (1024^2 log-normal 15.6 ms against 14.9), but where segments are few their warps' latency counts more
+    // (256^2 ramp 0.32 ms against 0.35).
+    const int part = nseg < 32LL * sms ? 4 : 8;
+    pixelwise_dense_kernel<<<(unsigned)ctas, kPwRegenThreads, 0, s>>>(a, bits, t.nw, t.segs, part, &counters->list[0],
+                                                                     u.count, u.list);
     return cudaGetLastError();
 }
 

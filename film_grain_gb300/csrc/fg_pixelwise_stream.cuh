@@ -27,7 +27,9 @@
 namespace fg {
 
 struct PwStream {
-    static constexpr int kThreads = 128;
+    // Eight warps share a tile's tables and bits: four take 1024^2 log-normal, N 256 from 14.9 to 16.4 ms, and leave
+    // the saturated tiles of small planes to fewer (200^2 ramp radius 0.2, N 200: 0.54 ms against 0.81).
+    static constexpr int kThreads = 256;
     static constexpr int kPairs = 256;               // a warp's queue of (grain, entry) candidates
 };
 
@@ -41,9 +43,9 @@ struct PwStreamShared {
     float4 ent[32 * NW];  // the offsets: o.x, o.y, o.x * zoom, o.y * zoom
     unsigned int mask[phase_table_words(NW)];  // [axis][class][bucket][word]
     PwStreamWarp warp[PwStream::kThreads / 32];
-    int tile, chunk;
+    int tile, chunk, unused[2];
     // then the tile's bits: pixel (x, y) of the footprint has words [(y * fw + x) * nw, +nw)
-    unsigned int bits[2];
+    __device__ __forceinline__ unsigned int *bits() { return reinterpret_cast<unsigned int *>(this + 1); }
 };
 
 // tile: edge in cells (a multiple of 32); ntx x nty tiles from cell (gi0, gj0); nw: words of a pixel's bits;
@@ -125,7 +127,7 @@ __device__ __forceinline__ void stream_test(const PixelwiseArgs &a, const PwStre
     if (!hit) return;
     const int x = (int)rx - fx0, y = (int)ry - fy0;
     if ((unsigned)x < (unsigned)fw && (unsigned)y < (unsigned)fh)  // else outside the plane
-        atomicOr(&S.bits[(y * fw + x) * g.nw + (e >> 5)], 1u << (e & 31));
+        atomicOr(S.bits() + (y * fw + x) * g.nw + (e >> 5), 1u << (e & 31));
 }
 
 // The candidates of 32 grains, one per lane (G.rr < 0: none): each lane intersects the two axes' words for its
@@ -180,16 +182,18 @@ __device__ __forceinline__ void stream_candidates(const PixelwiseArgs &a, const 
     }
 }
 
-// Dynamic shared memory: PwStreamShared with fp_words words of bits.
+// Dynamic shared memory: PwStreamShared and fp_words words of bits.
 template <int NW>
 __global__ void __launch_bounds__(PwStream::kThreads)
     pixelwise_stream_kernel(const __grid_constant__ PixelwiseArgs a, const __grid_constant__ PwStreamGrid g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PwStreamShared<NW> &S = *reinterpret_cast<PwStreamShared<NW> *>(smem_raw);
+    constexpr int nthreads = PwStream::kThreads;
     const int tid = threadIdx.x, lane = tid & 31;
     PwStreamWarp &W = S.warp[tid >> 5];
-    for (int e = tid; e < a.n; e += PwStream::kThreads) S.ent[e] = g.ent[e];
-    for (int b = tid; b < phase_table_words(NW); b += PwStream::kThreads) S.mask[b] = g.masks[b];
+    unsigned int *bits = S.bits();
+    for (int e = tid; e < a.n; e += nthreads) S.ent[e] = g.ent[e];
+    for (int b = tid; b < phase_table_words(NW); b += nthreads) S.mask[b] = g.masks[b];
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
     const int ntiles = g.ntx * g.nty, chunk_rows = g.tile >> 5;
     const bool any_dense = *g.dense_count != 0;
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(PwStream::kThreads)
         const int fw = fx1 - fx0 + 1, fh = fy1 - fy0 + 1;
         if (fw <= 0 || fh <= 0 || (long long)fw * fh * g.nw > g.fp_words) continue;  // (the plan's bound holds)
         const int row_words = fw * g.nw, words = row_words * fh;
-        for (int w = tid; w < words; w += PwStream::kThreads) S.bits[w] = 0u;
+        for (int w = tid; w < words; w += nthreads) bits[w] = 0u;
         __syncthreads();
 
         int head = 0, queued = 0, ghead = 0, grains = 0;  // the warp's rings; uniform
@@ -231,33 +235,38 @@ __global__ void __launch_bounds__(PwStream::kThreads)
             G.j = g.gj0 + 32 * tw + (int)(__float_as_uint(v.w) >> 16);
             stream_candidates<NW>(a, g, S, W, G, fx0, fy0, fw, fh);
         };
-        auto draw = [&](int count) {  // the first `count` cells, one per lane
-            const uint2 cell = W.cell[(head + (lane < count ? lane : 0)) & 63];
-            __syncwarp();
-            head += count;
-            queued -= count;
-            const int i = g.gi0 + (int)cell.x, j = g.gj0 + (int)cell.y;
-            const float at = __uint_as_float((cell.x - (unsigned)tc) | ((cell.y - 32u * (unsigned)tw) << 16));
-            Xoshiro rng;
-            uint32_t q = 0u;
-            if (lane < count) q = sparse_cell_count(a, i, j, &rng);
-            const float sx = FG_FMUL((float)i, a.delta), sy = FG_FMUL((float)j, a.delta);
-            while (__any_sync(0xffffffffu, q != 0u)) {
-                float4 v = make_float4(0.0f, 0.0f, -1.0f, at);
-                if (q != 0u) {
-                    q--;
-                    v.x = FG_FADD(sx, uniform_f32_from(U, rng.next()));
-                    v.y = FG_FADD(sy, uniform_f32_from(U, rng.next()));
-                    float r = radius_draw(a, rng);
-                    if (r > a.rm) r = a.rm;
-                    if (r > 0.0f) v.z = FG_FMUL(r, r);  // a radius <= 0 covers nothing
-                }
-                const unsigned have = __ballot_sync(0xffffffffu, v.z >= 0.0f);
-                if (v.z >= 0.0f) W.grain[(ghead + grains + __popc(have & ((1u << lane) - 1u))) & 63] = v;
-                grains += __popc(have);
-                __syncwarp();
-                if (grains >= 32) cover(32);
+        // Each lane draws the grains of one cell, one a step, and takes the next cell from the ring when it has
+        // no more: a lane whose cell holds several grains does not leave the others waiting.
+        Xoshiro rng = {0, 0, 0, 0};
+        uint32_t q = 0u;
+        float sx = 0.0f, sy = 0.0f, at = 0.0f;
+        auto step = [&]() {
+            const unsigned idle = __ballot_sync(0xffffffffu, q == 0u);
+            const int take = min(queued, __popc(idle)), rank = __popc(idle & ((1u << lane) - 1u));
+            if (q == 0u && rank < take) {
+                const uint2 cell = W.cell[(head + rank) & 63];
+                const int i = g.gi0 + (int)cell.x, j = g.gj0 + (int)cell.y;
+                at = __uint_as_float((cell.x - (unsigned)tc) | ((cell.y - 32u * (unsigned)tw) << 16));
+                sx = FG_FMUL((float)i, a.delta);
+                sy = FG_FMUL((float)j, a.delta);
+                q = sparse_cell_count(a, i, j, &rng);
             }
+            head += take;
+            queued -= take;
+            float4 v = make_float4(0.0f, 0.0f, -1.0f, at);
+            if (q != 0u) {
+                q--;
+                v.x = FG_FADD(sx, uniform_f32_from(U, rng.next()));
+                v.y = FG_FADD(sy, uniform_f32_from(U, rng.next()));
+                float r = radius_draw(a, rng);
+                if (r > a.rm) r = a.rm;
+                if (r > 0.0f) v.z = FG_FMUL(r, r);  // a radius <= 0 covers nothing
+            }
+            const unsigned have = __ballot_sync(0xffffffffu, v.z >= 0.0f);
+            if (v.z >= 0.0f) W.grain[(ghead + grains + __popc(have & ((1u << lane) - 1u))) & 63] = v;
+            grains += __popc(have);
+            __syncwarp();
+            if (grains >= 32) cover(32);
         };
         const int rows = 32 / g.sub;
         for (;;) {
@@ -295,31 +304,31 @@ __global__ void __launch_bounds__(PwStream::kThreads)
                 }
                 queued += __popc(pending);
                 __syncwarp();
-                if (queued >= 32) draw(32);
+                while (queued >= 32) step();  // (a step takes as many cells as lanes are idle)
             }
         }
-        if (queued > 0) draw(queued);
+        while (queued > 0 || __any_sync(0xffffffffu, q != 0u)) step();
         if (grains > 0) cover(grains);
         __syncthreads();
         if (tid == 0) {
             atomicAdd(&a.diag[3], 1ull);
             atomicAdd(&a.diag[5], 1ull);
         }
-        for (int w = tid; w < words; w += PwStream::kThreads) {
-            const unsigned v = S.bits[w];
+        for (int w = tid; w < words; w += nthreads) {
+            const unsigned v = bits[w];
             if (v)
                 atomicOr(g.bits + ((long long)(fy0 + w / row_words) * a.out_w + fx0) * g.nw + w % row_words, v);
         }
     }
 }
 
-// The segments left to the per-sample pass, their samples in parts of kDensePart: each warp takes the next part.
-constexpr int kDensePart = 8;
+// The segments left to the per-sample pass, their samples in parts of `part` (a divisor of 32): each warp takes the
+// next part.
 __global__ void __launch_bounds__(kPwRegenThreads)
-    pixelwise_dense_kernel(const __grid_constant__ PixelwiseArgs a, unsigned int *bits, int nw, int segs,
+    pixelwise_dense_kernel(const __grid_constant__ PixelwiseArgs a, unsigned int *bits, int nw, int segs, int part,
                            int *__restrict__ next, const int *__restrict__ count, const int *__restrict__ list) {
     __shared__ RegenQueue queues[kPwRegenThreads / 32];
-    const int lane = threadIdx.x & 31, parts = (a.n + kDensePart - 1) / kDensePart;
+    const int lane = threadIdx.x & 31, parts = (a.n + part - 1) / part;
     const long long n = (long long)*count * parts;
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
     unsigned long long done = 0;
@@ -329,7 +338,7 @@ __global__ void __launch_bounds__(kPwRegenThreads)
         i = __shfl_sync(0xffffffffu, i, 0);
         if (i < 0 || i >= n) break;
         const int seg = list[i / parts], y = seg / segs, x = 32 * (seg % segs) + lane;
-        const int k0 = i % parts * kDensePart, k1 = min(a.n, k0 + kDensePart);
+        const int k0 = i % parts * part, k1 = min(a.n, k0 + part);
         const bool valid = x < a.out_w;
         pixelwise_pixel_queue(a, U, x, y, valid, k0, k1, queues[threadIdx.x >> 5],
                               valid ? bits + ((long long)y * a.out_w + x) * nw : nullptr);

@@ -12,11 +12,12 @@
 // 0 .. 2.  Three accumulators (kx) stay in tensor memory over the CTA's whole share of the rows; the first one
 // has 16 more columns, for a constant slot whose channel 0 is one: their sum of g is the bias gradient.
 // A CTA (one per SM, three roles: loader, MMA issuer, and everyone for the end) walks a contiguous range of
-// row blocks through two stages, then adds its result up in shared memory and onto dW and db with one atomic
+// row blocks through two or four stages, then adds its result up in shared memory and onto dW and db with one atomic
 // per element (the sums over CTAs were f32 atomics before, too).
 //
 // Measured on 256 tiles of 64^2, 32 -> 32 channels (134 MB, 20 us at the measured copy rate): mma.sync with
-// operands staged channel by channel 267 us, this kernel 63 us.
+// operands staged channel by channel 267 us; this split 63 us; four stages of 64 columns 50 us; the end's sums
+// without shared-memory atomics 45 us.  What is left: the input rows, read 5/3 times, and the steps' copies.
 //
 // Waits are bounded as in fg_sg_tc.cu; a CTA whose wait ran out adds NaN to dW and db.
 #include <algorithm>
@@ -28,19 +29,19 @@
 namespace fg {
 
 constexpr int kWgThreads = 192;  // loader, MMA issuer, four warps that read the accumulators
-constexpr int kWgPx = 128;       // columns of a row tile
 
-template <int CG, int CX>  // channels of a gradient pixel (16 or 32) and of an input pixel in shared memory
-struct WgCfg {
+template <int CG, int CX, int PX>  // channels of a gradient pixel (16 or 32) and of an input pixel in shared
+struct WgCfg {                     // memory, columns of a row tile (128, or 64 for images no wider)
     static constexpr int kRows = CX == 32 ? 3 : 4;  // gradient rows per step
     static constexpr int kXRows = kRows + 2;
     static constexpr int kGSlots = 128 / CG;
-    static constexpr int kGRow = kWgPx * 2 * CG, kXRow = (kWgPx + 8) * 2 * CX;  // bytes of a row slot
+    static constexpr int kGRow = PX * 2 * CG, kXRow = (PX + 8) * 2 * CX;  // bytes of a row slot
     static constexpr int kX = kGSlots * kGRow;                                  // the input rows, then the ones
     static constexpr int kStage = (kX + (kXRows + 1) * kXRow + 1023) / 1024 * 1024;
     static constexpr int kN = kXRows * CX;
-    static constexpr int kBar = 2 * kStage;
-    static constexpr int kSmem = kBar + 64;
+    static constexpr int kStages = PX == 64 ? 4 : 2;
+    static constexpr int kBar = kStages * kStage;
+    static constexpr int kSmem = kBar + 16 * kStages + 32;
     static constexpr uint64_t kSwG = CG == 32 ? 4ull : 6ull, kSwX = CX == 32 ? 4ull : 6ull;
     static constexpr int kSum = 9 * CX * 33;  // the CTA's sums: [tap * CX + ci][33] by co, then db
     static_assert(3 * kN + 16 <= 512 && kSum * 4 + 128 <= kStage && kSmem <= 227 * 1024, "sizes");
@@ -54,19 +55,20 @@ struct WgArgs {
 
 __device__ int g_sg_wg_timeout;
 
-template <int CG, int CX>
+template <int CG, int CX, int PX>
 __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid_constant__ CUtensorMap tm_g,
                                                                     const __grid_constant__ CUtensorMap tm_x,
                                                                     const __grid_constant__ WgArgs a) {
-    using C = WgCfg<CG, CX>;
+    using C = WgCfg<CG, CX, PX>;
+    constexpr int kStages = C::kStages;
     extern __shared__ __align__(1024) unsigned char wg_sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sbase = smem_u32(wg_sm);
-    const uint32_t full = sbase + C::kBar, freed = full + 16, done = freed + 16, tmem_slot = done + 8;
-    volatile int *s_abort = reinterpret_cast<volatile int *>(wg_sm + C::kBar + 48);
+    const uint32_t full = sbase + C::kBar, freed = full + 8 * kStages, done = freed + 8 * kStages, tmem_slot = done + 8;
+    volatile int *s_abort = reinterpret_cast<volatile int *>(wg_sm + C::kBar + 16 * kStages + 16);
 
     if (tid == 0) {
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < kStages; i++) {
             mbar_init(full + 8 * i, 1);
             mbar_init(freed + 8 * i, 1);
         }
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     // the constant slots: channel 0 of every pixel one, in the input rows' swizzle
-    for (int e = tid; e < 2 * C::kXRow / 16; e += kWgThreads) {
+    for (int e = tid; e < kStages * C::kXRow / 16; e += kWgThreads) {
         const int st = e / (C::kXRow / 16), b = e - st * (C::kXRow / 16);
         constexpr int kCh = CX / 8;
         const int px = b / kCh, c = b - px * kCh;
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(wg_sm + C::kBar + 40);
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(wg_sm + C::kBar + 16 * kStages + 8);
 
     // the CTA's steps [t0, t1): kRows rows of one column tile each, down the columns of all images
     const int per_col = (a.H + C::kRows - 1) / C::kRows;
@@ -105,14 +107,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     if (warp == 0) {
         if (lane == 0) {
             for (long long t = t0; t < t1; t++) {
-                const int i = (int)(t - t0), s = i & 1;
-                if (i >= 2 && !mbar_wait(freed + 8 * s, (uint32_t)((i / 2 + 1) & 1), s_abort)) {
+                const int i = (int)(t - t0), s = i % kStages;
+                if (i >= kStages && !mbar_wait(freed + 8 * s, (uint32_t)((i / kStages + 1) & 1), s_abort)) {
                     *s_abort = 1;
                     break;
                 }
                 const long long col = t / per_col;
                 const int y0 = (int)(t - col * per_col) * C::kRows, img = (int)(col / a.tiles_x),
-                          x0 = (int)(col - (long long)img * a.tiles_x) * kWgPx;
+                          x0 = (int)(col - (long long)img * a.tiles_x) * PX;
                 mbar_expect_tx(full + 8 * s, (uint32_t)(C::kRows * a.g_px * 2 * CG + C::kXRows * a.x_px * 2 * CX));
                 const uint32_t dst = sbase + (uint32_t)(s * C::kStage);
                 auto load = [&](const CUtensorMap *tm, uint32_t to, int x, int y) {
@@ -132,16 +134,16 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
         const uint64_t g0 = tc_desc(sbase, C::kGRow, 16 * CG) | (C::kSwG << 61);
         const uint64_t x0d = tc_desc(sbase + C::kX, C::kXRow, 16 * CX) | (C::kSwX << 61);
         for (long long t = t0; t < t1; t++) {
-            const int i = (int)(t - t0), s = i & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, (uint32_t)((i / 2) & 1), s_abort));
+            const int i = (int)(t - t0), s = i % kStages;
+            ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, (uint32_t)((i / kStages) & 1), s_abort));
             if (!ok) {
                 *s_abort = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const long long col = t / per_col;
-            const int x0 = (int)(col % a.tiles_x) * kWgPx;
-            const int ksteps = (min(kWgPx, a.W - x0) + 15) / 16;  // the gradient is zero past the image's edge
+            const int x0 = (int)(col % a.tiles_x) * PX;
+            const int ksteps = (min(PX, a.W - x0) + 15) / 16;  // the gradient is zero past the image's edge
             const uint64_t gd = g0 + (uint64_t)(s * (C::kStage >> 4)), xd = x0d + (uint64_t)(s * (C::kStage >> 4));
             for (int k = 0; k < ksteps; k++) {
 #pragma unroll
@@ -166,8 +168,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
         if (tid == 0) {
             atomicExch(&g_sg_wg_timeout, 1);
             const int none = 0;
-            for (int i = max(0, issued - 2); i < issued; i++)
-                (void)mbar_wait(full + 8 * (i & 1), (uint32_t)((i / 2) & 1), &none);
+            for (int i = max(0, issued - kStages); i < issued; i++)
+                (void)mbar_wait(full + 8 * (i % kStages), (uint32_t)((i / kStages) & 1), &none);
             (void)mbar_wait(done, 0, &none);
         }
         __syncthreads();
@@ -176,32 +178,43 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     float *sum = reinterpret_cast<float *>(wg_sm), *sdb = sum + C::kSum;
     for (int e = tid; e < C::kSum + 32; e += kWgThreads) sum[e] = 0.0f;
     __syncthreads();
-    if (warp >= 2 && any && ok) {
-        const int quad = warp & 3, m = quad * 32 + lane, gy = m / CG, co = m % CG;
-        const bool mine = gy < C::kRows && co < a.cout;
-        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16);
-        for (int kx = 0; kx < 3; kx++) {
-            for (int c0 = 0; c0 < C::kN; c0 += 16) {
-                uint32_t v[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                    "%14, %15}, [%16];\n"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                    : "r"(base + (uint32_t)((kx == 0 ? 0 : 16 + kx * C::kN) + c0)));
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                const int ky = c0 / CX - gy, ci0 = c0 % CX;
-                if (mine && ky >= 0 && ky <= 2) {
+    // the quarters of the tensor memory (gradient rows) in turn: f32 additions to shared memory one after the
+    // other, which an atomic would make of each a compare-and-swap loop
+    for (int turn = 0; turn < 4; turn++) {
+        const int quad = warp & 3, m = quad * 32 + lane, gy = m / CG, co = m % CG, gy0 = quad * 32 / CG,
+                  gy1 = (quad * 32 + 31) / CG;
+        if (warp >= 2 && quad == turn && gy0 < C::kRows && any && ok) {
+            const bool mine = gy < C::kRows && co < a.cout;
+            const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16);
+            for (int kx = 0; kx < 3; kx++) {
+                for (int c0 = gy0 * CX; c0 < min(C::kN, (gy1 + 3) * CX); c0 += 16) {
+                    uint32_t v[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                        "%13, %14, %15}, [%16];\n"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                          "=r"(v[15])
+                        : "r"(base + (uint32_t)((kx == 0 ? 0 : 16 + kx * C::kN) + c0)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    const int ky = c0 / CX - gy, ci0 = c0 % CX;
+                    if (mine && ky >= 0 && ky <= 2) {
+                        float *to = sum + ((3 * ky + kx) * CX + ci0) * 33 + co;
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        atomicAdd(&sum[((3 * ky + kx) * CX + ci0 + j) * 33 + co], __uint_as_float(v[j]));
+                        for (int j = 0; j < 16; j++) to[33 * j] += __uint_as_float(v[j]);
+                    }
+                    __syncwarp();  // two gradient rows of a warp add to the same elements in different steps
                 }
             }
+            uint32_t b;
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(b) : "r"(base + (uint32_t)C::kN));
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            for (int g = gy0; g <= gy1; g++) {
+                if (mine && gy == g) sdb[co] += __uint_as_float(b);
+                __syncwarp();
+            }
         }
-        uint32_t b;
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(b) : "r"(base + (uint32_t)C::kN));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (mine) atomicAdd(&sdb[co], __uint_as_float(b));
+        __syncthreads();
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -219,13 +232,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     }
 }
 
-template <int CG, int CX>
-static cudaError_t launch_wg(const void *g, int g_cstride, const void *x, int x_cstride, WgArgs a, cudaStream_t s) {
-    using C = WgCfg<CG, CX>;
+template <int CG, int CX, int PX>
+static cudaError_t launch_wg_px(const void *g, int g_cstride, const void *x, int x_cstride, WgArgs a, cudaStream_t s) {
+    using C = WgCfg<CG, CX, PX>;
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (!encode) return cudaErrorNotSupported;
-    a.g_px = std::min(kWgPx, (a.W + 15) & ~15);          // whole K steps (zero past the image's edge)
-    a.x_px = std::min(kWgPx + 8, ((a.W + 15) & ~15) + 8);  // with the halo columns, in whole swizzle periods
+    a.tiles_x = (a.W + PX - 1) / PX;
+    a.g_px = std::min(PX, (a.W + 15) & ~15);          // whole K steps (zero past the image's edge)
+    a.x_px = std::min(PX + 8, ((a.W + 15) & ~15) + 8);  // with the halo columns, in whole swizzle periods
     CUtensorMap tm[2];
     for (int k = 0; k < 2; k++) {
         const cuuint64_t ch = (cuuint64_t)std::min(k ? CX : CG, k ? x_cstride : g_cstride);
@@ -243,12 +257,20 @@ static cudaError_t launch_wg(const void *g, int g_cstride, const void *x, int x_
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(sg_wgrad_tc_kernel<CG, CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+        e = cudaFuncSetAttribute(sg_wgrad_tc_kernel<CG, CX, PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
     if (e != cudaSuccess) return e;
     const long long steps = (long long)a.nb * a.tiles_x * ((a.H + C::kRows - 1) / C::kRows);
-    sg_wgrad_tc_kernel<CG, CX><<<(unsigned)std::min<long long>(steps, std::max(1, sms)), kWgThreads, C::kSmem, s>>>(
+    sg_wgrad_tc_kernel<CG, CX, PX><<<(unsigned)std::min<long long>(steps, std::max(1, sms)), kWgThreads, C::kSmem, s>>>(
         tm[0], tm[1], a);
     return cudaGetLastError();
+}
+
+// Images up to 64 pixels wide: rows of 64 columns in four stages instead of 128 in two, whose copies' latency
+// was most of a step (256 tiles of 64^2, 32 -> 32 channels: 63 -> 50 us).
+template <int CG, int CX>
+static cudaError_t launch_wg(const void *g, int g_cstride, const void *x, int x_cstride, const WgArgs &a, cudaStream_t s) {
+    return a.W <= 64 ? launch_wg_px<CG, CX, 64>(g, g_cstride, x, x_cstride, a, s)
+                     : launch_wg_px<CG, CX, 128>(g, g_cstride, x, x_cstride, a, s);
 }
 
 // The weight gradient of a conv kind (input, residual, output) on the tensor cores, added onto dw and db.
@@ -261,7 +283,6 @@ cudaError_t launch_sg_wgrad_tc(int kind, const void *g, int g_cstride, const voi
     a.dw = dw;
     a.db = db;
     a.nb = nb; a.H = H; a.W = W;
-    a.tiles_x = (W + kWgPx - 1) / kWgPx;
     a.cout = kind == FG_SG_CONV_OUTPUT ? 8 : 32;
     switch (kind) {
     case FG_SG_CONV_INPUT: return launch_wg<32, 16>(g, g_cstride, x, x_cstride, a, s);

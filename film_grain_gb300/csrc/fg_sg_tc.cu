@@ -28,6 +28,10 @@
 // neighbouring threads write eight bank groups) and leave by TMA, which also cuts them at the image's edge;
 // written directly, a thread's own 64 bytes would touch each 32-byte sector twice.
 //
+// Images narrower than a row tile's half share row tiles (tc_narrow): a tile's input is then the rows of two or more
+// images with their halo pixels, side by side as TMA lays them, read from wherever the tile begins; the
+// epilogue finds each position's pixel and stores it by plain stores, as a warp's pixels lie in several images.
+//
 // Measured, 32 -> 32 at 3 x 1024^2 pixels (403 MB, 60 us at the measured copy rate): 18 MMAs of N 32 per row
 // 128 us; this split with one epilogue group and rows as 16-byte TMA pieces 95 us; two groups 92 us; the MMAs
 // issued by a converged warp 78 us; with constant operands inside a run 72 us (call by call 139 -> 76 us).
@@ -49,19 +53,21 @@ namespace fg {
 
 constexpr int kTcPx = 128;          // output pixels of one row tile (the MMA's M)
 constexpr int kTcHalo = kTcPx + 2;  // input pixels of one row at most
-constexpr int kTcSlots = 6;         // input rows in flight
+constexpr int kTcNarrowPx = 208;    // input pixels of a row tile of narrow images at most
 constexpr int kTcAcc = 8;           // accumulator rows in tensor memory
 constexpr int kTcStageBytes = 2048; // a warp's 32 pixels of 32 channels
 constexpr int kTcThreads = 320;     // loader, MMA issuer, two groups of four epilogue warps
-// barriers: rows full, rows free (MMA), rows free (epilogue), accumulators full, accumulators free, drain
-constexpr int kTcBars = 3 * kTcSlots + 2 * kTcAcc + 1;
 __device__ int g_sg_tc_timeout;
 
 enum TcMode { kTcInput, kTcResidual, kTcResidualAux, kTcOutput, kTcDgrad, kTcDgradMasked, kTcLinear, kTcLinearMasked };
 
-// Sizes of a mode.  A row slot holds kTcHalo pixels, rounded up to what the swizzle repeats over (8 pixels).
-template <int MODE>
+// Sizes of a mode.  A row slot holds kTcHalo pixels, rounded up to what the swizzle repeats over (8 pixels), or
+// the rows of several narrow images.
+template <int MODE, bool NARROW>
 struct TcCfg {
+    static constexpr int kSlots = NARROW ? 4 : 6;  // input rows in flight
+    // barriers: rows full, rows free (MMA), rows free (epilogue), accumulators full, accumulators free, drain
+    static constexpr int kBars = 3 * kSlots + 2 * kTcAcc + 1;
     static constexpr bool kRelu = MODE == kTcInput || MODE == kTcResidual || MODE == kTcResidualAux;
     static constexpr bool kRes = MODE == kTcResidual || MODE == kTcResidualAux;       // the addend is the input row
     static constexpr bool kAdd = MODE == kTcDgrad || MODE == kTcDgradMasked;          // another tensor
@@ -72,16 +78,17 @@ struct TcCfg {
     static constexpr int kHalves = kCin / 16;        // MMAs' K steps per tap
     static constexpr int kChunks = kCin / 8;         // 16-byte channel chunks per pixel
     static constexpr int kPxBytes = 2 * kCin;
-    static constexpr int kRowBytes = (kTcHalo + 7) / 8 * 8 * kPxBytes;
+    static constexpr int kRowBytes = (NARROW ? kTcNarrowPx : (kTcHalo + 7) / 8 * 8) * kPxBytes;
     static constexpr int kCols = kF32 ? 16 : 32;     // accumulator columns of an output row
     static constexpr int kCout = kF32 ? 8 : 32;      // output channels the weights have
     static constexpr int kWRows = MODE == kTcLinearMasked ? 8 : 32;  // output channels of a masked gradient's layer
     static constexpr int kBlock = 3 * kCols * 16;    // weights of one (kx, chunk): rows ky = 2, 1, 0
     static constexpr uint64_t kSwizzle = kCin == 32 ? 4ull : 6ull;  // 64- or 32-byte swizzle
-    static constexpr int kWOff = kTcSlots * kRowBytes;
+    static constexpr int kWOff = kSlots * kRowBytes;
     static constexpr int kStageOff = (kWOff + 3 * kChunks * kBlock + 511) / 512 * 512;
     static constexpr int kBarOff = kStageOff + (kF32 ? 0 : 8 * (kTwo ? 2 : 1) * kTcStageBytes);
-    static constexpr int kSmem = kBarOff + 8 * kTcBars + 16 + 128;
+    static constexpr int kSmem = kBarOff + 8 * kBars + 16 + 128;
+    static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
     static constexpr uint32_t kTmemCols = kCols * kTcAcc;
 };
 
@@ -94,19 +101,29 @@ struct TcArgs {
     bf16 *out, *out2;        // out2: aux, or the masked gradient
     int nb, H, W, tiles_x;
     int box_px;              // pixels of an input row box (even, <= kTcHalo)
+    // narrow images: a row tile is `step` positions of the line of all images' rows of pitch W + 2 pixels, from the
+    // halo pixel on, loaded as the rows of `images` images; tiles_x counts the tiles of the whole line
+    int step, images;
 };
 
 // The CTA's rows: [t0, t1) of the nb * tiles_x * H row tiles, column-major, as runs of one column.
 struct TcRun {
-    int img, x0, y0, rows;
+    int img, x0, y0, rows;  // narrow: img the first image loaded, x0 the tile's first position in its row
 };
+template <bool NARROW>
 __device__ __forceinline__ bool tc_run(const TcArgs &a, long long &t, long long t1, TcRun &r) {
     if (t >= t1) return false;
     const long long col = t / a.H;
     r.y0 = (int)(t - col * a.H);
     r.rows = (int)min((long long)(a.H - r.y0), t1 - t);
-    r.img = (int)(col / a.tiles_x);
-    r.x0 = (int)(col - (long long)r.img * a.tiles_x) * kTcPx;
+    if (NARROW) {
+        const long long v = col * a.step;
+        r.img = (int)(v / (a.W + 2));
+        r.x0 = (int)(v - (long long)r.img * (a.W + 2));
+    } else {
+        r.img = (int)(col / a.tiles_x);
+        r.x0 = (int)(col - (long long)r.img * a.tiles_x) * kTcPx;
+    }
     t += r.rows;
     return true;
 }
@@ -133,13 +150,14 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {  // two f32 additio
     return *reinterpret_cast<float2 *>(&d);
 }
 
-template <int MODE>
+template <int MODE, bool NARROW>
 __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                      const __grid_constant__ CUtensorMap tmap_out,
                                                                      const __grid_constant__ CUtensorMap tmap_out2,
                                                                      const __grid_constant__ TcArgs a) {
     extern __shared__ __align__(1024) unsigned char tc_sm[];
-    using C = TcCfg<MODE>;
+    using C = TcCfg<MODE, NARROW>;
+    constexpr int kTcSlots = C::kSlots, kTcBars = C::kBars;
     constexpr bool kRes = C::kRes, kTwo = C::kTwo;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sbase = smem_u32(tc_sm);
@@ -201,9 +219,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tc_sm + C::kBarOff + 8 * kTcBars + 4);
 
-    const long long total = (long long)a.nb * a.tiles_x * a.H;
+    const long long total = (NARROW ? 1ll : (long long)a.nb) * a.tiles_x * a.H;
     const long long t0 = total * blockIdx.x / gridDim.x, t1 = total * (blockIdx.x + 1) / gridDim.x;
-    const uint32_t row_bytes = (uint32_t)a.box_px * C::kPxBytes;
+    const uint32_t row_bytes = (uint32_t)(NARROW ? a.images * (a.W + 2) : a.box_px) * C::kPxBytes;
     // Input rows are numbered q = 0, 1, ... over the CTA's runs (a run of R output rows has R + 2), output
     // rows n; row q is in slot q % kTcSlots, row n in accumulator n % kTcAcc.
     long long t = t0;
@@ -214,7 +232,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
         if (lane == 0) {
             int q = 0;
             bool ok = true;
-            while (ok && tc_run(a, t, t1, r)) {
+            while (ok && tc_run<NARROW>(a, t, t1, r)) {
                 for (int i = 0; i < r.rows + 2; i++, q++) {
                     const int s = q % kTcSlots;
                     if (q >= kTcSlots) {
@@ -230,7 +248,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     asm volatile(
                         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
                         "%3, %4, %5}], [%6];\n" ::"r"(sbase + (uint32_t)(s * C::kRowBytes)),
-                        "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(r.x0 - 1), "r"(r.y0 - 1 + i), "r"(r.img),
+                        "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(NARROW ? -1 : r.x0 - 1), "r"(r.y0 - 1 + i), "r"(r.img),
                         "r"(full + 8 * s)
                         : "memory");
                     issued = q + 1;
@@ -243,7 +261,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
         const uint64_t b0 = tc_desc(sbase + C::kWOff, C::kBlock, 128);
         int q = 0, n0 = 0;  // n0: output rows of the runs before
         bool ok = true;
-        while (ok && tc_run(a, t, t1, r)) {
+        while (ok && tc_run<NARROW>(a, t, t1, r)) {
             for (int i = 0; i < r.rows + 2; i++, q++) {
                 const int s = q % kTcSlots;
                 // the run's output rows that input row i reaches: o0 .. o1, tap ky = i - o
@@ -260,7 +278,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint64_t ad = a0 + (uint64_t)(s * (C::kRowBytes >> 4));
+                const uint64_t ad = a0 + (uint64_t)(s * (C::kRowBytes >> 4)) +
+                                    (NARROW ? (uint64_t)(r.x0 * (C::kPxBytes >> 4)) : 0ull);
                 // rows [o, o + cnt) of the window: accumulator columns from kCols ((n0 + o) % kTcAcc), weight
                 // rows from kCols (2 - ky)
                 const int w0 = (n0 + o0) % kTcAcc, cnt = o1 - o0 + 1, head = min(cnt, kTcAcc - w0);
@@ -337,12 +356,18 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
             if (ok) mbar_arrive(free_epi + 8 * (row % kTcSlots));
             else *s_abort = 1;
         };
-        while (tc_run(a, t, t1, r)) {
+        while (tc_run<NARROW>(a, t, t1, r)) {
             free_halo(q);
             for (int o = 0; o < r.rows; o++, n++) {
                 if ((n & 1) != group) continue;
-                const int x = r.x0 + m, y = r.y0 + o, acc = n % kTcAcc;
-                const size_t p = ((size_t)r.img * a.H + y) * a.W + x;
+                const int y = r.y0 + o, acc = n % kTcAcc;
+                int x = r.x0 + m, img = r.img;
+                if (NARROW) {
+                    img += x / (a.W + 2);
+                    x %= a.W + 2;
+                    if (m >= a.step || img >= a.nb) x = a.W;  // no pixel
+                }
+                const size_t p = ((size_t)img * a.H + y) * a.W + x;
                 uint4 rv[4], mv[4];
                 float uv = 0.0f;
                 if (x < a.W) {
@@ -394,10 +419,11 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     : "r"(tcol));
                 if (kRes) {
                     // chunk c of pixel i lies at chunk c ^ (i / 2 % 4) of its 64 bytes (the swizzle)
-                    const unsigned char *rp = tc_sm + s * C::kRowBytes + (m + 1) * 64;
+                    const int px = (NARROW ? r.x0 : 0) + m + 1;
+                    const unsigned char *rp = tc_sm + s * C::kRowBytes + px * 64;
 #pragma unroll
                     for (int c = 0; c < 4; c++)
-                        rv[c] = *reinterpret_cast<const uint4 *>(rp + ((c ^ (((m + 1) >> 1) & 3)) << 4));
+                        rv[c] = *reinterpret_cast<const uint4 *>(rp + ((c ^ ((px >> 1) & 3)) << 4));
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -439,11 +465,28 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
                     // arrival right behind the loads can pass them, and a halo row outside the image (filled
                     // with zeros at once) then overwrites what they are about to read.
                     if (kRes) mbar_arrive(free_epi + 8 * s);
-                    if (x < a.W) {  // the box is cut at the image's edge
+                    if (!NARROW && x < a.W) {  // the box is cut at the image's edge
                         if (!C::kMask || a.out) tma_store(&tmap_out, stage, x, y, r.img);
                         if (kTwo) tma_store(&tmap_out2, stage + kTcStageBytes, x, y, r.img);
                     }
                     asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                }
+                if (NARROW) {
+                    // a warp's 32 positions lie in up to three images: plain stores, four lanes to a pixel
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int px = 8 * k + (lane >> 2), c = lane & 3;
+                        const bool has = __shfl_sync(0xffffffffu, x < a.W ? 1 : 0, px) != 0;
+                        const size_t at = (size_t)__shfl_sync(0xffffffffu, (unsigned long long)p, px) * 32 + 8 * c;
+                        const unsigned char *from = stage + px * 64 + ((c ^ ((px >> 1) & 3)) << 4);
+                        if (has) {
+                            if (!C::kMask || a.out) *reinterpret_cast<uint4 *>(a.out + at) = *reinterpret_cast<const uint4 *>(from);
+                            if (kTwo)
+                                *reinterpret_cast<uint4 *>(a.out2 + at) =
+                                    *reinterpret_cast<const uint4 *>(from + kTcStageBytes);
+                        }
+                    }
+                    __syncwarp();  // the stage is written again for the next row
                 }
             }
             q += r.rows + 2;
@@ -476,9 +519,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) sg_conv32_tc_kernel(const __gri
     }
 }
 
-template <int MODE>
-static cudaError_t launch_tc(const void *in, int in_cstride, TcArgs a, cudaStream_t s) {
-    using C = TcCfg<MODE>;
+template <int MODE, bool NARROW>
+static cudaError_t launch_tc_as(const void *in, int in_cstride, TcArgs a, cudaStream_t s) {
+    using C = TcCfg<MODE, NARROW>;
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (!encode) return cudaErrorNotSupported;
     CUtensorMap tm[3];  // input rows, and 32-pixel boxes of the outputs
@@ -487,7 +530,8 @@ static cudaError_t launch_tc(const void *in, int in_cstride, TcArgs a, cudaStrea
         const cuuint64_t ch = k == 0 || C::kF32 ? C::kCin : 32, px = k == 0 || C::kF32 ? 2 * (cuuint64_t)in_cstride : 64;
         const cuuint64_t dims[4] = {ch, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.nb};
         const cuuint64_t strides[3] = {px, (cuuint64_t)a.W * px, (cuuint64_t)a.H * a.W * px};
-        const cuuint32_t box[4] = {(cuuint32_t)ch, k == 0 ? (cuuint32_t)a.box_px : 32u, 1, 1};
+        const cuuint32_t box[4] = {(cuuint32_t)ch, k == 0 ? (cuuint32_t)(NARROW ? a.W + 2 : a.box_px) : 32u, 1,
+                                   k == 0 && NARROW ? (cuuint32_t)a.images : 1u};
         const cuuint32_t estr[4] = {1, 1, 1, 1};
         if (encode(&tm[k], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base[k]), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
@@ -498,12 +542,40 @@ static cudaError_t launch_tc(const void *in, int in_cstride, TcArgs a, cudaStrea
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(sg_conv32_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+        e = cudaFuncSetAttribute(sg_conv32_tc_kernel<MODE, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
     if (e != cudaSuccess) return e;
-    const long long rows = (long long)a.nb * a.tiles_x * a.H;
+    const long long rows = (NARROW ? 1ll : (long long)a.nb) * a.tiles_x * a.H;
     const long long grid = std::min<long long>(rows, 2ll * std::max(1, sms));
-    sg_conv32_tc_kernel<MODE><<<(unsigned)grid, kTcThreads, C::kSmem, s>>>(tm[0], tm[1], tm[2], a);
+    sg_conv32_tc_kernel<MODE, NARROW><<<(unsigned)grid, kTcThreads, C::kSmem, s>>>(tm[0], tm[1], tm[2], a);
     return cudaGetLastError();
+}
+
+// Images so narrow that a row would leave half of the 128 accumulator rows empty share their row tiles: the
+// rows of all images stand in one line, each with its two halo pixels, and the line is cut every 128
+// positions -- or, where that would need more than kTcNarrowPx pixels loaded for a tile, every whole number of
+// images.  The halo positions' sums are dropped.
+// 256 tiles of 64^2, 32 -> 32 channels with the ReLU output (201 MB, 30 us at the measured copy rate): 51 -> 44 us,
+// the masked data gradient (335 MB, 50 us) 65 -> 58, the input conv 32 -> 25; 200 images of 50 x 33, a layer call by call: 35 us.
+static bool tc_narrow(TcArgs &a) {
+    const int pitch = a.W + 2;
+    if (a.nb < 2 || pitch > kTcNarrowPx / 3) return false;
+    const long long line = (long long)a.nb * pitch;
+    a.step = kTcPx;
+    int off = 0;  // the last first position of a tile in its image's row: the multiples of gcd(128, pitch)
+    for (int t = 0; t < pitch; t++) off = std::max(off, t * kTcPx % pitch);
+    a.images = (off + kTcHalo + pitch - 1) / pitch;
+    if (a.images * pitch > kTcNarrowPx) {
+        a.images = kTcPx / pitch;
+        if (a.images < 2) return false;
+        a.step = a.images * pitch;
+    }
+    a.tiles_x = (int)((line + a.step - 1) / a.step);
+    return true;
+}
+
+template <int MODE>
+static cudaError_t launch_tc(const void *in, int in_cstride, TcArgs a, cudaStream_t s) {
+    return tc_narrow(a) ? launch_tc_as<MODE, true>(in, in_cstride, a, s) : launch_tc_as<MODE, false>(in, in_cstride, a, s);
 }
 
 // A surrogate conv on the tensor cores, by the C-ABI's kinds.  For the residual kind res is the input itself; res

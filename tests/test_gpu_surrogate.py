@@ -305,3 +305,45 @@ def test_evaluator_matches_oracle(sg, cuda):
     assert abs(e["mae"] - 0.5) < 1e-6 and e["raps_max"] < 1e-6  # f32 rounding of img + 0.5
     e = sg.evaluate(2 * a, a)  # doubling the image quadruples its power
     assert abs(e["raps_max"] - 3.0) < 1e-9
+
+
+@pytest.mark.parametrize("nb,h,w", [(200, 3, 1), (9, 11, 24), (7, 5, 30), (2, 9, 62), (5, 8, 64), (6, 7, 65), (3, 40, 67),
+                                    (2, 5, 68)])
+def test_narrow_images_sharing_row_tiles(sg, cuda, fgl, nb, h, w):
+    """Images up to 67 pixels wide share row tiles, wherever the tiles cut them: every conv gives the bits that it
+    gives for each image on its own (one image takes a row tile alone, and a pixel's sum runs in the same
+    order)."""
+    torch = cuda
+    x, wt, b, res = _conv_inputs(torch, nb, h, w, 11)
+    dev = lambda a: torch.from_numpy(a).cuda().to(torch.bfloat16)
+    X, Wt, R, B = dev(x), dev(wt), dev(res), torch.from_numpy(b).cuda()
+    W16 = Wt[:, :, :16].contiguous()
+    X16 = X[..., :16].contiguous()
+    U = torch.rand((nb, h, w), device="cuda")
+    L, st = fgl.lib(), torch.cuda.current_stream().cuda_stream
+
+    def run(n, s):
+        sub = lambda t: t[s:s + n].contiguous()
+        xs, x16, rs, us = sub(X), sub(X16), sub(R), sub(U)
+        new = lambda: torch.empty_like(xs)
+        out = [new() for _ in range(8)] + [torch.empty_like(us)]
+        fwd = lambda kind, i, c, wgt, r, u, o, a, f: L.fg_sg_conv_forward(
+            kind, i.data_ptr(), c, wgt.data_ptr(), B.data_ptr(), None if r is None else r.data_ptr(),
+            None if u is None else u.data_ptr(), None if o is None else o.data_ptr(),
+            None if a is None else a.data_ptr(), None if f is None else f.data_ptr(), n, h, w, st)
+        assert fwd(sg.CONV_INPUT, x16, 16, W16, None, None, out[0], None, None) == 0
+        assert fwd(sg.CONV_RESIDUAL, xs, 32, Wt, xs, None, out[1], None, None) == 0
+        assert fwd(sg.CONV_RESIDUAL, xs, 32, Wt, xs, None, out[2], out[3], None) == 0
+        assert fwd(sg.CONV_OUTPUT, xs, 32, Wt[:8].contiguous(), None, us, None, None, out[8]) == 0
+        assert fwd(sg.CONV_DGRAD_RESIDUAL, xs, 32, Wt, rs, None, out[4], None, None) == 0
+        assert L.fg_sg_conv_dgrad(sg.CONV_DGRAD_RESIDUAL, xs.data_ptr(), 32, Wt.data_ptr(), rs.data_ptr(), xs.data_ptr(),
+                                  out[5].data_ptr(), out[6].data_ptr(), n, h, w, st) == 0
+        assert L.fg_sg_conv_dgrad(sg.CONV_DGRAD_OUTPUT, x16.data_ptr(), 16, Wt[:8].contiguous().data_ptr(), None,
+                                  rs.data_ptr(), None, out[7].data_ptr(), n, h, w, st) == 0
+        torch.cuda.synchronize()
+        return out
+
+    together = run(nb, 0)
+    for s in range(0, nb, max(1, nb // 5)):
+        for a, t in zip(run(1, s), together):
+            assert torch.equal(a[0], t[s])

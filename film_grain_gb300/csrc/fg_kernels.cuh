@@ -65,7 +65,7 @@ constexpr float kPwRegenKernel = 2.05f;
 // which the kernel splits the samples (96 x 64 N 32 without the split: 226 us).
 constexpr double kPwRegenSmallVisits = 4.5e6;
 constexpr float kPwRegenSmall = 5.0f;
-constexpr double kPwRegenWarps = 32.0;
+constexpr double kPwRegenWarps = 64.0;
 // The stream pass (fg_pixelwise_stream.cuh): planes of kPwStreamPixels output pixels and more, and the grains per
 // output pixel, in multiples of N, above which a segment's samples go to the per-sample kernel -- with ranges of
 // up to 4 cells an axis, and wider ones, whose samples look at more cells.  Log-normal 0.025 at 1024^2, N 256:

@@ -357,12 +357,13 @@ static cudaError_t launch_pixelwise_regen(const PixelwiseArgs &a, cudaStream_t s
     const long long grid = row_ctas * a.out_h;
     if (grid <= 0) return cudaSuccess;
     // A warp alone on its scheduler takes 3.6 us a sample, most of it waiting: with fewer warps than
-    // kPwRegenWarps per SM the samples are split, into parts of four and more (each part ends with a round
-    // of less than 32 cells).
+    // kPwRegenWarps per SM the samples are split, down to one by one where that is what fills the chip (a
+    // part's last round of cells is partly idle, but 96 x 64 N 32 takes 131 us a call in parts of four and
+    // 32 warps, 111 us so).
     const int sms = sm_count();
     const double warps = (double)((a.out_w + 31) / 32) * a.out_h;
     const double want = warps > 0 ? kPwRegenWarps * (double)std::max(1, sms) / warps : 1.0;
-    const int per = std::max(4, (int)std::ceil(a.n / std::max(1.0, want)));
+    const int per = std::max(1, (int)std::ceil(a.n / std::max(1.0, want)));
     const int parts = (a.n + per - 1) / per;
     pixelwise_regen_kernel<<<(unsigned)(grid * parts), kPwRegenThreads, 0, s>>>(a, (int)row_ctas, parts, per);
     return cudaGetLastError();

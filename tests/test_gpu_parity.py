@@ -309,7 +309,7 @@ def test_pixelwise_screened_cells(cuda, fgl, orc, w, h, radius, cell, zoom, n):
 
 @pytest.mark.parametrize("n", [1, 4, 5, 31, 33, 100])
 def test_pixelwise_small_plane_parts(cuda, fgl, orc, n):
-    """A small plane on the per-sample kernel, its samples in parts of four and more over several warps."""
+    """A small plane on the per-sample kernel, its samples in parts over several warps."""
     plane = _blobs(35, 9)
     p, d, *_ = _setup(fgl, orc, plane, radius=0.2, n=n, seed=3)
     if n <= 5:

@@ -263,6 +263,12 @@ static bool plan_stream(const PixelwiseArgs &a, const PwSparseGrid &g, int sms, 
             // parts of a tile's chunks: one or two for each of its eight warps
             const int chunks = (T / 32) * (T / 32);
             t->sub = chunks >= 16 ? 1 : chunks >= 4 ? 4 : 8;
+            t->cols = (t->gw + 31) / 32;
+            // no tiles (DIRECT) where they would be this small, unless a grain has many hits to gather
+            t->direct = T <= 64 && t->gw < 65536 && 32.0 * t->ghw < 65536.0 &&
+                        (double)a.out_w * a.out_h * t->nw < 0x1p31 &&
+                        a.n * 3.14 * a.radius_mean * a.radius_mean * a.zoom * a.zoom < 16.0;
+            if (t->direct) t->sub = 8;
             return (double)t->ntx * t->nty < 2.0e9;
         }
     }
@@ -374,17 +380,23 @@ static cudaError_t set_smem(K k, size_t smem) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-template <int NW>
-static cudaError_t launch_stream(const PixelwiseArgs &a, const PwStreamGrid &t, int sms, cudaStream_t s) {
-    const size_t smem = sizeof(PwStreamShared<NW>) + (size_t)t.fp_words * sizeof(unsigned int);
-    cudaError_t e = set_smem(pixelwise_stream_kernel<NW>, smem);
+template <int NW, bool DIRECT>
+static cudaError_t launch_stream_as(const PixelwiseArgs &a, const PwStreamGrid &t, int sms, cudaStream_t s) {
+    const size_t smem = sizeof(PwStreamShared<NW>) + (DIRECT ? 0 : (size_t)t.fp_words * sizeof(unsigned int));
+    cudaError_t e = set_smem(pixelwise_stream_kernel<NW, DIRECT>, smem);
     int per_sm = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pixelwise_stream_kernel<NW>, PwStream::kThreads, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pixelwise_stream_kernel<NW, DIRECT>, PwStream::kThreads, smem);
     if (e != cudaSuccess) return e;
-    const long long grid = std::min<long long>((long long)t.ntx * t.nty, (long long)sms * std::max(1, per_sm));
-    pixelwise_stream_kernel<NW><<<(unsigned)grid, PwStream::kThreads, smem, s>>>(a, t);
+    const long long work = DIRECT ? (long long)t.cols * t.ghw * t.sub * 32 / PwStream::kThreads + 1 : (long long)t.ntx * t.nty;
+    const long long grid = std::min<long long>(work, (long long)sms * std::max(1, per_sm));
+    pixelwise_stream_kernel<NW, DIRECT><<<(unsigned)grid, PwStream::kThreads, smem, s>>>(a, t);
     return cudaGetLastError();
+}
+
+template <int NW>
+static cudaError_t launch_stream(const PixelwiseArgs &a, const PwStreamGrid &t, int sms, cudaStream_t s) {
+    return t.direct ? launch_stream_as<NW, true>(a, t, sms, s) : launch_stream_as<NW, false>(a, t, sms, s);
 }
 
 // The plane's bits, its emptiness bitmask (g) written: the tables, the stream pass and the per-sample kernel over

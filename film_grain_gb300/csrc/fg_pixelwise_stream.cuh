@@ -59,6 +59,7 @@ struct PwStreamGrid {
     float near_rm;    // |dx| up to this: the sample's range holds the grain's cell
     float class_scale;  // a band's half-width times this: its radius class
     int tile, ntx, nty, nw, fp_words, sub;
+    int direct, cols;  // direct: no tiles, the hits go to the plane's bits; cols: chunks of a word row
     unsigned int *bits;  // [out_h * out_w * nw]
     int *next;           // the next tile
     const unsigned char *dense;  // per segment of 32 output pixels: left to the per-sample pass
@@ -102,7 +103,7 @@ struct StreamGrain {
 };
 template <int NW>
 __device__ __forceinline__ void stream_test(const PixelwiseArgs &a, const PwStreamGrid &g, PwStreamShared<NW> &S,
-                                            const StreamGrain &G, bool live, int src, int e, int fx0, int fy0, int fw,
+                                            unsigned int *bits, const StreamGrain &G, bool live, int src, int e, int fx0, int fy0, int fw,
                                             int fh) {
     const float gx = __shfl_sync(0xffffffffu, G.gx, src), gy = __shfl_sync(0xffffffffu, G.gy, src);
     const float rr = __shfl_sync(0xffffffffu, G.rr, src);
@@ -127,7 +128,7 @@ __device__ __forceinline__ void stream_test(const PixelwiseArgs &a, const PwStre
     if (!hit) return;
     const int x = (int)rx - fx0, y = (int)ry - fy0;
     if ((unsigned)x < (unsigned)fw && (unsigned)y < (unsigned)fh)  // else outside the plane
-        atomicOr(S.bits() + (y * fw + x) * g.nw + (e >> 5), 1u << (e & 31));
+        atomicOr(bits + (y * fw + x) * g.nw + (e >> 5), 1u << (e & 31));
 }
 
 // The candidates of 32 grains, one per lane (G.rr < 0: none): each lane intersects the two axes' words for its
@@ -135,8 +136,8 @@ __device__ __forceinline__ void stream_test(const PixelwiseArgs &a, const PwStre
 // of the counts, as many as the queue holds at a time, and tests them 32 at a time, every lane busy.
 template <int NW>
 __device__ __forceinline__ void stream_candidates(const PixelwiseArgs &a, const PwStreamGrid &g, PwStreamShared<NW> &S,
-                                                  PwStreamWarp &W, const StreamGrain &G, int fx0, int fy0, int fw,
-                                                  int fh) {
+                                                  PwStreamWarp &W, unsigned int *bits, const StreamGrain &G, int fx0,
+                                                  int fy0, int fw, int fh) {
     const int lane = threadIdx.x & 31;
     unsigned m[NW];
     int cnt = 0;
@@ -176,14 +177,19 @@ __device__ __forceinline__ void stream_candidates(const PixelwiseArgs &a, const 
         for (int i = 0; i < here; i += 32) {
             const bool live = i + lane < here;
             const unsigned pr = W.pairs[live ? i + lane : 0];
-            stream_test(a, g, S, G, live, (int)(pr >> 8), (int)(pr & 0xFFu), fx0, fy0, fw, fh);
+            stream_test(a, g, S, bits, G, live, (int)(pr >> 8), (int)(pr & 0xFFu), fx0, fy0, fw, fh);
         }
         __syncwarp();  // the queue is read before it is written again
     }
 }
 
 // Dynamic shared memory: PwStreamShared and fp_words words of bits.
-template <int NW>
+// DIRECT (small planes): the warps take chunks of the whole plane, keep their queues from one to the next and set
+// the hits' bits in global memory.  A tile of such a plane holds few grains a warp: 256^2 ramp radius 0.12, N 64,
+// where each tile's last steps ran with few lanes, 330 us a call in tiles, 255 us so; 700 x 900, N 100, zoom 1.5
+// 2.37 and 2.08 ms.  With many hits a grain the atomics show (200^2 radius 0.2, N 200, 25 hits: 0.52 and 0.58 ms), and
+// on large planes too (1080p radius 0.1, N 32: 1.87 and 2.30 ms).
+template <int NW, bool DIRECT>
 __global__ void __launch_bounds__(PwStream::kThreads)
     pixelwise_stream_kernel(const __grid_constant__ PixelwiseArgs a, const __grid_constant__ PwStreamGrid g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(PwStream::kThreads)
     constexpr int nthreads = PwStream::kThreads;
     const int tid = threadIdx.x, lane = tid & 31;
     PwStreamWarp &W = S.warp[tid >> 5];
-    unsigned int *bits = S.bits();
+    unsigned int *bits = DIRECT ? g.bits : S.bits();
     for (int e = tid; e < a.n; e += nthreads) S.ent[e] = g.ent[e];
     for (int b = tid; b < phase_table_words(NW); b += nthreads) S.mask[b] = g.masks[b];
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
@@ -199,27 +205,32 @@ __global__ void __launch_bounds__(PwStream::kThreads)
     const bool any_dense = *g.dense_count != 0;
     for (;;) {
         __syncthreads();  // the tables; the previous tile's bits are written out
-        if (tid == 0) {
-            const int t = atomicAdd(g.next, 1);
-            S.tile = (t < ntiles && !cancel_requested(a.cancel)) ? t : -1;
-            S.chunk = 0;
+        int tile = 0;
+        if (!DIRECT) {
+            if (tid == 0) {
+                const int t = atomicAdd(g.next, 1);
+                S.tile = (t < ntiles && !cancel_requested(a.cancel)) ? t : -1;
+                S.chunk = 0;
+            }
+            __syncthreads();
+            tile = S.tile;
+            if (tile < 0) return;
         }
-        __syncthreads();
-        const int tile = S.tile;
-        if (tile < 0) return;
         const int tc = (tile % g.ntx) * g.tile, tw = (tile / g.ntx) * chunk_rows;  // first column, first word row
         // the pixels whose samples its grains can reach, with a pixel of slack for the rounding
         const float X0 = (float)(g.gi0 + tc) * a.delta - a.rm, X1 = (float)(g.gi0 + tc + g.tile) * a.delta + a.rm;
         const float Y0 = (float)(g.gj0 + 32 * tw) * a.delta - a.rm, Y1 = (float)(g.gj0 + 32 * tw + g.tile) * a.delta + a.rm;
-        const int fx0 = max(0, (int)floorf((X0 + a.offx_min) * a.zoom - 0.5f) - 1);
-        const int fx1 = min(a.out_w - 1, (int)ceilf((X1 + a.offx_max) * a.zoom - 0.5f) + 1);
-        const int fy0 = max(0, (int)floorf((Y0 + a.offy_min) * a.zoom - 0.5f) - 1);
-        const int fy1 = min(a.out_h - 1, (int)ceilf((Y1 + a.offy_max) * a.zoom - 0.5f) + 1);
+        const int fx0 = DIRECT ? 0 : max(0, (int)floorf((X0 + a.offx_min) * a.zoom - 0.5f) - 1);
+        const int fx1 = DIRECT ? a.out_w - 1 : min(a.out_w - 1, (int)ceilf((X1 + a.offx_max) * a.zoom - 0.5f) + 1);
+        const int fy0 = DIRECT ? 0 : max(0, (int)floorf((Y0 + a.offy_min) * a.zoom - 0.5f) - 1);
+        const int fy1 = DIRECT ? a.out_h - 1 : min(a.out_h - 1, (int)ceilf((Y1 + a.offy_max) * a.zoom - 0.5f) + 1);
         const int fw = fx1 - fx0 + 1, fh = fy1 - fy0 + 1;
-        if (fw <= 0 || fh <= 0 || (long long)fw * fh * g.nw > g.fp_words) continue;  // (the plan's bound holds)
         const int row_words = fw * g.nw, words = row_words * fh;
-        for (int w = tid; w < words; w += nthreads) bits[w] = 0u;
-        __syncthreads();
+        if (!DIRECT) {
+            if (fw <= 0 || fh <= 0 || (long long)fw * fh * g.nw > g.fp_words) continue;  // (the plan's bound holds)
+            for (int w = tid; w < words; w += nthreads) bits[w] = 0u;
+            __syncthreads();
+        }
 
         int head = 0, queued = 0, ghead = 0, grains = 0;  // the warp's rings; uniform
         auto cover = [&](int count) {  // the first `count` grains, one per lane
@@ -233,7 +244,7 @@ __global__ void __launch_bounds__(PwStream::kThreads)
             G.rr = lane < count ? v.z : -1.0f;
             G.i = g.gi0 + tc + (int)(__float_as_uint(v.w) & 0xFFFFu);
             G.j = g.gj0 + 32 * tw + (int)(__float_as_uint(v.w) >> 16);
-            stream_candidates<NW>(a, g, S, W, G, fx0, fy0, fw, fh);
+            stream_candidates<NW>(a, g, S, W, bits, G, fx0, fy0, fw, fh);
         };
         // Each lane draws the grains of one cell, one a step, and takes the next cell from the ring when it has
         // no more: a lane whose cell holds several grains does not leave the others waiting.
@@ -268,15 +279,18 @@ __global__ void __launch_bounds__(PwStream::kThreads)
             __syncwarp();
             if (grains >= 32) cover(32);
         };
-        const int rows = 32 / g.sub;
+        const int rows = 32 / g.sub, across = DIRECT ? g.cols : chunk_rows;
+        const int chunks = across * (DIRECT ? g.ghw : chunk_rows) * g.sub;
+        int taken = 0;
         for (;;) {
-            int c = 0;
-            if (lane == 0) c = atomicAdd(&S.chunk, 1);
+            int c = chunks;
+            if (lane == 0 && !(DIRECT && cancel_requested(a.cancel))) c = atomicAdd(DIRECT ? g.next : &S.chunk, 1);
             c = __shfl_sync(0xffffffffu, c, 0);
-            if (c >= chunk_rows * chunk_rows * g.sub) break;
+            if (c >= chunks) break;
+            taken++;
             const int part = c % g.sub;
             c /= g.sub;
-            const int col = tc + 32 * (c % chunk_rows) + lane, k = tw + c / chunk_rows;
+            const int col = tc + 32 * (c % across) + lane, k = tw + c / across;
             if (any_dense) {
                 // nothing to do when every pixel whose samples the chunk's grains reach is left to the
                 // per-sample pass
@@ -309,6 +323,13 @@ __global__ void __launch_bounds__(PwStream::kThreads)
         }
         while (queued > 0 || __any_sync(0xffffffffu, q != 0u)) step();
         if (grains > 0) cover(grains);
+        if (DIRECT) {
+            if (lane == 0 && taken) {
+                atomicAdd(&a.diag[3], (unsigned long long)taken);
+                atomicAdd(&a.diag[5], (unsigned long long)taken);
+            }
+            return;
+        }
         __syncthreads();
         if (tid == 0) {
             atomicAdd(&a.diag[3], 1ull);

@@ -327,6 +327,8 @@ def test_pixelwise_small_plane_parts(cuda, fgl, orc, n):
     (41, 33, 0.12, "const", 3.0, 40, None),      # reach 0.36 of a pixel
     (120, 90, 0.3, "const", 1.0, 64, 1.0),       # cells of a pixel, the rejection regime
     (110, 90, 0.3, "const", 1.0, 20, 0.04),      # ranges of 16 cells: no per-sample kernel
+    (131, 67, 0.3, "const", 1.0, 128, None),     # 36 hits a grain: tiles and their footprints
+    (320, 250, 0.12, "const", 1.0, 40, 0.02),    # tiles of many chunks
 ])
 def test_pixelwise_stream_pass(cuda, fgl, orc, w, h, radius, dist, zoom, n, cell):
     """The stream pass: widths off the segments and tiles, every variant of words, dark, middle and saturated

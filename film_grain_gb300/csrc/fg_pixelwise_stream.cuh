@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(PwStream::kThreads)
         Xoshiro rng = {0, 0, 0, 0};
         uint32_t q = 0u;
         float sx = 0.0f, sy = 0.0f, at = 0.0f;
+        bool more = true;  // cells may still come
         auto step = [&]() {
             const unsigned idle = __ballot_sync(0xffffffffu, q == 0u);
             const int take = min(queued, __popc(idle)), rank = __popc(idle & ((1u << lane) - 1u));
@@ -277,52 +278,62 @@ __global__ void __launch_bounds__(PwStream::kThreads)
             if (v.z >= 0.0f) W.grain[(ghead + grains + __popc(have & ((1u << lane) - 1u))) & 63] = v;
             grains += __popc(have);
             __syncwarp();
-            if (grains >= 32) cover(32);
+            if (grains >= 32 || (!more && have == 0u)) cover(min(grains, 32));
         };
         const int rows = 32 / g.sub, across = DIRECT ? g.cols : chunk_rows;
         const int chunks = across * (DIRECT ? g.ghw : chunk_rows) * g.sub;
-        int taken = 0;
+        int taken = 0, col = 0, k = 0;
+        unsigned word = 0u, pending = 0u;
+        // Cells into the ring until it holds 32 or there are no more, then a step: one place for each, as the code of
+        // a step is what the instruction cache holds.
         for (;;) {
-            int c = chunks;
-            if (lane == 0 && !(DIRECT && cancel_requested(a.cancel))) c = atomicAdd(DIRECT ? g.next : &S.chunk, 1);
-            c = __shfl_sync(0xffffffffu, c, 0);
-            if (c >= chunks) break;
-            taken++;
-            const int part = c % g.sub;
-            c /= g.sub;
-            const int col = tc + 32 * (c % across) + lane, k = tw + c / across;
-            if (any_dense) {
-                // nothing to do when every pixel whose samples the chunk's grains reach is left to the
-                // per-sample pass
-                const float cx = (float)(g.gi0 + col - lane) * a.delta, cy = (float)(g.gj0 + 32 * k) * a.delta;
-                const int px0 = max(0, (int)floorf((cx - a.rm + a.offx_min) * a.zoom - 0.5f) - 1);
-                const int px1 = min(a.out_w - 1, (int)ceilf((cx + 32.0f * a.delta + a.rm + a.offx_max) * a.zoom - 0.5f) + 1);
-                const int py0 = max(0, (int)floorf((cy - a.rm + a.offy_min) * a.zoom - 0.5f) - 1);
-                const int py1 = min(a.out_h - 1, (int)ceilf((cy + 32.0f * a.delta + a.rm + a.offy_max) * a.zoom - 0.5f) + 1);
-                bool left = true;
-                if (px0 <= px1)
-                    for (int py = py0 + lane; py <= py1 && left; py += 32)
-                        for (int sg = px0 >> 5; sg <= px1 >> 5; sg++)
-                            left = left && g.dense[(long long)py * g.segs + sg] != 0;
-                if (__all_sync(0xffffffffu, left)) continue;
-            }
-            unsigned word = (col < g.gw && k < g.ghw) ? __ldg(g.cellmask + (long long)k * g.gw + col) : 0u;
-            if (g.sub > 1) word &= (0xffffffffu >> (32 - rows)) << (rows * part);
-            for (;;) {
-                const unsigned pending = __ballot_sync(0xffffffffu, word != 0u);
-                if (pending == 0u) break;
+            while (more && queued < 32) {
+                if (pending == 0u) {
+                    int c = chunks;
+                    if (lane == 0 && !(DIRECT && cancel_requested(a.cancel))) c = atomicAdd(DIRECT ? g.next : &S.chunk, 1);
+                    c = __shfl_sync(0xffffffffu, c, 0);
+                    if (c >= chunks) {
+                        more = false;
+                        break;
+                    }
+                    taken++;
+                    const int part = c % g.sub;
+                    c /= g.sub;
+                    col = tc + 32 * (c % across) + lane;
+                    k = tw + c / across;
+                    if (any_dense) {
+                        // nothing to do when every pixel whose samples the chunk's grains reach is left to the
+                        // per-sample pass
+                        const float cx = (float)(g.gi0 + col - lane) * a.delta, cy = (float)(g.gj0 + 32 * k) * a.delta;
+                        const float side = 32.0f * a.delta + a.rm;
+                        const int px0 = max(0, (int)floorf((cx - a.rm + a.offx_min) * a.zoom - 0.5f) - 1);
+                        const int px1 = min(a.out_w - 1, (int)ceilf((cx + side + a.offx_max) * a.zoom - 0.5f) + 1);
+                        const int py0 = max(0, (int)floorf((cy - a.rm + a.offy_min) * a.zoom - 0.5f) - 1);
+                        const int py1 = min(a.out_h - 1, (int)ceilf((cy + side + a.offy_max) * a.zoom - 0.5f) + 1);
+                        bool left = true;
+                        if (px0 <= px1)
+                            for (int py = py0 + lane; py <= py1 && left; py += 32)
+                                for (int sg = px0 >> 5; sg <= px1 >> 5; sg++)
+                                    left = left && g.dense[(long long)py * g.segs + sg] != 0;
+                        if (__all_sync(0xffffffffu, left)) continue;
+                    }
+                    word = (col < g.gw && k < g.ghw) ? __ldg(g.cellmask + (long long)k * g.gw + col) : 0u;
+                    if (g.sub > 1) word &= (0xffffffffu >> (32 - rows)) << (rows * part);
+                    pending = __ballot_sync(0xffffffffu, word != 0u);
+                    if (pending == 0u) continue;
+                }
                 if (word != 0u) {
                     W.cell[(head + queued + __popc(pending & ((1u << lane) - 1u))) & 63] =
                         make_uint2((unsigned)col, (unsigned)(32 * k + __ffs(word) - 1));
                     word &= word - 1u;
                 }
                 queued += __popc(pending);
+                pending = __ballot_sync(0xffffffffu, word != 0u);
                 __syncwarp();
-                while (queued >= 32) step();  // (a step takes as many cells as lanes are idle)
             }
+            if (queued == 0 && grains == 0 && !__any_sync(0xffffffffu, q != 0u)) break;
+            step();
         }
-        while (queued > 0 || __any_sync(0xffffffffu, q != 0u)) step();
-        if (grains > 0) cover(grains);
         if (DIRECT) {
             if (lane == 0 && taken) {
                 atomicAdd(&a.diag[3], (unsigned long long)taken);

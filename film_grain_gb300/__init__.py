@@ -465,8 +465,8 @@ def render_grainwise(lam, params: Params, derived: Derived, cancel: Optional[Cal
 
 def pixelwise_kernel_count(params: "Params", derived: "Derived") -> int:
     """Kernel launches one pixel-wise render of these params makes: 3 on the per-sample kernel, 6 on the
-    sparse block pass (with the plane's emptiness bitmask and the sorted offsets), 4 on the lean block
-    pass."""
+    stream pass (with the plane's emptiness bitmask, the offsets' phase masks and the dense segments) and on
+    the sparse block pass (with the bitmask and the sorted offsets), 4 on the lean block pass."""
     offs = np.ascontiguousarray(derived.offsets_input, np.float32)
     n = ctypes.c_int32()
     _raise(lib().fg_pixelwise_kernel_count(params.c, derived._c, offs.ctypes.data, ctypes.byref(n)))
@@ -482,8 +482,8 @@ def pixelwise_diagnostics() -> Tuple[int, int, int, int]:
 
 
 def pixelwise_sparse_forms() -> Tuple[int, int]:
-    """(sample-major, grain-major) blocks of the sparse block pass in this thread's last pixel-wise
-    render: the two forms of its sample step, which give identical counts."""
+    """(sample-major blocks of the sparse pass, grain-major tiles of the stream pass) in this thread's last
+    pixel-wise render: two forms of the same test, which give identical counts."""
     arr = (ctypes.c_ulonglong * 2)()
     lib().fg_pixelwise_sparse_forms(arr)
     return tuple(int(v) for v in arr)

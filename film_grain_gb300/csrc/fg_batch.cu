@@ -136,7 +136,10 @@ __global__ void __launch_bounds__(kPwRegenThreads)
     }
     __syncthreads();
     const long long local = b - R.first;
-    pixelwise_regen_pixels(s_pa, (int)(local % R.row_ctas) * kPwRegenThreads, (int)(local / R.row_ctas), 0, s_pa.n);
+    if (pixelwise_two_step(s_pa))
+        pixelwise_regen_pixels<true>(s_pa, (int)(local % R.row_ctas) * kPwRegenThreads, (int)(local / R.row_ctas), 0, s_pa.n);
+    else
+        pixelwise_regen_pixels<false>(s_pa, (int)(local % R.row_ctas) * kPwRegenThreads, (int)(local / R.row_ctas), 0, s_pa.n);
 }
 
 // Pixel-wise items in lean CTAs (256 threads, 4 per SM); the root blocks they leave to fat CTAs are

@@ -111,6 +111,14 @@ struct PixelwiseArgs {
     int cm_gi0, cm_gj0, cm_gw, cm_ghw;
 };
 
+// Whether the per-sample kernel screens this plane's samples in two steps: ranges of more than 4 cells an axis.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool pixelwise_two_step(const PixelwiseArgs &a) {
+    return floor(2.0 * (double)a.rm / (double)a.delta) + 2.0 > 4.0;
+}
+
 struct GrainwiseArgs {
     const float *lam;           // in_w x in_h
     const float2 *offs;         // offsets [n]

@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(PwFat::kThreads, PwFat::kCtasPerSm)
 // Per-sample kernel: one thread per output pixel and part of its samples (pixelwise_regen_pixels); no barriers.
 // CTA b covers pixels [256 (c % row_ctas), +256) of row c / row_ctas, c = b / parts, and samples
 // [per (b % parts), +per).
+template <bool kTwoStep>
 __global__ void __launch_bounds__(kPwRegenThreads) pixelwise_regen_kernel(const __grid_constant__ PixelwiseArgs a,
                                                                           int row_ctas, int parts, int per) {
     if (a.cancel) {  // once per warp: the warp's lanes work in step, so the whole warp stops
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(kPwRegenThreads) pixelwise_regen_kernel(const 
     }
     const unsigned c = blockIdx.x / (unsigned)parts;
     const int k0 = (int)(blockIdx.x % (unsigned)parts) * per;
-    pixelwise_regen_pixels(a, (int)(c % (unsigned)row_ctas) * kPwRegenThreads, (int)(c / (unsigned)row_ctas), k0,
+    pixelwise_regen_pixels<kTwoStep>(a, (int)(c % (unsigned)row_ctas) * kPwRegenThreads, (int)(c / (unsigned)row_ctas), k0,
                            min(a.n, k0 + per));
 }
 
@@ -371,7 +372,10 @@ static cudaError_t launch_pixelwise_regen(const PixelwiseArgs &a, cudaStream_t s
     const double want = warps > 0 ? kPwRegenWarps * (double)std::max(1, sms) / warps : 1.0;
     const int per = std::max(1, (int)std::ceil(a.n / std::max(1.0, want)));
     const int parts = (a.n + per - 1) / per;
-    pixelwise_regen_kernel<<<(unsigned)(grid * parts), kPwRegenThreads, 0, s>>>(a, (int)row_ctas, parts, per);
+    if (pixelwise_two_step(a))
+        pixelwise_regen_kernel<true><<<(unsigned)(grid * parts), kPwRegenThreads, 0, s>>>(a, (int)row_ctas, parts, per);
+    else
+        pixelwise_regen_kernel<false><<<(unsigned)(grid * parts), kPwRegenThreads, 0, s>>>(a, (int)row_ctas, parts, per);
     return cudaGetLastError();
 }
 
@@ -416,9 +420,9 @@ static cudaError_t launch_pixelwise_stream(const PixelwiseArgs &a, const PwSpars
     u.dense = reinterpret_cast<unsigned char *>(u.list + nseg);
     u.count = &counters->list[1];
     // the per-sample kernel's limits, as pixelwise_prefers_regen
-    const double axis = std::floor(2.0 * (double)a.rm / (double)a.delta) + 2.0;
+    const bool two = pixelwise_two_step(a);
     u.limit = std::isfinite(regen_reach(a))
-                  ? (axis > 4.0 ? kPwStreamDenseWide : kPwStreamDense) * (float)a.n * a.zoom * a.zoom
+                  ? (two ? kPwStreamDenseWide : kPwStreamDense) * (float)a.n * a.zoom * a.zoom
                   : HUGE_VALF;
     u.w_max = FG_FMUL(FG_FMUL(a.rm, a.zoom), 1.000008f) + t.eps;  // (stream_candidates' half-width of radius rm, rounded up)
     t.cellmask = g.cellmask;
@@ -443,8 +447,8 @@ static cudaError_t launch_pixelwise_stream(const PixelwiseArgs &a, const PwSpars
     // (1024^2 log-normal 15.6 ms against 14.9), but where segments are few their warps' latency counts more
     // (256^2 ramp 0.32 ms against 0.35).
     const int part = nseg < 32LL * sms ? 4 : 8;
-    pixelwise_dense_kernel<<<(unsigned)ctas, kPwRegenThreads, 0, s>>>(a, bits, t.nw, t.segs, part, &counters->list[0],
-                                                                     u.count, u.list);
+    auto *dense = two ? pixelwise_dense_kernel<true> : pixelwise_dense_kernel<false>;
+    dense<<<(unsigned)ctas, kPwRegenThreads, 0, s>>>(a, bits, t.nw, t.segs, part, &counters->list[0], u.count, u.list);
     return cudaGetLastError();
 }
 

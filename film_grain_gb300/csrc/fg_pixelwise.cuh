@@ -171,13 +171,16 @@ struct RegenQueue {
 //      one of them against its owner's sample.  What is left waits for the next sample's cells, so only
 //      the last round of 32 samples runs with idle lanes; a sample that turns out covered leaves its
 //      pending cells out;
-//   3. ranges wider than 3 x 3 cells (log-normal radii reach three times their mean) are screened in two
-//      steps: the middle cells of all 32 samples first, then the outer cells of the samples that are not
-//      covered yet, dealt to the lanes 32 samples at a time.
+//   3. (kTwoStep) ranges wider than 3 x 3 cells (log-normal radii reach three times their mean) are screened in
+//      two steps: the middle cells of all 32 samples first, then the outer cells of the samples that are not
+//      covered yet, dealt to the lanes 32 samples at a time.  Without it the code is smaller: 1021 x 763, ranges of
+//      3 cells, 2.85 ms against 3.11.  With it 700 x 500 log-normal 0.05 / 0.01, N 16 takes 1.14 ms; with its steps
+//      written out twice, 1.79 (the code of a regenerated cell then fills the instruction cache).
 // Coverage is an OR over the cells, so neither the order nor the dealing changes it.  A range wider
 // than 8 cells on an axis (outside the plane-level choice of this path) or than two lambda pixels runs the
 // plain loop instead.
 // What bounds it: the shifts, xors and multiplies of the screens' hashes and of the regenerated cells' draws.
+template <bool kTwoStep>
 __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a, const UniformF32 &U, int x, int y,
                                                           bool valid, int k0, int k1, RegenQueue &Q,
                                                           unsigned int *bits = nullptr) {
@@ -210,15 +213,47 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
             head += count;
             queued -= count;
         };
-        // Cells of sample ks of lane `owner` that may hold grains -- the middle 3 x 3 of its range, or the others --
-        // into the queue, rank by rank.  Returns whether its range is wider than that.
-        auto screen = [&](int owner, int ks, bool live, bool middle) -> bool {
+        // Turn by turn: first each of the 32 samples' middle 3 x 3 cells (without kTwoStep all its cells), a sample of
+        // every lane a turn, then (with wider ranges) the outer cells of the samples not covered by then, 32 of any lane and sample a turn.  A
+        // turn's cells that may hold grains go into the queue, rank by rank.  One place for each step: the code of
+        // a regenerated cell is what the instruction cache holds.
+        bool wide = false;
+        int turn = 0, scanned = 0, phead = 0, pairs = 0;
+        for (;;) {
+            int owner = lane, ks = turn;
+            bool live = valid, middle = true, last;
+            if (turn < nk) {
+                turn++;
+                last = turn == nk;
+            } else if constexpr (!kTwoStep) {
+                break;
+            } else {
+                if (!__any_sync(0xffffffffu, wide)) break;
+                for (; pairs < 32 && scanned < nk; scanned++) {
+                    const bool due = valid && !((Q.hit[scanned] >> lane) & 1u);
+                    const unsigned d = __ballot_sync(0xffffffffu, due);
+                    if (due)
+                        Q.pair[(phead + pairs + __popc(d & ((1u << lane) - 1u))) & 63] = (unsigned short)(lane | (scanned << 5));
+                    pairs += __popc(d);
+                }
+                if (pairs == 0 && queued == 0) break;
+                __syncwarp();
+                const int c = min(pairs, 32);  // (0: a turn that only empties the queue)
+                const unsigned pr = c > 0 ? Q.pair[(phead + (lane < c ? lane : 0)) & 63] : 0u;
+                __syncwarp();
+                phead += c;
+                pairs -= c;
+                owner = (int)(pr & 31u);
+                ks = (int)(pr >> 5);
+                live = lane < c;
+                middle = false;
+                last = pairs == 0 && scanned == nk;
+            }
             const int j0 = __shfl_sync(0xffffffffu, rows.j0, ks), nj = __shfl_sync(0xffffffffu, rows.nj, ks);
             const int iy0 = __shfl_sync(0xffffffffu, rows.iy0, ks);
             const unsigned up = __shfl_sync(0xffffffffu, rows.up, ks);
             int i0 = 0, mid = 0;
             unsigned long long m = 0ull;
-            bool wide = false;
             if (live && nj != 0) {  // nj == 0: no cell (src/pixelwise.rs:60-62)
                 const float xg = xg_of(x - lane + owner, a.inv_zoom, a.offs[kb + ks].x);
                 i0 = f2i_floor(FG_FDIV(FG_FSUB(xg, a.rm), a.delta));
@@ -236,12 +271,13 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
                     } else {
                         const int mi = (ni - 1) >> 1, mj = (nj - 1) >> 1;
                         mid = mi * 8 + mj;
-                        wide = ni > 3 || nj > 3;
+                        if (kTwoStep) wide = wide || ni > 3 || nj > 3;
                         const CellParam *row0 = a.cells + (long long)iy0 * a.in_w, *row1 = up ? row0 + a.in_w : row0;
                         uint32_t b0 = maybe_bound(row0[ix0].thresh), b1 = maybe_bound(row1[ix0].thresh);
                         int ix = ix0;
-                        const int di1 = middle ? min(mi + 2, ni) : ni, dj1 = middle ? min(mj + 2, nj) : nj;
-                        for (int di = middle ? max(mi - 1, 0) : 0; di < di1; di++) {
+                        const bool part = kTwoStep && middle;
+                        const int di1 = part ? min(mi + 2, ni) : ni, dj1 = part ? min(mj + 2, nj) : nj;
+                        for (int di = part ? max(mi - 1, 0) : 0; di < di1; di++) {
                             const int i = i0 + di;
                             if (ix != ix1 && cell_axis_pixel(i, a.delta, a.in_w) == ix1) {
                                 ix = ix1;
@@ -250,8 +286,8 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
                             }
                             const uint64_t colh = cell_col_hash(a.seed, i);
                             unsigned col = 0u;
-                            for (int dj = middle ? max(mj - 1, 0) : 0; dj < dj1; dj++) {
-                                if (!middle && abs(di - mi) <= 1 && abs(dj - mj) <= 1) continue;  // in the first step
+                            for (int dj = part ? max(mj - 1, 0) : 0; dj < dj1; dj++) {
+                                if (kTwoStep && !middle && abs(di - mi) <= 1 && abs(dj - mj) <= 1) continue;  // in the first step
                                 col |= (first_draw_maybe(cell_row_hash(colh, j0 + dj), ((up >> dj) & 1u) ? b1 : b0) ? 1u : 0u)
                                        << dj;
                             }
@@ -266,7 +302,6 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
             __syncwarp();
             for (;;) {
                 const unsigned pending = __ballot_sync(0xffffffffu, m != 0ull);
-                if (pending == 0u) break;
                 if (m != 0ull) {
                     const int pos = __ffsll((long long)m) - 1;
                     m &= m - 1ull;
@@ -277,37 +312,14 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
                 }
                 queued += __popc(pending);
                 __syncwarp();
-                if (queued >= 32) {
-                    run(32);
+                if (queued >= 32 || (last && pending == 0u && queued > 0)) {
+                    run(min(queued, 32));
                     if ((Q.hit[ks] >> owner) & 1u) m = 0ull;
-                }
-            }
-            return wide;
-        };
-        bool wide = false;
-        for (int ks = 0; ks < nk; ks++) wide = screen(lane, ks, valid, true) || wide;
-        if (__any_sync(0xffffffffu, wide)) {
-            if (queued > 0) run(queued);
-            int phead = 0, pairs = 0;
-            for (int ks = 0; ks < nk; ks++) {
-                const bool due = valid && !((Q.hit[ks] >> lane) & 1u);
-                const unsigned d = __ballot_sync(0xffffffffu, due);
-                if (due) Q.pair[(phead + pairs + __popc(d & ((1u << lane) - 1u))) & 63] = (unsigned short)(lane | (ks << 5));
-                pairs += __popc(d);
-                __syncwarp();
-                if (pairs >= 32 || (ks == nk - 1 && pairs > 0)) {
-                    do {
-                        const int c = min(pairs, 32);
-                        const unsigned pr = Q.pair[(phead + (lane < c ? lane : 0)) & 63];
-                        __syncwarp();
-                        phead += c;
-                        pairs -= c;
-                        screen((int)(pr & 31u), (int)(pr >> 5), lane < c, false);
-                    } while (ks == nk - 1 && pairs > 0);
+                } else if (pending == 0u) {
+                    break;
                 }
             }
         }
-        if (queued > 0) run(queued);
         // word ks holds sample ks's lanes: lane b counts the words with bit b
         const unsigned w = Q.hit[lane];
         __syncwarp();
@@ -331,6 +343,7 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
 // (lane- or rank-major), where a sample of 32 lanes left its last round of 32 cells half empty, and above 1.1 a
 // loop that visited one cell at a time.  GB300, radius 0.025, N 64: 1021 x 763 blobs 4.03 -> 2.82 ms,
 // 700 x 500 ramp 3.09 -> 1.86 ms (1.94 with the loop kept above 1.1).
+template <bool kTwoStep>
 __device__ __forceinline__ void pixelwise_regen_pixels(const PixelwiseArgs &a, int x0, int y, int k0, int k1) {
     __shared__ RegenQueue queues[kPwRegenThreads / 32];
     const int x = x0 + (int)threadIdx.x;
@@ -343,7 +356,7 @@ __device__ __forceinline__ void pixelwise_regen_pixels(const PixelwiseArgs &a, i
     if (x - (int)(threadIdx.x & 31) >= a.out_w) return;  // whole warps
     const bool valid = x < a.out_w;
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
-    const uint32_t hits = pixelwise_pixel_queue(a, U, x, y, valid, k0, k1, queues[threadIdx.x >> 5]);  // all 32 lanes
+    const uint32_t hits = pixelwise_pixel_queue<kTwoStep>(a, U, x, y, valid, k0, k1, queues[threadIdx.x >> 5]);  // all 32 lanes
     if (!valid) return;
     float *out = a.out + (long long)y * a.out_w + x;
     if (k1 - k0 == a.n) *out = (float)hits;

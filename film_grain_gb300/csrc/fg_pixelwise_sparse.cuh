@@ -9,7 +9,8 @@
 //   0. (cell_mask_kernel, before the pass) the emptiness of every cell of the plane's cell grid is one
 //      bit of a column-major bitmask in global memory: a thread owns one column and 32 rows (the column
 //      stage of the cell hash computed once) and stores one word; a cell is empty when its first
-//      uniform does not exceed its Knuth threshold (cell_count_h).  Every cell is hashed once per plane;
+//      uniform does not exceed its Knuth threshold, and the screen (first_draw_maybe) lists one in 2^8 of
+//      the empty ones too.  Every cell is hashed once per plane;
 //   1. the CTA copies the bits of its window -- the cells its owned samples can reach -- into shared
 //      memory (column-major: word k of window column c holds rows 32k .. 32k + 31);
 //   2. the set bits, ranked in column-major order, list the non-empty cells; their grain counts (the

@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(PwStream::kThreads)
 
 // The segments left to the per-sample pass, their samples in parts of `part` (a divisor of 32): each warp takes the
 // next part.
+template <bool kTwoStep>
 __global__ void __launch_bounds__(kPwRegenThreads)
     pixelwise_dense_kernel(const __grid_constant__ PixelwiseArgs a, unsigned int *bits, int nw, int segs, int part,
                            int *__restrict__ next, const int *__restrict__ count, const int *__restrict__ list) {
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(kPwRegenThreads)
         const int seg = list[i / parts], y = seg / segs, x = 32 * (seg % segs) + lane;
         const int k0 = i % parts * part, k1 = min(a.n, k0 + part);
         const bool valid = x < a.out_w;
-        pixelwise_pixel_queue(a, U, x, y, valid, k0, k1, queues[threadIdx.x >> 5],
+        pixelwise_pixel_queue<kTwoStep>(a, U, x, y, valid, k0, k1, queues[threadIdx.x >> 5],
                               valid ? bits + ((long long)y * a.out_w + x) * nw : nullptr);
         done += (unsigned long long)min(32, a.out_w - 32 * (seg % segs)) * (unsigned long long)(k1 - k0);
     }

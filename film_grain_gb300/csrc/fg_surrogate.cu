@@ -5,12 +5,13 @@
 //   h0  = relu(conv_in(x) + b_in)                     16 -> 32
 //   h_l = h_{l-1} + relu(conv_l(h_{l-1}) + b_l)       32 -> 32, l = 1..L
 //   y   = u + conv_out(h_L) + b_out                   32 -> 1 (8 computed channels, channel 0 kept), f32
-// Every conv is an implicit GEMM on the tensor cores (mma.sync m16n8k16, bf16 x bf16 -> f32): a CTA owns
-// an 8 x 32 pixel tile, stages the haloed input tile and all weights in shared memory, and each of its 8
-// warps computes one 32-pixel tile row for every output channel.  The backward pass reuses the forward
-// kernel for the data gradient (weights flipped and transposed) and has a persistent weight-gradient
-// kernel in which pixels are the reduction dimension.  No bit-exactness constraint applies here, so this
-// unit is compiled with FMA contraction.
+// The convs and the weight gradients run on tcgen05 (fg_sg_tc.cu, fg_sg_wgrad.cu); buffers or channel strides that
+// are not 16-byte aligned take this unit's kernels: implicit GEMMs on mma.sync m16n8k16 (bf16 x bf16 -> f32), a CTA
+// owning an 8 x 32 pixel tile, with the haloed input tile and all weights in shared memory, each of its 8
+// warps computing one 32-pixel tile row for every output channel; the data gradient by the forward kernel
+// (weights flipped and transposed), the weight gradient by a persistent kernel in which pixels are the
+// reduction dimension.  No bit-exactness constraint applies here, so this unit is compiled with FMA
+// contraction.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -347,3 +347,13 @@ def test_pixelwise_stream_all_dense_and_empty(cuda, fgl, orc):
     _check("pixel", fgl, orc, np.ones((96, 100), np.float32), radius=0.1, n=64, seed=3)
     assert fgl.pixelwise_diagnostics()[0] == 96 * 100 * 64  # every segment on the per-sample kernel
     _check("pixel", fgl, orc, np.zeros((96, 100), np.float32), radius=0.1, n=64, seed=3)
+
+
+@pytest.mark.parametrize("n", [2, 9, 33, 40])
+def test_pixelwise_two_step_ranges(cuda, fgl, orc, n):
+    """The per-sample kernel with ranges of five cells and more: samples that the middle cells leave uncovered,
+    from none to all of a warp's (dark, middle and saturated areas), in one and two batches of 32."""
+    plane = _blobs(70, 45)
+    plane[:15, :40] = 0.02
+    plane[30:, 20:] = 1.0
+    _check("pixel", fgl, orc, plane, radius=0.03, dist="lognorm", sd=0.012, n=n, seed=21)

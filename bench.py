@@ -204,12 +204,12 @@ def cpu_pixel_baseline(oracle, planes, wl, threads, rows=None):
 # --profile-once runs), per unit of work: sg_conv32_tc_kernel (the residual conv) on the 1024^2 x 3
 # surrogate input, 373.9 MB read+write for 3 x 1024^2 px; grainwise_persistent_kernel on a 512^2 ->
 # 1024^2 plane of the grain-wise blob frame, 18.25 MB per 1024^2 output pixels (the lambda plane plus the
-# sample-mask lines that miss L2); cell_mask_kernel + pixelwise_sparse_kernel on the 1024^2 flat plane
-# of the large frame's parameters, 170.3 + 247.6 MB per 1024^2 output pixels (the emptiness bitmask
-# written, then read with the cell table).
+# sample-mask lines that miss L2); cell_mask_kernel + pixelwise_stream_kernel on the 1024^2 flat plane
+# of the large frame's parameters, 172.9 + 288.4 MB per 1024^2 output pixels (the emptiness bitmask
+# written, then read with the cell table and the samples' bits).
 SG_CONV_DRAM_BYTES_PER_PX = 373.9e6 / (3 * 1024 * 1024)
 GRAINWISE_DRAM_BYTES_PER_OUT_PX = 18.25e6 / (1024 * 1024)
-PIXELWISE_DRAM_BYTES_PER_OUT_PX = (170.3e6 + 247.6e6) / (1024 * 1024)
+PIXELWISE_DRAM_BYTES_PER_OUT_PX = (172.9e6 + 288.4e6) / (1024 * 1024)
 
 # Algorithmic lane-ops of the pixel-wise path (an exact method that hashes every cell once): per cell
 # its hash and first uniform (~65: the row stage of mix3, one SplitMix64, ~24; the four PCG32 seed words
@@ -720,10 +720,10 @@ def plain_line(wl_name, steps, warmup, rank=0, world=1, dist=None, cpu=True, e2e
         line["roofline"] = {"bound": "sm_issue", "achieved": ach / 1e12, "peak": peak / 1e12, "unit": "Tlane-op/s",
                             "frac": ach / peak,
                             "traffic": PIXELWISE_DRAM_BYTES_PER_OUT_PX * ow * oh,
-                            "traffic_basis": "ncu dram bytes of cell_mask_kernel + pixelwise_sparse_kernel on the "
+                            "traffic_basis": "ncu dram bytes of cell_mask_kernel + pixelwise_stream_kernel on the "
                                              "1024^2 flat plane of the large frame's parameters, scaled by "
                                              "output pixels",
-                            "kernel": "cell_mask_kernel + pixelwise_sparse_kernel + pixelwise_deferred_kernel "
+                            "kernel": "cell_mask_kernel + pixelwise_stream_kernel + pixelwise_dense_kernel "
                                       "(launch_ms: the whole render call of a plane)", "launch_ms": launch_ms,
                             "lane_ops_per_launch": [o["total"] for o in ops], "model_terms": ops[0],
                             "peak_basis": peak_basis}

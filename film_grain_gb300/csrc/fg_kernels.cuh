@@ -68,9 +68,9 @@ constexpr float kPwRegenSmall = 5.0f;
 constexpr double kPwRegenWarps = 64.0;
 // The stream pass (fg_pixelwise_stream.cuh): planes of kPwStreamPixels output pixels and more, and the grains per
 // output pixel, in multiples of N, above which a segment's samples go to the per-sample kernel -- with ranges of
-// up to 4 cells an axis, and wider ones, whose samples look at more cells.  Log-normal 0.025 at 1024^2, N 256:
-// at 2 N 20.7 ms, 4 N 18.9, 6 N 20.2, 10 N 21.1; 1080p radius 0.1 N 32: at 1.3 N 2.19 ms, 2 N 2.10, 3 N 2.02;
-// 1000^2 ramp, the same grain: 1.68, 1.58, 1.70.
+// up to 4 cells an axis, and wider ones, whose samples look at more cells.  Log-normal 0.025 / 0.01, N 256:
+// 1024^2 blobs at 2.2 N 13.4 ms, 3 N 12.3, 4 N 13.1, a 1000^2 ramp 29.3, 24.1, 22.0; radius 0.1 N 32: 1080p at
+// 1.3 N 2.19 ms, 2 N 2.10, 3 N 2.02, a 1000^2 ramp 1.68, 1.58, 1.70.
 constexpr double kPwStreamPixels = 8192.0;
 constexpr float kPwStreamDense = 2.0f, kPwStreamDenseWide = 4.0f;
 

@@ -17,8 +17,8 @@
 // What bounds it: the instructions of the grains' draws (seed words, Poisson and position draws, the
 // log-normal radius) and of their candidates: 70 ps a grain on the log-normal plane below.  It replaced a form of the sparse pass that staged each block's grains in shared
 // memory, generating a window's margin again for every block, and the fat pass over the denser blocks: GB300,
-// 1024^2 log-normal 0.025 N 256 sparse + fat 32.6 ms, stream + per-sample 13.8; 1080p radius 0.1 N 32 2.49 and
-// 1.03; 256^2 ramp 0.12 N 64 0.30 and 0.23.
+// 1024^2 log-normal 0.025 N 256 sparse + fat 32.6 ms, stream + per-sample 9.8; 1080p radius 0.1 N 32 2.49 and
+// 1.00; 256^2 ramp 0.12 N 64 0.30 and 0.15.
 #pragma once
 
 #include "fg_phase.cuh"

@@ -21,6 +21,7 @@ struct GwTile {
     float flast_x, flast_y;          // last output column / row as floats
     unsigned int *gmask;             // the chunk's first word of out_w x out_h x gwords
     int gwords;
+    float eps;  // margin of the one-pixel form (gw_splat)
 };
 
 // floor / ceil of an f32.  With kSmall (every coordinate within +-2^22) they are one directed-rounding
@@ -53,11 +54,38 @@ __device__ __forceinline__ bool gw_range(float c, float r, float lo_t, float hi_
 // radius, offset o, sample k of the chunk.  Most pairs have one pixel or none in their bounds, so the loops
 // test their end after the body.  Pixels of the tile's rectangle are integers below 2^24, so their index is
 // taken in f32.
+// A radius below 0.45 (with T.eps, several ulps of the largest coordinate) leaves the nearest pixel alone: any
+// other centre is half a pixel away or more.  Where both distances are below the radius by T.eps the bounds
+// hold whatever their roundings, and only a pair nearer to its edge computes them.
+// 124 x 1024, radius 0.2, N 256 4.51 -> 4.24 ms; 1024^2 -> 2048^2 log-normal 0.05 6.47 -> 6.20 ms.
+__device__ __forceinline__ void gw_set(const GwTile &T, unsigned int *mask, float fx, float fy, int k) {
+    const float lx = FG_FSUB(fx, T.frx0), ly = FG_FSUB(fy, T.fry0);
+    const unsigned bit = 1u << (k & 31);
+    if (lx >= 0.0f && lx < T.frw && ly >= 0.0f && ly < T.frh)
+        atomicOr(mask + (int)FG_FADD(FG_FMUL(ly, T.frw), lx) * T.words + (k >> 5), bit);
+    else
+        atomicOr(T.gmask + ((long long)(int)fy * T.out_w + (int)fx) * T.gwords + (k >> 5), bit);
+}
 template <bool kSmall>
 __device__ __forceinline__ void gw_splat(const GwTile &T, unsigned int *mask, float czx, float czy, float ro,
                                          const float2 o, int k) {
     const float tx = FG_FADD(czx, o.x), ty = FG_FADD(czy, o.y);
     float y0, y1, x0, x1;
+    if (kSmall && FG_FADD(ro, T.eps) < 0.45f) {
+        constexpr float kRint = 12582912.0f;  // 1.5 * 2^23: adding and removing it rounds to an integer
+        const float fx = FG_FSUB(FG_FADD(FG_FSUB(tx, 0.5f), kRint), kRint);
+        const float fy = FG_FSUB(FG_FADD(FG_FSUB(ty, 0.5f), kRint), kRint);
+        const float dx = FG_FSUB(FG_FADD(fx, 0.5f), tx), dy = FG_FSUB(FG_FADD(fy, 0.5f), ty);
+        if (!(FG_FADD(FG_FMUL(dx, dx), FG_FMUL(dy, dy)) <= FG_FMUL(ro, ro))) return;
+        if (!(fx >= 0.0f && fx <= T.flast_x && fy >= 0.0f && fy <= T.flast_y)) return;
+        if (fmaxf(fabsf(dx), fabsf(dy)) > FG_FSUB(ro, T.eps)) {
+            if (!(gw_range<kSmall>(ty, ro, 0.0f, T.flast_y, y0, y1) && gw_range<kSmall>(tx, ro, 0.0f, T.flast_x, x0, x1)))
+                return;
+            if (fx < x0 || fx > x1 || fy < y0 || fy > y1) return;
+        }
+        gw_set(T, mask, fx, fy, k);
+        return;
+    }
     const bool in_y = gw_range<kSmall>(ty, ro, 0.0f, T.flast_y, y0, y1);
     const bool in_x = gw_range<kSmall>(tx, ro, 0.0f, T.flast_x, x0, x1);
     if (!(in_x && in_y)) return;
@@ -68,14 +96,7 @@ __device__ __forceinline__ void gw_splat(const GwTile &T, unsigned int *mask, fl
         if (dysq <= rsq) {
             for (float fx = x0;;) {
                 const float dx = FG_FSUB(FG_FADD(fx, 0.5f), tx);
-                if (FG_FADD(FG_FMUL(dx, dx), dysq) <= rsq) {
-                    const float lx = FG_FSUB(fx, T.frx0), ly = FG_FSUB(fy, T.fry0);
-                    const unsigned bit = 1u << (k & 31);
-                    if (lx >= 0.0f && lx < T.frw && ly >= 0.0f && ly < T.frh)
-                        atomicOr(mask + (int)FG_FADD(FG_FMUL(ly, T.frw), lx) * T.words + (k >> 5), bit);
-                    else
-                        atomicOr(T.gmask + ((long long)(int)fy * T.out_w + (int)fx) * T.gwords + (k >> 5), bit);
-                }
+                if (FG_FADD(FG_FMUL(dx, dx), dysq) <= rsq) gw_set(T, mask, fx, fy, k);
                 if (!(fx < x1)) break;
                 fx = FG_FADD(fx, 1.0f);
             }
@@ -200,6 +221,7 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
     T.frh = (float)T.rh;
     T.words = W;
     T.out_w = a.out_w;
+    T.eps = 2.0f * a.frac_eps;  // eight ulps of the largest coordinate and more
     T.flast_x = (float)(a.out_w - 1);
     T.flast_y = (float)(a.out_h - 1);
     T.gmask = a.gmask + chunk * a.chunk_words;

@@ -357,3 +357,14 @@ def test_pixelwise_two_step_ranges(cuda, fgl, orc, n):
     plane[:15, :40] = 0.02
     plane[30:, 20:] = 1.0
     _check("pixel", fgl, orc, plane, radius=0.03, dist="lognorm", sd=0.012, n=n, seed=21)
+
+
+@pytest.mark.parametrize("radius,zoom,n", [(0.22, 2.0, 40), (0.2249, 2.0, 70), (0.2251, 2.0, 70), (0.004, 1.0, 64),
+                                           (0.00002, 1.0, 33), (0.4, 1.0, 130)])
+def test_grainwise_one_pixel_form(cuda, fgl, orc, radius, zoom, n):
+    """Zoomed radii up to and beyond 0.45, where a pair's bounds can hold more than the nearest pixel, and radii
+    around the coordinates' rounding, where every hit computes its bounds; the plane's edges."""
+    plane = _blobs(37, 29)
+    plane[:, -3:] = 0.9
+    dim = 1e-7 if radius < 0.001 else 1e-3 if radius < 0.01 else 1.0  # grains a pixel: not too many
+    _check("grain", fgl, orc, (plane * dim).astype(np.float32), radius=radius, zoom=zoom, n=n, seed=5)

@@ -230,6 +230,12 @@ static size_t stream_list_at(const PwSparseGrid &g, int n) {
 // pixel of an offset is exact while that reach plus the f32 rounding of the pixel coordinates (eps: a few
 // ulps of the largest coordinate) stays below half a pixel, and the rounding to an integer by adding
 // 1.5 * 2^23 needs coordinates below 2^22.
+// Reach: up to 0.44, which leaves the candidate room for the rounding (500 x 400, constant radius 0.42, N 64: 478 us
+// here, 518 us on the sparse pass; at 0.21, zoom 2, N 22 on 276 x 565: 411 and 641).
+// Hits: the walk over a grain's hits costs per hit, the block passes per sample of a block, so those win where a
+// grain covers many samples.  500 x 400 to 600 x 500, a ramp, here and on the block passes: 36 hits 862 and 968 us,
+// 45 hits 1127 and 1423 (radius 0.3) or 747 and 828 (0.38), 55 hits 796 and 794 (0.42), 58 hits 1035 and 881, 72 hits
+// 2123 and 1662; 116 hits (400 x 400, radius 0.19, zoom 2, N 256) 4799 and 2885.  Hence 48.
 // Planes below kPwStreamPixels stay with the sparse and fat passes, whose forms the tests hold against the oracle
 // there.
 // Tiles: the largest of 512 .. 32 cells an edge whose footprint's bits leave room for many CTAs an SM and whose
@@ -240,7 +246,9 @@ static bool plan_stream(const PixelwiseArgs &a, const PwSparseGrid &g, int sms, 
                                  std::fabs(a.offy_max)});
     const double coord = (double)std::max(a.out_w, a.out_h) + ext * a.zoom + 2.0;
     const double eps = coord * 0x1p-21 + 0x1p-20;
-    if (!(coord < 0x1p21) || !((double)a.rm * a.zoom + eps <= 0.4)) return false;
+    if (!(coord < 0x1p21) || !((double)a.rm * a.zoom + eps <= 0.44)) return false;
+    const double hits = a.n * 3.14 * a.radius_mean * a.radius_mean * a.zoom * a.zoom;
+    if (!(hits < 48.0)) return false;
     t->eps = (float)eps;
     // the roundings of xg, of xg +- rm, of the cell's origin and of the divisions: a few ulps of the largest
     // input coordinate
@@ -267,7 +275,7 @@ static bool plan_stream(const PixelwiseArgs &a, const PwSparseGrid &g, int sms, 
             // no tiles (DIRECT) where they would be this small, unless a grain has many hits to gather
             t->direct = T <= 64 && t->gw < 65536 && 32.0 * t->ghw < 65536.0 &&
                         (double)a.out_w * a.out_h * t->nw < 0x1p31 &&
-                        a.n * 3.14 * a.radius_mean * a.radius_mean * a.zoom * a.zoom < 16.0;
+                        hits < 16.0;
             if (t->direct) t->sub = 8;
             return (double)t->ntx * t->nty < 2.0e9;
         }

@@ -325,6 +325,7 @@ def test_pixelwise_small_plane_parts(cuda, fgl, orc, n):
     (103, 91, 0.05, "lognorm", 1.0, 256, None),
     (200, 180, 0.7, "const", 0.5, 50, None),     # grains wider than an input pixel
     (41, 33, 0.12, "const", 3.0, 40, None),      # reach 0.36 of a pixel
+    (67, 49, 0.21, "const", 2.0, 22, None),      # reach 0.42
     (120, 90, 0.3, "const", 1.0, 64, 1.0),       # cells of a pixel, the rejection regime
     (110, 90, 0.3, "const", 1.0, 20, 0.04),      # ranges of 16 cells: no per-sample kernel
     (131, 67, 0.3, "const", 1.0, 128, None),     # 36 hits a grain: tiles and their footprints

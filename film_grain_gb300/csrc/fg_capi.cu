@@ -294,10 +294,14 @@ fg_status enqueue_pixelwise(const float *d_lam, const fg_params &p, const fg_der
                             int *d_cancel) {
     const int in_w = (int)d.input_width, in_h = (int)d.input_height;
     const int out_w = (int)d.output_width, out_h = (int)d.output_height;
+    const long long n_in = (long long)in_w * in_h, n_out = (long long)out_w * out_h;
+    // An output that shares memory with lambda (a render in place) is cleared only once the cell table is made.
+    const bool in_place = !w.bits && d_out < d_lam + n_in && d_lam < d_out + n_out;
     FG_CUDA(launch_cell_params(d_lam, in_w, in_h, d.delta, w.cells,
                                w.bits ? w.bits : reinterpret_cast<unsigned int *>(d_out),
-                               w.bits ? (long long)(w.bits_bytes / sizeof(int)) : (long long)out_w * out_h, w.counters, s),
+                               w.bits ? (long long)(w.bits_bytes / sizeof(int)) : (in_place ? 0 : n_out), w.counters, s),
             "cell params");
+    if (in_place) FG_CUDA(cudaMemsetAsync(d_out, 0, sizeof(float) * n_out, s), "clear output");
     PixelwiseArgs a = pixelwise_args(p, d, pl, d_lam, w.cells, w.offs, d_out, w.counters->diag);
     a.cancel = d_cancel;
     FG_CUDA(launch_pixelwise(a, pl.nby, w.listed ? w.counters : nullptr, w.mask, w.bits, s), "pixelwise kernel");

@@ -369,3 +369,31 @@ def test_grainwise_one_pixel_form(cuda, fgl, orc, radius, zoom, n):
     plane[:, -3:] = 0.9
     dim = 1e-7 if radius < 0.001 else 1e-3 if radius < 0.01 else 1.0  # grains a pixel: not too many
     _check("grain", fgl, orc, (plane * dim).astype(np.float32), radius=radius, zoom=zoom, n=n, seed=5)
+
+
+@pytest.mark.parametrize("w,h,radius,zoom,n,kernels", [
+    (96, 64, 0.1, 1.0, 32, 3),    # per-sample kernel
+    (160, 128, 0.1, 1.0, 64, 6),  # stream pass
+    (160, 128, 0.45, 1.0, 64, 6),  # sparse and fat passes
+    (160, 128, 0.45, 0.5, 64, 6),  # an output smaller than lambda
+    (160, 128, 0.2, 1.0, 300, 4),  # lean and fat passes
+])
+def test_pixelwise_in_place(cuda, fgl, w, h, radius, zoom, n, kernels):
+    """An output that is lambda's own memory, or shares its end, gets what a separate one gets, through every
+    pixel-wise entry point."""
+    torch = cuda
+    L = fgl.lib()
+    p = fgl.ParamsBuilder(radius_mean=radius, zoom=zoom, n_samples=n, seed=3).build()
+    d = fgl.derive_common(p, (w, h))
+    lam = torch.from_numpy(fgl.lambda_plane(fgl.normalize_plane(_blobs(w, h))[0], d.inv_e_pi_r2)).cuda()
+    assert fgl.pixelwise_kernel_count(p, d) == kernels
+    want = fgl.render_pixelwise(lam, p, d).flatten()
+    offs = np.ascontiguousarray(d.offsets_input, np.float32)
+    st = torch.cuda.current_stream().cuda_stream
+    for name in ("fg_render_pixelwise", "fg_render_pixelwise_async", "fg_render_pixelwise_noalloc"):
+        for at in (0, w * h - 7):  # the output's first float in lambda
+            buf = torch.cat([lam.flatten(), torch.full((want.numel(),), 0.5, device="cuda")])
+            args = [buf.data_ptr(), p.c, d._c, offs.ctypes.data, buf[at:].data_ptr()]
+            args += [None, st] if name == "fg_render_pixelwise" else [st]
+            assert getattr(L, name)(*args) == 0, L.fg_last_error_message().decode()
+            assert torch.equal(buf[at:at + want.numel()], want), (name, at)

@@ -76,14 +76,27 @@ constexpr float kPwStreamDense = 2.0f, kPwStreamDenseWide = 4.0f;
 
 // In-launch cancellation: `cancel` is null or two words of mapped pinned host memory.  Word 0 is set
 // by the waiting host thread once the caller's cancel flag turns non-zero; the persistent passes
-// read it once per work item they pull (the block passes once per block) and stop, and a CTA that
-// stops on it sets word 1.
+// read it once per work item they pull (the block passes once per block, the per-sample kernel once per CTA)
+// and stop, and a CTA that stops on it sets word 1.  Reads of host memory go one after the other, about 7 ns
+// each, so warps whose items are short look at it by the clock (CancelPoll).
 #ifdef __CUDACC__
 __device__ __forceinline__ bool cancel_requested(int *cancel) {
     if (!cancel || *(volatile int *)cancel == 0) return false;
     *(volatile int *)(cancel + 1) = 1;
     return true;
 }
+// A warp's look at the flag every 200 us.  512 x 512, radius 0.1, N 32, with a flag, looking once per item of
+// the stream and dense passes: 1.92 ms a call against 0.40 without a flag.
+struct CancelPoll {
+    static constexpr long long kCycles = 400000;
+    long long last;
+    __device__ __forceinline__ void begin() { last = clock64(); }
+    __device__ __forceinline__ bool requested(int *cancel) {
+        if (!cancel || clock64() - last < kCycles) return false;
+        last = clock64();
+        return cancel_requested(cancel);
+    }
+};
 #endif
 
 struct PixelwiseArgs {

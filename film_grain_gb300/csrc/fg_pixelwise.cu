@@ -321,17 +321,13 @@ __global__ void __launch_bounds__(PwFat::kThreads, PwFat::kCtasPerSm)
     }
 }
 
-// Per-sample kernel: one thread per output pixel and part of its samples (pixelwise_regen_pixels); no barriers.
+// Per-sample kernel: one thread per output pixel and part of its samples (pixelwise_regen_pixels).
 // CTA b covers pixels [256 (c % row_ctas), +256) of row c / row_ctas, c = b / parts, and samples
 // [per (b % parts), +per).
 template <bool kTwoStep>
 __global__ void __launch_bounds__(kPwRegenThreads) pixelwise_regen_kernel(const __grid_constant__ PixelwiseArgs a,
                                                                           int row_ctas, int parts, int per) {
-    if (a.cancel) {  // once per warp: the warp's lanes work in step, so the whole warp stops
-        int stop = 0;
-        if ((threadIdx.x & 31) == 0) stop = cancel_requested(a.cancel) ? 1 : 0;
-        if (__shfl_sync(0xffffffffu, stop, 0)) return;
-    }
+    if (a.cancel && __syncthreads_or(threadIdx.x == 0 && cancel_requested(a.cancel))) return;
     const unsigned c = blockIdx.x / (unsigned)parts;
     const int k0 = (int)(blockIdx.x % (unsigned)parts) * per;
     pixelwise_regen_pixels<kTwoStep>(a, (int)(c % (unsigned)row_ctas) * kPwRegenThreads, (int)(c / (unsigned)row_ctas), k0,

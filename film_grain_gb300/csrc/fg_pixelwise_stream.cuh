@@ -203,6 +203,8 @@ __global__ void __launch_bounds__(PwStream::kThreads)
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
     const int ntiles = g.ntx * g.nty, chunk_rows = g.tile >> 5;
     const bool any_dense = *g.dense_count != 0;
+    CancelPoll poll;  // (DIRECT)
+    poll.begin();
     for (;;) {
         __syncthreads();  // the tables; the previous tile's bits are written out
         int tile = 0;
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(PwStream::kThreads)
             while (more && queued < 32) {
                 if (pending == 0u) {
                     int c = chunks;
-                    if (lane == 0 && !(DIRECT && cancel_requested(a.cancel))) c = atomicAdd(DIRECT ? g.next : &S.chunk, 1);
+                    if (lane == 0 && !(DIRECT && poll.requested(a.cancel))) c = atomicAdd(DIRECT ? g.next : &S.chunk, 1);
                     c = __shfl_sync(0xffffffffu, c, 0);
                     if (c >= chunks) {
                         more = false;
@@ -365,9 +367,11 @@ __global__ void __launch_bounds__(kPwRegenThreads)
     const long long n = (long long)*count * parts;
     const UniformF32 U = uniform_f32_new(0.0f, a.delta);
     unsigned long long done = 0;
+    CancelPoll poll;
+    poll.begin();
     for (;;) {
         int i = -1;
-        if (lane == 0 && !cancel_requested(a.cancel)) i = atomicAdd(next, 1);
+        if (lane == 0 && !poll.requested(a.cancel)) i = atomicAdd(next, 1);
         i = __shfl_sync(0xffffffffu, i, 0);
         if (i < 0 || i >= n) break;
         const int seg = list[i / parts], y = seg / segs, x = 32 * (seg % segs) + lane;

@@ -55,8 +55,7 @@ __global__ void __launch_bounds__(kGwThreads, 2) grainwise_persistent_kernel(con
 }
 
 // Expected lane-ops of each input tile and sample chunk (one warp per tile): its grains (sum of lambda) and
-// its pixels' Poisson set-up (two grain steps: kGwPixelCost).
-constexpr float kGwPixelCost = 800.0f;
+// its pixels' Poisson set-up.
 __global__ void grainwise_costs_kernel(const float *__restrict__ lam, int in_w, int in_h, int tin_w, int tin_h, int ntx,
                                        int ntiles, float grain_cost, float *__restrict__ cost) {
     const int tile = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
@@ -73,21 +72,15 @@ __global__ void grainwise_costs_kernel(const float *__restrict__ lam, int in_w, 
 }
 
 // The work list: tiles by descending cost (a bitonic sort in shared memory, one CTA, for up to kGwSortMax
-// tiles; larger grids keep the natural order), each cut into parts of at most `target` lane-ops, the cost
-// an item has when every CTA slot gets kGwItemsPerSlot.  Without the cut, the saturated spots of a blob
-// plane (3 % of the pixels, half of the grains) held the kernel to the end: 1024^2 -> 2048^2, N 128, the
-// heaviest tile ran 14.7 ms while the CTAs were done in 6.6 ms on average; finer cuts than two items per slot
-// repeat the items' set-up and share pixels among more lanes (3 or 4 per slot: 6.5 -> 7.2, 8.0 ms).  A part has no less
-// than kGwItemFloor lane-ops (an item's set-up, about 10 us of a CTA) and a pixel per warp.
+// tiles; larger grids keep the natural order), each cut into parts (gw_parts).
 // work[1] = items, then int2 (tile, part | parts << 16).
 constexpr int kGwSortMax = 4096;
-constexpr int kGwItemsPerSlot = 2;
-constexpr float kGwItemFloor = 2.0e6f;
 __global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__restrict__ cost, int ntiles, int slots,
                                                                int chunks, int most_parts, int *__restrict__ work) {
     __shared__ float key[kGwSortMax];
     __shared__ int idx[kGwSortMax];
     __shared__ float wsum[32];
+    __shared__ float wshare[kGwStretches][32];
     __shared__ int wcnt[33];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool sorted = ntiles <= kGwSortMax;
@@ -127,7 +120,29 @@ __global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__re
     __syncthreads();
     float total = 0.0f;
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) total += wsum[w];
-    const float target = fmaxf(kGwItemFloor, total * (float)chunks / (float)(slots * kGwItemsPerSlot));
+    float target = fmaxf(kGwItemFloor, total * (float)chunks / (float)(slots * kGwItemsPerSlot));
+    if (target > kGwItemFloor) {  // (else the items are fewer than the slots' turns)
+        float share[kGwStretches];
+#pragma unroll
+        for (int k = 0; k < kGwStretches; k++) share[k] = 0.0f;
+        for (int i = tid; i < ntiles; i += blockDim.x)
+#pragma unroll
+            for (int k = 0; k < kGwStretches; k++) share[k] += gw_slot_share(cost[i], target * gw_stretch(k), most_parts);
+#pragma unroll
+        for (int k = 0; k < kGwStretches; k++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) share[k] += __shfl_xor_sync(0xffffffffu, share[k], o);
+            if (lane == 0) wshare[k][warp] = share[k];
+        }
+        __syncthreads();
+        int fits = 0;
+        for (int k = kGwStretches - 1; k >= 0; k--) {
+            float sum_k = 0.0f;
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) sum_k += wshare[k][w];
+            if (sum_k * (float)chunks <= (float)slots) fits = k;
+        }
+        target *= gw_stretch(fits);
+    }
     int2 *items = reinterpret_cast<int2 *>(work + 2);
     int base = 0;  // items of the tiles before this round's
     for (int i0 = 0; i0 < ntiles; i0 += blockDim.x) {
@@ -136,7 +151,7 @@ __global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__re
         if (i < ntiles) {
             tile = sorted ? idx[i] : i;
             const float c = sorted ? key[i] : cost[i];
-            parts = max(1, min(most_parts, (int)fminf(ceilf(c / target), 65535.0f)));
+            parts = gw_parts(c, target, most_parts);
         }
         int incl = parts;
 #pragma unroll

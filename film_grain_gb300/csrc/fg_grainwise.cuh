@@ -178,20 +178,24 @@ __device__ __forceinline__ void gw_process(const GwTile &T, unsigned int *mask, 
     }
 }
 
-// Chunk `chunk` of the samples over part `part` of `parts` of a tile: a contiguous range of its pixels (a
-// heavy tile is split over several CTAs, each with its own copy of the tile's masks; OR makes the result
-// the same).  Each step of a warp draws one grain per lane.  In a part with enough pixels for the CTA's
-// warps a lane has a pixel of its own; in a smaller one g = 2 .. 32 lanes share a pixel: they hold the same
-// stream, draw its next g grains one after another, and each keeps one.  The draws (36 lane-ops for the
-// centre, about 90 with a log-normal radius) are then repeated in g lanes, but a pixel's grains are a serial
-// chain of whole steps, and a step's filter and pairs cost several times its draws (311x205, N 400: 4.9 -> 1.7 ms; 128x96, N 32:
+// Chunk `chunk` of the samples over part `part` of `parts` of a tile: every parts-th of its pixels (a heavy
+// tile is split over several CTAs, each with its own copy of the tile's masks; OR makes the result the same).  Taken
+// in turn, not as ranges, the parts of a tile that is bright on one side cost the same: with ranges, the CTAs of
+// 262 x 1186 blobs, radius 0.047, N 113, zoom 0.25 ran 9.7 ms, so 8.1.
+// Each step of a warp draws one grain per lane.  In a part with enough pixels for the CTA's
+// warps a lane has a pixel of its own; in a smaller one g = 2 .. 32 lanes share a pixel, until `fill` lanes have
+// one: they hold the same stream, draw its next g grains one after another, and each keeps one (128x96, N 32:
 // 0.88 -> 0.39 ms; filling the warps 1.5 or 2 times over instead of once was slower, 6.5 -> 7.0 and 8.0 ms
-// on the 1024^2 -> 2048^2 plane).
+// on the 1024^2 -> 2048^2 plane, and so was half a filling, 7.1 ms).
+// With a constant radius a grain is two draws of the stream, so each lane stands at its own grain and steps over the
+// other lanes' without forming their values: half of the repeated draws' instructions, which were a third of all
+// on saturated planes (7000 grains a pixel, one pair a grain: 123 x 1024, radius 0.025, N 64 19.4 -> 14.0 ms with the
+// above; N 128 23.0 -> 17.1, N 256 27.5 -> 23.2).  A log-normal draw has to be decided to know its length.
 // A group whose pixel is done takes the next one once half of the warp's groups wait (the Poisson set-up runs
 // for all of them at once), so that pixels of unequal lambda keep the lanes busy.
 template <bool kSmall, int MW>
 __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int tile_x, int tile_y,
-                                                    unsigned char *smem_raw, int part, int parts, int chunk) {
+                                                    unsigned char *smem_raw, int part, int parts, int chunk, int fill) {
     const int k0 = 32 * chunk * a.chunk_words;                 // the chunk's samples: [k0, k0 + n)
     const int n = min(a.n - k0, 32 * a.chunk_words);
     const int W = (n + 31) >> 5;
@@ -239,11 +243,10 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
     }
     for (int t = tid; t < region_words; t += kGwThreads) mask[t] = 0u;
     const int fw = ix1 - ix0, total = fw * (iy1 - iy0);
-    const int px_begin = (int)(((long long)total * part) / parts);
-    const int px_end = (int)(((long long)total * (part + 1)) / parts);
-    if (tid == 0) *next_px = px_begin;
+    const int px_end = (total - part + parts - 1) / parts;  // pixels part, part + parts, ... of the tile
+    if (tid == 0) *next_px = 0;
     int g = 1;  // lanes per pixel
-    while (g < 32 && g * (px_end - px_begin) < kGwThreads) g *= 2;
+    while (g < 32 && g * px_end < fill) g *= 2;
     const int sub = lane & (g - 1);
     // level 0: two buckets each
     for (int t = tid; t < kGbBuckets * S; t += kGwThreads) tabx[t] = taby[t] = 0u;
@@ -288,10 +291,13 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
             more = base + want < px_end;
             const int pi = base + __popc(idle & ((1u << (lane & ~(g - 1))) - 1u)) / g;
             if (((idle >> lane) & 1u) && pi < px_end) {
-                px = ix0 + pi % fw;
-                py = iy0 + pi / fw;
+                const int ti = part + pi * parts;
+                px = ix0 + ti % fw;
+                py = iy0 + ti / fw;
                 const float lv = a.lam[(long long)py * a.in_w + px];
                 if (lv > 0.0f) left = poisson_count(mix3(a.seed, kPixelStream, px, py), lv, rng);
+                if (!a.lognorm)  // to the lane's own grain
+                    for (int t = 0; t < 2 * sub; t++) rng.next();
             }
             continue;
         }
@@ -301,17 +307,27 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
             bool have = false;
             float ux = 0.0f, uy = 0.0f;
             RadiusDraw rd = {0ull, -1.0f};
-            for (int t = 0; t < g; t++) {
-                if (left > 0) {
-                    left--;
-                    const float vx = uniform_f32_from(U, rng.next()), vy = uniform_f32_from(U, rng.next());
-                    RadiusDraw vd = {0ull, -1.0f};
-                    if (a.lognorm) vd = lognormal_draw(a.log_mu, a.log_sigma, rng);
-                    if (t == sub) {
-                        have = true;
-                        ux = vx;
-                        uy = vy;
-                        rd = vd;
+            if (!a.lognorm) {
+                have = (uint32_t)sub < left;
+                ux = uniform_f32_from(U, rng.next());
+                uy = uniform_f32_from(U, rng.next());
+                for (int t = 1; t < g; t++) {
+                    rng.next();
+                    rng.next();
+                }
+                left = left > (uint32_t)g ? left - (uint32_t)g : 0u;
+            } else {
+                for (int t = 0; t < g; t++) {
+                    if (left > 0) {
+                        left--;
+                        const float vx = uniform_f32_from(U, rng.next()), vy = uniform_f32_from(U, rng.next());
+                        const RadiusDraw vd = lognormal_draw(a.log_mu, a.log_sigma, rng);
+                        if (t == sub) {
+                            have = true;
+                            ux = vx;
+                            uy = vy;
+                            rd = vd;
+                        }
                     }
                 }
             }
@@ -437,6 +453,34 @@ inline size_t grainwise_tile_smem_bytes(const GrainwiseArgs &a) {
 // The most CTAs a tile of `px` pixels is split over: one pixel for each warp.
 inline int grainwise_most_parts(int px) { return std::max(1, std::min(px / kGwWarps, 0x7FFF)); }
 
+// How tiles are cut into items: a tile of `cost` lane-ops into parts of at most `target` of them, the cost an item
+// has when every CTA slot gets kGwItemsPerSlot.  Without the cut, the saturated spots of a blob
+// plane (3 % of the pixels, half of the grains) held the kernel to the end: 1024^2 -> 2048^2, N 128, the
+// heaviest tile ran 14.7 ms while the CTAs were done in 6.6 ms on average; finer cuts than two items per slot
+// repeat the items' set-up and share pixels among more lanes (3 or 4 per slot: 6.5 -> 7.2, 8.0 ms).  A part has no less
+// than kGwItemFloor lane-ops (an item's set-up, about 10 us of a CTA) and a pixel per warp.
+// Rounding the parts up makes more items than the slots take in kGwItemsPerSlot turns, and where most of them cost the
+// same (a plane that is mostly saturated) the few left over take a whole turn more.  So the target is the smallest of
+// kGwStretches times that cost at which the items fit, an item taking the share of its slot that as many of its
+// size as fit into the slot leave it: 1024 x 123, radius 0.025, N 256 25.3 -> 21.5 ms, 600 x 400 of one intensity,
+// log-normal 0.03, N 256 12.2 -> 10.7.
+constexpr int kGwItemsPerSlot = 2;
+constexpr float kGwItemFloor = 2.0e6f;
+constexpr float kGwPixelCost = 800.0f;  // a pixel's Poisson set-up, in lane-ops (two grain steps)
+constexpr int kGwStretches = 8;
+__host__ __device__ inline float gw_stretch(int k) {
+    return k == 0 ? 1.0f : k == 1 ? 1.02f : k == 2 ? 1.05f : k == 3 ? 1.09f : k == 4 ? 1.14f : k == 5 ? 1.2f : k == 6 ? 1.3f : 1.45f;
+}
+__host__ __device__ inline int gw_parts(float cost, float target, int most_parts) {
+    const float p = fminf(ceilf(cost / target), (float)most_parts);
+    return p > 1.0f ? (int)p : 1;
+}
+__host__ __device__ inline float gw_slot_share(float cost, float target, int most_parts) {
+    const int parts = gw_parts(cost, target, most_parts);
+    const float fit = floorf((float)kGwItemsPerSlot * target * (float)parts / fmaxf(cost, 1.0f));
+    return (float)parts / fmaxf(fit, 1.0f);
+}
+
 // The tile variant for chunks of `words` mask words: the words a grain's candidate mask holds in registers.
 __host__ __device__ inline int grainwise_variant(int words) {
     return words <= 1 ? 1 : words <= 2 ? 2 : words <= 4 ? 4 : kGbMaxWords;
@@ -446,10 +490,11 @@ __host__ __device__ inline int grainwise_variant(int words) {
 // kVariant: grainwise_variant(a.chunk_words), or -1 to dispatch at run time (the batched kernel).
 template <bool kSmall, int kVariant = -1>
 __device__ __forceinline__ void grainwise_tile(const GrainwiseArgs &a, int tile_x, int tile_y,
-                                               unsigned char *smem_raw, int part, int parts, int chunk) {
-    if (kVariant > 0) grainwise_tile_bits<kSmall, kVariant < 0 ? 1 : kVariant>(a, tile_x, tile_y, smem_raw, part, parts, chunk);
-    else if (kSmall && a.chunk_words <= 2) grainwise_tile_bits<kSmall, 2>(a, tile_x, tile_y, smem_raw, part, parts, chunk);
-    else grainwise_tile_bits<kSmall, kGbMaxWords>(a, tile_x, tile_y, smem_raw, part, parts, chunk);
+                                               unsigned char *smem_raw, int part, int parts, int chunk,
+                                               int fill = kGwThreads) {
+    if (kVariant > 0) grainwise_tile_bits<kSmall, kVariant < 0 ? 1 : kVariant>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
+    else if (kSmall && a.chunk_words <= 2) grainwise_tile_bits<kSmall, 2>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
+    else grainwise_tile_bits<kSmall, kGbMaxWords>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
 }
 
 }  // namespace fg

@@ -142,6 +142,14 @@ __global__ void __launch_bounds__(kPwRegenThreads)
         pixelwise_regen_pixels<false>(s_pa, (int)(local % R.row_ctas) * kPwRegenThreads, (int)(local / R.row_ctas), 0, s_pa.n);
 }
 
+// A batch's grain-wise items: their number per CTA slot and the lanes that a part's pixels are spread over
+// (grainwise_tile_bits).  The images' tiles differ more than one plane's, so more items than in a single render; and
+// the items beside them keep an SM busy, so that repeating fewer draws counts for more than full warps.  A batch of
+// 19 images up to 1024^2, one of them saturated at radius 0.025, and one of 19 up to 256^2: 2 items and 512 lanes
+// 34.5 and 12.5 ms, 4 and 512 34.2 and 7.3, 6 and 384 29.7 and 7.9.
+constexpr int kBatchItemsPerSlot = 6;
+constexpr int kBatchFill = 384;
+
 // Pixel-wise items in lean CTAs (256 threads, 4 per SM); the root blocks they leave to fat CTAs are
 // appended to `deferred` for the persistent kernel.
 __global__ void __launch_bounds__(PwLean::kThreads, PwLean::kCtasPerSm)
@@ -195,8 +203,8 @@ __global__ void __launch_bounds__(512, 2) batch_persistent_kernel(const BatchIma
         __syncthreads();
         if (threadIdx.x == 0) s_image = w.image;
         if (s_img.algo == FG_ALGO_PIXEL) pixelwise_block<PwFat>(s_img.pa, w.x, w.y, smem_raw);
-        else if (s_img.small) grainwise_tile<true>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk);
-        else grainwise_tile<false>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk);
+        else if (s_img.small) grainwise_tile<true>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk, kBatchFill);
+        else grainwise_tile<false>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk, kBatchFill);
         __syncthreads();
     }
 }
@@ -371,12 +379,12 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
                     const int x1 = std::min(a.in_w, x0 + a.tin_w), y1 = std::min(a.in_h, y0 + a.tin_h);
                     if (im.h_lambda) {
                         for (int y = y0; y < y1; y++)
-                            for (int x = x0; x < x1; x++) lam_sum += im.h_lambda[(long long)y * a.in_w + x];
+                            for (int x = x0; x < x1; x++)  // (clamped: the cuts need finite costs)
+                                lam_sum += std::fmin(std::fmax(im.h_lambda[(long long)y * a.in_w + x], 0.0f), 1.0e6f);
                     } else {
                         lam_sum = 50.0 * (x1 - x0) * (y1 - y0);
                     }
-                    const int n_chunk = std::min((int)p.n_samples, 32 * a.chunk_words);
-                    const double cost = lam_sum * (60.0 + 0.3 * n_chunk) + 20.0 * (x1 - x0) * (y1 - y0);
+                    const double cost = lam_sum * a.grain_cost + (double)kGwPixelCost * (x1 - x0) * (y1 - y0);
                     const int most = grainwise_most_parts((x1 - x0) * (y1 - y0));
                     for (int c = 0; c < a.chunks; c++)
                         grain_tiles.push_back(GrainTile{cost, BatchItem{i, tx, ty, 0, c}, most});
@@ -385,19 +393,18 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
         }
     }
     if (request > 200 * 1024) return fail(set_error(FG_ERR_UNSUPPORTED, "batch tile needs too much shared memory"));
-    // Heavy grain-wise tiles are split over CTAs (part | parts << 16 in the item's last word) so that no
-    // item is far above the average share of an SM slot: a tile of cost c gets ceil(c / target) parts,
-    // at most grainwise_most_parts.
+    // Heavy grain-wise tiles are split over CTAs (part | parts << 16 in the item's word), as a single render's are
+    // (gw_parts, by the same costs), but into kBatchItemsPerSlot items a slot.
     {
         double total_cost = 0.0;
         for (const GrainTile &g : grain_tiles) total_cost += g.cost;
-        for (const CostItem &c : px_work) total_cost += c.cost;
         int dev = 0, sms = 0;
         FG_BCUDA(cudaGetDevice(&dev), "device");
         FG_BCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-        const double target = total_cost / (8.0 * std::max(1, sms) * std::max(1, tun.ctas_per_sm)) + 1.0;
+        const double slots = (double)std::max(1, sms) * std::max(1, tun.ctas_per_sm);
+        const float target = std::max(kGwItemFloor, (float)(total_cost / (slots * kBatchItemsPerSlot)));
         for (const GrainTile &g : grain_tiles) {
-            const int parts = (int)std::max(1.0, std::min((double)g.most_parts, std::ceil(g.cost / target)));
+            const int parts = gw_parts((float)g.cost, target, g.most_parts);
             for (int q = 0; q < parts; q++) {
                 BatchItem it = g.it;
                 it.part = q | (parts << 16);

@@ -430,3 +430,19 @@ def test_grainwise_saturated_strip_keeps_pace(cuda, fgl, n):
         dl = torch.from_numpy(lam).cuda()
         rate.append(_fastest(torch, lambda: fgl.render_grainwise(dl, p, d)) / float(lam.astype(np.float64).sum()))
     assert rate[1] < 1.85 * rate[0], [r * 1e12 for r in rate]
+
+
+def test_batch_not_slower_than_its_images(cuda, fgl):
+    """One launch over images whose grains cost very different amounts (radius 0.025 with one candidate pair a grain,
+    radius 0.2 with 44) takes no longer than the images one after the other (a tenth for noise)."""
+    torch = cuda
+    items, alone = [], 0.0
+    for w, h, radius in ((123, 1024, 0.025), (500, 400, 0.2), (250, 1024, 0.1)):
+        plane = workloads.blobs_plane(w, h, 3, scale=max(w, h) / 1536)
+        p, d, lam = _grain_plane(fgl, plane, radius_mean=radius, n_samples=256, seed=5)
+        dl = torch.from_numpy(lam).cuda()
+        items.append((dl, p, d, fgl.Algo.Grain, lam))
+        alone += _fastest(torch, lambda: fgl.render_grainwise(dl, p, d))
+    batch = fgl.Batch(items)
+    together = _fastest(torch, batch.run)
+    assert together < 1.1 * alone, f"{together * 1e3:.1f} ms together, {alone * 1e3:.1f} ms one by one"

@@ -9,15 +9,21 @@
 //            slot is not loaded when kRows = 3; what it holds reaches only its own rows of the result);
 //   N      : the channels of the kRows + 2 input rows around them, shifted by kx - 1 pixels (a start address).
 // The result's block (gradient row, input row) belongs to tap ky = their distance, and is dropped outside
-// 0 .. 2.  Three accumulators (kx) stay in tensor memory over the CTA's whole share of the rows; the first one
+// 0 .. 2.  Three accumulators (kx) stay in tensor memory over a segment of the CTA's rows; the first one
 // has 16 more columns, for a constant slot whose channel 0 is one: their sum of g is the bias gradient.
-// A CTA (one per SM, three roles: loader, MMA issuer, and everyone for the end) walks a contiguous range of
-// row blocks through two or four stages, then adds its result up in shared memory and onto dW and db with one atomic
-// per element (the sums over CTAs were f32 atomics before, too).
+// A CTA (one per SM, three roles: loader, MMA issuer, four warps that read the accumulators) walks a contiguous range
+// of row blocks through two or four stages.  At the end of a segment the accumulators are added, rounded to nearest, to
+// sums in shared memory, and those at the end onto dW and db with one atomic per element.
+// A segment is short because the accumulators' additions cut the sum's low bits off, so that sums of one sign fall
+// behind by half a bit per addition: over a CTA's whole share (148 additions on 256 tiles of 64^2) the gradient was
+// 2.0e-6 from 64 bits (one sign; 9.2e-7 with both), further than mma.sync's 1.6e-6 (7.7e-7); now 3.7e-7 (3.0e-7).  The
+// CTAs' shares grow with the batch, and so did mma.sync's sums, faster than a quarter of a share: hence at most four
+// segments.  The loads run on while the accumulators are read.
 //
 // Measured on 256 tiles of 64^2, 32 -> 32 channels (134 MB, 20 us at the measured copy rate): mma.sync with
-// operands staged channel by channel 267 us; this split 63 us; four stages of 64 columns 50 us; the end's sums
-// without shared-memory atomics 45 us.  What is left: the input rows, read 5/3 times, and the steps' copies.
+// operands staged channel by channel 267 us; this split 63 us; four stages of 64 columns 50 us; the sums
+// without shared-memory atomics 45 us; in four segments the same (flushed L2 51.8 us before and after; the output conv's,
+// whose gradient rows share warps, 45.7 -> 51.8).  What is left: the input rows, read 5/3 times, and the steps' copies.
 //
 // Waits are bounded as in fg_sg_tc.cu; a CTA whose wait ran out adds NaN to dW and db.
 #include <algorithm>
@@ -29,6 +35,8 @@
 namespace fg {
 
 constexpr int kWgThreads = 192;  // loader, MMA issuer, four warps that read the accumulators
+constexpr int kWgChain = 48;     // MMAs that add to an accumulator in a row, up to kWgSegments segments
+constexpr int kWgSegments = 4;
 
 template <int CG, int CX, int PX>  // channels of a gradient pixel (16 or 32) and of an input pixel in shared
 struct WgCfg {                     // memory, columns of a row tile (128, or 64 for images no wider)
@@ -40,17 +48,21 @@ struct WgCfg {                     // memory, columns of a row tile (128, or 64 
     static constexpr int kStage = (kX + (kXRows + 1) * kXRow + 1023) / 1024 * 1024;
     static constexpr int kN = kXRows * CX;
     static constexpr int kStages = PX == 64 ? 4 : 2;
-    static constexpr int kBar = kStages * kStage;
-    static constexpr int kSmem = kBar + 16 * kStages + 32;
+    // the CTA's sums: [tap * CX + ci][33] by co, a ky's 16 words further (so that the two gradient rows of a warp
+    // meet on different banks), then db
+    static constexpr int kSum = 9 * CX * 33 + 32;
+    static constexpr int kSumOff = kStages * kStage;
+    static constexpr int kBar = kSumOff + (kSum + 32) * 4;
+    static constexpr int kSmem = kBar + 16 * kStages + 48;
     static constexpr uint64_t kSwG = CG == 32 ? 4ull : 6ull, kSwX = CX == 32 ? 4ull : 6ull;
-    static constexpr int kSum = 9 * CX * 33;  // the CTA's sums: [tap * CX + ci][33] by co, then db
-    static_assert(3 * kN + 16 <= 512 && kSum * 4 + 128 <= kStage && kSmem <= 227 * 1024, "sizes");
+    static_assert(3 * kN + 16 <= 512 && kBar % 16 == 0 && kSmem <= 227 * 1024, "sizes");
 };
 
 struct WgArgs {
     float *dw, *db;
     int nb, H, W, tiles_x, cout;
     int g_px, x_px;  // pixels of the loaded boxes
+    int seg_steps;   // steps of kWgChain MMAs
 };
 
 __device__ int g_sg_wg_timeout;
@@ -64,8 +76,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     extern __shared__ __align__(1024) unsigned char wg_sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sbase = smem_u32(wg_sm);
-    const uint32_t full = sbase + C::kBar, freed = full + 8 * kStages, done = freed + 8 * kStages, tmem_slot = done + 8;
-    volatile int *s_abort = reinterpret_cast<volatile int *>(wg_sm + C::kBar + 16 * kStages + 16);
+    const uint32_t full = sbase + C::kBar, freed = full + 8 * kStages, done = freed + 8 * kStages, acc_full = done + 8,
+                   acc_free = acc_full + 8, tmem_slot = acc_free + 8;
+    volatile int *s_abort = reinterpret_cast<volatile int *>(wg_sm + C::kBar + 16 * kStages + 32);
+    float *sum = reinterpret_cast<float *>(wg_sm + C::kSumOff), *sdb = sum + C::kSum;
 
     if (tid == 0) {
         for (int i = 0; i < kStages; i++) {
@@ -73,9 +87,12 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
             mbar_init(freed + 8 * i, 1);
         }
         mbar_init(done, 1);
+        mbar_init(acc_full, 1);
+        mbar_init(acc_free, 4);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    for (int e = tid; e < C::kSum + 32; e += kWgThreads) sum[e] = 0.0f;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tmem_slot), "r"(512u)
                      : "memory");
@@ -96,12 +113,15 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(wg_sm + C::kBar + 16 * kStages + 8);
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(wg_sm + C::kBar + 16 * kStages + 24);
 
     // the CTA's steps [t0, t1): kRows rows of one column tile each, down the columns of all images
     const int per_col = (a.H + C::kRows - 1) / C::kRows;
     const long long total = (long long)a.nb * a.tiles_x * per_col;
     const long long t0 = total * blockIdx.x / gridDim.x, t1 = total * (blockIdx.x + 1) / gridDim.x;
+    const int steps = (int)(t1 - t0);
+    const int seg_steps = (steps - 1) / min(kWgSegments, (steps - 1) / a.seg_steps + 1) + 1;  // (nearly) equal segments
+    const int segs = (steps - 1) / seg_steps + 1;
     bool ok = true;
     int issued = 0;  // the loader's stages, for the wind-down
     if (warp == 0) {
@@ -133,8 +153,19 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
     } else if (warp == 1) {
         const uint64_t g0 = tc_desc(sbase, C::kGRow, 16 * CG) | (C::kSwG << 61);
         const uint64_t x0d = tc_desc(sbase + C::kX, C::kXRow, 16 * CX) | (C::kSwX << 61);
-        for (long long t = t0; t < t1; t++) {
+        int seg = 0, in_seg = 0;  // segments before this one, its steps so far
+        for (long long t = t0; t < t1; t++, in_seg++) {
             const int i = (int)(t - t0), s = i % kStages;
+            if (in_seg == seg_steps) {
+                tc_commit(acc_full);
+                ok = __all_sync(0xffffffffu, mbar_wait(acc_free, (uint32_t)(seg & 1), s_abort));
+                if (!ok) {
+                    *s_abort = 1;
+                    break;
+                }
+                seg++;
+                in_seg = 0;
+            }
             ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, (uint32_t)((i / kStages) & 1), s_abort));
             if (!ok) {
                 *s_abort = 1;
@@ -150,18 +181,82 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
                 for (int kx = 0; kx < 3; kx++) {
                     const uint32_t d = tmem + (uint32_t)(kx == 0 ? 0 : 16 + kx * C::kN);
                     tc_mma(d, gd + (uint64_t)(k * 2 * CG), xd + (uint64_t)(((16 * k + kx) * 2 * CX) >> 4),
-                           tc_idesc((uint32_t)(kx == 0 ? C::kN + 16 : C::kN), true), i > 0 || k > 0);
+                           tc_idesc((uint32_t)(kx == 0 ? C::kN + 16 : C::kN), true), in_seg > 0 || k > 0);
                 }
             }
             tc_commit(freed + 8 * s);
         }
+        if (ok) tc_commit(acc_full);
         tc_commit(done);
         __syncwarp();
+    } else {
+        // the segments' results onto the sums, a quarter of the tensor memory (gradient rows) per warp: plain f32
+        // additions to shared memory (an atomic would make of each a compare-and-swap loop), the warps at
+        // different kx, or at the bias, at a time
+        const int quad = warp & 3, m = quad * 32 + lane, gy = m / CG, co = m % CG, gy0 = quad * 32 / CG,
+                  gy1 = (quad * 32 + 31) / CG;
+        const bool mine = gy < C::kRows && co < a.cout;
+        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16);
+        for (int seg = 0; seg < segs; seg++) {
+            int stop = mbar_wait(acc_full, (uint32_t)(seg & 1), s_abort) ? 0 : 1;
+            // the four warps go on together or not at all
+            asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %0, 0;\n barrier.cta.red.or.pred q, 1, 128, p;\n"
+                         " selp.s32 %0, 1, 0, q;\n}\n"
+                         : "+r"(stop)
+                         :
+                         : "memory");
+            if (stop) {
+                *s_abort = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            // every warp reads something in the last turn; after that the next segment may overwrite
+            auto release = [&](int turn) {
+                if (turn < 3) return;
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_free);
+            };
+            for (int turn = 0; turn < 4; turn++) {
+                const int kx = (quad + turn) & 3;
+                if (gy0 < C::kRows && kx < 3) {
+                    // the input rows around the warp's gradient rows, all of them before the first is added
+                    constexpr int kXr = 128 / CG > 4 ? 4 : 3;
+                    uint32_t v[kXr][CX];
+#pragma unroll
+                    for (int x = 0; x < kXr; x++)
+                        tc_load(v[x], base + (uint32_t)((kx == 0 ? 0 : 16 + kx * C::kN) + min(gy0 + x, C::kXRows - 1) * CX));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    release(turn);
+#pragma unroll
+                    for (int x = 0; x < kXr; x++) {
+                        const int ky = gy0 + x - gy;
+                        if (mine && ky >= 0 && ky <= 2) {
+                            float *to = sum + (3 * ky + kx) * CX * 33 + 16 * ky + co;
+#pragma unroll
+                            for (int j = 0; j < CX; j++) to[33 * j] += __uint_as_float(v[x][j]);
+                        }
+                        __syncwarp();  // two gradient rows of a warp add to the same elements in different steps
+                    }
+                } else if (gy0 < C::kRows) {
+                    uint32_t b;
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n"
+                                 : "=r"(b)
+                                 : "r"(base + (uint32_t)C::kN));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    release(turn);
+                    for (int g = gy0; g <= gy1; g++) {
+                        if (mine && gy == g) sdb[co] += __uint_as_float(b);
+                        __syncwarp();
+                    }
+                } else {
+                    release(turn);  // a quarter without gradient rows
+                }
+                asm volatile("barrier.cta.sync 1, 128;\n" ::: "memory");
+            }
+        }
     }
-    // ---- the end: sums in shared memory (the stages are free), then one atomic per element
-    const bool any = t1 > t0;
-    ok = mbar_wait(done, 0, s_abort) && !*s_abort;
-    if (!ok) *s_abort = 1;
+    // ---- the end: one atomic per element
     __syncthreads();
     ok = *s_abort == 0;
     if (!ok) {
@@ -174,55 +269,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) sg_wgrad_tc_kernel(const __grid
         }
         __syncthreads();
     }
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    float *sum = reinterpret_cast<float *>(wg_sm), *sdb = sum + C::kSum;
-    for (int e = tid; e < C::kSum + 32; e += kWgThreads) sum[e] = 0.0f;
-    __syncthreads();
-    // the quarters of the tensor memory (gradient rows) in turn: f32 additions to shared memory one after the
-    // other, which an atomic would make of each a compare-and-swap loop
-    for (int turn = 0; turn < 4; turn++) {
-        const int quad = warp & 3, m = quad * 32 + lane, gy = m / CG, co = m % CG, gy0 = quad * 32 / CG,
-                  gy1 = (quad * 32 + 31) / CG;
-        if (warp >= 2 && quad == turn && gy0 < C::kRows && any && ok) {
-            const bool mine = gy < C::kRows && co < a.cout;
-            const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16);
-            for (int kx = 0; kx < 3; kx++) {
-                for (int c0 = gy0 * CX; c0 < min(C::kN, (gy1 + 3) * CX); c0 += 16) {
-                    uint32_t v[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                        "%13, %14, %15}, [%16];\n"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                          "=r"(v[15])
-                        : "r"(base + (uint32_t)((kx == 0 ? 0 : 16 + kx * C::kN) + c0)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                    const int ky = c0 / CX - gy, ci0 = c0 % CX;
-                    if (mine && ky >= 0 && ky <= 2) {
-                        float *to = sum + ((3 * ky + kx) * CX + ci0) * 33 + co;
-#pragma unroll
-                        for (int j = 0; j < 16; j++) to[33 * j] += __uint_as_float(v[j]);
-                    }
-                    __syncwarp();  // two gradient rows of a warp add to the same elements in different steps
-                }
-            }
-            uint32_t b;
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(b) : "r"(base + (uint32_t)C::kN));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            for (int g = gy0; g <= gy1; g++) {
-                if (mine && gy == g) sdb[co] += __uint_as_float(b);
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (any) {
+    {
         const float nan = __int_as_float(0x7fc00000);
         for (int e = tid; e < a.cout * 9 * CX; e += kWgThreads) {
             const int co = e / (9 * CX), r = e - co * (9 * CX);
-            atomicAdd(&a.dw[e], ok ? sum[r * 33 + co] : nan);
+            atomicAdd(&a.dw[e], ok ? sum[r * 33 + 16 * (r / (3 * CX)) + co] : nan);
         }
         if (tid < a.cout) atomicAdd(&a.db[tid], ok ? sdb[tid] : nan);
     }
@@ -240,6 +291,7 @@ static cudaError_t launch_wg_px(const void *g, int g_cstride, const void *x, int
     a.tiles_x = (a.W + PX - 1) / PX;
     a.g_px = std::min(PX, (a.W + 15) & ~15);          // whole K steps (zero past the image's edge)
     a.x_px = std::min(PX + 8, ((a.W + 15) & ~15) + 8);  // with the halo columns, in whole swizzle periods
+    a.seg_steps = kWgChain / (a.g_px / 16);
     CUtensorMap tm[2];
     for (int k = 0; k < 2; k++) {
         const cuuint64_t ch = (cuuint64_t)std::min(k ? CX : CG, k ? x_cstride : g_cstride);

@@ -347,3 +347,24 @@ def test_narrow_images_sharing_row_tiles(sg, cuda, fgl, nb, h, w):
     for s in range(0, nb, max(1, nb // 5)):
         for a, t in zip(run(1, s), together):
             assert torch.equal(a[0], t[s])
+
+
+@pytest.mark.parametrize("nb,h,w", [(256, 64, 64), (1, 720, 1280), (900, 24, 31), (3, 7, 9)])
+def test_weight_gradient_of_long_sums(sg, cuda, fgl, nb, h, w):
+    """Sums of one sign over up to a million pixels stay within 8e-7 plus 8e-7 a million pixels of 64 bits (relative
+    L2), what the mma.sync kernels reach: a tensor-core accumulator cuts bits off at each addition, half of the last
+    one on average, so a CTA may not keep adding to one for its whole share."""
+    torch = cuda
+    L, st = fgl.lib(), torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    for kind, co, ci, cg in ((sg.CONV_RESIDUAL, 32, 32, 32), (sg.CONV_INPUT, 32, 16, 32), (sg.CONV_OUTPUT, 8, 32, 16)):
+        g = torch.rand((nb, h, w, cg), generator=gen, device="cuda").to(torch.bfloat16)
+        x = torch.rand((nb, h, w, ci), generator=gen, device="cuda").to(torch.bfloat16)
+        dw, db = torch.zeros((co, 9, ci), device="cuda"), torch.zeros(co, device="cuda")
+        assert L.fg_sg_conv_wgrad(kind, g.data_ptr(), cg, x.data_ptr(), ci, dw.data_ptr(), db.data_ptr(), nb, h, w, st) == 0
+        gd = g[..., :co].double().reshape(-1, co)
+        xp = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1))
+        want = torch.stack([gd.T @ xp[:, t // 3:t // 3 + h, t % 3:t % 3 + w].reshape(-1, ci) for t in range(9)], dim=1)
+        bound = 8e-7 * (1 + nb * h * w / 1e6)
+        for got, ref in ((dw, want), (db, gd.sum(0))):
+            assert float((got.double() - ref).norm() / ref.norm()) < bound, kind

@@ -252,7 +252,8 @@ struct Layout {
 };
 
 // A pixel-wise plane's scratch: the counters and the deferred list (its header beside them, so that both
-// are cleared together), the offsets, the cell table and, last, the sparse pass's bitmask.
+// are cleared together), the offsets, the cell table and, last, the sparse pass's bitmask and the stream pass's bits
+// (without the bits, the bitmask's part has room for the sparse pass's sorted offsets too).
 struct PwScratch {
     PwPlan plan;
     size_t diag, offs, cells, mask, mask_bytes, bits, bits_bytes;
@@ -267,13 +268,21 @@ struct PwScratch {
         bits_bytes = mask_bytes ? pixelwise_stream_bytes(a, plan.nby) : 0;
         bits = l->add(bits_bytes);
     }
-    // the layout's allocation, without the bitmask where that finds no room (the plane takes the lean pass)
+    // the layout's allocation: without the bits where that finds no room (the plane takes the sparse pass), and then
+    // without the bitmask (the lean pass)
     cudaError_t alloc(DevBuf *b, const Layout &l, cudaStream_t s) {
         cudaError_t e = b->alloc(l.bytes, s);
-        if (e != cudaErrorMemoryAllocation || !mask_bytes) return e;
-        cudaGetLastError();
-        mask_bytes = bits_bytes = 0;
-        return b->alloc(mask, s);
+        if (e == cudaErrorMemoryAllocation && bits_bytes) {
+            cudaGetLastError();
+            bits_bytes = 0;
+            e = b->alloc(bits, s);
+        }
+        if (e == cudaErrorMemoryAllocation && mask_bytes) {
+            cudaGetLastError();
+            mask_bytes = 0;
+            e = b->alloc(mask, s);
+        }
+        return e;
     }
     PwBuffers at(void *base) const {
         char *c = static_cast<char *>(base);

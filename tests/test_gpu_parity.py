@@ -4,6 +4,9 @@ Every case renders the same seeded plane through the library's C-ABI (host lambd
 integrator) and through the oracle (a C restatement of src/pixelwise.rs / src/grainwise.rs), and
 requires the f32 output planes to be bit-identical (coverage counts equal, the same count * (1/N)).
 """
+import os
+import subprocess
+import sys
 import time
 
 import numpy as np
@@ -446,3 +449,44 @@ def test_batch_not_slower_than_its_images(cuda, fgl):
     batch = fgl.Batch(items)
     together = _fastest(torch, batch.run)
     assert together < 1.1 * alone, f"{together * 1e3:.1f} ms together, {alone * 1e3:.1f} ms one by one"
+
+
+# A render whose device memory comes from a pool of a given size (the driver API's struct CUmemPoolProps).
+_LIMITED_POOL = """
+import ctypes, sys
+import numpy as np, torch
+import film_grain_gb300 as fg
+from film_grain_gb300 import workloads
+
+class Props(ctypes.Structure):
+    _fields_ = [("alloc_type", ctypes.c_int), ("handle_types", ctypes.c_int), ("loc_type", ctypes.c_int),
+                ("loc_id", ctypes.c_int), ("security", ctypes.c_void_p), ("max_size", ctypes.c_size_t),
+                ("usage", ctypes.c_ushort), ("reserved", ctypes.c_ubyte * 54)]
+
+p = fg.ParamsBuilder(radius_mean=0.2, n_samples=256, seed=3).build()
+d = fg.derive_common(p, (4096, 4096))
+plane = workloads.ramp_noise(4096, 4096, 5)
+lam = torch.from_numpy(fg.lambda_plane(plane, d.inv_e_pi_r2)).cuda()
+want = fg.render_pixelwise(lam, p, d)
+assert fg.pixelwise_sparse_forms()[0] == 0 and fg.pixelwise_sparse_forms()[1] > 0
+cu = ctypes.CDLL("libcuda.so.1")
+props = Props(alloc_type=1, loc_type=1, loc_id=0, max_size=int(sys.argv[1]) << 20)
+pool = ctypes.c_void_p()
+assert cu.cuMemPoolCreate(ctypes.byref(pool), ctypes.byref(props)) == 0
+assert cu.cuDeviceSetMemPool(0, pool) == 0
+got = fg.render_pixelwise(lam, p, d)
+assert torch.equal(got, want)
+print("forms", *fg.pixelwise_sparse_forms(), "blocks", fg.pixelwise_diagnostics()[3])
+"""
+
+
+@pytest.mark.parametrize("mib,sparse", [(512, True), (288, False)])
+def test_pixelwise_with_little_memory(cuda, fgl, mib, sparse):
+    """4096^2, N 256: 256 MiB of cells, 50 of bitmask, 512 of the samples' bits.  Without room for the bits the plane
+    takes the sparse pass, without room for the bitmask the lean pass."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _LIMITED_POOL, str(mib)], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    forms = r.stdout.split()
+    assert int(forms[2]) == 0 and (int(forms[1]) > 0) == sparse and int(forms[4]) > 0, r.stdout

@@ -104,14 +104,16 @@ class HostSide {
         }
         dev_ = static_cast<int *>(d);
     }
-    // An early return waits here: the kernels and the counters' copy write the line.
+    // An early return waits here once something may be queued: the kernels and the counters' copy write the line.
+    // A refused request does not wait for what the caller has on the stream.
     ~HostSide() {
-        if (!waited_) cudaStreamSynchronize(stream_);
+        if (queued_ && !waited_) cudaStreamSynchronize(stream_);
         if (line_) HostLines::get().release(line_);
     }
     HostSide(const HostSide &) = delete;
     HostSide &operator=(const HostSide &) = delete;
     int *cancel_words() const { return dev_; }
+    void queued() { queued_ = true; }
     // where the counters' copy lands: pinned when there is a line
     unsigned long long *diag() {
         return line_ ? reinterpret_cast<unsigned long long *>(line_ + 2) : diag_;
@@ -138,7 +140,7 @@ class HostSide {
     const volatile int32_t *cancel_;
     cudaStream_t stream_;
     int *line_;
-    bool waited_ = false;
+    bool queued_ = false, waited_ = false;
     int *dev_ = nullptr;
     unsigned long long diag_[kPwDiagWords];
 };
@@ -500,6 +502,7 @@ static fg_status render_plane_sync(int algo, const float *lambda, const fg_param
     if (algo == FG_ALGO_PIXEL) {
         PwScratch scratch(p, d, h_offs, &l);
         FG_CUDA(scratch.alloc(&b, l, s), "alloc render");
+        host.queued();
         const PwBuffers w = scratch.at(b.p);
         FG_CUDA(cudaMemcpyAsync(w.offs, h_offs, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
         if ((st = planes(&d_lam, &d_out)) != FG_OK) return st;
@@ -514,6 +517,7 @@ static fg_status render_plane_sync(int algo, const float *lambda, const fg_param
         if ((st = grainwise_work_bytes(a, &work_bytes, &sms)) != FG_OK) return st;
         const size_t at_offs = l.add(off_bytes), at_work = l.add(work_bytes), at_mask = l.add(grainwise_mask_bytes(p, d));
         FG_CUDA(b.alloc(l.bytes, s), "alloc render");
+        host.queued();
         char *base = static_cast<char *>(b.p);
         FG_CUDA(cudaMemcpyAsync(base + at_offs, h_offs, off_bytes, cudaMemcpyHostToDevice, s), "offsets H2D");
         if ((st = planes(&d_lam, &d_out)) != FG_OK) return st;
@@ -659,6 +663,7 @@ FG_API fg_status fg_render_image(const float *rgb, int64_t width, int64_t height
         at_mask = l.add(mask_bytes * nplanes);
         FG_CUDA(b.alloc(l.bytes, s), "alloc render");
     }
+    host.queued();
     char *base = static_cast<char *>(b.p);
     float *d_rgb = reinterpret_cast<float *>(base + at_rgb), *d_planes = reinterpret_cast<float *>(base + at_planes);
     float *d_lam = reinterpret_cast<float *>(base + at_lam), *d_out = reinterpret_cast<float *>(base + at_out);

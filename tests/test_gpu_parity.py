@@ -490,3 +490,28 @@ def test_pixelwise_with_little_memory(cuda, fgl, mib, sparse):
     assert r.returncode == 0, r.stderr[-2000:]
     forms = r.stdout.split()
     assert int(forms[2]) == 0 and (int(forms[1]) > 0) == sparse and int(forms[4]) > 0, r.stdout
+
+
+def test_refused_request_does_not_wait(cuda, fgl):
+    """A request that is refused (too many samples for the grain-wise tile) returns while the caller's stream is still
+    busy: an image and a plane behind a kernel of about 0.4 s."""
+    torch = cuda
+    p = fgl.ParamsBuilder(radius_mean=0.1, n_samples=20000, seed=3, algo=fgl.Algo.Grain).build()
+    d = fgl.derive_common(p, (64, 48))
+    lam = torch.from_numpy(fgl.lambda_plane(fgl.normalize_plane(_blobs(64, 48))[0], d.inv_e_pi_r2)).cuda()
+    rgb = np.ascontiguousarray(workloads.blobs_rgb(64, 48, 3, scale=workloads.small_scale(64, 48)), np.float32)
+    out = np.empty((48, 64, 3), np.uint8)
+    stream = torch.cuda.Stream()
+    for plane in (True, False):
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(800_000_000)
+            done = torch.cuda.Event()
+            done.record()
+            if plane:
+                with pytest.raises(fgl.RenderError, match="too large"):
+                    fgl.render_grainwise(lam, p, d)
+            else:
+                assert fgl.lib().fg_render_image(rgb.ctypes.data, 64, 48, p.c, out.ctypes.data, None, None,
+                                                 stream.cuda_stream) != 0
+            assert not done.query()
+        torch.cuda.synchronize()

@@ -197,6 +197,7 @@ SIGNATURES = {
                                         ctypes.c_int32, ctypes.c_int32, _vp]),
     "fg_sg_conv_wgrad": (ctypes.c_int, [ctypes.c_int32, _vp, ctypes.c_int32, _vp, ctypes.c_int32, _vp, _vp,
                                         ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, _vp]),
+    "fg_sg_check": (ctypes.c_int, []),
     "fg_sg_mask_grad": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int64, _vp]),
     "fg_sg_flip_weights": (ctypes.c_int, [_vp, _vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                           _vp]),

@@ -617,15 +617,11 @@ cudaError_t launch_sg_conv_tc(int kind, const void *in, int in_cstride, const vo
 }
 
 // Whether a tensor-core conv ran out of an mbarrier wait since the last call (and clears the flag).
-int sg_conv32_tc_timeouts() {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_sg_tc_timeout, sizeof v) != cudaSuccess) {
-        cudaGetLastError();
-        return -1;
-    }
+cudaError_t sg_conv_tc_timeouts(int *v) {
     const int z = 0;
-    cudaMemcpyToSymbol(g_sg_tc_timeout, &z, sizeof z);
-    return v;
+    cudaError_t e = cudaMemcpyFromSymbol(v, g_sg_tc_timeout, sizeof *v);
+    if (e == cudaSuccess && *v) e = cudaMemcpyToSymbol(g_sg_tc_timeout, &z, sizeof z);
+    return e;
 }
 
 }  // namespace fg

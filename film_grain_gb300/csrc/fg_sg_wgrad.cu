@@ -344,4 +344,12 @@ cudaError_t launch_sg_wgrad_tc(int kind, const void *g, int g_cstride, const voi
     }
 }
 
+// As sg_conv_tc_timeouts, for the weight gradients.
+cudaError_t sg_wgrad_tc_timeouts(int *v) {
+    const int z = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(v, g_sg_wg_timeout, sizeof *v);
+    if (e == cudaSuccess && *v) e = cudaMemcpyToSymbol(g_sg_wg_timeout, &z, sizeof z);
+    return e;
+}
+
 }  // namespace fg

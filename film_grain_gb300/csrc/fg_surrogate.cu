@@ -475,6 +475,9 @@ cudaError_t launch_sg_conv_tc(int kind, const void *in, int in_cstride, const vo
 cudaError_t launch_sg_wgrad_tc(int kind, const void *g, int g_cstride, const void *x, int x_cstride, float *dw, float *db,
                                int nb, int H, int W, cudaStream_t s);
 
+cudaError_t sg_conv_tc_timeouts(int *v);
+cudaError_t sg_wgrad_tc_timeouts(int *v);
+
 static fg_status launch_conv(int32_t kind, const SgConvArgs &a, int nb, cudaStream_t s) {
     const long long blocks = (long long)nb * a.tiles_per_img;
     if (blocks > 0x7FFFFFFFll) return set_error(FG_ERR_UNSUPPORTED, "surrogate batch too large");
@@ -586,6 +589,17 @@ FG_API fg_status fg_sg_conv_wgrad(int32_t kind, const void *gout, int32_t g_cstr
     }
     e = cudaGetLastError();
     return e == cudaSuccess ? FG_OK : cuda_error(e, "surrogate wgrad launch");
+}
+
+FG_API fg_status fg_sg_check(void) {
+    int conv = 0, wgrad = 0;
+    cudaError_t e = sg_conv_tc_timeouts(&conv);
+    if (e == cudaSuccess) e = sg_wgrad_tc_timeouts(&wgrad);
+    if (e != cudaSuccess) return cuda_error(e, "surrogate check");
+    if (conv || wgrad)
+        return set_error(FG_ERR_INTERNAL, std::string("surrogate: a ") + (conv ? "conv" : "weight gradient") +
+                                              " gave up waiting for its copies; its outputs are NaN");
+    return FG_OK;
 }
 
 FG_API fg_status fg_sg_mask_grad(const void *dh, const void *relu, void *g, int64_t n, void *stream) {

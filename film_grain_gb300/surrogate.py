@@ -453,7 +453,9 @@ def train(net: SurrogateNet, u, radius, target, steps: int, batch: int = 256, lr
             else:
                 history.append((s + 1, float(loss.item()) / tb.numel()))
                 log(f"step {s + 1}: mse {history[-1][1]:.3e}")
+            _raise(lib().fg_sg_check())
         if checkpoint and checkpoint_every and (s + 1) % checkpoint_every == 0:
+            _raise(lib().fg_sg_check())
             net.save(checkpoint)
     return history
 

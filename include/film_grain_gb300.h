@@ -300,6 +300,9 @@ FG_API fg_status fg_sg_conv_dgrad(int32_t kind, const void *g, int32_t g_cstride
  * bias, channel stride g_cstride), x the conv input (channel stride x_cstride). */
 FG_API fg_status fg_sg_conv_wgrad(int32_t kind, const void *gout, int32_t g_cstride, const void *x, int32_t x_cstride,
                                   float *dw, float *db, int32_t nb, int32_t height, int32_t width, void *stream);
+/* FG_ERR_INTERNAL when a tensor-core kernel of the surrogate that has finished gave up a wait (each is bounded at
+ * about a second) since the last call: it wrote NaN.  Synchronises; for the places that read a result anyway. */
+FG_API fg_status fg_sg_check(void);
 /* g[i] = relu[i] > 0 ? dh[i] : 0 over n bf16 elements. */
 FG_API fg_status fg_sg_mask_grad(const void *dh, const void *relu, void *g, int64_t n, void *stream);
 /* wt[ci][8 - tap][co] = w[co][tap][ci] (zero in the padding), the weights of the data-gradient conv. */

@@ -191,6 +191,7 @@ extern "C" {
                             stream: *mut c_void) -> i32;
     pub fn fg_sg_conv_wgrad(kind: i32, gout: *const c_void, g_cstride: i32, x: *const c_void, x_cstride: i32,
                             dw: *mut f32, db: *mut f32, nb: i32, height: i32, width: i32, stream: *mut c_void) -> i32;
+    pub fn fg_sg_check() -> i32;
     pub fn fg_sg_mask_grad(dh: *const c_void, relu: *const c_void, g: *mut c_void, n: i64, stream: *mut c_void) -> i32;
     pub fn fg_sg_flip_weights(w: *const c_void, wt: *mut c_void, cout: i32, cin: i32, cout_pad: i32, cin_pad: i32,
                               stream: *mut c_void) -> i32;

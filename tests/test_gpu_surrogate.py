@@ -368,3 +368,24 @@ def test_weight_gradient_of_long_sums(sg, cuda, fgl, nb, h, w):
         bound = 8e-7 * (1 + nb * h * w / 1e6)
         for got, ref in ((dw, want), (db, gd.sum(0))):
             assert float((got.double() - ref).norm() / ref.norm()) < bound, kind
+
+
+def test_a_wait_given_up_ends_training(sg, cuda, fgl, monkeypatch, tmp_path):
+    """The flag that a kernel sets when a wait runs out is clear after a pass, and training raises where it reads a
+    result (and writes no checkpoint) when the library reports it."""
+    torch = cuda
+    net = _random_net(sg, torch, n_res=1)
+    u, r, t = _inputs(torch, 2, 16, 32)
+    sg.train(net, u, r, t, steps=1, batch=2, log_every=1, log=lambda s: None)
+    assert fgl.lib().fg_sg_check() == 0
+
+    class Reporting:
+        def __getattr__(self, name):
+            return (lambda: 7) if name == "fg_sg_check" else getattr(fgl.lib(), name)  # FG_ERR_INTERNAL
+
+    monkeypatch.setattr(sg, "lib", Reporting)
+    path = tmp_path / "ck.npz"
+    for kw in (dict(log_every=1), dict(checkpoint=str(path), checkpoint_every=1)):
+        with pytest.raises(fgl.RenderError):
+            sg.train(net, u, r, t, steps=net.step + 1, batch=2, log=lambda s: None, **kw)
+    assert not path.exists()

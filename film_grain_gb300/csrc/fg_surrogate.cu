@@ -488,7 +488,7 @@ static fg_status launch_conv(int32_t kind, const SgConvArgs &a, int nb, cudaStre
     const void *res = kind == FG_SG_CONV_RESIDUAL || kind == FG_SG_CONV_DGRAD_RESIDUAL ? a.res : nullptr;
     cudaError_t e = launch_sg_conv_tc(kind, a.in, a.in_cstride, a.w, a.bias, res, a.res_f32, nullptr, a.out, aux, a.out_f32,
                                       nb, a.H, a.W, s);
-    if (e == cudaErrorNotSupported) {  // e.g. an input that is its own output's buffer, or a residual of another tensor
+    if (e == cudaErrorNotSupported) {  // e.g. a misaligned output, or a residual of another tensor
         cudaGetLastError();
         switch (kind) {
         case FG_SG_CONV_INPUT: e = launch_conv_t<16, 32, kSgRelu>(a, total, s); break;
@@ -522,6 +522,9 @@ FG_API fg_status fg_sg_conv_forward(int32_t kind, const void *in, int32_t in_cst
         ((kind == FG_SG_CONV_INPUT || kind == FG_SG_CONV_RESIDUAL) && !bias) ||
         ((kind == FG_SG_CONV_RESIDUAL || kind == FG_SG_CONV_DGRAD_RESIDUAL) && !res))
         return set_error(FG_ERR_INVALID, "surrogate conv: missing buffer");
+    // (a pixel is read by the CTAs of its neighbours, which may not have started when it is written)
+    if (!f32_out && (in == out || (kind == FG_SG_CONV_RESIDUAL && in == aux)))
+        return set_error(FG_ERR_INVALID, "surrogate conv: the input cannot be an output");
     const int need_c = (kind == FG_SG_CONV_INPUT || kind == FG_SG_CONV_DGRAD_OUTPUT) ? 16 : 32;
     if (in_cstride < need_c) return set_error(FG_ERR_INVALID, "surrogate conv: input channel stride too small");
     const SgConvArgs a = conv_args(in, w, bias, res, res_f32, out, aux, out_f32, height, width, in_cstride);

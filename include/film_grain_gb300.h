@@ -283,7 +283,7 @@ typedef struct fg_sg_net {
 } fg_sg_net;
 
 /* One 3x3 conv over nb images of height x width (kind above; in_cstride = input channel stride, a
- * multiple of 8 and at least the kind's input channels; in and w 16-byte aligned). */
+ * multiple of 8 and at least the kind's input channels; in and w 16-byte aligned; in is neither out nor aux). */
 FG_API fg_status fg_sg_conv_forward(int32_t kind, const void *in, int32_t in_cstride, const void *w, const float *bias,
                                     const void *res, const float *res_f32, void *out, void *aux, float *out_f32,
                                     int32_t nb, int32_t height, int32_t width, void *stream);

@@ -1,5 +1,6 @@
 """CPU tests of the library's host side: the C-ABI exports, parameter resolution and the host
 arithmetic, each against the oracle (no GPU calls)."""
+import ctypes
 import os
 import re
 
@@ -194,3 +195,13 @@ def test_render_requires_gpu_and_fails_loudly(fgl):
     d = fgl.derive_common(p, (8, 8))
     with pytest.raises(fgl.GpuError):
         fgl.render_pixelwise(np.ones((8, 8), np.float32), p, d)
+
+
+def test_surrogate_conv_refuses_its_input_as_output(fgl):
+    """A 3x3 conv onto its own input races with the neighbouring tiles' reads, so it is refused, before any device
+    call (the addresses are never followed); the data gradient's residual may be its output."""
+    L = fgl.lib()
+    a, b, c, w = (ctypes.c_void_p(0x10000 * k) for k in (1, 2, 3, 4))
+    for kind, out, aux in ((0, a, None), (1, a, None), (1, b, a), (3, a, None), (4, a, None)):
+        assert L.fg_sg_conv_forward(kind, a, 32, w, w, c, None, out, aux, None, 1, 8, 8, None) == 4  # FG_ERR_INVALID
+        assert b"cannot be an output" in L.fg_last_error_message()

@@ -10,6 +10,7 @@ render of the same plane is bit-identical to an uncancelled one.  No GPU fault i
 kernels read a flag and return.
 """
 import ctypes
+import threading
 import time
 
 import numpy as np
@@ -112,3 +113,62 @@ def test_looking_at_the_flag_costs_little(cuda, fgl, size, radius):
 
     without, clear = best(None), best(ctypes.addressof(flag))
     assert clear < 1.5 * without + 100e-6, f"{without * 1e6:.0f} us without a flag, {clear * 1e6:.0f} us with one"
+
+
+@pytest.mark.parametrize("kernels,kw", [
+    (6, dict(radius_mean=0.5, n_samples=256)),  # the sparse pass and the fat pass over what it leaves
+    (4, dict(radius_mean=0.2, n_samples=300)),  # the lean pass
+])
+def test_cancel_stops_the_block_passes(cuda, fgl, kernels, kw):
+    """As above, on the block passes, at the first plane size that takes 0.12 s."""
+    torch = cuda
+    p = fgl.ParamsBuilder(seed=9, algo=fgl.Algo.Pixel, **kw).build()
+    for size in (2048, 4096, 8192, 12288):
+        d = fgl.derive_common(p, (size, size))
+        lam = torch.from_numpy(fgl.lambda_plane(workloads.ramp_noise(size, size, 3), d.inv_e_pi_r2)).cuda()
+        fgl.render_pixelwise(lam, p, d)
+        t0 = time.perf_counter()
+        want = fgl.render_pixelwise(lam, p, d)
+        full = time.perf_counter() - t0
+        if full > 0.12:
+            break
+    assert fgl.pixelwise_kernel_count(p, d) == kernels
+    assert fgl.pixelwise_sparse_forms()[1] == 0 and (fgl.pixelwise_sparse_forms()[0] > 0) == (kernels == 6)
+    start = time.perf_counter()
+    with pytest.raises(fgl.CancelledError) as err:
+        fgl.render_pixelwise(lam, p, d, cancel=lambda: time.perf_counter() - start > 0.25 * full)
+    assert "inside a kernel" in str(err.value)
+    assert time.perf_counter() - start < 0.75 * full
+    assert torch.equal(fgl.render_pixelwise(lam, p, d), want)
+
+
+def test_cancel_stops_short_items(cuda, fgl):
+    """The stream pass without tiles and the pass over its dense segments, whose warps look at the flag by the clock:
+    a flag set a third of the way into a render of some milliseconds."""
+    torch = cuda
+    L = fgl.lib()
+    p = fgl.ParamsBuilder(radius_mean=0.1, n_samples=256, seed=9).build()
+    d = fgl.derive_common(p, (850, 850))
+    lam = torch.from_numpy(fgl.lambda_plane(workloads.ramp_noise(850, 850, 3), d.inv_e_pi_r2)).cuda()
+    out = torch.empty((d.output_height, d.output_width), device="cuda")
+    offs = np.ascontiguousarray(d.offsets_input, np.float32)
+    flag = ctypes.c_int32(0)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call():
+        return L.fg_render_pixelwise(lam.data_ptr(), p.c, d._c, offs.ctypes.data, out.data_ptr(),
+                                     ctypes.addressof(flag), stream)
+
+    assert call() == 0
+    t0 = time.perf_counter()
+    assert call() == 0
+    full = time.perf_counter() - t0
+    assert full > 1.5e-3 and fgl.pixelwise_sparse_forms()[1] > 0
+    want = out.clone()
+    setter = threading.Timer(full / 3, lambda: setattr(flag, "value", 1))
+    setter.start()
+    assert call() == 2  # FG_ERR_CANCELLED
+    setter.join()
+    assert b"inside a kernel" in L.fg_last_error_message()
+    flag.value = 0
+    assert call() == 0 and torch.equal(out, want)

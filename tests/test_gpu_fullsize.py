@@ -69,3 +69,35 @@ def test_pixelwise_large_frame_4096(cuda, fgl, orc):
         got = out[y0:y0 + 24, x0:x0 + 24]
         diff = np.count_nonzero(got.view(np.uint32) != want.view(np.uint32))
         assert diff == 0, f"tile ({x0},{y0}): {diff} pixels differ"
+
+
+@pytest.mark.parametrize("w,h,side,kw", [
+    (2000, 1900, 32, dict(radius=0.5, n=16)),
+    (2900, 2800, 64, dict(radius=0.5, n=16)),
+    (1500, 1490, 32, dict(radius=0.3, n=64, zoom=2.0)),  # reach above 0.44 of an output pixel
+    (1500, 1490, 32, dict(radius=0.4, n=128)),           # 64 hits a grain
+    (2900, 2800, 32, dict(radius=0.45, dist="lognorm", sd=0.1, n=33)),
+    (700, 650, 16, dict(radius=0.5, n=200)),
+])
+def test_sparse_pass_with_larger_blocks(cuda, fgl, orc, w, h, side, kw):
+    """The sparse pass over blocks of 32 and 64 pixels, which it takes on planes that still give every CTA slot
+    several, the blocks that it splits, and the fat pass over what it leaves; on tiles at the corners, across block
+    edges and at the brightest pixel.  Sparse, not stream; an almost empty plane, where no block is split, tells the
+    blocks' size by their number."""
+    torch = cuda
+    dark = np.full((h, w), 0.01, np.float32)
+    p, d, lam, op, od, offs, offs_in = _plane_setup(fgl, orc, dark, seed=8, **kw)
+    fgl.render_pixelwise(torch.from_numpy(fgl.lambda_plane(dark, d.inv_e_pi_r2)).cuda(), p, d)
+    grid = (w / side + 3) * (h / side + 3)
+    assert 0.5 * grid < fgl.pixelwise_sparse_forms()[0] < 1.2 * grid
+    p, d, lam, op, od, offs, offs_in = _plane_setup(fgl, orc, workloads.blobs_plane(w, h, 4), seed=8, **kw)
+    out = fgl.render_pixelwise(torch.from_numpy(lam).cuda(), p, d).cpu().numpy()
+    sparse, stream = fgl.pixelwise_sparse_forms()
+    assert stream == 0 and sparse > 0
+    zoom = kw.get("zoom", 1.0)
+    iy, ix = np.unravel_index(int(np.argmax(lam)), lam.shape)
+    oh, ow = out.shape
+    for x0, y0 in ((0, 0), (ow - 20, oh - 20), (int(640 * zoom) - 10, int(576 * zoom) - 10),
+                   (min(int(ix * zoom), ow - 20), min(int(iy * zoom), oh - 20))):
+        want, _ = orc.render("pixel", lam, op, od, offs_in, rect=(x0, y0, x0 + 20, y0 + 20))
+        assert np.array_equal(out[y0:y0 + 20, x0:x0 + 20].view(np.uint32), want.view(np.uint32)), (x0, y0)

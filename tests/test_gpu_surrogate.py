@@ -389,3 +389,66 @@ def test_a_wait_given_up_ends_training(sg, cuda, fgl, monkeypatch, tmp_path):
         with pytest.raises(fgl.RenderError):
             sg.train(net, u, r, t, steps=net.step + 1, batch=2, log=lambda s: None, **kw)
     assert not path.exists()
+
+
+def _misaligned(torch, shape, skip, fill=None):
+    """A bf16 tensor of `shape` that starts `skip` elements behind a 16-byte boundary."""
+    n = int(np.prod(shape))
+    buf = torch.zeros(n + skip, dtype=torch.bfloat16, device="cuda")
+    view = buf[skip:].view(shape)
+    assert view.data_ptr() % 16
+    if fill is not None:
+        view.copy_(fill)
+    return view
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 9, 33), (3, 17, 70)])
+def test_mma_sync_kernels_match_oracle(sg, cuda, fgl, shape):
+    """The kernels that take what the tensor-core ones refuse: outputs off a 16-byte boundary, a residual of another
+    tensor, gradients off a boundary or of an odd channel stride; and the two passes that the backward pass ran beside
+    them.  Bounds as for the tensor-core kernels."""
+    torch = cuda
+    nb, h, w = shape
+    x, wt, b, res = _conv_inputs(torch, nb, h, w, 21)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda().to(torch.bfloat16)
+    X, X16, Wt, R, B = dev(x), dev(x[..., :16]), dev(wt), dev(res), torch.from_numpy(b).cuda()
+    L, st = fgl.lib(), torch.cuda.current_stream().cuda_stream
+    close = lambda got, want: np.all(np.abs(got.float().cpu().numpy() - want) <= 2.0**-7 * np.abs(want) + 2e-5)
+    ptr = lambda t: None if t is None else t.data_ptr()
+    call = lambda kind, i, c, wgt, r, o, a: L.fg_sg_conv_forward(kind, ptr(i), c, ptr(wgt), ptr(B), ptr(r), None, ptr(o),
+                                                                  ptr(a), None, nb, h, w, st)
+    z, relu = sr.conv(x, wt), np.maximum(sr.conv(x, wt) + b, 0)
+    z16 = sr.conv(x[..., :16], wt[:, :, :16])
+    out, aux = _misaligned(torch, X.shape, 2), _misaligned(torch, X.shape, 2)
+    assert call(sg.CONV_RESIDUAL, X, 32, Wt, X, out, aux) == 0 and close(out, x + relu) and close(aux, relu)
+    assert call(sg.CONV_DGRAD_RESIDUAL, X, 32, Wt, R, out, None) == 0 and close(out, res + z)
+    W16 = Wt[:, :, :16].contiguous()
+    assert call(sg.CONV_INPUT, X16, 16, W16, None, out, None) == 0 and close(out, np.maximum(z16 + b, 0))
+    assert call(sg.CONV_DGRAD_OUTPUT, X16, 16, W16, None, out, None) == 0 and close(out, z16)
+    whole, aux = torch.empty_like(X), torch.empty_like(X)
+    assert call(sg.CONV_RESIDUAL, X, 32, Wt, R, whole, aux) == 0 and close(whole, res + relu) and close(aux, relu)
+
+    g = sr.bf16_round(np.random.default_rng(22).normal(0, 1, (nb, h, w, 32)).astype(np.float32))
+    bound = nb * h * w * 2.0**-23
+    for skip, cs in ((4, 32), (0, 36)):
+        G = torch.zeros(nb * h * w * cs + skip, dtype=torch.bfloat16, device="cuda")
+        gv = G[skip:].view(nb, h, w, cs)
+        gv[..., :32].copy_(dev(g))
+        for kind, xin, co, ci in ((sg.CONV_RESIDUAL, X, 32, 32), (sg.CONV_INPUT, X16, 32, 16), (sg.CONV_OUTPUT, X, 8, 32)):
+            dw, db = torch.zeros((co, 9, ci), device="cuda"), torch.zeros(co, device="cuda")
+            assert L.fg_sg_conv_wgrad(kind, gv.data_ptr(), cs, xin.data_ptr(), ci, dw.data_ptr(), db.data_ptr(), nb, h, w,
+                                      st) == 0
+            gn, xn = g[..., :co].astype(np.float64), xin.float().cpu().numpy().astype(np.float64)
+            assert np.all(np.abs(dw.cpu().numpy() - sr.conv_wgrad(gn, xn)) <= bound * sr.conv_wgrad(np.abs(gn), np.abs(xn)))
+            flat = gn.reshape(-1, co)
+            assert np.all(np.abs(db.cpu().numpy() - flat.sum(0)) <= bound * np.abs(flat).sum(0))
+
+    masked = torch.empty_like(X)
+    assert L.fg_sg_mask_grad(R.data_ptr(), X.data_ptr(), masked.data_ptr(), X.numel(), st) == 0
+    assert torch.equal(masked, torch.where(X > 0, R, torch.zeros_like(R)))
+    flipped = torch.empty((32, 9, 16), dtype=torch.bfloat16, device="cuda")
+    W8 = Wt[:8].contiguous()
+    assert L.fg_sg_flip_weights(W8.data_ptr(), flipped.data_ptr(), 8, 32, 16, 32, st) == 0
+    want = torch.zeros_like(flipped)
+    want[:, :, :8] = W8.flip(1).permute(2, 1, 0)
+    assert torch.equal(flipped, want)

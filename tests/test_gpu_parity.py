@@ -515,3 +515,15 @@ def test_refused_request_does_not_wait(cuda, fgl):
                                                  stream.cuda_stream) != 0
             assert not done.query()
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("w,h,zoom,radius,n", [
+    (61, 9, 1.0, 0.02, 33),    # a saturated ramp end: parts of a few pixels, 2 to 32 lanes to a pixel
+    (97, 3, 2.0, 0.015, 20),   # parts that do not divide the tile
+    (40, 1, 1.0, 0.01, 5),     # 32 lanes to a pixel of many thousand grains
+    (130, 95, 0.5, 0.03, 64),  # one tile, groups of 1 and 2
+])
+def test_grainwise_parts_and_skipped_draws(cuda, fgl, orc, w, h, zoom, radius, n):
+    """Constant radius: the lanes of a pixel stand at their own grains of its stream, in parts that take the tile's
+    pixels in turn."""
+    _check("grain", fgl, orc, workloads.ramp_noise(w, h, 5), radius=radius, n=n, zoom=zoom, seed=17)

@@ -723,7 +723,7 @@ FG_API void fg_pixelwise_diagnostics(unsigned long long out[4]) {
     for (int i = 0; i < 4; i++) out[i] = g_pw_diag[i];
 }
 
-// The sparse pass's blocks of that render by the form of their sample step: sample-major, grain-major.
+// That render's blocks of the sparse pass, and tiles (or parts of chunks) of the stream pass.
 FG_API void fg_pixelwise_sparse_forms(unsigned long long out[2]) {
     out[0] = g_pw_diag[4];
     out[1] = g_pw_diag[5];

@@ -2,22 +2,23 @@
 //
 // The reference walks input pixels, draws Poisson(lambda) grains from each pixel's stream, and for
 // every grain and offset k ORs bit k into the 64-bit sample masks of the output pixels whose centres
-// fall in the offset disk (AtomicU64::fetch_or), then popcounts the masks.  Here one CTA owns an
-// output tile and keeps its N-bit masks in shared memory (ceil(N/32) words per pixel).  It
-// regenerates the grains of every input pixel whose offset disks can reach the tile (pixel streams
-// are deterministic, so tiles never exchange grains), rasterises them with the reference's exact
-// bounds() and centre test, and finishes with the popcount * (1/N) epilogue -- optionally fused
-// with the luma colour recombination and u8 packing.
+// fall in the offset disk (AtomicU64::fetch_or), then popcounts the masks.  Here a work item is a tile of
+// input pixels, or a part of one, and a chunk of the samples; its CTA keeps the sample masks (ceil(N/32) words per
+// pixel) of the output rectangle that the tile maps to in shared memory, draws the tile's grains, rasterises them
+// with the reference's exact bounds() and centre test, and ORs the masks into the plane's; bits that fall outside
+// the rectangle go to the plane's masks at once (so tiles never exchange grains).  The popcount * (1/N) epilogue is
+// optionally fused with the luma colour recombination and u8 packing.
 //
 // Work organisation:
-//   - each warp takes 32 footprint pixels at a time (one per lane, Poisson set-up in step) and draws
-//     their grains one per lane per step;
+//   - persistent CTAs pull the items, heaviest tiles first (grainwise_order_kernel);
+//   - the lanes of a warp take one grain each a step, of a pixel of their own or of one that a group of lanes shares
+//     (fg_grainwise.cuh);
 //   - an offset can put a pixel centre inside a grain's disk only if frac(czx + offx) lies within
 //     radius_out of 1/2 (and likewise for y).  Each lane turns both tests, widened by a rounding margin
 //     and rounded out to 1/128 buckets, into a bitmask over the sample index (two lookups per axis in
-//     per-tile sparse OR tables), ANDs them, and the set bits -- about 1.2x the true candidates -- are
-//     dealt over the warp's lanes for stage B: the reference's exact bounds() and centre tests on one
-//     pair per lane.  Above 256 samples a work item takes one chunk of them (fg_grainwise.cuh);
+//     per-tile sparse OR tables), ANDs them, and the set bits -- about 1.2x the true candidates -- go to the
+//     warp's queue, from which 32 pairs at a time get stage B: the reference's exact bounds() and centre tests,
+//     one pair per lane.  Above 256 samples a work item takes one chunk of them;
 //   - the lognormal radius is evaluated with the double-float exp (exp_f64_to_f32).
 // Bits are set with shared-memory atomicOr; OR is idempotent and commutative, so the result does not
 // depend on the order.

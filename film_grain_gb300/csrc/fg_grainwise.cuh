@@ -469,7 +469,14 @@ constexpr float kGwItemFloor = 2.0e6f;
 constexpr float kGwPixelCost = 800.0f;  // a pixel's Poisson set-up, in lane-ops (two grain steps)
 constexpr int kGwStretches = 8;
 __host__ __device__ inline float gw_stretch(int k) {
-    return k == 0 ? 1.0f : k == 1 ? 1.02f : k == 2 ? 1.05f : k == 3 ? 1.09f : k == 4 ? 1.14f : k == 5 ? 1.2f : k == 6 ? 1.3f : 1.45f;
+    return k == 0   ? 1.0f
+           : k == 1 ? 1.02f
+           : k == 2 ? 1.05f
+           : k == 3 ? 1.09f
+           : k == 4 ? 1.14f
+           : k == 5 ? 1.2f
+           : k == 6 ? 1.3f
+                    : 1.45f;
 }
 __host__ __device__ inline int gw_parts(float cost, float target, int most_parts) {
     const float p = fminf(ceilf(cost / target), (float)most_parts);
@@ -492,8 +499,10 @@ template <bool kSmall, int kVariant = -1>
 __device__ __forceinline__ void grainwise_tile(const GrainwiseArgs &a, int tile_x, int tile_y,
                                                unsigned char *smem_raw, int part, int parts, int chunk,
                                                int fill = kGwThreads) {
-    if (kVariant > 0) grainwise_tile_bits<kSmall, kVariant < 0 ? 1 : kVariant>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
-    else if (kSmall && a.chunk_words <= 2) grainwise_tile_bits<kSmall, 2>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
+    if (kVariant > 0)
+        grainwise_tile_bits<kSmall, kVariant < 0 ? 1 : kVariant>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
+    else if (kSmall && a.chunk_words <= 2)
+        grainwise_tile_bits<kSmall, 2>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
     else grainwise_tile_bits<kSmall, kGbMaxWords>(a, tile_x, tile_y, smem_raw, part, parts, chunk, fill);
 }
 

@@ -104,7 +104,7 @@ struct PixelwiseArgs {
     const CellParam *cells;     // in_w x in_h
     const float2 *offs;         // offsets_input [n]
     float *out;                 // out_w x out_h, accumulates hit counts (pre-zeroed)
-    unsigned long long *diag;   // [4] counters: regenerated samples, unstaged blocks, subdivisions, blocks
+    unsigned long long *diag;   // [kPwDiagWords] counters
     int in_w, in_h, out_w, out_h;
     int n;
     float rm, delta, inv_zoom, zoom;

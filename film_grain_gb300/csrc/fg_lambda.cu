@@ -45,7 +45,8 @@ __device__ __forceinline__ float div_like_host(float v, float den, uint32_t host
 
 // log(x) rounded to f32 as f32(log((double)x)) is, for 1e-6 <= x <= 1, on the f32 pipe.  (The f64 pipe, 1/32 of the
 // f32 one's rate, bound the prelude: 127 us for 2 million pixels.)  After Tang (ACM TOMS 16, 1990): x = 2^e m with
-// m in [0.7, 1.4), 128 intervals of m, each with a c near its middle (1 next to 1) whose 1/c has 10 bits;
+// m in [0.7, 1.4) (m and e by subtracting the bits of 0.7 and masking the exponent, as logf of ARM's Optimized Routines
+// does), 128 intervals of m, each with a c near its middle (1 next to 1) whose 1/c has 10 bits;
 // m / c = 1 + r exactly as a pair of floats, and log x = e log 2 + log c + log1p(r), summed as pairs.  The pair is
 // within 2^-36 of log x relatively, and where that leaves the rounding open (one x in 2^11) f64 decides.
 struct LogInterval {

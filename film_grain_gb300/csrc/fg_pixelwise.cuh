@@ -158,8 +158,9 @@ struct RegenQueue {
 
 // Hit count of output pixel (x, y) over its samples [k0, k1) by the reference's per-sample loop
 // (src/pixelwise.rs:30-38 around evaluate_indicator, src/pixelwise.rs:47-106), and when `bits` is given (the
-// pixel's words; the samples then lie in one word) the hits' bits.  Called by all 32 lanes of a warp (neighbouring pixels; `valid` false for
-// lanes past the row's end, which take part without samples); the lanes take the samples in step:
+// pixel's words; the samples then lie in one word) the hits' bits.  Called by all 32 lanes of a warp (neighbouring
+// pixels; `valid` false for lanes past the row's end, which take part without samples); the lanes take the samples in
+// step:
 //   1. every cell of a sample's range gets the emptiness screen alone (first_draw_maybe): the same short work
 //      on every lane, one column hash per column; the cells that may hold grains go to a 64-bit mask, cell
 //      (i0 + di, j0 + dj) at bit di * 8 + dj with the middle cell swapped into bit 0.  The rows of a sample
@@ -214,9 +215,9 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
             queued -= count;
         };
         // Turn by turn: first each of the 32 samples' middle 3 x 3 cells (without kTwoStep all its cells), a sample of
-        // every lane a turn, then (with wider ranges) the outer cells of the samples not covered by then, 32 of any lane and sample a turn.  A
-        // turn's cells that may hold grains go into the queue, rank by rank.  One place for each step: the code of
-        // a regenerated cell is what the instruction cache holds.
+        // every lane a turn, then (with wider ranges) the outer cells of the samples not covered by then, 32 of any
+        // lane and sample a turn.  A turn's cells that may hold grains go into the queue, rank by rank.  One place for
+        // each step: the code of a regenerated cell is what the instruction cache holds.
         bool wide = false;
         int turn = 0, scanned = 0, phead = 0, pairs = 0;
         for (;;) {
@@ -233,7 +234,8 @@ __device__ __forceinline__ uint32_t pixelwise_pixel_queue(const PixelwiseArgs &a
                     const bool due = valid && !((Q.hit[scanned] >> lane) & 1u);
                     const unsigned d = __ballot_sync(0xffffffffu, due);
                     if (due)
-                        Q.pair[(phead + pairs + __popc(d & ((1u << lane) - 1u))) & 63] = (unsigned short)(lane | (scanned << 5));
+                        Q.pair[(phead + pairs + __popc(d & ((1u << lane) - 1u))) & 63] =
+                            (unsigned short)(lane | (scanned << 5));
                     pairs += __popc(d);
                 }
                 if (pairs == 0 && queued == 0) break;

@@ -15,10 +15,10 @@
 // Segments of 32 output pixels that hold many grains are left to the per-sample kernel (stream_classify).
 //
 // What bounds it: the instructions of the grains' draws (seed words, Poisson and position draws, the
-// log-normal radius) and of their candidates: 70 ps a grain on the log-normal plane below.  It replaced a form of the sparse pass that staged each block's grains in shared
-// memory, generating a window's margin again for every block, and the fat pass over the denser blocks: GB300,
-// 1024^2 log-normal 0.025 N 256 sparse + fat 32.6 ms, stream + per-sample 9.8; 1080p radius 0.1 N 32 2.49 and
-// 1.00; 256^2 ramp 0.12 N 64 0.30 and 0.15.
+// log-normal radius) and of their candidates: 70 ps a grain on the log-normal plane below.  It replaced a form of the
+// sparse pass that staged each block's grains in shared memory, generating a window's margin again for every block,
+// and the fat pass over the denser blocks: GB300, 1024^2 log-normal 0.025 N 256 sparse + fat 32.6 ms, stream +
+// per-sample 9.8; 1080p radius 0.1 N 32 2.49 and 1.00; 256^2 ramp 0.12 N 64 0.30 and 0.15.
 #pragma once
 
 #include "fg_phase.cuh"
@@ -103,8 +103,8 @@ struct StreamGrain {
 };
 template <int NW>
 __device__ __forceinline__ void stream_test(const PixelwiseArgs &a, const PwStreamGrid &g, PwStreamShared<NW> &S,
-                                            unsigned int *bits, const StreamGrain &G, bool live, int src, int e, int fx0, int fy0, int fw,
-                                            int fh) {
+                                            unsigned int *bits, const StreamGrain &G, bool live, int src, int e, int fx0,
+                                            int fy0, int fw, int fh) {
     const float gx = __shfl_sync(0xffffffffu, G.gx, src), gy = __shfl_sync(0xffffffffu, G.gy, src);
     const float rr = __shfl_sync(0xffffffffu, G.rr, src);
     const float4 O = S.ent[e];

@@ -555,7 +555,8 @@ static cudaError_t launch_tc_as(const void *in, int in_cstride, TcArgs a, cudaSt
 // positions -- or, where that would need more than kTcNarrowPx pixels loaded for a tile, every whole number of
 // images.  The halo positions' sums are dropped.
 // 256 tiles of 64^2, 32 -> 32 channels with the ReLU output (201 MB, 30 us at the measured copy rate): 51 -> 44 us,
-// the masked data gradient (335 MB, 50 us) 65 -> 58, the input conv 32 -> 25; 200 images of 50 x 33, a layer call by call: 35 us.
+// the masked data gradient (335 MB, 50 us) 65 -> 58, the input conv 32 -> 25; 200 images of 50 x 33, a layer call by
+// call: 35 us.
 static bool tc_narrow(TcArgs &a) {
     const int pitch = a.W + 2;
     if (a.nb < 2 || pitch > kTcNarrowPx / 3) return false;
@@ -580,8 +581,9 @@ static cudaError_t launch_tc(const void *in, int in_cstride, TcArgs a, cudaStrea
 
 // A surrogate conv on the tensor cores, by the C-ABI's kinds.  For the residual kind res is the input itself; res
 // may be out in the data gradient; out2 (may be null) is the ReLU output (residual) or the gradient masked by
-// `relu` (then w are the layer's own weights, else already turned around, and out may be null).  Returns cudaErrorNotSupported when the buffers overlap otherwise or are not 16-byte aligned, or
-// the tensor maps cannot be made (the caller's mma.sync kernels run instead).
+// `relu` (then w are the layer's own weights, else already turned around, and out may be null).  Returns
+// cudaErrorNotSupported when the buffers overlap otherwise or are not 16-byte aligned, or the tensor maps cannot be
+// made (the caller's mma.sync kernels run instead).
 cudaError_t launch_sg_conv_tc(int kind, const void *in, int in_cstride, const void *w, const float *bias, const void *res,
                               const float *u, const void *relu, void *out, void *out2, float *out_f32, int nb, int H,
                               int W, cudaStream_t s) {

@@ -180,8 +180,9 @@ __device__ __forceinline__ void gw_process(const GwTile &T, unsigned int *mask, 
 
 // Chunk `chunk` of the samples over part `part` of `parts` of a tile: every parts-th of its pixels (a heavy
 // tile is split over several CTAs, each with its own copy of the tile's masks; OR makes the result the same).  Taken
-// in turn, not as ranges, the parts of a tile that is bright on one side cost the same: with ranges, the CTAs of
-// 262 x 1186 blobs, radius 0.047, N 113, zoom 0.25 ran 9.7 ms, so 8.1.
+// in turn, not as ranges, the parts of a tile that is bright on one side cost the same (262 x 1186 blobs, radius 0.047,
+// N 113, zoom 0.25: 9.7 ms with ranges, 8.1 so; a plane of few grains a pixel pays for the scattered loads, 256 x 256,
+// radius 0.1, N 32 at intensity 0.03 31 -> 36 us).
 // Each step of a warp draws one grain per lane.  In a part with enough pixels for the CTA's
 // warps a lane has a pixel of its own; in a smaller one g = 2 .. 32 lanes share a pixel, until `fill` lanes have
 // one: they hold the same stream, draw its next g grains one after another, and each keeps one (128x96, N 32:
@@ -243,7 +244,16 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
     }
     for (int t = tid; t < region_words; t += kGwThreads) mask[t] = 0u;
     const int fw = ix1 - ix0, total = fw * (iy1 - iy0);
-    const int px_end = (total - part + parts - 1) / parts;  // pixels part, part + parts, ... of the tile
+    // the part's pixels: of each `parts` of the tile in a row one, where that would be a few of the tile's columns the
+    // next one each time
+    int gcd = fw, step = parts;
+    while (step) {
+        const int rest = gcd % step;
+        gcd = step;
+        step = rest;
+    }
+    const bool turn = fw < 8 * gcd;
+    const int px_end = total / parts + ((turn ? (part + total / parts) % parts : part) < total % parts ? 1 : 0);
     if (tid == 0) *next_px = 0;
     int g = 1;  // lanes per pixel
     while (g < 32 && g * px_end < fill) g *= 2;
@@ -291,7 +301,7 @@ __device__ __forceinline__ void grainwise_tile_bits(const GrainwiseArgs &a, int 
             more = base + want < px_end;
             const int pi = base + __popc(idle & ((1u << (lane & ~(g - 1))) - 1u)) / g;
             if (((idle >> lane) & 1u) && pi < px_end) {
-                const int ti = part + pi * parts;
+                const int ti = pi * parts + (turn ? (part + pi) % parts : part);
                 px = ix0 + ti % fw;
                 py = iy0 + ti / fw;
                 const float lv = a.lam[(long long)py * a.in_w + px];
@@ -462,22 +472,13 @@ inline int grainwise_most_parts(int px) { return std::max(1, std::min(px / kGwWa
 // Rounding the parts up makes more items than the slots take in kGwItemsPerSlot turns, and where most of them cost the
 // same (a plane that is mostly saturated) the few left over take a whole turn more.  So the target is the smallest of
 // kGwStretches times that cost at which the items fit, an item taking the share of its slot that as many of its
-// size as fit into the slot leave it: 1024 x 123, radius 0.025, N 256 25.3 -> 21.5 ms, 600 x 400 of one intensity,
-// log-normal 0.03, N 256 12.2 -> 10.7.
+// size as fit into the slot leave it: 1024 x 123, radius 0.025, N 256 25.3 -> 21.5 ms.  (Stretched further, up to 1.45,
+// fewer and larger parts left slots idle: 153 x 771, radius 0.066, N 233, zoom 2 8.5 -> 10.8.)
 constexpr int kGwItemsPerSlot = 2;
 constexpr float kGwItemFloor = 2.0e6f;
 constexpr float kGwPixelCost = 800.0f;  // a pixel's Poisson set-up, in lane-ops (two grain steps)
-constexpr int kGwStretches = 8;
-__host__ __device__ inline float gw_stretch(int k) {
-    return k == 0   ? 1.0f
-           : k == 1 ? 1.02f
-           : k == 2 ? 1.05f
-           : k == 3 ? 1.09f
-           : k == 4 ? 1.14f
-           : k == 5 ? 1.2f
-           : k == 6 ? 1.3f
-                    : 1.45f;
-}
+constexpr int kGwStretches = 4;
+__host__ __device__ inline float gw_stretch(int k) { return k == 0 ? 1.0f : k == 1 ? 1.02f : k == 2 ? 1.05f : 1.09f; }
 __host__ __device__ inline int gw_parts(float cost, float target, int most_parts) {
     const float p = fminf(ceilf(cost / target), (float)most_parts);
     return p > 1.0f ? (int)p : 1;

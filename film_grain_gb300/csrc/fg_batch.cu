@@ -44,7 +44,7 @@ struct BatchImage {
 
 struct BatchItem {
     int image, x, y;
-    int part;   // grain-wise: part | parts << 16
+    int part;   // grain-wise: part | even << 15 | parts << 16
     int chunk;  // grain-wise: sample chunk
 };
 
@@ -203,10 +203,11 @@ __global__ void __launch_bounds__(512, 2) batch_persistent_kernel(const BatchIma
         __syncthreads();
         if (threadIdx.x == 0) s_image = w.image;
         if (s_img.algo == FG_ALGO_PIXEL) pixelwise_block<PwFat>(s_img.pa, w.x, w.y, smem_raw);
-        else if (s_img.small)
-            grainwise_tile<true>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk, kBatchFill);
-        else
-            grainwise_tile<false>(s_img.ga, w.x, w.y, smem_raw, w.part & 0xFFFF, w.part >> 16, w.chunk, kBatchFill);
+        else {
+            const int part = w.part & 0x7FFF, parts = w.part >> 16, fill = (w.part & 0x8000) ? kGwEvenFill : kBatchFill;
+            if (s_img.small) grainwise_tile<true>(s_img.ga, w.x, w.y, smem_raw, part, parts, w.chunk, fill);
+            else grainwise_tile<false>(s_img.ga, w.x, w.y, smem_raw, part, parts, w.chunk, fill);
+        }
         __syncthreads();
     }
 }
@@ -293,7 +294,8 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
     struct GrainTile {
         double cost;
         BatchItem it;
-        int most_parts;
+        int px;
+        bool even;
     };
     std::vector<GrainTile> grain_tiles;
     std::vector<RegenRange> regen;
@@ -377,19 +379,24 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
             for (int ty = 0; ty < nty; ty++) {
                 for (int tx = 0; tx < ntx; tx++) {
                     double lam_sum = 0.0;
+                    float lam_max = 0.0f;
                     const int x0 = tx * a.tin_w, y0 = ty * a.tin_h;
                     const int x1 = std::min(a.in_w, x0 + a.tin_w), y1 = std::min(a.in_h, y0 + a.tin_h);
                     if (im.h_lambda) {
                         for (int y = y0; y < y1; y++)
-                            for (int x = x0; x < x1; x++)  // (clamped: the cuts need finite costs)
-                                lam_sum += std::fmin(std::fmax(im.h_lambda[(long long)y * a.in_w + x], 0.0f), 1.0e6f);
+                            for (int x = x0; x < x1; x++) {  // (clamped: the cuts need finite costs)
+                                const float l = std::fmin(std::fmax(im.h_lambda[(long long)y * a.in_w + x], 0.0f), 1.0e6f);
+                                lam_sum += l;
+                                lam_max = std::fmax(lam_max, l);
+                            }
                     } else {
                         lam_sum = 50.0 * (x1 - x0) * (y1 - y0);
                     }
                     const double cost = lam_sum * a.grain_cost + (double)kGwPixelCost * (x1 - x0) * (y1 - y0);
-                    const int most = grainwise_most_parts((x1 - x0) * (y1 - y0));
+                    const int px = (x1 - x0) * (y1 - y0);
+                    const bool even = im.h_lambda && gw_even((float)lam_sum, lam_max, px);
                     for (int c = 0; c < a.chunks; c++)
-                        grain_tiles.push_back(GrainTile{cost, BatchItem{i, tx, ty, 0, c}, most});
+                        grain_tiles.push_back(GrainTile{cost, BatchItem{i, tx, ty, 0, c}, px, even});
                 }
             }
         }
@@ -406,10 +413,12 @@ static fg_status batch_build(const fg_batch_image *imgs, int n, const fg_batch_t
         const double slots = (double)std::max(1, sms) * std::max(1, tun.ctas_per_sm);
         const float target = std::max(kGwItemFloor, (float)(total_cost / (slots * kBatchItemsPerSlot)));
         for (const GrainTile &g : grain_tiles) {
-            const int parts = gw_parts((float)g.cost, target, g.most_parts);
+            const int most = grainwise_most_parts(g.px);
+            const int parts = g.even ? gw_even_parts((float)g.cost, target, most, g.px, images[g.it.image].ga.lognorm != 0)
+                                     : gw_parts((float)g.cost, target, most);
             for (int q = 0; q < parts; q++) {
                 BatchItem it = g.it;
-                it.part = q | (parts << 16);
+                it.part = q | (g.even ? 0x8000 : 0) | (parts << 16);
                 work.push_back(CostItem{g.cost / parts, it});
             }
         }

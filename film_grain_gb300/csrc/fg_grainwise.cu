@@ -49,8 +49,9 @@ __global__ void __launch_bounds__(kGwThreads, 2) grainwise_persistent_kernel(con
         __syncthreads();
         const int i = s_item;
         if (i < 0) break;
-        const int2 it = items[i / a.chunks];  // (tile, part | parts << 16)
-        grainwise_tile<kSmall, kVariant>(a, it.x % ntx, it.x / ntx, smem_raw, it.y & 0xFFFF, it.y >> 16, i % a.chunks);
+        const int2 it = items[i / a.chunks];  // (tile, part | even << 15 | parts << 16)
+        grainwise_tile<kSmall, kVariant>(a, it.x % ntx, it.x / ntx, smem_raw, it.y & 0x7FFF, it.y >> 16, i % a.chunks,
+                                         (it.y & 0x8000) ? kGwEvenFill : kGwThreads);
         __syncthreads();
     }
 }
@@ -63,21 +64,38 @@ __global__ void grainwise_costs_kernel(const float *__restrict__ lam, int in_w, 
     if (tile >= ntiles) return;
     const int x0 = (tile % ntx) * tin_w, y0 = (tile / ntx) * tin_h;
     const int w = min(x0 + tin_w, in_w) - x0, n = w * (min(y0 + tin_h, in_h) - y0);
-    float sum = 0.0f;
+    float sum = 0.0f, most = 0.0f;
     // (clamped: the work list's bound needs finite costs, whatever plane the caller passes)
-    for (int i = lane; i < n; i += 32)
-        sum += fminf(fmaxf(lam[(long long)(y0 + i / w) * in_w + x0 + i % w], 0.0f), 1.0e6f);
+    for (int i = lane; i < n; i += 32) {
+        const float l = fminf(fmaxf(lam[(long long)(y0 + i / w) * in_w + x0 + i % w], 0.0f), 1.0e6f);
+        sum += l;
+        most = fmaxf(most, l);
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) cost[tile] = grain_cost * sum + kGwPixelCost * (float)n;
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+    }
+    // the cost's last bit: the tile is even
+    if (lane == 0)
+        cost[tile] = __uint_as_float((__float_as_uint(grain_cost * sum + kGwPixelCost * (float)n) & ~1u) |
+                                     (gw_even(sum, most, n) ? 1u : 0u));
 }
 
 // The work list: tiles by descending cost (a bitonic sort in shared memory, one CTA, for up to kGwSortMax
 // tiles; larger grids keep the natural order), each cut into parts (gw_parts).
-// work[1] = items, then int2 (tile, part | parts << 16).
+// work[1] = items, then int2 (tile, part | even << 15 | parts << 16).
 constexpr int kGwSortMax = 4096;
-__global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__restrict__ cost, int ntiles, int slots,
-                                                               int chunks, int most_parts, int *__restrict__ work) {
+__global__ void __launch_bounds__(1024) grainwise_order_kernel(const __grid_constant__ GrainwiseArgs a,
+                                                               const float *__restrict__ cost, int ntx, int ntiles,
+                                                               int slots, int most_parts) {
+    int *work = a.work;
+    const int chunks = a.chunks;
+    auto cut = [&](float c, int tile, float target) {
+        if (!(__float_as_uint(c) & 1u)) return gw_parts(c, target, most_parts);
+        const int w = min(a.tin_w, a.in_w - tile % ntx * a.tin_w), h = min(a.tin_h, a.in_h - tile / ntx * a.tin_h);
+        return gw_even_parts(c, target, most_parts, w * h, a.lognorm != 0);
+    };
     __shared__ float key[kGwSortMax];
     __shared__ int idx[kGwSortMax];
     __shared__ float wsum[32];
@@ -128,7 +146,10 @@ __global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__re
         for (int k = 0; k < kGwStretches; k++) share[k] = 0.0f;
         for (int i = tid; i < ntiles; i += blockDim.x)
 #pragma unroll
-            for (int k = 0; k < kGwStretches; k++) share[k] += gw_slot_share(cost[i], target * gw_stretch(k), most_parts);
+            for (int k = 0; k < kGwStretches; k++) {
+                const float t = target * gw_stretch(k);
+                share[k] += gw_slot_share(cost[i], t, cut(cost[i], i, t));
+            }
 #pragma unroll
         for (int k = 0; k < kGwStretches; k++) {
 #pragma unroll
@@ -148,11 +169,12 @@ __global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__re
     int base = 0;  // items of the tiles before this round's
     for (int i0 = 0; i0 < ntiles; i0 += blockDim.x) {
         const int i = i0 + tid;
-        int tile = 0, parts = 0;
+        int tile = 0, parts = 0, even = 0;
         if (i < ntiles) {
             tile = sorted ? idx[i] : i;
             const float c = sorted ? key[i] : cost[i];
-            parts = gw_parts(c, target, most_parts);
+            parts = cut(c, tile, target);
+            even = (__float_as_uint(c) & 1u) << 15;
         }
         int incl = parts;
 #pragma unroll
@@ -167,7 +189,7 @@ __global__ void __launch_bounds__(1024) grainwise_order_kernel(const float *__re
             if (w < warp) first += wcnt[w];
             round += wcnt[w];
         }
-        for (int q = 0; q < parts; q++) items[first + q] = make_int2(tile, q | (parts << 16));
+        for (int q = 0; q < parts; q++) items[first + q] = make_int2(tile, q | even | (parts << 16));
         base += round;
         __syncthreads();
     }
@@ -230,9 +252,10 @@ int grainwise_tile_count(const GrainwiseArgs &a) {
 }
 
 // The scheduler's area: item counter, items, then the list -- every tile's share above the first is a target's
-// worth of lane-ops, so there are at most slots * kGwItemsPerSlot of those -- and the tiles' costs.
+// worth of lane-ops, so there are at most slots * kGwItemsPerSlot of those (twice as many items, of even tiles) -- and
+// the tiles' costs.
 static size_t grainwise_list_items(const GrainwiseArgs &a, int sms) {
-    return (size_t)grainwise_tile_count(a) + (size_t)2 * sms * kGwItemsPerSlot + 1;
+    return 2 * ((size_t)grainwise_tile_count(a) + (size_t)2 * sms * kGwItemsPerSlot + 1);
 }
 size_t grainwise_work_ints(const GrainwiseArgs &a, int sms) {
     return 2 + 2 * grainwise_list_items(a, sms) + (size_t)grainwise_tile_count(a);
@@ -249,8 +272,7 @@ cudaError_t launch_grainwise(const GrainwiseArgs &a, int sms, cudaStream_t s) {
     float *cost = reinterpret_cast<float *>(a.work + 2 + 2 * grainwise_list_items(a, sms));
     grainwise_costs_kernel<<<(ntiles + 7) / 8, 256, 0, s>>>(a.lam, a.in_w, a.in_h, a.tin_w, a.tin_h, ntx, ntiles,
                                                             a.grain_cost, cost);
-    grainwise_order_kernel<<<1, 1024, 0, s>>>(cost, ntiles, slots, a.chunks, grainwise_most_parts(a.tin_w * a.tin_h),
-                                              a.work);
+    grainwise_order_kernel<<<1, 1024, 0, s>>>(a, cost, ntx, ntiles, slots, grainwise_most_parts(a.tin_w * a.tin_h));
     void (*k)(GrainwiseArgs, int);
     if (!small) k = grainwise_persistent_kernel<false, kGbMaxWords>;  // coordinates beyond 2^22: one variant
     else if (v == 1) k = grainwise_persistent_kernel<true, 1>;

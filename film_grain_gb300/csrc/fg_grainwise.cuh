@@ -483,8 +483,37 @@ __host__ __device__ inline int gw_parts(float cost, float target, int most_parts
     const float p = fminf(ceilf(cost / target), (float)most_parts);
     return p > 1.0f ? (int)p : 1;
 }
-__host__ __device__ inline float gw_slot_share(float cost, float target, int most_parts) {
-    const int parts = gw_parts(cost, target, most_parts);
+// A tile whose pixels hold about the same (many) grains: each lane group's first pixel takes as long as every other's,
+// so a part whose groups do not fit the CTA's lanes at once, or leave many of them out, wastes them to its end.  Its
+// parts are sized for that (gw_even_parts: about as many, up to twice, by the share of the lanes that work) and its
+// groups as large as fit at once.
+__host__ __device__ inline bool gw_even(float lam_sum, float lam_max, int px) {
+    return lam_sum >= 0.75f * lam_max * (float)px && lam_sum >= 50.0f * (float)px;
+}
+constexpr int kGwEvenFill = kGwThreads / 2 + 1;  // grainwise_tile_bits' fill: the most lanes that are no more than all
+__host__ __device__ inline int gw_even_parts(float cost, float target, int most_parts, int px, bool lognorm) {
+    int best = gw_parts(cost, target, most_parts);
+    if (best == 1) return 1;
+    const int lo = gw_parts(cost, 1.25f * target, most_parts), hi = best * 2 < most_parts ? best * 2 : most_parts;
+    float best_score = 0.0f;
+    const int first = best;
+    for (int k = -1; k <= 5; k++) {  // as cut by cost, and filled by groups of 1 .. 32
+        const int parts = k < 0 ? first : (int)((((long long)px << k) + kGwThreads - 1) / kGwThreads);
+        if (parts < lo || parts > hi) continue;
+        const int n = (px + parts - 1) / parts;
+        int g = 1;
+        while (g < 32 && 2 * g * n <= kGwThreads) g *= 2;
+        const int rounds = (n * g + kGwThreads - 1) / kGwThreads;
+        const float repeated = (lognorm ? 0.12f : 0.04f) * (float)(g - 1);  // the draws that g lanes repeat
+        const float score = (float)n * (float)g / ((float)rounds * (float)kGwThreads) / (1.0f + repeated);
+        if (score > 1.02f * best_score) {
+            best_score = score;
+            best = parts;
+        }
+    }
+    return best;
+}
+__host__ __device__ inline float gw_slot_share(float cost, float target, int parts) {
     const float fit = floorf((float)kGwItemsPerSlot * target * (float)parts / fmaxf(cost, 1.0f));
     return (float)parts / fmaxf(fit, 1.0f);
 }

@@ -527,3 +527,23 @@ def test_grainwise_parts_and_skipped_draws(cuda, fgl, orc, w, h, zoom, radius, n
     """Constant radius: the lanes of a pixel stand at their own grains of its stream, in parts that take the tile's
     pixels in turn."""
     _check("grain", fgl, orc, workloads.ramp_noise(w, h, 5), radius=radius, n=n, zoom=zoom, seed=17)
+
+
+@pytest.mark.parametrize("w,h,n,dist", [(37, 29, 33, "const"), (37, 29, 40, "lognorm"), (90, 31, 20, "const"),
+                                        (23, 40, 200, "const")])
+def test_grainwise_even_tiles(cuda, fgl, orc, w, h, n, dist):
+    """Saturated planes, whose tiles are cut into parts that fill the lanes at once."""
+    _check("grain", fgl, orc, np.ones((h, w), np.float32), radius=0.04, dist=dist, sd=0.012 if dist == "lognorm" else 0.0,
+           n=n, seed=23)
+
+
+def test_grainwise_fewer_samples_cost_less(cuda, fgl):
+    """A saturated plane at N 128 takes less time than at N 256: the same grains with half of the samples.  Cut by cost
+    alone, its parts of 675 pixels left a third of the lanes waiting, and it took 86 ms against 81."""
+    torch = cuda
+    times = []
+    for n in (128, 256):
+        p, d, lam = _grain_plane(fgl, np.ones((512, 1024), np.float32), radius_mean=0.025, n_samples=n, seed=5)
+        dl = torch.from_numpy(lam).cuda()
+        times.append(_fastest(torch, lambda: fgl.render_grainwise(dl, p, d), 3))
+    assert times[0] < 0.95 * times[1], times

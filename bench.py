@@ -202,13 +202,14 @@ def cpu_pixel_baseline(oracle, planes, wl, threads, rows=None):
 
 # DRAM bytes per launch from ncu captures of the dominant kernels on their profiling cases (the
 # --profile-once runs), per unit of work: sg_conv32_tc_kernel (the residual conv) on the 1024^2 x 3
-# surrogate input, 373.9 MB read+write for 3 x 1024^2 px; grainwise_persistent_kernel on a 512^2 ->
-# 1024^2 plane of the grain-wise blob frame, 18.25 MB per 1024^2 output pixels (the lambda plane plus the
+# surrogate input, 211.8 MB read for 3 x 1024^2 px, and its output written once (158.5 of 201.3 MB there: the
+# rest was still in the L2, which a larger frame does not fit); grainwise_persistent_kernel on a 512^2 ->
+# 1024^2 plane of the grain-wise blob frame, 18.4 MB per 1024^2 output pixels (the lambda plane plus the
 # sample-mask lines that miss L2); cell_mask_kernel + pixelwise_stream_kernel on the 1024^2 flat plane
 # of the large frame's parameters, 172.9 + 288.4 MB per 1024^2 output pixels (the emptiness bitmask
 # written, then read with the cell table and the samples' bits).
-SG_CONV_DRAM_BYTES_PER_PX = 373.9e6 / (3 * 1024 * 1024)
-GRAINWISE_DRAM_BYTES_PER_OUT_PX = 18.25e6 / (1024 * 1024)
+SG_CONV_DRAM_BYTES_PER_PX = 211.8e6 / (3 * 1024 * 1024) + 64
+GRAINWISE_DRAM_BYTES_PER_OUT_PX = 18.4e6 / (1024 * 1024)
 PIXELWISE_DRAM_BYTES_PER_OUT_PX = (172.9e6 + 288.4e6) / (1024 * 1024)
 
 # Algorithmic lane-ops of the pixel-wise path (an exact method that hashes every cell once): per cell
